@@ -92,8 +92,14 @@ struct adscf_batch {
   void* d_f32 = nullptr;                // FilmDev<float>[n]
   void* d_f64 = nullptr;                // FilmDev<double>[n]
   int* d_list32 = nullptr;              // films sweeping in FP32 / FP64, by contour length
-  int* d_items32 = nullptr;             // (film << 1) | chain of the FP32 films, same order
   int* d_list64 = nullptr;
+  // line sweeps by precision (0 FP32, 1 FP64) and warps per line (0: one warp
+  // per line; 1..4: 4, 8, 16, 32 warps): (film << 1) | chain, longest
+  // contours first; lines past 4096 rows are in d_long
+  int* d_fsweep[2][5] = {};
+  int n_fsweep[2][5] = {};
+  int* d_long[2] = {};                  // films of more than 4096 rows
+  int n_long[2] = {};
   int n32 = 0, n64 = 0;
   // shared-memory line sweeps: rows per line (max gz + 1 of the list) and
   // lanes per block (0: the list sweeps on global memory)
@@ -798,13 +804,24 @@ int build_film(adscf_batch* b) {
   };
   std::stable_sort(l32.begin(), l32.end(), by_work);
   std::stable_sort(l64.begin(), l64.end(), by_work);
+  std::vector<int> sweep[2][5], longl[2];
+  for (int f64p = 0; f64p < 2; ++f64p)
+    for (int f : f64p ? l64 : l32) {
+      const int rows = b->npts[f];
+      int k = 0;
+      if (rows > kFilmGroupRows) { longl[f64p].push_back(f); continue; }
+      if (rows > kFilmWarpRows)
+        for (k = 1; (2 << k) < film_group_warps(rows);) ++k;
+      sweep[f64p][k].push_back(f << 1);
+      sweep[f64p][k].push_back((f << 1) | 1);
+    }
   long long max_npts = 0;
   for (int i = 0; i < n; ++i) max_npts = std::max<long long>(max_npts, b->npts[i]);
   b->film_cl_threads = closure_threads(max_npts);
   b->n32 = (int)l32.size();
   b->n64 = (int)l64.size();
-  // layout of the shared-memory sweeps: one thread per (film, chain) runs a
-  // serial recurrence, so the first `per_warp` lanes of each warp work and
+  // layout of the shared-memory sweeps of lines past 4096 rows: one thread
+  // per (film, chain) runs a serial recurrence, so the first `per_warp` lanes of each warp work and
   // a block holds `warps` warps: W = warps * per_warp lines share the
   // block's shared memory.  ADSCF_FILM_LANES / ADSCF_FILM_WARPS override.
   {
@@ -824,8 +841,8 @@ int build_film(adscf_batch* b) {
       W = warps * b->film_per_warp;
       if (warps == 0) W = 0;
     };
-    lanes(l32, sizeof(float), b->zcap32, b->lanes32);
-    lanes(l64, sizeof(double), b->zcap64, b->lanes64);
+    lanes(longl[0], sizeof(float), b->zcap32, b->lanes32);
+    lanes(longl[1], sizeof(double), b->zcap64, b->lanes64);
     BK(cudaFuncSetAttribute(k_film1d_chains_sm<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
     BK(cudaFuncSetAttribute(k_film1d_chains_sm<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
   }
@@ -837,12 +854,17 @@ int build_film(adscf_batch* b) {
   BK(cudaMalloc(&b->d_list64, std::max<size_t>(1, l64.size()) * sizeof(int)));
   if (!l32.empty())
     BK(cudaMemcpyAsync(b->d_list32, l32.data(), l32.size() * sizeof(int), cudaMemcpyHostToDevice, b->stream));
-  {  // (film, chain) items of the warp sweep, in the order of l32
-    std::vector<int> items;
-    for (int f : l32) { items.push_back(f << 1); items.push_back((f << 1) | 1); }
-    BK(cudaMalloc(&b->d_items32, std::max<size_t>(1, items.size()) * sizeof(int)));
-    if (!items.empty())
-      BK(cudaMemcpyAsync(b->d_items32, items.data(), items.size() * sizeof(int), cudaMemcpyHostToDevice, b->stream));
+  auto up = [&](const std::vector<int>& v, int*& d, int& cnt) -> int {
+    cnt = (int)v.size();
+    if (v.empty()) return ADSCF_OK;
+    BK(cudaMalloc(&d, v.size() * sizeof(int)));
+    BK(cudaMemcpyAsync(d, v.data(), v.size() * sizeof(int), cudaMemcpyHostToDevice, b->stream));
+    return ADSCF_OK;
+  };
+  for (int p = 0; p < 2; ++p) {
+    int rc = up(longl[p], b->d_long[p], b->n_long[p]);
+    for (int k = 0; k < 5 && !rc; ++k) rc = up(sweep[p][k], b->d_fsweep[p][k], b->n_fsweep[p][k]);
+    if (rc) return rc;
   }
   if (!l64.empty())
     BK(cudaMemcpyAsync(b->d_list64, l64.data(), l64.size() * sizeof(int), cudaMemcpyHostToDevice, b->stream));
@@ -856,32 +878,37 @@ int build_film(adscf_batch* b) {
   return ADSCF_OK;
 }
 
+// chains of a batch's films of one precision: a warp per (film, chain) up to
+// 256 rows, 4 to 32 warps up to 4096, a thread per (film, chain) beyond
+template <typename T>
+void film_sweeps(adscf_batch* b) {
+  cudaStream_t s = b->stream;
+  constexpr int p = sizeof(T) == 8;
+  const FilmDev<T>* F = static_cast<const FilmDev<T>*>(p ? b->d_f64 : b->d_f32);
+  if (const int n = b->n_fsweep[p][0]) k_film1d_warp_b<T><<<(n + 3) / 4, 128, 0, s>>>(F, b->d_S, b->d_fsweep[p][0], n);
+  for (int k = 1; k < 5; ++k) {
+    const int n = b->n_fsweep[p][k], threads = 32 * (2 << k);
+    if (!n) continue;
+    if (threads <= 256) k_film1d_group_b<T, 256><<<n, threads, 0, s>>>(F, b->d_S, b->d_fsweep[p][k]);
+    else k_film1d_group_b<T, 1024><<<n, threads, 0, s>>>(F, b->d_S, b->d_fsweep[p][k]);
+  }
+  if (const int n = b->n_long[p]) {
+    const int W = p ? b->lanes64 : b->lanes32, zcap = p ? b->zcap64 : b->zcap32, pw = b->film_per_warp;
+    if (W)
+      k_film1d_chains_sm<T><<<dim3((n + W - 1) / W, 2), 32 * (W / pw), film_sweep_smem(zcap, W, sizeof(T)), s>>>(
+          F, b->d_S, b->d_long[p], n, zcap, pw);
+    else
+      k_film1d_chains_b<T><<<dim3((n + FILM_THREADS - 1) / FILM_THREADS, 2), FILM_THREADS, 0, s>>>(
+          F, b->d_S, b->d_long[p], n);
+  }
+}
+
 int enqueue_film(adscf_batch* b) {
   cudaStream_t s = b->stream;
   const FilmDev<float>* f32 = static_cast<const FilmDev<float>*>(b->d_f32);
   const FilmDev<double>* f64 = static_cast<const FilmDev<double>*>(b->d_f64);
-  const int pw = b->film_per_warp;
-  if (b->n32 && b->zcap32 <= 32 * kFilmWarpM) {
-    // one warp per (film, chain), longest contours first
-    k_film1d_warp_b<<<(2 * b->n32 + 3) / 4, 128, 0, s>>>(f32, b->d_S, b->d_items32, 2 * b->n32);
-  } else if (b->n32 && b->lanes32) {
-    const int W = b->lanes32;
-    k_film1d_chains_sm<float><<<dim3((b->n32 + W - 1) / W, 2), 32 * (W / pw),
-                                film_sweep_smem(b->zcap32, W, sizeof(float)), s>>>(
-        f32, b->d_S, b->d_list32, b->n32, b->zcap32, pw);
-  } else if (b->n32) {
-    k_film1d_chains_b<float><<<dim3((b->n32 + FILM_THREADS - 1) / FILM_THREADS, 2), FILM_THREADS, 0, s>>>(
-        f32, b->d_S, b->d_list32, b->n32);
-  }
-  if (b->n64 && b->lanes64) {
-    const int W = b->lanes64;
-    k_film1d_chains_sm<double><<<dim3((b->n64 + W - 1) / W, 2), 32 * (W / pw),
-                                 film_sweep_smem(b->zcap64, W, sizeof(double)), s>>>(
-        f64, b->d_S, b->d_list64, b->n64, b->zcap64, pw);
-  } else if (b->n64) {
-    k_film1d_chains_b<double><<<dim3((b->n64 + FILM_THREADS - 1) / FILM_THREADS, 2), FILM_THREADS, 0, s>>>(
-        f64, b->d_S, b->d_list64, b->n64);
-  }
+  film_sweeps<float>(b);
+  film_sweeps<double>(b);
   // one-line films: blocks of 128 points, twice as many resident films as
   // with 256 (a longer line takes its points in passes)
   if (b->n32) k_film_contour_b<float><<<b->n32, 128, 0, s>>>(f32, b->d_list32);
@@ -1337,7 +1364,11 @@ int adscf_batch_destroy(adscf_batch* b) {
   cudaFree(b->pool); cudaFree(b->d_inst); cudaFree(b->d_S);
   cudaFree(b->d_tw); cudaFree(b->d_fk); cudaFree(b->d_g64);
   for (auto& C : b->cls) { cudaFree(C.wx); cudaFree(C.wy); cudaFree(C.wz); }
-  cudaFree(b->d_f32); cudaFree(b->d_f64); cudaFree(b->d_list32); cudaFree(b->d_list64); cudaFree(b->d_items32);
+  cudaFree(b->d_f32); cudaFree(b->d_f64); cudaFree(b->d_list32); cudaFree(b->d_list64);
+  for (int p = 0; p < 2; ++p) {
+    cudaFree(b->d_long[p]);
+    for (int* d : b->d_fsweep[p]) cudaFree(d);
+  }
   cudaFree(b->d_items); cudaFree(b->d_ctl); cudaFree(b->d_ranges);
   cudaFree(b->d_tabf);
   if (b->h_pinned) cudaFreeHost(b->h_pinned);
@@ -1410,7 +1441,14 @@ int adscf_batch_results(adscf_batch* b, adscf_iter_result* out) {
 
 int adscf_batch_launches(const adscf_batch* b) {
   if (!b) return -1;
-  if (b->film) return 2 * ((b->n32 > 0) + (b->n64 > 0)) + 3;
+  if (b->film) {
+    int k = (b->n32 > 0) + (b->n64 > 0) + 3;   // contours, closure, solve, mix
+    for (int p = 0; p < 2; ++p) {
+      k += b->n_long[p] > 0;
+      for (int c : b->n_fsweep[p]) k += c > 0;
+    }
+    return k;
+  }
   if (b->sweep) return 5;   // sweep, contour, closure, solve, mix (and a memset of the counters)
   int k = 4;   // contour, closure, solve, mix
   for (const auto& C : b->cls) {

@@ -285,20 +285,49 @@ int adi_tune(adscf_ctx* ctx, FilmState* F, const FilmDev<float>& D, const FieldR
   return ADSCF_OK;
 }
 
-// 1D chains of every line: FP32 sweeps on lines of up to 32 * kFilmWarpM
-// planes with one warp per (line, chain) (film_warp.cuh); FP64 sweeps (the
-// reference's serial Thomas) and longer lines with one thread per (line,
-// chain).
+// Contour kernel of a film: 32 points a block with the nodes dealt to its
+// warps while those blocks fit the SMs in one wave (two of 1024 threads on
+// each of 152), one thread per point beyond, where the points alone fill them.
+constexpr int kFewPoints = 32 * 2 * 152;
+bool film_few_points(int npts) { return npts <= kFewPoints; }
+
+// FP32 copy of the field for the ADI sweeps
+void field_f32(const FilmDev<float>& D, const FieldRef& fr, size_t n, cudaStream_t s) {
+  k_film_wconv<<<(int)std::min<size_t>((n + 255) / 256, 152 * 4), 256, 0, s>>>(fr, D.wf, n);
+}
+
+// 1D chains of every line (film_warp.cuh): one warp per (line, chain) up to
+// 256 rows, several warps up to 4096, one thread per (line, chain) beyond.
+// FP64 lines whose warps find enough idle SMs spread them over a cluster
+// (one FP64 pipe per SM); with more (line, chain) pairs than that the SMs
+// are busy anyway and a line's warps share a CTA, whose barrier is cheaper.
 template <typename T>
-void launch_chains_1d(const FilmDev<T>& D, const FieldRef& fr, int chains, cudaStream_t s) {
-  if constexpr (sizeof(T) == 4) {
-    if (D.gz + 1 <= 32 * kFilmWarpM) {
-      k_film1d_warp<<<dim3((D.nlines + 3) / 4, chains), 128, 0, s>>>(D);
-      return;
-    }
+int launch_chains_1d(adscf_ctx* ctx, const FilmDev<T>& D, const FieldRef& fr, int chains, cudaStream_t s) {
+  const int n = D.gz + 1;
+  if (n <= kFilmWarpRows) {
+    k_film1d_warp<T><<<dim3((D.nlines + 3) / 4, chains), 128, 0, s>>>(D, fr);
+  } else if (n <= kFilmGroupRows) {
+    const int W = film_group_warps(n);
+    const bool spread = sizeof(T) == 8 && (long long)D.nlines * chains * std::min(W, 8) <= 152;
+    const int csize = spread ? std::min(W, 8) : 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(D.nlines * csize, chains);
+    cfg.blockDim = dim3(32 * (W / csize));
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = csize;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = csize > 1 ? 1 : 0;
+    if (cfg.blockDim.x <= 256) CK(cudaLaunchKernelEx(&cfg, k_film1d_group<T, 256>, D, fr, csize));
+    else CK(cudaLaunchKernelEx(&cfg, k_film1d_group<T, 1024>, D, fr, csize));
+  } else {
+    const dim3 g((D.nlines + FILM_THREADS - 1) / FILM_THREADS, chains);
+    k_film1d_chains<T><<<g, FILM_THREADS, 0, s>>>(D, fr);
   }
-  const dim3 g((D.nlines + FILM_THREADS - 1) / FILM_THREADS, chains);
-  k_film1d_chains<T><<<g, FILM_THREADS, 0, s>>>(D, fr);
+  return ADSCF_OK;
 }
 
 template <typename T>
@@ -310,21 +339,15 @@ int chains_t(adscf_ctx* ctx, const double* d_w) {
   if (ctx->geometry == ADSCF_FILM_3D) {
     // node 0 of both chains = 1, then ns Douglas ADI steps (three sweeps each)
     k_film_fill<T><<<std::max(1, (D.npts + 255) / 256), 256, 0, s>>>(D.q, D.qd, D.npts);
-    if (sizeof(T) == 4) {
-      const size_t n = (size_t)ctx->ntypes * D.npts;
-      k_film_wconv<<<(int)std::min<size_t>((n + 255) / 256, 152 * 4), 256, 0, s>>>(fr, D.wf, n);
-    }
     if constexpr (sizeof(T) == 4) {
+      field_f32(D, fr, (size_t)ctx->ntypes * D.npts, s);
       if (!F->adi_set) adi_defaults(F, D);
     }
     const AdiLaunch A = adi_launch<T>(F, D, 2);
     for (int st = 1; st <= D.ns; ++st) adi_step<T>(A, D, fr, st, 2, s);
   } else {
-    if (sizeof(T) == 4) {
-      const size_t n = (size_t)ctx->ntypes * D.npts;
-      k_film_wconv<<<(int)std::min<size_t>((n + 255) / 256, 152 * 4), 256, 0, s>>>(fr, D.wf, n);
-    }
-    launch_chains_1d<T>(D, fr, 2, s);
+    const int rc = launch_chains_1d<T>(ctx, D, fr, 2, s);
+    if (rc) return rc;
   }
   CK(cudaGetLastError());
   return ADSCF_OK;
@@ -333,7 +356,8 @@ int chains_t(adscf_ctx* ctx, const double* d_w) {
 template <typename T>
 int contour_t(adscf_ctx* ctx) {
   FilmDev<T> D = fdev<T>(ctx->film);
-  k_film_contour<T><<<ctx->contour_blocks, 256, 0, ctx->stream>>>(D);
+  if (film_few_points(D.npts)) k_film_contour_s<T><<<ctx->contour_blocks, 1024, 0, ctx->stream>>>(D);
+  else k_film_contour<T><<<ctx->contour_blocks, 256, 0, ctx->stream>>>(D);
   CK(cudaGetLastError());
   return ADSCF_OK;
 }
@@ -364,17 +388,15 @@ int step_single_t(adscf_ctx* ctx, double* d_prop, const double* d_w, double ds) 
   FieldRef fr{};
   fr.direct = d_w;
   if (ctx->geometry == ADSCF_FILM_3D) {
-    if (sizeof(T) == 4)   // one field (type 0) of npts values
-      k_film_wconv<<<(int)std::min<size_t>((n + 255) / 256, 152 * 4), 256, 0, s>>>(fr, D.wf, n);
     if constexpr (sizeof(T) == 4) {
+      field_f32(D, fr, n, s);   // one field (type 0) of npts values
       if (!F->adi_set) adi_defaults(F, fdev<float>(F));
     }
     const AdiLaunch A = adi_launch<T>(F, D, 1);
     adi_step<T>(A, D, fr, 1, 1, s);
   } else {
-    if (sizeof(T) == 4)   // one field (type 0) of npts values
-      k_film_wconv<<<(int)std::min<size_t>((n + 255) / 256, 152 * 4), 256, 0, s>>>(fr, D.wf, n);
-    launch_chains_1d<T>(D, fr, 1, s);
+    const int rc = launch_chains_1d<T>(ctx, D, fr, 1, s);
+    if (rc) return rc;
   }
   k_convert<double, T><<<std::max<size_t>(1, (n + 255) / 256), 256, 0, s>>>(D.q + n, d_prop, n);
   CK(cudaGetLastError());
@@ -508,9 +530,10 @@ int film_create(adscf_ctx* ctx, const adscf_params* p) {
     }
     CK(cudaMalloc(&F->d_alf, f3.size() * sizeof(float)));
     CK(cudaMemcpy(F->d_alf, f3.data(), f3.size() * sizeof(float), cudaMemcpyHostToDevice));
-    CK(cudaMalloc(&F->d_wf, (size_t)ctx->ntypes * ctx->npts * sizeof(float)));
+    if (ctx->geometry == ADSCF_FILM_3D) CK(cudaMalloc(&F->d_wf, (size_t)ctx->ntypes * ctx->npts * sizeof(float)));
   }
-  ctx->contour_blocks = (int)std::min<size_t>(((size_t)ctx->npts + 255) / 256, 152 * 4);
+  ctx->contour_blocks = film_few_points(ctx->npts) ? (ctx->npts + 31) / 32
+                                                   : (int)std::min<size_t>(((size_t)ctx->npts + 255) / 256, 152 * 4);
   CK(cudaMalloc(&ctx->d_qpart, ctx->contour_blocks * sizeof(double)));
   int rc = F->t64 ? alloc_t<double>(ctx, F, gam_elems) : alloc_t<float>(ctx, F, gam_elems);
   if (rc) return rc;
@@ -528,7 +551,7 @@ int film_create(adscf_ctx* ctx, const adscf_params* p) {
     CK(cudaMemsetAsync(ctx->d_tmp, 0, n * sizeof(double), ctx->stream));
     const FieldRef fr = make_ref(ctx, ctx->d_tmp);
     k_film_fill<float><<<std::max(1, (D.npts + 255) / 256), 256, 0, ctx->stream>>>(D.q, D.qd, D.npts);
-    k_film_wconv<<<(int)std::min<size_t>((n + 255) / 256, 152 * 4), 256, 0, ctx->stream>>>(fr, D.wf, n);
+    field_f32(D, fr, n, ctx->stream);
     CK(cudaGetLastError());
     return adi_tune(ctx, F, D, fr);
   }

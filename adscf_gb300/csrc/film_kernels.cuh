@@ -59,8 +59,8 @@ struct FilmDev {
   // ADI (Film_3D) only
   double dx, dy;
   T* w1;                 // [2][npts] intermediate q*, q** of the ADI sweeps
-  // FP32 line sweeps (1D chains): FP32 copies of the mesh factors and, for
-  // single contexts, of the field ([ntypes][npts], filled per propagation)
+  // FP32 sweeps: FP32 copies of the mesh factors and, for the ADI sweeps, of
+  // the field ([ntypes][npts], filled per propagation)
   const float* alf;
   const float* bef;
   const float* gaf;
@@ -208,7 +208,6 @@ __device__ __forceinline__ void film1d_chain(const FilmDev<T>& F, const double* 
     const CnStep st = cn_step(film_ds(F.dss, dir, s, F.ns));
     const int ty = (F.brush || F.single) ? 0 : film_type(dir, s, F.ns, F.na);
     const double* w = field + (size_t)ty * F.npts;
-    const float* wl = sizeof(T) == 4 ? F.wf + (size_t)ty * F.npts : nullptr;
     const T* qp = chain + (size_t)(s - 1) * F.npts;
     T* qn = chain + (size_t)s * F.npts;
     // forward elimination (increment form for FP32 sweeps, see cn_rhs)
@@ -224,7 +223,7 @@ __device__ __forceinline__ void film1d_chain(const FilmDev<T>& F, const double* 
         const T q_jp1 = qp[(size_t)(j + 1) * L + line];
         const size_t i = (size_t)j * L + line;
         T b, hw;
-        cn_row<T>(F, st, j, sizeof(T) == 4 ? 0.0 : w[i], sizeof(T) == 4 ? wl[i] : 0.f, a, c, b, hw);
+        cn_row<T>(F, st, j, w[i], (float)w[i], a, c, b, hw);
         diag = r_add(r_add((T)1, b), hw);
         rhs = cn_rhs<T>(a, b, c, hw, q_jm1, q_j, q_jp1);
         q_jm1 = q_j;
@@ -547,6 +546,7 @@ __device__ __forceinline__ void film_contour_body(const FilmDev<T>& F, int bid, 
   } else {
     for (int p = bid * blockDim.x + threadIdx.x; p < F.npts; p += nb * blockDim.x) {
       double a0 = 0.0, a1 = 0.0;
+#pragma unroll 4
       for (int s = 0; s <= N; ++s) {
         const double pr = (double)F.q[(size_t)s * np + p] * (double)F.qd[(size_t)(N - s) * np + p];
         a0 += F.wA[s] * pr;
@@ -567,6 +567,64 @@ __device__ __forceinline__ void film_contour_body(const FilmDev<T>& F, int bid, 
 template <typename T>
 __global__ void __launch_bounds__(256)
 k_film_contour(FilmDev<T> F) { film_contour_body<T>(F, blockIdx.x, gridDim.x); }
+
+// The same for a film of few points: with one thread per point a 1001-point
+// line has four blocks, each thread waiting on Ns + 1 slice loads in turn.
+// Here a block takes 32 points and deals the nodes to its 32 warps (node s to
+// warp s mod 32), each summing as above; the 32 partial sums of a point are
+// added in FP64 in the order of the warps.
+template <typename T>
+__global__ void __launch_bounds__(1024)
+k_film_contour_s(FilmDev<T> F) {
+  __shared__ double part[2][32][33];
+  const int lane = threadIdx.x & 31, g = threadIdx.x >> 5;
+  const int p = blockIdx.x * 32 + lane;
+  const int N = F.ns;
+  const size_t np = F.npts;
+  double a0 = 0.0, a1 = 0.0;
+  if (p < F.npts) {
+    if constexpr (sizeof(T) == 4) {
+      float ah = 0.f, al = 0.f, bh = 0.f, bl = 0.f;
+#pragma unroll 4
+      for (int s = g; s <= N; s += 32) {
+        const float x = F.q[(size_t)s * np + p], y = F.qd[(size_t)(N - s) * np + p];
+        const double wa = F.wA[s], wb = F.ntypes == 2 ? F.wB[s] : 0.0;
+        const float wah = (float)wa, wbh = (float)wb;
+        ffw_add(ah, al, x, y, make_float2(wah, (float)(wa - (double)wah)));
+        if (F.ntypes == 2) ffw_add(bh, bl, x, y, make_float2(wbh, (float)(wb - (double)wbh)));
+      }
+      a0 = (double)ah + (double)al;
+      a1 = (double)bh + (double)bl;
+    } else {
+#pragma unroll 4
+      for (int s = g; s <= N; s += 32) {
+        const double pr = (double)F.q[(size_t)s * np + p] * (double)F.qd[(size_t)(N - s) * np + p];
+        a0 += F.wA[s] * pr;
+        if (F.ntypes == 2) a1 += F.wB[s] * pr;
+      }
+    }
+  }
+  part[0][g][lane] = a0;
+  part[1][g][lane] = a1;
+  __syncthreads();
+  if (g < F.ntypes && p < F.npts) {   // warp 0: block A (or homopolymer), warp 1: block B
+    double t = 0.0;
+#pragma unroll
+    for (int k = 0; k < 32; ++k) t += part[g][k][lane];
+    F.dist[(size_t)g * np + p] = t;
+  }
+  if (g == 0) {
+    double qn = 0.0;
+    if (p < F.npts) {
+      qn = (double)F.q[(size_t)N * np + p];
+      if (F.brush) qn *= (double)F.qd[p];
+      qn *= F.wz[p / F.nlines];
+    }
+#pragma unroll
+    for (int o = 16; o; o >>= 1) qn += __shfl_xor_sync(0xffffffffu, qn, o);
+    if (lane == 0) F.qpart[blockIdx.x] = qn;
+  }
+}
 
 // ---------------------------------------------------------------------------
 // Film batches: many independent one-line films (Film_1D or brush), each

@@ -1,5 +1,5 @@
-// film_warp.cuh -- warp-cooperative tridiagonal line solves for the FP32
-// (split precision) Crank-Nicolson sweeps of films and brushes.
+// film_warp.cuh -- cooperative tridiagonal line solves for the Crank-Nicolson
+// sweeps of films and brushes: a warp, part of one, or several warps per line.
 //
 // The reference solves every line with a serial Thomas recurrence (tridiag,
 // Film_CK_AD/Film_3D/Geometry_Modules/mod_realspace.f90:184-215; the 1D CN
@@ -21,15 +21,49 @@
 //  - the interior unknowns then follow from their lane's two separators.
 //
 // The matrix is that of the reference; only the elimination order differs,
-// so the result equals the serial solve up to FP32 rounding (the systems are
-// diagonally dominant: 1 + hw > 0 beyond the off-diagonals).  Pivots are FP32
-// reciprocals (rcp.approx, as the serial FP32 sweeps); a zero pivot sets the
-// error flag like the serial solve.  The sweeps solve for the increment
-// u = q' - q of the step (see cn_rhs), so Dirichlet rows give u = -q.
+// so the result equals the serial solve up to rounding (the systems are
+// diagonally dominant: 1 + hw > 0 beyond the off-diagonals).  Pivots are
+// multiplied by their reciprocals (FP32: rcp.approx, as the serial FP32
+// sweeps); a zero pivot sets the error flag like the serial solve.  The FP32
+// sweeps solve for the increment u = q' - q of the step (see cn_rhs), so
+// Dirichlet rows give u = -q.
 #pragma once
 #include "film_kernels.cuh"
 
 namespace fw {
+
+// pivots: the hardware reciprocal in FP32 (see rcp_hw), correctly rounded in FP64
+__device__ __forceinline__ float rcp(float x) { return rcp_hw(x); }
+__device__ __forceinline__ double rcp(double x) { return __drcp_rn(x); }
+
+// Local elimination of the interior rows 0..K-2 of a lane with three
+// right-hand sides -- r, -a_0 at the first row, -c_{K-2} at the last row: on
+// return row i is x_i + y_i u(left separator) + z_i u(own separator).
+template <typename T, int K>
+__device__ __forceinline__ void eliminate(const T (&a)[K], const T (&d)[K], const T (&c)[K], const T (&r)[K],
+                                          T (&x)[K - 1], T (&y)[K - 1], T (&z)[K - 1], int* err) {
+  T g[K - 1];
+  T bet = (T)1;
+#pragma unroll
+  for (int i = 0; i < K - 1; ++i) {
+    const int im = i > 0 ? i - 1 : 0;
+    const T gi = i == 0 ? (T)0 : r_mul(c[im], bet);
+    const T piv = i == 0 ? d[0] : r_fma(-a[i], gi, d[i]);
+    if (piv == (T)0) atomicOr(err, 1);
+    bet = rcp(piv);
+    g[i] = gi;
+    x[i] = r_mul(i == 0 ? r[0] : r_fma(-a[i], x[im], r[i]), bet);
+    y[i] = r_mul(i == 0 ? -a[0] : r_mul(-a[i], y[im]), bet);
+    const T zr = i == K - 2 ? -c[i] : (T)0;
+    z[i] = r_mul(i == 0 ? zr : r_fma(-a[i], z[im], zr), bet);
+  }
+#pragma unroll
+  for (int i = K - 3; i >= 0; --i) {
+    x[i] = r_fma(-g[i + 1], x[i + 1], x[i]);
+    y[i] = r_fma(-g[i + 1], y[i + 1], y[i]);
+    z[i] = r_fma(-g[i + 1], z[i + 1], z[i]);
+  }
+}
 
 // One line system on the G-lane group of the calling lane.  Lane l of the
 // group owns K consecutive rows (rows past the line's end are identity rows
@@ -40,111 +74,128 @@ namespace fw {
 // separator through a, and that separator to row 0 through c (all G lanes
 // own rows).  K is a compile-time constant so that every row stays in
 // registers.  All G lanes of the group must call it together.
-template <int G, int K>
-__device__ __forceinline__ void solve(const float (&a)[K], const float (&d)[K], const float (&c)[K],
-                                      float (&r)[K], bool periodic, int* err) {
+template <int G, int K, typename T>
+__device__ __forceinline__ void solve(const T (&a)[K], const T (&d)[K], const T (&c)[K],
+                                      T (&r)[K], bool periodic, int* err) {
   static_assert(K >= 2, "a lane needs an interior row and a separator");
   const int lane = threadIdx.x & 31;
   const int gl = lane & (G - 1);          // lane within the group
   const int base = lane - gl;
   const unsigned mask = 0xffffffffu;
-  float x[K - 1], y[K - 1], z[K - 1], g[K - 1];
-  // local elimination of the interior rows 0..K-2 with three right-hand
-  // sides: r, -a_0 at the first row, -c_{K-2} at the last row
-  float bet = 1.f;
-#pragma unroll
-  for (int i = 0; i < K - 1; ++i) {
-    const int im = i > 0 ? i - 1 : 0;
-    const float gi = i == 0 ? 0.f : __fmul_rn(c[im], bet);
-    const float piv = i == 0 ? d[0] : __fmaf_rn(-a[i], gi, d[i]);
-    if (piv == 0.f) atomicOr(err, 1);
-    bet = rcp_hw(piv);
-    g[i] = gi;
-    x[i] = __fmul_rn(i == 0 ? r[0] : __fmaf_rn(-a[i], x[im], r[i]), bet);
-    y[i] = __fmul_rn(i == 0 ? -a[0] : __fmul_rn(-a[i], y[im]), bet);
-    const float zr = i == K - 2 ? -c[i] : 0.f;
-    z[i] = __fmul_rn(i == 0 ? zr : __fmaf_rn(-a[i], z[im], zr), bet);
-  }
-#pragma unroll
-  for (int i = K - 3; i >= 0; --i) {
-    x[i] = __fmaf_rn(-g[i + 1], x[i + 1], x[i]);
-    y[i] = __fmaf_rn(-g[i + 1], y[i + 1], y[i]);
-    z[i] = __fmaf_rn(-g[i + 1], z[i + 1], z[i]);
-  }
+  T x[K - 1], y[K - 1], z[K - 1];
+  eliminate<T, K>(a, d, c, r, x, y, z, err);
   // the separator row in its neighbours' terms: the last interior row of this
   // lane and the first interior row of the next lane
   constexpr int S = K - 1, Li = K - 2;
   const int nx = base + ((gl + 1) & (G - 1));
-  float xn = __shfl_sync(mask, x[0], nx), yn = __shfl_sync(mask, y[0], nx), zn = __shfl_sync(mask, z[0], nx);
-  if (!periodic && gl == G - 1) { xn = 0.f; yn = 0.f; zn = 0.f; }
-  float A = __fmul_rn(a[S], y[Li]);
-  float B = __fmaf_rn(c[S], yn, __fmaf_rn(a[S], z[Li], d[S]));
-  float C = __fmul_rn(c[S], zn);
-  float R = __fmaf_rn(-c[S], xn, __fmaf_rn(-a[S], x[Li], r[S]));
+  T xn = __shfl_sync(mask, x[0], nx), yn = __shfl_sync(mask, y[0], nx), zn = __shfl_sync(mask, z[0], nx);
+  if (!periodic && gl == G - 1) { xn = (T)0; yn = (T)0; zn = (T)0; }
+  T A = r_mul(a[S], y[Li]);
+  T B = r_fma(c[S], yn, r_fma(a[S], z[Li], d[S]));
+  T C = r_mul(c[S], zn);
+  T R = r_fma(-c[S], xn, r_fma(-a[S], x[Li], r[S]));
   // parallel cyclic reduction over the group (identity beyond its ends
   // unless periodic)
 #pragma unroll
   for (int st = 1; st < G; st *= 2) {
     const int su = base + ((gl - st) & (G - 1)), sd = base + ((gl + st) & (G - 1));
-    float Au = __shfl_sync(mask, A, su), Bu = __shfl_sync(mask, B, su);
-    float Cu = __shfl_sync(mask, C, su), Ru = __shfl_sync(mask, R, su);
-    float Ad = __shfl_sync(mask, A, sd), Bd = __shfl_sync(mask, B, sd);
-    float Cd = __shfl_sync(mask, C, sd), Rd = __shfl_sync(mask, R, sd);
-    if (!periodic && gl - st < 0) { Au = 0.f; Bu = 1.f; Cu = 0.f; Ru = 0.f; }
-    if (!periodic && gl + st >= G) { Ad = 0.f; Bd = 1.f; Cd = 0.f; Rd = 0.f; }
-    if (Bu == 0.f || Bd == 0.f) atomicOr(err, 1);
-    const float kl = __fmul_rn(A, rcp_hw(Bu));
-    const float kr = __fmul_rn(C, rcp_hw(Bd));
-    const float nB = __fmaf_rn(-kr, Ad, __fmaf_rn(-kl, Cu, B));
-    const float nR = __fmaf_rn(-kr, Rd, __fmaf_rn(-kl, Ru, R));
-    A = __fmul_rn(-kl, Au);
-    C = __fmul_rn(-kr, Cd);
+    T Au = __shfl_sync(mask, A, su), Bu = __shfl_sync(mask, B, su);
+    T Cu = __shfl_sync(mask, C, su), Ru = __shfl_sync(mask, R, su);
+    T Ad = __shfl_sync(mask, A, sd), Bd = __shfl_sync(mask, B, sd);
+    T Cd = __shfl_sync(mask, C, sd), Rd = __shfl_sync(mask, R, sd);
+    if (!periodic && gl - st < 0) { Au = (T)0; Bu = (T)1; Cu = (T)0; Ru = (T)0; }
+    if (!periodic && gl + st >= G) { Ad = (T)0; Bd = (T)1; Cd = (T)0; Rd = (T)0; }
+    if (Bu == (T)0 || Bd == (T)0) atomicOr(err, 1);
+    const T kl = r_mul(A, rcp(Bu));
+    const T kr = r_mul(C, rcp(Bd));
+    const T nB = r_fma(-kr, Ad, r_fma(-kl, Cu, B));
+    const T nR = r_fma(-kr, Rd, r_fma(-kl, Ru, R));
+    A = r_mul(-kl, Au);
+    C = r_mul(-kr, Cd);
     B = nB;
     R = nR;
   }
   // after log2 G steps the reduced equation couples only to the lane itself:
   // periodic lines reach it through both neighbours, open lines never
-  const float den = periodic ? __fadd_rn(__fadd_rn(A, C), B) : B;
-  if (den == 0.f) atomicOr(err, 1);
-  const float v = __fmul_rn(R, rcp_hw(den));          // u at this lane's separator
-  float vl = __shfl_sync(mask, v, base + ((gl - 1) & (G - 1)));
-  if (!periodic && gl == 0) vl = 0.f;
+  const T den = periodic ? r_add(r_add(A, C), B) : B;
+  if (den == (T)0) atomicOr(err, 1);
+  const T v = r_mul(R, rcp(den));          // u at this lane's separator
+  T vl = __shfl_sync(mask, v, base + ((gl - 1) & (G - 1)));
+  if (!periodic && gl == 0) vl = (T)0;
 #pragma unroll
-  for (int i = 0; i < K - 1; ++i) r[i] = __fmaf_rn(z[i], v, __fmaf_rn(y[i], vl, x[i]));
+  for (int i = 0; i < K - 1; ++i) r[i] = r_fma(z[i], v, r_fma(y[i], vl, x[i]));
   r[S] = v;
 }
 
 }  // namespace fw
 
 // ---------------------------------------------------------------------------
-// 1D CN chain (Film_1D / brush, FP32 increment form) with one warp per
-// (line, chain): lane l owns rows [l K, l K + K - 1] of the line's gz + 1
-// rows (K = film_warp_rows; rows past the wall are identity padding), keeps
-// their q in registers for the whole contour, exchanges edge values by
-// shuffles, and solves each step with fw::solve.  Per-warp shared
-// memory `sm` holds, by row: the FP32 mesh factors alpha, gamma, the FP32
-// field of types 0 and 1, and a staging row through which each finished
-// slice goes to global memory (coalesced for one-line films).  `chain`:
-// slices [(ns+1)][npts] of the chain, rows of this line at stride `stride`.
+// 1D CN chain (Film_1D / brush) with one warp per (line, chain): lane l owns
+// rows [l K, l K + K - 1] of the line's gz + 1 rows (K = film_warp_rows; rows
+// past the wall are identity padding), keeps their q in registers for the
+// whole contour, and solves each step with fw::solve.  `chain`: slices
+// [(ns+1)][npts] of the chain, rows of this line at stride `stride`.
+//
+// FP32 solves for the increment u = q' - q (see cn_rhs).  FP64 writes the
+// step (1 + ds M) q' = (1 - ds M) q as (1 + ds M) v = q, q' = 2 v - q (on the
+// walls v = q / 2, so q' = 0): the right-hand side is q itself, which spares
+// five FP64 operations a row and the neighbours' values on GB300's narrow
+// FP64 pipe.  The matrix is the reference's; the elimination order is not,
+// so results equal the serial Thomas solve to rounding.
+//
+// Bound: FP64 issue (a warp instruction per 64 cycles on each SM quarter), in
+// FP32 the latency of the solve's dependent operations.
+//
+// Per-warp shared memory `sm` holds, by row: the mesh factors alpha, gamma,
+// the term of types 0 and 1 that multiplies the step (FP32: the field, FP64:
+// beta + w / 2), and a staging row through which each finished slice goes to
+// global memory (coalesced for one-line films).
 // ---------------------------------------------------------------------------
 constexpr int kFilmWarpM = 8;                 // rows per lane at most: lines up to 32 * 8 planes
 constexpr int kFilmWarpRows = 32 * kFilmWarpM;
+template <typename T>
 struct FilmWarpSm {
-  float al[kFilmWarpRows], ga[kFilmWarpRows], w0[kFilmWarpRows], w1[kFilmWarpRows], stage[kFilmWarpRows];
+  T al[kFilmWarpRows], ga[kFilmWarpRows], w0[kFilmWarpRows], w1[kFilmWarpRows], stage[kFilmWarpRows];
 };
 
-template <int K>
-__device__ __forceinline__ void film1d_chain_warp(const FilmDev<float>& F, int dir, float* chain,
-                                                  size_t stride, FilmWarpSm& sm) {
+// One CN row of a step: matrix and right-hand side from the mesh factors al,
+// ga and the step's term w (FP32: field, FP64: beta + w / 2); qm, q0, qp: q
+// of the row and its neighbours (FP64 reads q0 only)
+template <typename T>
+__device__ __forceinline__ void cn_line_row(const CnStep& st, T al, T ga, T w, T qm, T q0, T qp,
+                                            T& a, T& d, T& c, T& r) {
+  if constexpr (sizeof(T) == 4) {
+    const float hw = __fmul_rn(st.hdsf, w);
+    a = __fmul_rn(-st.dsf, al);
+    c = __fmul_rn(-st.dsf, ga);
+    const float b = -__fadd_rn(a, c);
+    d = __fadd_rn(__fadd_rn(1.f, b), hw);
+    r = cn_rhs<float>(a, b, c, hw, qm, q0, qp);
+  } else {
+    a = r_mul(-st.ds, al);
+    c = r_mul(-st.ds, ga);
+    d = r_fma(st.ds, w, 1.0);
+    r = q0;
+  }
+}
+// right-hand side of a wall row, and the new q of a row from its solution u
+__device__ __forceinline__ float cn_wall_rhs(float q) { return -q; }
+__device__ __forceinline__ double cn_wall_rhs(double q) { return r_mul(0.5, q); }
+__device__ __forceinline__ float cn_new_q(float q, float u) { return __fadd_rn(q, u); }
+__device__ __forceinline__ double cn_new_q(double q, double u) { return r_fma(2.0, u, -q); }
+
+template <int K, typename T>
+__device__ __forceinline__ void film1d_chain_warp(const FilmDev<T>& F, int dir, T* chain,
+                                                  size_t stride, FilmWarpSm<T>& sm) {
   const int lane = threadIdx.x & 31;
   const int n = F.gz + 1;
   const int s0 = lane * K;                    // this lane's rows s0 .. s0 + K - 1
-  float q[K];
+  T q[K];
 #pragma unroll
   for (int i = 0; i < K; ++i) {
     const int j = s0 + i;
-    float v = 0.f;
-    if (j < n) v = F.single ? chain[(size_t)j * stride] : (dir == 1 && F.brush) ? (float)F.graft[j] : 1.f;
+    T v = (T)0;
+    if (j < n) v = F.single ? chain[(size_t)j * stride] : (dir == 1 && F.brush) ? (T)F.graft[j] : (T)1;
     q[i] = v;
   }
   if (!F.single) {
@@ -158,37 +209,33 @@ __device__ __forceinline__ void film1d_chain_warp(const FilmDev<float>& F, int d
   for (int s = 1; s <= F.ns; ++s) {
     const CnStep st = cn_step(film_ds(F.dss, dir, s, F.ns));
     const int ty = (F.brush || F.single) ? 0 : film_type(dir, s, F.ns, F.na);
-    const float* wl = ty == 0 ? sm.w0 : sm.w1;
-    // edge values of the neighbouring lanes' rows
-    const float qprev = __shfl_up_sync(0xffffffffu, q[K - 1], 1);
-    const float qnext = __shfl_down_sync(0xffffffffu, q[0], 1);
-    float a[K], d[K], c[K], r[K];
+    const T* wl = ty == 0 ? sm.w0 : sm.w1;
+    // FP32: edge values of the neighbouring lanes' rows
+    T qprev = (T)0, qnext = (T)0;
+    if constexpr (sizeof(T) == 4) {
+      qprev = __shfl_up_sync(0xffffffffu, q[K - 1], 1);
+      qnext = __shfl_down_sync(0xffffffffu, q[0], 1);
+    }
+    T a[K], d[K], c[K], r[K];
 #pragma unroll
     for (int i = 0; i < K; ++i) {
       const int j = s0 + i;
-      a[i] = 0.f; d[i] = 1.f; c[i] = 0.f; r[i] = 0.f;
+      a[i] = (T)0; d[i] = (T)1; c[i] = (T)0; r[i] = (T)0;
       if (j < n) {
         if (j == 0 || j == n - 1) {
-          r[i] = -q[i];                        // Dirichlet wall: q' = 0
+          r[i] = cn_wall_rhs(q[i]);            // Dirichlet wall: q' = 0
         } else {
-          const float qm = i == 0 ? qprev : q[i > 0 ? i - 1 : 0];
-          const float qp = i == K - 1 ? qnext : q[i + 1 < K ? i + 1 : i];
-          const float ai = __fmul_rn(-st.dsf, sm.al[j]);
-          const float ci = __fmul_rn(-st.dsf, sm.ga[j]);
-          const float bi = -__fadd_rn(ai, ci);
-          const float hw = __fmul_rn(st.hdsf, wl[j]);
-          a[i] = ai;
-          c[i] = ci;
-          d[i] = __fadd_rn(__fadd_rn(1.f, bi), hw);
-          r[i] = cn_rhs<float>(ai, bi, ci, hw, qm, q[i], qp);
+          const T qm = i == 0 ? qprev : q[i > 0 ? i - 1 : 0];
+          const T qp = i == K - 1 ? qnext : q[i + 1 < K ? i + 1 : i];
+          cn_line_row<T>(st, sm.al[j], sm.ga[j], wl[j], qm, q[i], qp, a[i], d[i], c[i], r[i]);
         }
       }
     }
     fw::solve<32, K>(a, d, c, r, false, F.err);
-    float* qn = chain + (size_t)s * F.npts;
+    T* qn = chain + (size_t)s * F.npts;
 #pragma unroll
     for (int i = 0; i < K; ++i) {
-      q[i] = __fadd_rn(q[i], r[i]);
+      q[i] = cn_new_q(q[i], r[i]);
       if (s0 + i < n) sm.stage[s0 + i] = q[i];
     }
     __syncwarp();
@@ -200,8 +247,9 @@ __device__ __forceinline__ void film1d_chain_warp(const FilmDev<float>& F, int d
 // rows per lane of an n-row line: the smallest K >= 2 with 32 K >= n
 __host__ __device__ __forceinline__ int film_warp_rows(int n) { return n <= 64 ? 2 : (n + 31) / 32; }
 
-__device__ __forceinline__ void film1d_chain_warp_any(const FilmDev<float>& F, int dir, float* chain,
-                                                      size_t stride, FilmWarpSm& sm) {
+template <typename T>
+__device__ __forceinline__ void film1d_chain_warp_any(const FilmDev<T>& F, int dir, T* chain,
+                                                      size_t stride, FilmWarpSm<T>& sm) {
   switch (film_warp_rows(F.gz + 1)) {
     case 2: film1d_chain_warp<2>(F, dir, chain, stride, sm); break;
     case 3: film1d_chain_warp<3>(F, dir, chain, stride, sm); break;
@@ -213,57 +261,359 @@ __device__ __forceinline__ void film1d_chain_warp_any(const FilmDev<float>& F, i
   }
 }
 
-// mesh factors and FP32 field of one line into the warp's shared memory
-__device__ __forceinline__ void film_warp_tables(const FilmDev<float>& F, const float* w0, const float* w1,
-                                                 size_t wstride, FilmWarpSm& sm) {
+// mesh factors al, ga of row j and the term of field value w there (see
+// cn_line_row); w32: the FP32 copy of the field value
+template <typename T>
+__device__ __forceinline__ T cn_mesh(const FilmDev<T>& F, int j, bool up) {
+  if constexpr (sizeof(T) == 4) return up ? F.gaf[j] : F.alf[j];
+  else return up ? F.gamma[j] : F.alpha[j];
+}
+template <typename T>
+__device__ __forceinline__ T cn_term(const FilmDev<T>& F, int j, double w) {
+  if constexpr (sizeof(T) == 4) return (float)w;
+  else return r_fma(0.5, w, F.beta[j]);
+}
+
+// mesh factors and field terms of one line into the warp's shared memory;
+// `field`: [ntypes][npts], rows of the line at stride `wstride` (FP32: the
+// rounding to FP32 that k_film_wconv makes)
+template <typename T>
+__device__ __forceinline__ void film_warp_tables(const FilmDev<T>& F, const double* field, size_t wstride,
+                                                 FilmWarpSm<T>& sm) {
   const int lane = threadIdx.x & 31;
   for (int j = lane; j <= F.gz; j += 32) {
-    sm.al[j] = F.alf[j];
-    sm.ga[j] = F.gaf[j];
-    sm.w0[j] = w0[(size_t)j * wstride];
-    sm.w1[j] = w1 ? w1[(size_t)j * wstride] : 0.f;
+    sm.al[j] = cn_mesh<T>(F, j, false);
+    sm.ga[j] = cn_mesh<T>(F, j, true);
+    sm.w0[j] = cn_term<T>(F, j, field[(size_t)j * wstride]);
+    sm.w1[j] = F.ntypes == 2 && !F.single ? cn_term<T>(F, j, field[F.npts + (size_t)j * wstride]) : (T)0;
   }
   __syncwarp();
 }
 
+// Whether every system of a line's chains is diagonally dominant: 1 + ds w / 2
+// >= 0.01 for the largest step and the lowest field value (the mesh terms
+// are, b = |a| + |c|).  Then no elimination order meets a zero pivot.  Where
+// it is not, the order decides which pivots vanish and how far rounding
+// grows, and the chain runs the reference's serial recurrence instead
+// (film1d_chain).  Every lane of a warp calls it; the answer is uniform over
+// the warps of a line.
+template <typename T>
+__device__ __forceinline__ bool film_line_dominant(const FilmDev<T>& F, const double* field, size_t wstride) {
+  double lo = 0.0;
+  const int types = F.single ? 1 : F.ntypes;
+  for (int t = 0; t < types; ++t)
+    for (int j = threadIdx.x & 31; j <= F.gz; j += 32) lo = fmin(lo, field[(size_t)t * F.npts + (size_t)j * wstride]);
+#pragma unroll
+  for (int o = 16; o; o >>= 1) lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+  if (lo >= 0.0) return true;
+  double ds = 0.0;
+  for (int s = 1 + (threadIdx.x & 31); s <= F.ns; s += 32) ds = fmax(ds, F.dss[s]);
+#pragma unroll
+  for (int o = 16; o; o >>= 1) ds = fmax(ds, __shfl_xor_sync(0xffffffffu, ds, o));
+  return 1.0 + 0.5 * ds * lo >= 0.01;
+}
+
 // Single context (Film_1D / brush lines of one film): one warp per (line,
 // chain); blockIdx.y = chain.
-static __global__ void __launch_bounds__(128)
-k_film1d_warp(FilmDev<float> F) {
-  __shared__ FilmWarpSm sm_all[4];
+template <typename T>
+__global__ void __launch_bounds__(128)
+k_film1d_warp(FilmDev<T> F, FieldRef fr) {
+  __shared__ FilmWarpSm<T> sm_all[4];
   const int wib = threadIdx.x >> 5;
   const int line = blockIdx.x * 4 + wib;
   if (line >= F.nlines) return;
   const int dir = blockIdx.y;
   const size_t L = F.nlines;
-  FilmWarpSm& sm = sm_all[wib];
-  film_warp_tables(F, F.wf + line, F.ntypes == 2 ? F.wf + F.npts + line : nullptr, L, sm);
-  film1d_chain_warp_any(F, dir, (dir == 0 ? F.q : F.qd) + line, L, sm);
+  FilmWarpSm<T>& sm = sm_all[wib];
+  if (sizeof(T) == 8 && !film_line_dominant<T>(F, fr.get() + line, L)) {
+    if ((threadIdx.x & 31) == 0) film1d_chain<T>(F, fr.get(), line, dir);
+    return;
+  }
+  film_warp_tables<T>(F, fr.get() + line, L, sm);
+  film1d_chain_warp_any<T>(F, dir, (dir == 0 ? F.q : F.qd) + line, L, sm);
 }
 
 // Batch: one warp per (film, chain) of `items` ((film << 1) | chain, longest
 // contours first), the field from the film's current SCF history slot.
-static __global__ void __launch_bounds__(128)
-k_film1d_warp_b(const FilmDev<float>* __restrict__ Fs, const ScfDev* __restrict__ Ss,
+template <typename T>
+__global__ void __launch_bounds__(128)
+k_film1d_warp_b(const FilmDev<T>* __restrict__ Fs, const ScfDev* __restrict__ Ss,
                 const int* __restrict__ items, int nitems) {
-  __shared__ FilmWarpSm sm_all[4];
+  __shared__ FilmWarpSm<T> sm_all[4];
   const int wib = threadIdx.x >> 5;
   const int it = blockIdx.x * 4 + wib;
   if (it >= nitems) return;
   const int f = items[it] >> 1, dir = items[it] & 1;
-  const FilmDev<float> F = Fs[f];
+  const FilmDev<T> F = Fs[f];
   const ScfDev& S = Ss[f];
   const double* field = S.hx + (size_t)((*S.iter) % S.slots) * ((size_t)S.ntypes * S.npts);
-  FilmWarpSm& sm = sm_all[wib];
-  const int lane = threadIdx.x & 31;
-  for (int j = lane; j <= F.gz; j += 32) {
-    sm.al[j] = F.alf[j];
-    sm.ga[j] = F.gaf[j];
-    sm.w0[j] = (float)field[j];
-    sm.w1[j] = F.ntypes == 2 ? (float)field[F.npts + j] : 0.f;
+  FilmWarpSm<T>& sm = sm_all[wib];
+  if (sizeof(T) == 8 && !film_line_dominant<T>(F, field, 1)) {
+    if ((threadIdx.x & 31) == 0) film1d_chain<T>(F, field, 0, dir);
+    return;
   }
-  __syncwarp();
-  film1d_chain_warp_any(F, dir, dir == 0 ? F.q : F.qd, 1, sm);
+  film_warp_tables<T>(F, field, 1, sm);
+  film1d_chain_warp_any<T>(F, dir, dir == 0 ? F.q : F.qd, 1, sm);
+}
+
+// ---------------------------------------------------------------------------
+// Longer lines (257 .. 4096 rows): W warps per (line, chain), K = 4 rows per
+// lane, W the power of two >= rows / 128.  Each warp reduces its 128 rows to
+// one equation in the last rows of itself and its neighbours:
+//  - lanes eliminate their interior rows (fw::eliminate), then the warp's 31
+//    first separators by cyclic reduction with the warp's two boundary
+//    unknowns as extra right-hand sides, so every row of the warp is
+//    x + y U(previous warp) + z U(this warp), U = solution at a warp's last row;
+//  - the warps exchange seven numbers each (their last row's equation and
+//    their first row's x, y, z) and every warp solves the W equations in U
+//    itself, one lane per equation: one barrier per contour step.
+// The exchange slots are double buffered by step parity: a warp writes the
+// slots of step s + 2 only after the barrier of step s + 1, which every warp
+// passes after its reads of step s.
+//
+// A single line puts its warps in different CTAs of a cluster (at most 8),
+// since FP64 instructions of warps on one SM share one narrow pipe: the
+// exchange goes to every CTA's shared memory and the barrier is the
+// cluster's.  Many lines keep their warps in one CTA (clusters of one).  The
+// arithmetic is the same either way: K and W depend on the line length alone.
+// Bound: FP64 issue, one warp instruction per 64 cycles on each SM quarter.
+// Measured (GB300, FP64, against one thread per line and chain): brush of
+// 1001 rows and 1200 steps 1368 -> 11.6 ms; an SCF iteration of a 501-row
+// film with 100 steps 56.8 -> 0.95 ms.
+// ---------------------------------------------------------------------------
+constexpr int kFilmGroupK = 4;
+constexpr int kFilmGroupMaxW = 32;
+constexpr int kFilmGroupRows = kFilmGroupMaxW * 32 * kFilmGroupK;
+__host__ __device__ __forceinline__ int film_group_warps(int n) {
+  int w = 2;
+  while (w * 32 * kFilmGroupK < n) w *= 2;
+  return w;
+}
+
+namespace fw {
+
+__device__ __forceinline__ unsigned cluster_map(const void* p, int rank) {
+  unsigned a = (unsigned)__cvta_generic_to_shared(p), r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void cluster_store(unsigned addr, double v) {
+  asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(addr), "d"(v) : "memory");
+}
+__device__ __forceinline__ void cluster_store(unsigned addr, float v) {
+  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
+}
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+}  // namespace fw
+
+template <typename T>
+struct FilmGroupSm {
+  T ex[2][7][kFilmGroupMaxW];           // by step parity: A, B, R, c, x0, y0, z0 of every warp
+};
+
+// `chain`, `stride`, `field`, `wstride` as film1d_chain_warp / film_warp_tables;
+// csize: CTAs of the cluster, W = csize * (blockDim.x / 32) warps.
+template <typename T>
+__device__ __forceinline__ void film1d_chain_group(const FilmDev<T>& F, int dir, T* chain, size_t stride,
+                                                   const double* field, size_t wstride, int crank, int csize,
+                                                   FilmGroupSm<T>& sm) {
+  constexpr int K = kFilmGroupK, S = K - 1, Li = K - 2;
+  const unsigned mask = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const int W = csize * (blockDim.x >> 5);
+  const int w = crank * (blockDim.x >> 5) + (threadIdx.x >> 5);   // this warp of the line
+  const int n = F.gz + 1;
+  const int s0 = (w * 32 + lane) * K;
+  T q[K], al[K], ga[K], t0[K], t1[K];
+#pragma unroll
+  for (int i = 0; i < K; ++i) {
+    const int j = s0 + i;
+    T v = (T)0;
+    al[i] = ga[i] = t0[i] = t1[i] = (T)0;
+    if (j < n) {
+      v = F.single ? chain[(size_t)j * stride] : (dir == 1 && F.brush) ? (T)F.graft[j] : (T)1;
+      al[i] = cn_mesh<T>(F, j, false);
+      ga[i] = cn_mesh<T>(F, j, true);
+      t0[i] = cn_term<T>(F, j, field[(size_t)j * wstride]);
+      if (F.ntypes == 2 && !F.single) t1[i] = cn_term<T>(F, j, field[F.npts + (size_t)j * wstride]);
+      if (!F.single) chain[(size_t)j * stride] = v;
+    }
+    q[i] = v;
+  }
+  // FP32: q of the previous warp's last row and the next warp's first row
+  T qlo = (T)0, qhi = (T)0;
+  if constexpr (sizeof(T) == 4) {
+    auto q0_of = [&](int j) {
+      if (j < 0 || j >= n) return (T)0;
+      return F.single ? chain[(size_t)j * stride] : (dir == 1 && F.brush) ? (T)F.graft[j] : (T)1;
+    };
+    qlo = q0_of(w * 32 * K - 1);
+    qhi = q0_of((w + 1) * 32 * K);
+  }
+  for (int s = 1; s <= F.ns; ++s) {
+    const CnStep st = cn_step(film_ds(F.dss, dir, s, F.ns));
+    const int ty = (F.brush || F.single) ? 0 : film_type(dir, s, F.ns, F.na);
+    T qprev = (T)0, qnext = (T)0;
+    if constexpr (sizeof(T) == 4) {
+      qprev = __shfl_up_sync(mask, q[K - 1], 1);
+      qnext = __shfl_down_sync(mask, q[0], 1);
+      if (lane == 0) qprev = qlo;
+      if (lane == 31) qnext = qhi;
+    }
+    T a[K], d[K], c[K], r[K];
+#pragma unroll
+    for (int i = 0; i < K; ++i) {
+      const int j = s0 + i;
+      a[i] = (T)0; d[i] = (T)1; c[i] = (T)0; r[i] = (T)0;
+      if (j < n) {
+        if (j == 0 || j == n - 1) {
+          r[i] = cn_wall_rhs(q[i]);
+        } else {
+          const T qm = i == 0 ? qprev : q[i > 0 ? i - 1 : 0];
+          const T qp = i == K - 1 ? qnext : q[i + 1 < K ? i + 1 : i];
+          cn_line_row<T>(st, al[i], ga[i], ty == 0 ? t0[i] : t1[i], qm, q[i], qp, a[i], d[i], c[i], r[i]);
+        }
+      }
+    }
+    T x[K - 1], y[K - 1], z[K - 1];
+    fw::eliminate<T, K>(a, d, c, r, x, y, z, F.err);
+    // separator equations of lanes 0..30 in the warp's boundary unknowns:
+    // lane 0's left neighbour is the previous warp's last row (right-hand
+    // side Y), lane 30's right neighbour this warp's last row (Z); lane 31
+    // takes no part (identity)
+    const T xn = __shfl_down_sync(mask, x[0], 1), yn = __shfl_down_sync(mask, y[0], 1),
+            zn = __shfl_down_sync(mask, z[0], 1);
+    const T As = r_mul(a[S], y[Li]);
+    const T Bs = r_fma(a[S], z[Li], d[S]);
+    const T Rs = r_fma(-a[S], x[Li], r[S]);
+    T A = As, B = r_fma(c[S], yn, Bs), C = r_mul(c[S], zn), R = r_fma(-c[S], xn, Rs), Y = (T)0, Z = (T)0;
+    if (lane == 0) { Y = -A; A = (T)0; }
+    if (lane == 30) { Z = -C; C = (T)0; }
+    if (lane == 31) { A = (T)0; B = (T)1; C = (T)0; R = (T)0; }
+#pragma unroll
+    for (int sp = 1; sp < 32; sp *= 2) {
+      if (B == (T)0) atomicOr(F.err, 1);
+      const T iB = fw::rcp(B);
+      const int su = (lane - sp) & 31, sd = (lane + sp) & 31;
+      T Au = __shfl_sync(mask, A, su), Iu = __shfl_sync(mask, iB, su), Cu = __shfl_sync(mask, C, su);
+      T Ru = __shfl_sync(mask, R, su), Yu = __shfl_sync(mask, Y, su), Zu = __shfl_sync(mask, Z, su);
+      T Ad = __shfl_sync(mask, A, sd), Id = __shfl_sync(mask, iB, sd), Cd = __shfl_sync(mask, C, sd);
+      T Rd = __shfl_sync(mask, R, sd), Yd = __shfl_sync(mask, Y, sd), Zd = __shfl_sync(mask, Z, sd);
+      // beyond the ends A or C is zero, so the wrapped values drop out
+      const T kl = r_mul(A, Iu), kr = r_mul(C, Id);
+      B = r_fma(-kr, Ad, r_fma(-kl, Cu, B));
+      R = r_fma(-kr, Rd, r_fma(-kl, Ru, R));
+      Y = r_fma(-kr, Yd, r_fma(-kl, Yu, Y));
+      Z = r_fma(-kr, Zd, r_fma(-kl, Zu, Z));
+      A = r_mul(-kl, Au);
+      C = r_mul(-kr, Cd);
+    }
+    if (B == (T)0) atomicOr(F.err, 1);
+    const T iB = fw::rcp(B);
+    T X = r_mul(R, iB);
+    Y = r_mul(Y, iB);
+    Z = r_mul(Z, iB);
+    if (lane == 31) { X = (T)0; Y = (T)0; Z = (T)1; }   // its separator is U itself
+    // the warp's numbers: its last row's equation (lane 31, in the terms of
+    // lane 30's separator) and its first row (lane 0)
+    const T X30 = __shfl_sync(mask, X, 30), Y30 = __shfl_sync(mask, Y, 30), Z30 = __shfl_sync(mask, Z, 30);
+    const T eA = __shfl_sync(mask, r_mul(As, Y30), 31), eB = __shfl_sync(mask, r_fma(As, Z30, Bs), 31);
+    const T eR = __shfl_sync(mask, r_fma(-As, X30, Rs), 31), eC = __shfl_sync(mask, c[S], 31);
+    const T fx = __shfl_sync(mask, r_fma(z[0], X, x[0]), 0), fy = __shfl_sync(mask, r_fma(z[0], Y, y[0]), 0);
+    const T fz = __shfl_sync(mask, r_mul(z[0], Z), 0);
+    T (*ex)[kFilmGroupMaxW] = sm.ex[s & 1];
+    for (int k = lane; k < 7 * csize; k += 32) {
+      const int which = k % 7, to = k / 7;
+      const T v = which == 0 ? eA : which == 1 ? eB : which == 2 ? eR : which == 3 ? eC : which == 4 ? fx : which == 5 ? fy : fz;
+      if (csize == 1) ex[which][w] = v;
+      else fw::cluster_store(fw::cluster_map(&ex[which][w], to), v);
+    }
+    if (csize == 1) __syncthreads();
+    else fw::cluster_barrier();
+    // every warp solves the W equations, lane l the one of warp l
+    T gA = (T)0, gB = (T)1, gC = (T)0, gR = (T)0, hx = (T)0, hy = (T)0, hz = (T)0;
+    if (lane < W) {
+      gA = ex[0][lane]; gB = ex[1][lane]; gR = ex[2][lane];
+      if (lane + 1 < W) { hx = ex[4][lane + 1]; hy = ex[5][lane + 1]; hz = ex[6][lane + 1]; }
+      const T cc = ex[3][lane];
+      gB = r_fma(cc, hy, gB);
+      gR = r_fma(-cc, hx, gR);
+      gC = r_mul(cc, hz);
+      if (lane == 0) gA = (T)0;
+    }
+    for (int sp = 1; sp < W; sp *= 2) {
+      if (gB == (T)0) atomicOr(F.err, 1);
+      const T i0 = fw::rcp(gB);
+      const int su = (lane - sp) & 31, sd = (lane + sp) & 31;
+      const T Au = __shfl_sync(mask, gA, su), Iu = __shfl_sync(mask, i0, su), Cu = __shfl_sync(mask, gC, su),
+              Ru = __shfl_sync(mask, gR, su);
+      const T Ad = __shfl_sync(mask, gA, sd), Id = __shfl_sync(mask, i0, sd), Cd = __shfl_sync(mask, gC, sd),
+              Rd = __shfl_sync(mask, gR, sd);
+      const T kl = r_mul(gA, Iu), kr = r_mul(gC, Id);
+      gB = r_fma(-kr, Ad, r_fma(-kl, Cu, gB));
+      gR = r_fma(-kr, Rd, r_fma(-kl, Ru, gR));
+      gA = r_mul(-kl, Au);
+      gC = r_mul(-kr, Cd);
+    }
+    if (gB == (T)0) atomicOr(F.err, 1);
+    const T U = r_mul(gR, fw::rcp(gB));
+    const T UL = w > 0 ? __shfl_sync(mask, U, w > 0 ? w - 1 : 0) : (T)0;
+    const T UR = __shfl_sync(mask, U, w);
+    // separators of the lanes, then their interior rows
+    const T v = r_fma(Z, UR, r_fma(Y, UL, X));
+    T vl = __shfl_up_sync(mask, v, 1);
+    if (lane == 0) vl = UL;
+    T* qn = chain + (size_t)s * F.npts;
+#pragma unroll
+    for (int i = 0; i < K; ++i) {
+      const T u = i == S ? v : r_fma(z[i < S ? i : 0], v, r_fma(y[i < S ? i : 0], vl, x[i < S ? i : 0]));
+      q[i] = cn_new_q(q[i], u);
+      if (s0 + i < n) qn[(size_t)(s0 + i) * stride] = q[i];
+    }
+    if constexpr (sizeof(T) == 4) {   // the neighbouring warps' edge rows
+      const T UN = __shfl_sync(mask, U, w + 1 < W ? w + 1 : w);
+      const T nx_ = __shfl_sync(mask, hx, w), ny_ = __shfl_sync(mask, hy, w), nz_ = __shfl_sync(mask, hz, w);
+      qlo = cn_new_q(qlo, UL);
+      if (w + 1 < W) qhi = cn_new_q(qhi, r_fma(nz_, UN, r_fma(ny_, UR, nx_)));
+    }
+  }
+}
+
+// Single context: clusters of csize CTAs, one cluster per line; blockIdx.y =
+// chain.  MAXT: 256 threads keep every value of an FP64 row in registers,
+// 1024 (lines of more than 1024 rows in one CTA) spill some.
+template <typename T, int MAXT>
+__global__ void __launch_bounds__(MAXT)
+k_film1d_group(FilmDev<T> F, FieldRef fr, int csize) {
+  __shared__ FilmGroupSm<T> sm;
+  if (csize > 1) fw::cluster_barrier();   // every CTA of the cluster runs before its memory is written
+  const int line = blockIdx.x / csize, dir = blockIdx.y;
+  const size_t L = F.nlines;
+  if (!film_line_dominant<T>(F, fr.get() + line, L)) {
+    if (threadIdx.x == 0 && blockIdx.x % csize == 0) film1d_chain<T>(F, fr.get(), line, dir);
+    return;
+  }
+  film1d_chain_group<T>(F, dir, (dir == 0 ? F.q : F.qd) + line, L, fr.get() + line, L, blockIdx.x % csize, csize, sm);
+}
+
+// Batch: one CTA per (film, chain) of `items`, all with blockDim.x / 32 warps
+// per line.
+template <typename T, int MAXT>
+__global__ void __launch_bounds__(MAXT)
+k_film1d_group_b(const FilmDev<T>* __restrict__ Fs, const ScfDev* __restrict__ Ss, const int* __restrict__ items) {
+  __shared__ FilmGroupSm<T> sm;
+  const int f = items[blockIdx.x] >> 1, dir = items[blockIdx.x] & 1;
+  const FilmDev<T> F = Fs[f];
+  const ScfDev& S = Ss[f];
+  const double* field = S.hx + (size_t)((*S.iter) % S.slots) * ((size_t)S.ntypes * S.npts);
+  if (!film_line_dominant<T>(F, field, 1)) {
+    if (threadIdx.x == 0) film1d_chain<T>(F, field, 0, dir);
+    return;
+  }
+  film1d_chain_group<T>(F, dir, dir == 0 ? F.q : F.qd, 1, field, 1, 0, 1, sm);
 }
 
 // ---------------------------------------------------------------------------
