@@ -754,7 +754,7 @@ int adscf_set_pass_plan(adscf_ctx* ctx, int y, int z, int x) {
 int adscf_stage_launches(const adscf_ctx* ctx, int stage) {
   if (!ctx) return -1;
   int prop, contour = 1, update = 3;
-  if (ctx->geometry == ADSCF_BULK) prop = 1 + (ctx->plan_x == PK_FUSED ? 2 : 4) * ctx->ns;
+  if (ctx->geometry == ADSCF_BULK) prop = bulk_chain_launches(ctx);
   else prop = ctx->film_launches;
   if (ctx->geometry != ADSCF_BULK) contour = ctx->film_contour_launches;
   switch (stage) {

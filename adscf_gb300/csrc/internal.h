@@ -69,6 +69,7 @@ struct adscf_ctx {
   int xy_grid = 0;
   int* d_flags = nullptr;             // device error flags (bounded-wait expiry)
   float2* d_dcin = nullptr;           // fused XY plan: [2][gz] (0,0) pencils entering the z pass, [gz] convolved
+  struct BulkMx* mx = nullptr;        // mixed-radix passes (bulk_mx.cuh), null where the register FFT runs
   // kernel per pass of a double step (PK_*), chosen by the autotuner
   int plan_y = PK_PLAIN, plan_z = PK_PLAIN, plan_x = PK_PLAIN;
   int autotune = 1;
@@ -155,6 +156,7 @@ int d2h(adscf_ctx* ctx, double* h, const double* d, size_t n);
 int bulk_create(adscf_ctx* ctx);
 void bulk_destroy(adscf_ctx* ctx);
 int bulk_enqueue_propagate(adscf_ctx* ctx);     // from E to dist + qpart
+int bulk_chain_launches(const adscf_ctx* ctx);
 int bulk_enqueue_chains(adscf_ctx* ctx);        // both chains, all steps
 int bulk_enqueue_contour(adscf_ctx* ctx);       // contour integral + Q
 int bulk_enqueue_expfield(adscf_ctx* ctx, const double* d_w);
