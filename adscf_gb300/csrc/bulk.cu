@@ -1,5 +1,4 @@
 // bulk.cu -- plans, tables and launch sequences of the bulk propagator.
-#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -12,27 +11,8 @@
 #include "internal.h"
 #include "bulk_reg.cuh"
 #include "bulk_tma.cuh"
-#include "bulk_mx.cuh"
 #include "bulk_host.h"
-
-// Launch geometry and tables of the mixed-radix passes of one context.
-struct BulkMx {
-  mxk::Axis a[3];               // x, y, z
-  bool can_fuse = false;        // a z plane fits a block
-  bool fused = false;           // Yi + X + Yf as one plane pass
-  int rows = 1, thr_x = 32, thr_p = 256;        // x pass: rows and threads of a block; plane pass threads
-  int cols_y = 1, thr_y = 32, tiles_y = 0;      // y passes
-  int cols_z = 1, thr_z = 32, tiles_z = 0, dc_blocks = 0;
-  size_t sm_x = 0, sm_p = 0, sm_y = 0, sm_z = 0;
-  void* d_tw = nullptr;         // twiddles (cplx<T>)
-  void* d_fk = nullptr;         // diffusion factors by position (T)
-  float2* d_dc = nullptr;       // [3][gz]: dcin, dcout, kernel
-  template <typename T> mxk::Dev<T>& dev();
-  mxk::Dev<float> d32{};
-  mxk::Dev<double> d64{};
-};
-template <> mxk::Dev<float>& BulkMx::dev<float>() { return d32; }
-template <> mxk::Dev<double>& BulkMx::dev<double>() { return d64; }
+#include "launch_pdl.h"
 
 namespace {
 
@@ -218,184 +198,6 @@ int setup_tma(adscf_ctx* ctx, void* spec) {
   return ADSCF_OK;
 }
 
-// ---- mixed-radix passes (bulk_mx.cuh) ---------------------------------------
-// Radices of an n-point line, at most rmax each (at least 5): the fewest
-// stages, then the smallest largest radix; the largest comes last, where it
-// needs no twiddles.
-bool mx_axis(int n, int rmax, mxk::Axis& A) {
-  static const int kRad[] = {16, 15, 12, 10, 9, 8, 6, 5, 4, 3, 2};
-  A = mxk::Axis{};
-  A.n = n;
-  std::vector<int> best, cur;
-  auto better = [&](const std::vector<int>& c) {
-    if (best.empty()) return true;
-    if (c.size() != best.size()) return c.size() < best.size();
-    return *std::max_element(c.begin(), c.end()) < *std::max_element(best.begin(), best.end());
-  };
-  auto dfs = [&](auto&& self, int m, int cap) -> void {
-    if (m == 1) {
-      if (better(cur)) best = cur;
-      return;
-    }
-    if ((int)cur.size() == mxk::kMaxStages) return;
-    for (int r : kRad)
-      if (r <= cap && m % r == 0) {
-        cur.push_back(r);
-        self(self, m / r, r);
-        cur.pop_back();
-      }
-  };
-  if (n > 1024) return false;
-  if (n > 1) {
-    dfs(dfs, n, std::max(5, rmax));
-    if (best.empty()) return false;
-  }
-  std::sort(best.begin(), best.end());
-  A.nst = (int)best.size();
-  int m = n;
-  for (int i = 0; i < A.nst; ++i) {
-    A.rad[i] = best[i];
-    A.m[i] = m;
-    m /= best[i];
-    A.mg[i] = (1u << 20) / (unsigned)m + 1;
-  }
-  return true;
-}
-int mx_min_radix(const mxk::Axis& A) { return A.nst ? A.rad[0] : 1; }
-// frequency of position p of a line
-int mx_freq(const mxk::Axis& A, int p) {
-  int k = 0, f = 1, m = A.n;
-  for (int i = 0; i < A.nst; ++i) {
-    m /= A.rad[i];
-    k += f * (p / m);
-    p %= m;
-    f *= A.rad[i];
-  }
-  return k;
-}
-
-// diffusion factors by position, from the natural-order tables of append_tables
-template <typename T>
-int mx_factors(adscf_ctx* ctx, const std::vector<T>& fk, const std::vector<double>& g64) {
-  BulkMx* M = ctx->mx;
-  const int gx = ctx->gx, gy = ctx->gy, gz = ctx->gz;
-  const size_t nxy = (size_t)gx * gy;
-  std::vector<T> out(2 * nxy + 2 * (size_t)gz);
-  for (int h = 0; h < 2; ++h) {
-    for (int y = 0; y < gy; ++y)
-      for (int x = 0; x < gx; ++x)
-        out[h * nxy + (size_t)y * gx + x] = fk[h * nxy + (size_t)mx_freq(M->a[1], y) * gx + mx_freq(M->a[0], x)];
-    for (int z = 0; z < gz; ++z) out[2 * nxy + (size_t)h * gz + z] = fk[2 * nxy + (size_t)h * gz + mx_freq(M->a[2], z)];
-  }
-  CK(cudaMemcpy(M->d_fk, out.data(), out.size() * sizeof(T), cudaMemcpyHostToDevice));
-  if (sizeof(T) == 4) {
-    std::vector<float2> c(gz);
-    for (int i = 0; i < gz; ++i) {
-      const float h = (float)g64[i];
-      c[i] = make_float2(h, (float)(g64[i] - (double)h));
-    }
-    CK(cudaMemcpy(M->d_dc + 2 * (size_t)gz, c.data(), gz * sizeof(float2), cudaMemcpyHostToDevice));
-  }
-  return ADSCF_OK;
-}
-
-// Plans and launch geometry.  Blocks: about two per SM (152 SMs) before they
-// grow, at most 4096 (strided: 8192 FP32) points each, and one thread per
-// butterfly of the smallest radix.  FP32 radices up to 16: the fewest stages.
-// FP64 radices: npts / 19456 (the 608 SM quarters times 32 lanes), 5 at
-// least: with fewer butterflies than lanes a larger radix only lengthens
-// each quarter's program.
-template <typename T>
-int mx_setup(adscf_ctx* ctx, BulkDev<T>& I, const std::vector<T>& fk, const std::vector<double>& g64) {
-  BulkMx* M = new (std::nothrow) BulkMx();
-  if (!M) return set_err(ctx, ADSCF_E_OOM, "mixed-radix plan");
-  ctx->mx = M;
-  const int gx = ctx->gx, gy = ctx->gy, gz = ctx->gz;
-  const int rmax = sizeof(T) == 4 ? 16 : std::max(5, std::min(16, ctx->npts / 19456));
-  if (!mx_axis(gx, rmax, M->a[0]) || !mx_axis(gy, rmax, M->a[1]) || !mx_axis(gz, rmax, M->a[2])) {
-    delete M;
-    ctx->mx = nullptr;
-    return ADSCF_OK;
-  }
-  int optin = 0;
-  CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->dev));
-  const size_t es = sizeof(cplx<T>);
-  auto threads = [](size_t work, int cap) { return (int)std::min<size_t>(cap, std::max<size_t>(32, (work + 31) / 32 * 32)); };
-  const int pitch = gx | 1;
-  const int nrows = gy * gz;
-  M->rows = std::max(1, std::min((nrows + 303) / 304, std::max(1, 4096 / gx)));
-  M->thr_x = threads((size_t)M->rows * gx / mx_min_radix(M->a[0]), 256);
-  M->sm_x = ((size_t)M->rows * pitch + gx) * es;
-  auto strided = [&](int n, const mxk::Axis& A, auto&& tiles, int& cols, int& thr, int& nt) {
-    const int cmin = sizeof(T) == 8 ? 2 : 4;
-    cols = 16;
-    while (cols > cmin && (tiles(cols) < 304 || (size_t)n * cols > 65536 / sizeof(cplx<T>))) cols /= 2;
-    while (cols > 1 && tiles(cols) < 152) cols /= 2;
-    nt = tiles(cols);
-    thr = threads((size_t)n * cols / mx_min_radix(A), 256);
-  };
-  strided(gz, M->a[2], [&](int c) { return (gx * gy + c - 1) / c; }, M->cols_z, M->thr_z, M->tiles_z);
-  M->sm_z = ((size_t)gz * M->cols_z + gz) * es + 2 * (size_t)gz * sizeof(T);
-  if (sizeof(T) == 4) {
-    M->dc_blocks = (gz + M->thr_z / 32 - 1) / (M->thr_z / 32);
-    M->sm_z = std::max(M->sm_z, 2 * (size_t)gz * sizeof(float2));
-  }
-  if (gy > 1) {
-    strided(gy, M->a[1], [&](int c) { return (gx + c - 1) / c * gz; }, M->cols_y, M->thr_y, M->tiles_y);
-    M->sm_y = ((size_t)gy * M->cols_y + gy) * es;
-    M->sm_p = ((size_t)gy * pitch + gx + gy) * es;
-    M->can_fuse = M->sm_p <= (size_t)optin;
-    M->thr_p = threads((size_t)gx * gy / std::min(mx_min_radix(M->a[0]), mx_min_radix(M->a[1])), 512);
-  }
-  if (std::max(M->sm_x, std::max(M->sm_y, M->sm_z)) > (size_t)optin) {
-    delete M;
-    ctx->mx = nullptr;
-    return ADSCF_OK;
-  }
-  CK(cudaFuncSetAttribute(k_mx_xy<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
-  CK(cudaFuncSetAttribute(k_mx_xy<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
-  CK(cudaFuncSetAttribute(k_mx_s<T, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
-  CK(cudaFuncSetAttribute(k_mx_s<T, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
-  CK(cudaFuncSetAttribute(k_mx_s<T, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
-  std::vector<cplx<T>> tw;
-  std::vector<std::pair<int, int>> seen;
-  for (int d = 0; d < 3; ++d) M->a[d].tw_off = bulkhost::twiddle_offset<T>(M->a[d].n, tw, seen);
-  CK(cudaMalloc(&M->d_tw, tw.size() * es));
-  CK(cudaMemcpy(M->d_tw, tw.data(), tw.size() * es, cudaMemcpyHostToDevice));
-  CK(cudaMalloc(&M->d_fk, (2 * (size_t)gx * gy + 2 * (size_t)gz) * sizeof(T)));
-  if (sizeof(T) == 4) {
-    CK(cudaMalloc(&M->d_dc, 3 * (size_t)gz * sizeof(float2)));
-    CK(cudaMemset(M->d_dc, 0, 3 * (size_t)gz * sizeof(float2)));
-  }
-  const int rc = mx_factors<T>(ctx, fk, g64);
-  if (rc) return rc;
-  mxk::Dev<T>& D = M->dev<T>();
-  D.gx = gx; D.gy = gy; D.gz = gz;
-  D.ax = M->a[0]; D.ay = M->a[1]; D.az = M->a[2];
-  D.tw = static_cast<const cplx<T>*>(M->d_tw);
-  D.fk = static_cast<const T*>(M->d_fk);
-  D.spec = I.spec;
-  D.E = I.E;
-  D.dcin = M->d_dc;
-  D.dcout = M->d_dc + gz;
-  D.dcc = M->d_dc + 2 * (size_t)gz;
-  D.pitch = pitch;
-  D.mgx = mxk::div_magic(gx);
-  D.mgj = mxk::div_magic(gx / (M->a[0].nst ? M->a[0].rad[0] : 1));
-  // few planes leave SMs idle; FP64 is bound by how many quarters work
-  M->fused = M->can_fuse && sizeof(T) == 4;
-  return ADSCF_OK;
-}
-
-void mx_destroy(adscf_ctx* ctx) {
-  if (!ctx->mx) return;
-  cudaFree(ctx->mx->d_tw);
-  cudaFree(ctx->mx->d_fk);
-  cudaFree(ctx->mx->d_dc);
-  delete ctx->mx;
-  ctx->mx = nullptr;
-}
-
 template <typename T>
 int tune_t(adscf_ctx* ctx);
 
@@ -540,15 +342,14 @@ int create_t(adscf_ctx* ctx) {
   hb<T>(ctx) = I;
   // Mixed-radix passes where a line length has no register FFT.  Of the
   // shapes that have one on every axis, FP64 takes them too unless the axes
-  // are equal (64 x 32 x 128: 81 against 99 us a double step; FP32 20.7
-  // against 18.8, so it stays) and at 32^3, whose 1024 lines are 16
-  // register-FFT blocks on 152 SMs (42 against 60 us).
+  // are equal (one_reg; its FP32 passes at 64 x 32 x 128 take 18.8 us a double
+  // step against 20.7), and at 32^3, whose 1024 lines are 16 register-FFT
+  // blocks on 152 SMs (23 against 60 us).
   const bool all_reg = ctx->regx && ctx->regy && ctx->regz;
   const bool one_reg = all_reg && ctx->regx == ctx->regy && ctx->regx == ctx->regz;
   const bool mixed = sizeof(T) == 8 ? !one_reg || ctx->regx == 32 : !all_reg;
   if (mixed && !ctx->use_generic) {
     if ((rc = mx_setup<T>(ctx, I, fk, g64))) return rc;
-    if (ctx->mx) ctx->mx->dev<T>().I = static_cast<const BulkDev<T>*>(ctx->d_inst);
   }
   // default plan: the most specialised kernel available for each pass (the
   // fused plane pass where the TMA passes run: the tuner's choice at 64^3 and
@@ -565,49 +366,6 @@ int create_t(adscf_ctx* ctx) {
 // the same arithmetic on the same natural-order spectrum.
 template <typename T>
 int expfield_t(adscf_ctx* ctx, const double* d_w);
-
-// Launch with programmatic stream serialisation: the kernel may start while
-// the previous kernel on the stream finishes; the TMA passes wait for it
-// (griddepcontrol.wait) before they touch its output.
-template <typename... KArgs, typename... Args>
-void launch_pdl(void (*kern)(KArgs...), int grid, int block, size_t smem, cudaStream_t s,
-                Args&&... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(block);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);
-}
-
-// mixed-radix passes: real-space pass of node t (with the y transforms of its
-// planes when fused), and a whole double step
-template <typename T>
-void mx_real(adscf_ctx* ctx, int t) {
-  const BulkMx* M = ctx->mx;
-  mxk::Dev<T> D = ctx->mx->dev<T>();
-  D.slices = hb<T>(ctx).slices;
-  if (M->fused)
-    launch_pdl(k_mx_xy<T, true>, ctx->gz, M->thr_p, M->sm_p, ctx->stream, D, t, ctx->gy, mxk::div_magic(ctx->gy));
-  else
-    launch_pdl(k_mx_xy<T, false>, (ctx->gy * ctx->gz + M->rows - 1) / M->rows, M->thr_x, M->sm_x, ctx->stream, D, t,
-               M->rows, mxk::div_magic(M->rows));
-}
-template <typename T>
-void mx_step(adscf_ctx* ctx, int t) {
-  const BulkMx* M = ctx->mx;
-  mxk::Dev<T> D = ctx->mx->dev<T>();
-  const bool y = ctx->gy > 1 && !M->fused;
-  if (y) launch_pdl(k_mx_s<T, 0>, M->tiles_y, M->thr_y, M->sm_y, ctx->stream, D, M->cols_y, M->tiles_y);
-  launch_pdl(k_mx_s<T, 2>, M->tiles_z + M->dc_blocks, M->thr_z, M->sm_z, ctx->stream, D, M->cols_z, M->tiles_z);
-  if (y) launch_pdl(k_mx_s<T, 1>, M->tiles_y, M->thr_y, M->sm_y, ctx->stream, D, M->cols_y, M->tiles_y);
-  mx_real<T>(ctx, t);
-}
 
 // fused XY plane pass of step t (t = 0: the initial plane)
 template <int NN>
@@ -679,7 +437,7 @@ void step_nn(adscf_ctx* ctx, int t) {
 template <typename T>
 void step_t(adscf_ctx* ctx, int t) {
   if (ctx->mx) {
-    mx_step<T>(ctx, t);
+    mx_step(ctx, t);
     return;
   }
   // persistent and TMA passes need one register line length on all axes
@@ -703,7 +461,7 @@ template <typename T>
 int chains_t(adscf_ctx* ctx) {
   const XAux none{nullptr, nullptr, nullptr};
   if (ctx->mx) {
-    mx_real<T>(ctx, 0);
+    mx_real(ctx, 0);
   } else if (sizeof(T) == 4 && ctx->plan_x == PK_FUSED) {
     // the initial plane pass also does Yf of step 1
     if (ctx->tma == 64) xy_pass<64>(ctx, 0);
@@ -742,56 +500,13 @@ const char* pk_name(int k) {
   return k == PK_FUSED ? "fused-xy" : k == PK_TMA ? "tma" : k == PK_PERSISTENT ? "persistent" : "plain";
 }
 
-// plane pass or separate y passes of the mixed-radix plan, timed like the
-// candidates below (both do the same arithmetic)
-template <typename T>
-int mx_tune(adscf_ctx* ctx) {
-  BulkMx* M = ctx->mx;
-  if (!M->can_fuse) return ADSCF_OK;
-  const TuneKey key{ctx->dev, ctx->gx, ctx->gy, ctx->gz, ctx->prec, 16};
-  {
-    std::lock_guard<std::mutex> lk(g_tune_mu);
-    auto it = g_tune.find(key);
-    if (it != g_tune.end()) {
-      M->fused = it->second.x == PK_FUSED;
-      ctx->tune_report = it->second.report + " (cached)";
-      return ADSCF_OK;
-    }
-  }
-  CK(cudaMemsetAsync(ctx->d_tmp, 0, 2 * (size_t)ctx->npts * sizeof(double), ctx->stream));
-  int rc = expfield_t<T>(ctx, ctx->d_tmp);
-  if (rc) return rc;
-  const int steps = std::min(ctx->ns, 6);
-  EventPair ev;
-  CK(ev.create());
-  float us[2] = {1e30f, 1e30f};
-  for (int round = 0; round < 3; ++round)
-    for (int f = 0; f < 2; ++f) {
-      M->fused = f == 1;
-      mx_real<T>(ctx, 0);
-      mx_step<T>(ctx, 1);
-      cudaEventRecord(ev.a, ctx->stream);
-      for (int t = 1; t <= steps; ++t) mx_step<T>(ctx, t);
-      cudaEventRecord(ev.b, ctx->stream);
-      CK(cudaEventSynchronize(ev.b));
-      float ms = 0.f;
-      cudaEventElapsedTime(&ms, ev.a, ev.b);
-      us[f] = std::min(us[f], 1000.f * ms / steps);
-    }
-  CK(cudaGetLastError());
-  M->fused = us[1] < us[0];
-  char line[128];
-  std::snprintf(line, sizeof(line), "mixed radix %s; y passes apart %.2f us/double step, plane pass %.2f",
-                M->fused ? "plane pass" : "y passes apart", us[0], us[1]);
-  ctx->tune_report = line;
-  std::lock_guard<std::mutex> lk(g_tune_mu);
-  g_tune[key] = TuneVal{PK_PLAIN, PK_PLAIN, M->fused ? PK_FUSED : PK_PLAIN, line};
-  return ADSCF_OK;
-}
-
 template <typename T>
 int tune_t(adscf_ctx* ctx) {
-  if (ctx->mx) return mx_tune<T>(ctx);
+  if (ctx->mx) {   // unit Boltzmann factors from a zero field, as below
+    CK(cudaMemsetAsync(ctx->d_tmp, 0, 2 * (size_t)ctx->npts * sizeof(double), ctx->stream));
+    const int rc = expfield_t<T>(ctx, ctx->d_tmp);
+    return rc ? rc : mx_tune(ctx);
+  }
   const int avail = (ctx->tma ? 1 : 0) | (ctx->pgrid_y ? 2 : 0) | (ctx->pgrid_x ? 4 : 0) |
                     (ctx->use_generic ? 8 : 0);
   const TuneKey key{ctx->dev, ctx->gx, ctx->gy, ctx->gz, ctx->prec, avail};
@@ -1080,7 +795,7 @@ int bulk_hold_slices(adscf_ctx* ctx, bool full) {
 }
 // kernel launches of a propagation's contour steps and its first pass
 int bulk_chain_launches(const adscf_ctx* ctx) {
-  const bool two = ctx->mx ? ctx->mx->fused || ctx->gy == 1 : ctx->plan_x == PK_FUSED;
+  const bool two = ctx->mx || ctx->plan_x == PK_FUSED;
   return 1 + (two ? 2 : 4) * ctx->ns;
 }
 // bound of the TMA passes' pipeline waits (0: every wait gives up at once)

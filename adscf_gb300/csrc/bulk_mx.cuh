@@ -1,55 +1,87 @@
-// bulk_mx.cuh -- mixed-radix line passes of the bulk propagator for grids the
+// bulk_mx.cuh -- mixed-radix passes of the bulk propagator for grids the
 // register FFT does not cover (lines of 2, 3 and 5 factors, unequal axes,
 // two-dimensional grids), and for FP64 grids too small to fill the GPU there.
 //
-// Same double step as bulk_kernels.cuh (X, Yf, Z, Yi).  A line of
-// n = R_1 R_2 ... R_S points is transformed in place in shared memory, one
-// stage per radix: stage s takes the R_s points at stride M / R_s of each
-// block of M points (M = n, n / R_1, ...), transforms them in registers and
-// writes them back where they were, times W_M^(j k).  Frequency
+// Same double step as bulk_kernels.cuh in two passes over the spectrum.  A
+// line of n = R_1 R_2 ... R_S points is transformed in place in shared
+// memory, one stage per radix: stage s takes the R_s points at stride M / R_s
+// of each block of M points (M = n, n / R_1, ...), transforms them in
+// registers and writes them back where they were, times W_M^(j k).  Frequency
 // k = k_1 + R_1 (k_2 + R_2 (...)) ends at position (... (k_1) R_2 + k_2) R_3
 // + ...; the inverse runs the stages backwards from there.  Nothing is
 // reordered in between: the diffusion factors are tabulated by position, and
-// position 0 is frequency 0.  In-place stages need one buffer, so a whole
-// z plane (up to ~28000 FP32 points) fits one block and
-//   k_mx_xy : Yi, X and the next step's Yf in one trip of a plane, and
-//   k_mx_s  : the z pass (and, where a plane does not fit or there are too
-//             few planes for the SMs, the separate y passes)
-// make a double step two launches.  Radices up to 16 are compile-time
-// butterflies chosen by a switch that is uniform over the block.
+// position 0 is frequency 0.
 //
-// Bound: FP32 the latency of the stages (a barrier each) and of the launches,
-// FP64 the FP64 pipe: one warp instruction per 64 cycles on each SM quarter,
-// so FP64 plans with fewer points than lanes take small radices, which leave
-// every quarter a short program.
+// The y transform is cut between two of its stages.  Its first stages couple
+// the R_o rows y = j + M' r of a z plane (M' = gy / R_o), its last ones the M'
+// neighbouring rows of a block of positions, so
+//   k_mx_a (one block per row set (j, z)): outer inverse y stages, inverse x,
+//          node t of both chains, forward x, outer forward y stages;
+//   k_mx_b (one block per (row block, columns)): inner y stages, forward z,
+//          exp(-ds k^2) / N, inverse z, inner inverse y stages
+// are a whole double step: the spectrum is read and written twice, by blocks
+// of a few hundred to a few thousand points whatever the grid.  Butterflies
+// are compile-time radices up to 16 behind a switch that is uniform over the
+// block; the outermost stages of a pass read and write global memory.
+//
+// The FP32 (0, 0) pencil (see DcPencil): k_mx_a leaves every row's kx = 0
+// entry in dcin, blocks of their own in k_mx_b add them up over y and convolve
+// the sums into dcout, the table's factor of that pencil is zero, and the next
+// k_mx_a adds dcout to the kx = 0 entry of every row.  Neither the cut nor the
+// launch geometry changes an operation, so the tuner's choice does not either.
+//
+// Bound: FP32 the latency of the stages (a barrier each), FP64 the FP64 pipe:
+// one warp instruction per 64 cycles on each SM quarter, so FP64 plans with
+// fewer points than lanes take small radices, which leave every quarter a
+// short program.
 #pragma once
 #include "bulk_tma.cuh"
 
 namespace mxk {
 
 constexpr int kMaxStages = 6;
-struct Axis {
+struct Axis {                   // radices and block lengths of an axis's stages
   int n, nst, tw_off;
-  int rad[kMaxStages];
-  int m[kMaxStages];            // block length M of the stage
-  unsigned mg[kMaxStages];      // 2^20 / (M / R) + 1: division by M / R of u < n <= 1024
+  int rad[kMaxStages], m[kMaxStages];
+};
+
+// One stage over `lines` lines of a tile.  Task t: line l = t mod lines, then
+// b = u / mp, j = u mod mp of u = t / lines; its points are b m + j + r mp.
+struct Step {
+  int R, m, mp, total;          // radix, block length and stride in the tile, tasks
+  unsigned mg, mgl;             // 2^20 / mp + 1, div_magic(lines)
+  int lines, lmask, lsh;        // line l at (l & lmask) ls + (l >> lsh) ls2
+  int ls, ls2, es;              // pitches in shared memory
+  int gls, gls2, ges;           // pitches in global memory (first and last steps)
+  int tw, tws, jmul, jin;       // twiddle table, W index = (jmul j + jin tile j) tws k
+};
+constexpr int kMaxSteps = 8;
+struct Prog {
+  int n;
+  Step s[kMaxSteps];            // in forward order
 };
 
 template <typename T>
 struct Dev {
   int gx, gy, gz;
-  Axis ax, ay, az;
-  const cplx<T>* tw;            // twiddle tables (offsets in the axes)
+  int ro, mi;                   // outer rows of a tile (R_o), rows of an inner block (M')
+  int pitch;                    // row pitch of k_mx_a's tile (odd)
+  int cols, lc, ctiles;         // columns of k_mx_b's tile (a power of two, its log), tiles along x
+  int ntiles;                   // blocks of columns of k_mx_b (the rest convolve the pencil)
+  Prog a, b;                    // steps around the real-space visit / the diffusion factor
+  int rx, rz;                   // radices of those visits (1: none)
+  int nxs;                      // x steps of program a (its first ones)
+  unsigned mgj, mgz;            // divisions by gx / rx, and by the z lines of a tile
+  int tw_x, tw_y, tw_z;         // twiddle tables in `tw`
+  const cplx<T>* tw;
   const T* fk;                  // by position: g_xy hi, lo [gy gx] each, g_z / N hi, lo [gz] each
   const BulkDev<T>* I;
   cplx<T>* spec;
   cplx<T>* slices;
   const T* E;
-  float2* dcin;                 // [gz] FP32 (0, 0) pencil before the z pass, kept by the pass before it
+  float2* dcin;                 // [gz][gy] FP32 kx = 0 entries of the rows before the y and z transforms
   float2* dcout;                // [gz] the pencil convolved by the z pass
   const float2* dcc;            // [gz] its kernel, (hi, lo)
-  int pitch;                    // row pitch of a plane in shared memory (odd)
-  unsigned mgx, mgj;            // divisions by gx, and by gx over the first x radix (div_magic)
 };
 
 __host__ __device__ __forceinline__ unsigned div_magic(int d) {
@@ -117,75 +149,6 @@ __device__ __forceinline__ void dft(cplx<T>* v, int sg) {
   else dft_c<T, R>(v, sg);
 }
 
-// One stage over `lines` lines at pitch ls (point pitch es), twiddle table
-// W_n at element `tw` of shared memory: forward (SG = 1) transforms, then
-// multiplies by W_M^(j k); inverse (SG = -1) multiplies by the conjugate, then
-// transforms.  The points are read at element `buf` of shared memory and
-// written back there, except that SRC_G reads them from, and DST_G writes
-// them to, global memory (gp, pitches gls and ges); dc: FP32 value that
-// replaces point 0 of line 0 on the way in (SRC_G) or receives it (DST_G).
-struct Geo {
-  int n, R, M;
-  unsigned mg;
-  int lines;
-  unsigned mgl;
-  int ls, es;
-};
-template <typename T>
-struct Glob {
-  cplx<T>* p;
-  int ls, es;
-  float2* dc;
-};
-enum { IO_SMEM = 0, SRC_G = 1, DST_G = 2 };
-
-template <typename T, int SG, int R, int IO>
-__device__ __forceinline__ void stage_r(int buf, int tw, const Geo& g, const Glob<T>& G) {
-  extern __shared__ __align__(16) unsigned char smraw[];
-  cplx<T>* sm = reinterpret_cast<cplx<T>*>(smraw);
-  const int Mp = g.M / R, tws = g.n / g.M;
-  const int total = g.n / R * g.lines;
-  const int st = Mp * g.es;
-  for (int t = threadIdx.x; t < total; t += blockDim.x) {
-    const int u = fdiv(t, g.mgl), l = t - u * g.lines;
-    const int b = (int)(((unsigned)u * g.mg) >> 20), j = u - b * Mp;
-    const int at = b * g.M + j;
-    cplx<T>* p = sm + buf + l * g.ls + at * g.es;
-    cplx<T> v[R];
-    if constexpr (IO == SRC_G) {
-      const cplx<T>* q = G.p + (size_t)l * G.ls + (size_t)at * G.es;
-#pragma unroll
-      for (int r = 0; r < R; ++r) v[r] = q[(size_t)(r * Mp) * G.es];
-      if constexpr (sizeof(T) == 4)
-        if (t == 0 && G.dc) v[0] = *G.dc;
-    } else {
-#pragma unroll
-      for (int r = 0; r < R; ++r) v[r] = p[r * st];
-    }
-    const cplx<T>* w = sm + tw;
-    const int ji = j * tws;
-    if (SG < 0 && j) {
-#pragma unroll
-      for (int r = 1; r < R; ++r) v[r] = cmulc<T>(v[r], w[ji * r]);
-    }
-    dft<T, R>(v, SG);
-    if (SG > 0 && j) {
-#pragma unroll
-      for (int r = 1; r < R; ++r) v[r] = cmul<T>(v[r], w[ji * r]);
-    }
-    if constexpr (IO == DST_G) {
-      cplx<T>* q = G.p + (size_t)l * G.ls + (size_t)at * G.es;
-#pragma unroll
-      for (int r = 0; r < R; ++r) q[(size_t)(r * Mp) * G.es] = v[r];
-      if constexpr (sizeof(T) == 4)
-        if (t == 0 && G.dc) *G.dc = v[0];
-    } else {
-#pragma unroll
-      for (int r = 0; r < R; ++r) p[r * st] = v[r];
-    }
-  }
-}
-
 #define ADSCF_MX_SWITCH(R_, CALL)                                                        \
   switch (R_) {                                                                          \
     case 2: CALL(2); break;                                                              \
@@ -201,59 +164,89 @@ __device__ __forceinline__ void stage_r(int buf, int tw, const Geo& g, const Glo
     default: CALL(16); break;                                                            \
   }
 
-template <typename T, int SG>
-__device__ __noinline__ void stage(int buf, int tw, Geo g) {
-  const Glob<T> none{};
-#define ADSCF_MX_CALL(R_) stage_r<T, SG, R_, IO_SMEM>(buf, tw, g, none)
-  ADSCF_MX_SWITCH(g.R, ADSCF_MX_CALL)
-#undef ADSCF_MX_CALL
-}
-template <typename T, int SG, int IO>
-__device__ __noinline__ void stage_io(int buf, int tw, Geo g, Glob<T> G) {
-#define ADSCF_MX_CALL(R_) stage_r<T, SG, R_, IO>(buf, tw, g, G)
-  ADSCF_MX_SWITCH(g.R, ADSCF_MX_CALL)
-#undef ADSCF_MX_CALL
-}
-
-__device__ __forceinline__ Geo geo(const Axis& A, int s, int lines, unsigned mgl, int ls, int es) {
-  return Geo{A.n, A.rad[s], A.m[s], A.mg[s], lines, mgl, ls, es};
-}
-// stages [s0, s1) of the lines in shared memory, a barrier after each; the
-// inverse runs them from s1 - 1 down
-template <typename T, int SG>
-__device__ __forceinline__ void stages(int buf, int tw, const Axis& A, int s0, int s1, int lines, unsigned mgl,
-                                       int ls, int es) {
-  for (int i = s0; i < s1; ++i) {
-    stage<T, SG>(buf, tw, geo(A, SG > 0 ? i : s1 - 1 - (i - s0), lines, mgl, ls, es));
-    __syncthreads();
+// One stage of the tile: forward (SG = 1) transforms, then multiplies by
+// W^(j k); inverse (SG = -1) multiplies by the conjugate, then transforms.
+// g: global memory the points come from (inverse of k_mx_a, forward of
+// k_mx_b) or go to, null for shared memory; lines with (l & lmask) >= nl do
+// not exist there.  dc (the x step next to the row's end, FP32): value added
+// to point 0 of every line (SG < 0), or where point 0 of line l is left, at
+// dc[l dcs] (SG > 0).
+template <typename T, int SG, bool SRC, int R>
+__device__ __forceinline__ void stage_r(const Step& S, cplx<T>* sm, int tile_j, cplx<T>* g, int nl, float2* dc,
+                                        int dcs) {
+  for (int t = threadIdx.x; t < S.total; t += blockDim.x) {
+    const int u = fdiv(t, S.mgl), l = t - u * S.lines;
+    const int b = (int)(((unsigned)u * S.mg) >> 20), j = u - b * S.mp;
+    const int at = b * S.m + j, lo = l & S.lmask, hi = l >> S.lsh;
+    cplx<T>* p = sm + lo * S.ls + hi * S.ls2 + at * S.es;
+    cplx<T>* q = g ? g + (size_t)lo * S.gls + (size_t)hi * S.gls2 + (size_t)at * S.ges : nullptr;
+    const int st = S.mp * S.es;
+    const size_t gst = (size_t)S.mp * S.ges;
+    cplx<T> v[R];
+    if (SRC && g) {
+      if (lo < nl) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) v[r] = q[r * gst];
+      } else {
+#pragma unroll
+        for (int r = 0; r < R; ++r) v[r] = mk<T>((T)0, (T)0);
+      }
+    } else {
+#pragma unroll
+      for (int r = 0; r < R; ++r) v[r] = p[r * st];
+    }
+    if constexpr (sizeof(T) == 4 && SG < 0)
+      if (dc && at == 0) v[0] = cadd<T>(v[0], *dc);
+    const int ji = (S.jmul * j + S.jin * tile_j) * S.tws;
+    const cplx<T>* w = sm + S.tw;
+    if (SG < 0 && ji) {
+#pragma unroll
+      for (int r = 1; r < R; ++r) v[r] = cmulc<T>(v[r], w[ji * r]);
+    }
+    dft<T, R>(v, SG);
+    if (SG > 0 && ji) {
+#pragma unroll
+      for (int r = 1; r < R; ++r) v[r] = cmul<T>(v[r], w[ji * r]);
+    }
+    if constexpr (sizeof(T) == 4 && SG > 0)
+      if (dc && at == 0) dc[(size_t)l * dcs] = v[0];
+    if (!SRC && g) {
+      if (lo < nl) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) q[r * gst] = v[r];
+      }
+    } else {
+#pragma unroll
+      for (int r = 0; r < R; ++r) p[r * st] = v[r];
+    }
   }
 }
 
 // Last forward stage, diffusion factor and first inverse stage of the z lines
-// in one visit of the points (both stages have M = R, no twiddles).  fz: the
-// g_z / N factors by position at byte offset of shared memory (hi [n], lo
-// [n]); fxy: the columns' g_xy (hi, with lo at + nxy).
+// in one visit of the points (both stages have M = R, no twiddles).  Lines
+// (row yy of the block, column c); fz: the g_z / N factors by position (hi
+// [n], lo [n]); fxy: the tile's g_xy (rows gx apart, lo parts at + nxy).
 template <typename T, int R>
-__device__ __forceinline__ void mid_r(int buf, const Geo& g, int fz_off, const T* fxy, int nxy) {
-  extern __shared__ __align__(16) unsigned char smraw[];
-  cplx<T>* sm = reinterpret_cast<cplx<T>*>(smraw);
-  const T* fz = reinterpret_cast<const T*>(smraw + fz_off);
-  const int total = g.n / R * g.lines;
+__device__ __forceinline__ void mid_r(const Dev<T>& D, cplx<T>* sm, const T* fz, const T* fxy, int nl) {
+  const int gz = D.gz, lines = D.mi << D.lc, nxy = D.gx * D.gy;
+  const int total = gz / R * lines;
   for (int t = threadIdx.x; t < total; t += blockDim.x) {
-    const int u = fdiv(t, g.mgl), l = t - u * g.lines;
-    cplx<T>* p = sm + buf + l * g.ls + u * R * g.es;
-    const T ah = __ldg(fxy + l);
+    const int u = fdiv(t, D.mgz), l = t - u * lines;
+    const int c = l & (D.cols - 1), yy = l >> D.lc;
+    if (c >= nl) continue;
+    cplx<T>* p = sm + ((yy * gz + u * R) << D.lc) + c;
+    const T ah = __ldg(fxy + (size_t)yy * D.gx + c);
     T al = (T)0;
-    if constexpr (sizeof(T) == 4) al = __ldg(fxy + nxy + l);
+    if constexpr (sizeof(T) == 4) al = __ldg(fxy + nxy + (size_t)yy * D.gx + c);
     cplx<T> v[R];
 #pragma unroll
-    for (int r = 0; r < R; ++r) v[r] = p[r * g.es];
+    for (int r = 0; r < R; ++r) v[r] = p[r << D.lc];
     if constexpr (R > 1) dft<T, R>(v, +1);
 #pragma unroll
     for (int r = 0; r < R; ++r) {
       const T bh = fz[u * R + r];
       if constexpr (sizeof(T) == 4) {   // compensated product, one rounding
-        const float bl = fz[g.n + u * R + r];
+        const float bl = fz[gz + u * R + r];
         const float gh = ah * bh;
         const float gl = fmaf(ah, bh, -gh) + fmaf(ah, bl, al * bh);
         v[r] = mk<T>(fmaf(v[r].x, gh, v[r].x * gl), fmaf(v[r].y, gh, v[r].y * gl));
@@ -264,44 +257,36 @@ __device__ __forceinline__ void mid_r(int buf, const Geo& g, int fz_off, const T
     }
     if constexpr (R > 1) dft<T, R>(v, -1);
 #pragma unroll
-    for (int r = 0; r < R; ++r) p[r * g.es] = v[r];
+    for (int r = 0; r < R; ++r) p[r << D.lc] = v[r];
   }
-}
-template <typename T>
-__device__ __noinline__ void mid(int buf, Geo g, int fz_off, const T* fxy, int nxy) {
-  if (g.R == 1) {
-    mid_r<T, 1>(buf, g, fz_off, fxy, nxy);
-    return;
-  }
-#define ADSCF_MX_CALL(R_) mid_r<T, R_>(buf, g, fz_off, fxy, nxy)
-  ADSCF_MX_SWITCH(g.R, ADSCF_MX_CALL)
-#undef ADSCF_MX_CALL
 }
 
 // Last inverse stage of the x rows, node t of both chains and the first
 // forward stage in one visit (both stages have M = n: a task holds points
 // j + r n / R of a row; tasks of a row are neighbours, so the Boltzmann
 // factors and the slice move in runs of n / R points).  E, sl: factors and
-// slice at the tile's first point, rows gx apart; f: bits 0-3 = forward /
+// slice at the tile's first row, its rows M' gx apart; f: bits 0-3 = forward /
 // backward chain takes the A factor at node t, at node t + 1; bit 4: t <
-// Ns, the forward stage follows; init: no inverse, slice = (1, 1).
+// Ns, the forward stage follows; init: no inverse, slice = (1, 1); dco, dci:
+// as dc of stage_r where this is the rows' only stage, else null.
 template <typename T, int R>
-__device__ __forceinline__ void real_r(int buf, int tw, const Geo& g, unsigned mgj, const T* E, cplx<T>* sl,
-                                       unsigned f, bool init) {
-  extern __shared__ __align__(16) unsigned char smraw[];
-  cplx<T>* sm = reinterpret_cast<cplx<T>*>(smraw);
-  const int Mp = g.n / R;
-  const int total = Mp * g.lines;
+__device__ __forceinline__ void real_r(const Dev<T>& D, cplx<T>* sm, const T* E, cplx<T>* sl, unsigned f, bool init,
+                                       float2* dco, float2* dci) {
+  const int Mp = D.gx / R;
+  const int total = Mp * D.ro;
+  const size_t rs = (size_t)D.mi * D.gx;
   const bool fA = f & 1, bA = f & 2, fA2 = f & 4, bA2 = f & 8, more = f & 16;
+  const cplx<T>* w = sm + D.ro * D.pitch;
   for (int t = threadIdx.x; t < total; t += blockDim.x) {
-    const int l = fdiv(t, mgj), j = t - l * Mp;
-    cplx<T>* p = sm + buf + l * g.ls + j;
-    const size_t gp = (size_t)l * g.n + j;
-    const cplx<T>* w = sm + tw;
+    const int l = fdiv(t, D.mgj), j = t - l * Mp;
+    cplx<T>* p = sm + l * D.pitch + j;
+    const size_t gp = l * rs + j;
     cplx<T> v[R];
     if (!init) {
 #pragma unroll
       for (int r = 0; r < R; ++r) v[r] = p[r * Mp];
+      if constexpr (sizeof(T) == 4)
+        if (dco) v[0] = cadd<T>(v[0], *dco);   // the only stage: j = 0
       if constexpr (R > 1) {
         if (j) {
 #pragma unroll
@@ -312,14 +297,14 @@ __device__ __forceinline__ void real_r(int buf, int tw, const Geo& g, unsigned m
     }
 #pragma unroll
     for (int r = 0; r < R; ++r) {
-      const EPt<T> ev = load_ept(E, gp + (size_t)r * Mp);
+      const EPt<T> ev = load_ept(E, gp + r * Mp);
       if (init) {
         v[r] = mk<T>(fA ? ev.a : ev.b, bA ? ev.a : ev.b);
-        sl[gp + (size_t)r * Mp] = mk<T>((T)1, (T)1);
+        sl[gp + r * Mp] = mk<T>((T)1, (T)1);
       } else {
         const cplx<T> q = mk<T>(emul(v[r].x, fA ? ev.a : ev.b, fA ? ev.al : ev.bl),
                                 emul(v[r].y, bA ? ev.a : ev.b, bA ? ev.al : ev.bl));
-        sl[gp + (size_t)r * Mp] = q;
+        sl[gp + r * Mp] = q;
         v[r] = mk<T>(emul(q.x, fA2 ? ev.a : ev.b, fA2 ? ev.al : ev.bl),
                      emul(q.y, bA2 ? ev.a : ev.b, bA2 ? ev.al : ev.bl));
       }
@@ -332,230 +317,198 @@ __device__ __forceinline__ void real_r(int buf, int tw, const Geo& g, unsigned m
         for (int r = 1; r < R; ++r) v[r] = cmul<T>(v[r], w[j * r]);
       }
     }
+    if constexpr (sizeof(T) == 4)
+      if (dci) dci[(size_t)l * D.mi] = v[0];
 #pragma unroll
     for (int r = 0; r < R; ++r) p[r * Mp] = v[r];
   }
-}
-template <typename T>
-__device__ __noinline__ void real_mid(int buf, int tw, Geo g, unsigned mgj, const T* E, cplx<T>* sl, unsigned f,
-                                      bool init) {
-  if (g.R == 1) {
-    real_r<T, 1>(buf, tw, g, mgj, E, sl, f, init);
-    return;
-  }
-#define ADSCF_MX_CALL(R_) real_r<T, R_>(buf, tw, g, mgj, E, sl, f, init)
-  ADSCF_MX_SWITCH(g.R, ADSCF_MX_CALL)
-#undef ADSCF_MX_CALL
-}
-
-template <typename T>
-__device__ __forceinline__ void load_tw(cplx<T>* dst, const Dev<T>& D, const Axis& A) {
-  for (int i = threadIdx.x; i < A.n; i += blockDim.x) dst[i] = D.tw[A.tw_off + i];
 }
 
 }  // namespace mxk
 
 // ---------------------------------------------------------------------------
-// Real-space pass of `rows` x-rows per block: [inverse y,] inverse x, node t
-// of both chains (slice store), times E(t + 1), forward x [, forward y].
-// PLANES: the rows are one z plane (rows = gy > 1, blockIdx.x = z) and the y
-// transforms belong to the pass; their outermost stages read and write the
-// spectrum directly.  Otherwise rows [blockIdx.x rows, + rows) of the grid, x
-// only.  t = 0 starts the chains: slice 0 = (1, 1).
-// Where the block handles whole (0, 0) pencil entries -- planes, or every row
-// of a one-point y axis -- it takes their values of the z pass from D.dcout
-// and leaves those for the next one in D.dcin (FP32).
-// Shared memory: rows pitch + gx + (PLANES ? gy : 0) points.
+// Real-space pass of the row set (j, z): block j + M' z.  t = 0 starts the
+// chains: slice 0 = (1, 1).  Shared memory: R_o pitch + gx + gy points.
 // ---------------------------------------------------------------------------
-template <typename T, bool PLANES>
-__global__ void __launch_bounds__(512)
-k_mx_xy(const __grid_constant__ mxk::Dev<T> D, int t, int rows, unsigned mg_rows) {
+template <typename T>
+__global__ void __launch_bounds__(128, sizeof(T) == 4 ? 6 : 4)
+k_mx_a(const __grid_constant__ mxk::Dev<T> D, int t) {
   extern __shared__ __align__(16) unsigned char smraw[];
-  cplx<T>* tile = reinterpret_cast<cplx<T>*>(smraw);
+  cplx<T>* sm = reinterpret_cast<cplx<T>*>(smraw);
   const BulkDev<T>& I = *D.I;
-  const int gx = D.gx, pitch = D.pitch;
-  const int row0 = blockIdx.x * rows;
-  const int nr = PLANES ? rows : min(rows, D.gy * D.gz - row0);
-  const unsigned mgl = nr == rows ? mg_rows : mxk::div_magic(nr);
-  const int ne = nr * gx;
-  const int o_twx = rows * pitch, o_twy = o_twx + gx;
-  const size_t base = (size_t)row0 * gx;
+  const int gx = D.gx, ro = D.ro, mi = D.mi;
+  const int z = blockIdx.x / mi, j = blockIdx.x - z * mi;
+  const size_t base = ((size_t)z * D.gy + j) * gx;
+  const size_t rs = (size_t)mi * gx;
   const int ns = I.ns;
   tmak::pdl_launch_dependents();
-  mxk::load_tw<T>(tile + o_twx, D, D.ax);
-  if constexpr (PLANES) mxk::load_tw<T>(tile + o_twy, D, D.ay);
+  {
+    cplx<T>* tw = sm + ro * D.pitch;
+    for (int i = threadIdx.x; i < gx; i += blockDim.x) tw[i] = D.tw[D.tw_x + i];
+    if (ro > 1)
+      for (int i = threadIdx.x; i < D.gy; i += blockDim.x) tw[gx + i] = D.tw[D.tw_y + i];
+  }
   const int tt = t == 0 ? 1 : t;
   const bool more = t == 0 || t < ns;
   const unsigned f = (chain_type_fwd(I, tt) == 0 ? 1u : 0u) | (chain_type_bwd(I, tt) == 0 ? 2u : 0u) |
                      (chain_type_fwd(I, t + 1) == 0 ? 4u : 0u) | (chain_type_bwd(I, t + 1) == 0 ? 8u : 0u) |
                      (more ? 16u : 0u);
-  const bool dcrow = sizeof(T) == 4 && (PLANES || D.gy == 1);
   cplx<T>* sl = D.slices + (size_t)t * (size_t)I.npts + base;
   const T* E = D.E + base * (sizeof(T) == 4 ? 4 : 2);
-  const int nx = D.ax.nst, ny = D.ay.nst;
+  cplx<T>* g = D.spec + base;
+  // the x step where a row's kx = 0 entry is complete (none: the real visit)
+  const int xs = sizeof(T) == 4 ? D.nxs - 1 : -2;
+  float2* dci = sizeof(T) == 4 ? D.dcin + (size_t)z * D.gy + j : nullptr;
+  float2* dco = sizeof(T) == 4 ? D.dcout + z : nullptr;
   tmak::pdl_wait();
-  if constexpr (PLANES) __syncthreads();   // twiddles
+  __syncthreads();
   if (t > 0) {
-    {  // the tile's Boltzmann factors on their way to L1 while it is transformed
-      const char* e0 = reinterpret_cast<const char*>(E);
-      for (int i = threadIdx.x * 128; i < ne * 16; i += blockDim.x * 128) tmak::prefetch_l1(e0 + i);
+    // the tile's Boltzmann factors on their way to L1 while it is transformed
+    for (int r = 0; r < ro; ++r) {
+      const char* e0 = reinterpret_cast<const char*>(E) + r * rs * 16;
+      for (int i = threadIdx.x * 128; i < gx * 16; i += blockDim.x * 128) tmak::prefetch_l1(e0 + i);
     }
-    if constexpr (PLANES) {
-      const mxk::Glob<T> G{D.spec + base, 1, gx, dcrow ? D.dcout + blockIdx.x : nullptr};
-      mxk::stage_io<T, -1, mxk::SRC_G>(0, o_twy, mxk::geo(D.ay, ny - 1, gx, D.mgx, 1, pitch), G);
-      __syncthreads();
-      mxk::stages<T, -1>(0, o_twy, D.ay, 0, ny - 1, gx, D.mgx, 1, pitch);
-    } else {
-#pragma unroll 4
-      for (int e = threadIdx.x; e < ne; e += blockDim.x) {
-        const int r = mxk::fdiv(e, D.mgx), x = e - r * gx;
-        tile[r * pitch + x] = D.spec[base + e];
-      }
-      if constexpr (sizeof(T) == 4) {
-        if (dcrow) {
-          __syncthreads();
-          for (int r = threadIdx.x; r < nr; r += blockDim.x) tile[r * pitch] = D.dcout[row0 + r];
-        }
-      }
+    if (D.a.n == 0) {
+      for (int x = threadIdx.x; x < gx; x += blockDim.x) sm[x] = g[x];
       __syncthreads();
     }
-    mxk::stages<T, -1>(0, o_twx, D.ax, 1, nx, nr, mgl, pitch, 1);
-  } else if constexpr (!PLANES) {
-    __syncthreads();   // twiddles
+    for (int i = D.a.n - 1; i >= 0; --i) {
+      const mxk::Step& S = D.a.s[i];
+      cplx<T>* src = i == D.a.n - 1 ? g : nullptr;
+#define ADSCF_MX_CALL(R_) mxk::stage_r<T, -1, true, R_>(S, sm, j, src, gx, i == xs ? dco : nullptr, 0)
+      ADSCF_MX_SWITCH(S.R, ADSCF_MX_CALL)
+#undef ADSCF_MX_CALL
+      __syncthreads();
+    }
   }
-  {
-    mxk::Geo g = nx ? mxk::geo(D.ax, 0, nr, mgl, pitch, 1) : mxk::Geo{1, 1, 1, 0u, nr, mgl, pitch, 1};
-    mxk::real_mid<T>(0, o_twx, g, D.mgj, E, sl, f, t == 0);
+  if (D.rx == 1) {
+    mxk::real_r<T, 1>(D, sm, E, sl, f, t == 0, xs == -1 ? dco : nullptr, xs == -1 ? dci : nullptr);
+  } else {
+#define ADSCF_MX_CALL(R_) \
+  mxk::real_r<T, R_>(D, sm, E, sl, f, t == 0, xs == -1 ? dco : nullptr, xs == -1 ? dci : nullptr)
+    ADSCF_MX_SWITCH(D.rx, ADSCF_MX_CALL)
+#undef ADSCF_MX_CALL
   }
   if (!more) return;
   __syncthreads();
-  mxk::stages<T, +1>(0, o_twx, D.ax, 1, nx, nr, mgl, pitch, 1);
-  if constexpr (PLANES) {
-    mxk::stages<T, +1>(0, o_twy, D.ay, 0, ny - 1, gx, D.mgx, 1, pitch);
-    const mxk::Glob<T> G{D.spec + base, 1, gx, dcrow ? D.dcin + blockIdx.x : nullptr};
-    mxk::stage_io<T, +1, mxk::DST_G>(0, o_twy, mxk::geo(D.ay, ny - 1, gx, D.mgx, 1, pitch), G);
-  } else {
-#pragma unroll 4
-    for (int e = threadIdx.x; e < ne; e += blockDim.x) {
-      const int r = mxk::fdiv(e, D.mgx), x = e - r * gx;
-      D.spec[base + e] = tile[r * pitch + x];
-    }
-    if constexpr (sizeof(T) == 4) {
-      if (dcrow)
-        for (int r = threadIdx.x; r < nr; r += blockDim.x) D.dcin[row0 + r] = tile[r * pitch];
-    }
+  for (int i = 0; i < D.a.n; ++i) {
+    const mxk::Step& S = D.a.s[i];
+    cplx<T>* dst = i == D.a.n - 1 ? g : nullptr;
+#define ADSCF_MX_CALL(R_) mxk::stage_r<T, +1, false, R_>(S, sm, j, dst, gx, i == xs ? dci : nullptr, mi)
+    ADSCF_MX_SWITCH(S.R, ADSCF_MX_CALL)
+#undef ADSCF_MX_CALL
+    if (!dst) __syncthreads();
+  }
+  if (D.a.n == 0) {
+    __syncthreads();
+    for (int x = threadIdx.x; x < gx; x += blockDim.x) g[x] = sm[x];
   }
 }
 
 // ---------------------------------------------------------------------------
-// Strided passes: tiles of `cols` (a power of two) neighbouring columns.
-// KIND 0 forward y, 1 inverse y (columns x of plane z, tiles do not cross
-// planes), 2 z (columns (y, x)).  The outermost stages read and write the
-// spectrum directly.  The z pass has `ntiles` blocks of columns, then blocks
-// whose warps convolve the FP32 (0, 0) pencil, one output per warp, from
-// D.dcin into D.dcout (the columns' own result for it is replaced by the next
-// pass).  The y passes keep and replace the pencil's entries.
-// Shared memory: n cols + n points, and 2 n factors (z).
+// Diffusion pass of the row block k (positions [k M', (k + 1) M') of y) and a
+// tile of `cols` columns: block k ctiles + tile.  Blocks from ntiles on: one
+// output of the FP32 (0, 0) pencil per warp.  Shared memory: M' gz cols + gy
+// + gz points and 2 gz factors.
 // ---------------------------------------------------------------------------
-template <typename T, int KIND>
-__global__ void __launch_bounds__(256)
-k_mx_s(const __grid_constant__ mxk::Dev<T> D, int cols, int ntiles) {
+template <typename T, int BT>
+__global__ void __launch_bounds__(BT, BT == 512 ? 1 : sizeof(T) == 4 ? 3 : 2)
+k_mx_b(const __grid_constant__ mxk::Dev<T> D) {
   extern __shared__ __align__(16) unsigned char smraw[];
-  cplx<T>* tile = reinterpret_cast<cplx<T>*>(smraw);
-  constexpr bool zdir = KIND == 2;
-  const mxk::Axis& A = zdir ? D.az : D.ay;
-  const int n = A.n, gx = D.gx, nxy = gx * D.gy, ns = A.nst;
+  cplx<T>* sm = reinterpret_cast<cplx<T>*>(smraw);
+  const int gx = D.gx, gz = D.gz, mi = D.mi, nxy = gx * D.gy;
   tmak::pdl_launch_dependents();
-  if constexpr (zdir && sizeof(T) == 4) {
-    if ((int)blockIdx.x >= ntiles) {
+  if constexpr (sizeof(T) == 4) {
+    if ((int)blockIdx.x >= D.ntiles) {
       float2* in = reinterpret_cast<float2*>(smraw);
-      float2* c = in + n;
-      for (int i = threadIdx.x; i < n; i += blockDim.x) c[i] = D.dcc[i];
+      float2* c = in + ((gz + 1) & ~1);
+      for (int i = threadIdx.x; i < gz; i += blockDim.x) c[i] = D.dcc[i];
       tmak::pdl_wait();
-      for (int i = threadIdx.x; i < n; i += blockDim.x) in[i] = D.dcin[i];
+      // row sums in float-float, eight threads per plane (rows y = k, k + 8,
+      // ... each, then over k): many loads are in flight
+      constexpr int kParts = 8;
+      float4* part = reinterpret_cast<float4*>(c + ((gz + 1) & ~1));
+      for (int i = threadIdx.x; i < gz * kParts; i += blockDim.x) {
+        float xh = 0.f, xl = 0.f, yh = 0.f, yl = 0.f;
+        const float2* row = D.dcin + (size_t)(i / kParts) * D.gy;
+#pragma unroll 4
+        for (int y = i % kParts; y < D.gy; y += kParts) {
+          const float2 v = row[y];
+          ff_add(xh, xl, v.x, 0.f);
+          ff_add(yh, yl, v.y, 0.f);
+        }
+        part[i] = make_float4(xh, xl, yh, yl);
+      }
       __syncthreads();
-      const int nw = blockDim.x >> 5;
-      const int z = ((int)blockIdx.x - ntiles) * nw + (threadIdx.x >> 5);
-      if (z < n) {
-        const float2 o = tmak::dc_point(in, c, n, z);
+      for (int i = threadIdx.x; i < gz; i += blockDim.x) {
+        float4 s = part[i * kParts];
+#pragma unroll
+        for (int k = 1; k < kParts; ++k) {
+          const float4 v = part[i * kParts + k];
+          ff_add(s.x, s.y, v.x, v.y);
+          ff_add(s.z, s.w, v.z, v.w);
+        }
+        in[i] = make_float2(s.x + s.y, s.z + s.w);
+      }
+      __syncthreads();
+      const int z = ((int)blockIdx.x - D.ntiles) * (blockDim.x >> 5) + (threadIdx.x >> 5);
+      if (z < gz) {
+        const float2 o = tmak::dc_point(in, c, gz, z);
         if ((threadIdx.x & 31) == 0) D.dcout[z] = o;
       }
       return;
     }
   }
-  const int o_tw = n * cols;
-  const int fz_off = (o_tw + n) * (int)sizeof(cplx<T>);
-  mxk::load_tw<T>(tile + o_tw, D, A);
-  if constexpr (zdir) {
-    T* fz = reinterpret_cast<T*>(smraw + fz_off);
+  const int k = blockIdx.x / D.ctiles, c0 = (blockIdx.x - k * D.ctiles) << D.lc;
+  const int nl = min(D.cols, gx - c0);
+  const int pts = (mi * gz) << D.lc;
+  T* fz = reinterpret_cast<T*>(sm + pts + D.gy + gz);
+  if (mi > 1)
+    for (int i = threadIdx.x; i < D.gy; i += blockDim.x) sm[pts + i] = D.tw[D.tw_y + i];
+  for (int i = threadIdx.x; i < gz; i += blockDim.x) sm[pts + D.gy + i] = D.tw[D.tw_z + i];
+  {
     const T* gzt = D.fk + 2 * (size_t)nxy;
-    for (int i = threadIdx.x; i < 2 * n; i += blockDim.x) fz[i] = gzt[i];
+    for (int i = threadIdx.x; i < 2 * gz; i += blockDim.x) fz[i] = gzt[i];
   }
-  const int lc = __ffs(cols) - 1;
-  size_t base;
-  int nl, es;
-  int z = 0, x0 = 0;
-  if constexpr (zdir) {
-    const int L0 = blockIdx.x * cols;
-    base = L0;
-    nl = min(cols, nxy - L0);
-    es = nxy;
-  } else {
-    const int tpp = (gx + cols - 1) >> lc;
-    z = blockIdx.x / tpp;
-    x0 = (blockIdx.x - z * tpp) << lc;
-    base = (size_t)z * nxy + x0;
-    nl = min(cols, gx - x0);
-    es = gx;
-  }
-  const unsigned mgl = nl == cols ? (lc ? 1u << (32 - lc) : 0u) : mxk::div_magic(nl);
-  const bool dcl = sizeof(T) == 4 && !zdir && x0 == 0;
-  const mxk::Glob<T> in{D.spec + base, 1, es, dcl && KIND == 1 ? D.dcout + z : nullptr};
-  const mxk::Glob<T> out{D.spec + base, 1, es, dcl && KIND == 0 ? D.dcin + z : nullptr};
+  cplx<T>* g = D.spec + (size_t)k * mi * gx + c0;
+  const T* fxy = D.fk + (size_t)k * mi * gx + c0;
   tmak::pdl_wait();
   __syncthreads();
-  if constexpr (KIND < 2) {
-    constexpr int SG = KIND == 0 ? +1 : -1;
-    const int first = SG > 0 ? 0 : ns - 1, last = SG > 0 ? ns - 1 : 0;
-    if (ns == 1) {   // one stage: through shared memory, then out
-      mxk::stage_io<T, SG, mxk::SRC_G>(0, o_tw, mxk::geo(A, 0, nl, mgl, 1, cols), in);
-      __syncthreads();
-      for (int e = threadIdx.x; e < n << lc; e += blockDim.x) {
-        const int j = e >> lc, c = e & (cols - 1);
-        if (c < nl) D.spec[base + (size_t)j * es + c] = tile[e];
-      }
-      if constexpr (sizeof(T) == 4 && KIND == 0) {
-        if (dcl && threadIdx.x == 0) D.dcin[z] = tile[0];
-      }
-      return;
+  if (D.b.n == 0) {
+    for (int e = threadIdx.x; e < pts; e += blockDim.x) {
+      const int c = e & (D.cols - 1), zz = e >> D.lc;
+      if (c < nl) sm[e] = g[(size_t)zz * nxy + c];
     }
-    mxk::stage_io<T, SG, mxk::SRC_G>(0, o_tw, mxk::geo(A, first, nl, mgl, 1, cols), in);
     __syncthreads();
-    mxk::stages<T, SG>(0, o_tw, A, 1, ns - 1, nl, mgl, 1, cols);
-    mxk::stage_io<T, SG, mxk::DST_G>(0, o_tw, mxk::geo(A, last, nl, mgl, 1, cols), out);
+  }
+  for (int i = 0; i < D.b.n; ++i) {
+    const mxk::Step& S = D.b.s[i];
+    cplx<T>* src = i == 0 ? g : nullptr;
+#define ADSCF_MX_CALL(R_) mxk::stage_r<T, +1, true, R_>(S, sm, 0, src, nl, nullptr, 0)
+    ADSCF_MX_SWITCH(S.R, ADSCF_MX_CALL)
+#undef ADSCF_MX_CALL
+    __syncthreads();
+  }
+  if (D.rz == 1) {
+    mxk::mid_r<T, 1>(D, sm, fz, fxy, nl);
   } else {
-    if (ns < 2) {   // the middle visit only: through shared memory
-      for (int e = threadIdx.x; e < n << lc; e += blockDim.x) {
-        const int j = e >> lc, c = e & (cols - 1);
-        if (c < nl) tile[e] = D.spec[base + (size_t)j * es + c];
-      }
-      __syncthreads();
-    } else {
-      mxk::stage_io<T, +1, mxk::SRC_G>(0, o_tw, mxk::geo(A, 0, nl, mgl, 1, cols), in);
-      __syncthreads();
-      mxk::stages<T, +1>(0, o_tw, A, 1, ns - 1, nl, mgl, 1, cols);
-    }
-    const int R = ns ? A.rad[ns - 1] : 1;
-    mxk::mid<T>(0, mxk::Geo{n, R, R, 0u, nl, mgl, 1, cols}, fz_off, D.fk + base, nxy);
-    __syncthreads();
-    if (ns < 2) {
-      for (int e = threadIdx.x; e < n << lc; e += blockDim.x) {
-        const int j = e >> lc, c = e & (cols - 1);
-        if (c < nl) D.spec[base + (size_t)j * es + c] = tile[e];
-      }
-    } else {
-      mxk::stages<T, -1>(0, o_tw, A, 1, ns - 1, nl, mgl, 1, cols);
-      mxk::stage_io<T, -1, mxk::DST_G>(0, o_tw, mxk::geo(A, 0, nl, mgl, 1, cols), out);
+#define ADSCF_MX_CALL(R_) mxk::mid_r<T, R_>(D, sm, fz, fxy, nl)
+    ADSCF_MX_SWITCH(D.rz, ADSCF_MX_CALL)
+#undef ADSCF_MX_CALL
+  }
+  __syncthreads();
+  for (int i = D.b.n - 1; i >= 0; --i) {
+    const mxk::Step& S = D.b.s[i];
+    cplx<T>* dst = i == 0 ? g : nullptr;
+#define ADSCF_MX_CALL(R_) mxk::stage_r<T, -1, false, R_>(S, sm, 0, dst, nl, nullptr, 0)
+    ADSCF_MX_SWITCH(S.R, ADSCF_MX_CALL)
+#undef ADSCF_MX_CALL
+    if (!dst) __syncthreads();
+  }
+  if (D.b.n == 0) {
+    for (int e = threadIdx.x; e < pts; e += blockDim.x) {
+      const int c = e & (D.cols - 1), zz = e >> D.lc;
+      if (c < nl) g[(size_t)zz * nxy + c] = sm[e];
     }
   }
 }

@@ -157,6 +157,16 @@ int bulk_create(adscf_ctx* ctx);
 void bulk_destroy(adscf_ctx* ctx);
 int bulk_enqueue_propagate(adscf_ctx* ctx);     // from E to dist + qpart
 int bulk_chain_launches(const adscf_ctx* ctx);
+// mixed-radix passes (bulk_mx.cu): plan and tables (ctx->mx stays null for a
+// grid they do not take), tables of a new box, geometry tuner, launches
+template <typename T>
+int mx_setup(adscf_ctx* ctx, const BulkDev<T>& I, const std::vector<T>& fk, const std::vector<double>& g64);
+template <typename T>
+int mx_factors(adscf_ctx* ctx, const std::vector<T>& fk, const std::vector<double>& g64);
+int mx_tune(adscf_ctx* ctx);
+void mx_real(adscf_ctx* ctx, int t);
+void mx_step(adscf_ctx* ctx, int t);
+void mx_destroy(adscf_ctx* ctx);
 int bulk_enqueue_chains(adscf_ctx* ctx);        // both chains, all steps
 int bulk_enqueue_contour(adscf_ctx* ctx);       // contour integral + Q
 int bulk_enqueue_expfield(adscf_ctx* ctx, const double* d_w);
