@@ -270,8 +270,7 @@ int adscf_forward(adscf_ctx* ctx, const double* field, double* free_energy) {
   }
   if ((rc = check_ctx(ctx)) || (rc = adj_setup(ctx))) return rc;
   const size_t nv = 2 * (size_t)ctx->npts;
-  std::vector<double> tmp(field, field + nv);
-  CK(cudaMemcpyAsync(ctx->adj->d_w, tmp.data(), nv * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
+  if ((rc = h2d(ctx, ctx->adj->d_w, field, nv))) return rc;
   return forward_core(ctx, free_energy, nullptr);
 }
 

@@ -139,10 +139,16 @@ struct EventPair {
   }
 };
 // host helpers (capi.cu): blocks for n items, capped; host <-> device copies of
-// n doubles through the context's page-locked staging buffer (synchronous)
+// n doubles (synchronous): page-locked caller memory by DMA directly, other
+// memory through the context's page-locked staging buffer
 int grid_blocks(size_t n, int per, int cap);
 int ensure_pinned(adscf_ctx* ctx, size_t bytes);
 bool host_pinned(const void* p);
+// copies of `bytes` through the page-locked buffer `pin` of that size, in
+// chunks, so that the DMA of one chunk runs beside the memcpy of the next;
+// staged_h2d returns with the copies enqueued, staged_d2h when all is in h
+cudaError_t staged_h2d(cudaStream_t s, void* d, const void* h, size_t bytes, void* pin);
+cudaError_t staged_d2h(cudaStream_t s, void* h, const void* d, size_t bytes, void* pin);
 int h2d(adscf_ctx* ctx, double* d, const double* h, size_t n);
 int d2h(adscf_ctx* ctx, double* h, const double* d, size_t n);
 #define CK(call)                                                              \
