@@ -44,6 +44,8 @@ struct FilmState {
   // per line), from the autotuner or the defaults
   AdiShape adi[3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
   bool adi_fuse = false;        // x and y sweeps as one plane kernel (shape adi[0])
+  bool any_ok = false;          // the sweeps on lines of any length (film_any.cuh) take this film
+  bool adi_any = false;         // and run it
   bool adi_set = false;
 };
 
@@ -53,6 +55,8 @@ AdiShape adi_default_shape(int dim, const FilmDev<float>& D);
 void adi_warp_sweep(int dim, AdiShape sh, const FilmDev<float>& D, int step, int chains, cudaStream_t s);
 bool adi_fused_ok(AdiShape x, AdiShape y, const FilmDev<float>& D);
 void adi_fused_sweep(AdiShape sh, const FilmDev<float>& D, int step, int chains, cudaStream_t s);
+template <typename T> bool adi_any_ok(const FilmDev<T>& D, int optin);
+template <typename T> void adi_any_step(const FilmDev<T>& D, const FieldRef& fr, int step, int chains, cudaStream_t s);
 
 namespace {
 
@@ -100,6 +104,7 @@ struct AdiLaunch {
   size_t sx, sy, sz;
   AdiShape sh[3];   // FP32 warp-solver shapes (g = 0: the kernels above)
   bool fuse = false;  // FP32: x and y sweeps in one plane kernel of shape sh[0]
+  bool any = false;   // sweeps on lines of any length
 };
 template <typename T>
 AdiLaunch adi_launch(const FilmState* F, const FilmDev<T>& D, int chains) {
@@ -121,6 +126,7 @@ AdiLaunch adi_launch(const FilmState* F, const FilmDev<T>& D, int chains) {
   A.gz = dim3((D.nlines + A.wz - 1) / A.wz, chains);
   for (int d = 0; d < 3; ++d) A.sh[d] = sizeof(T) == 4 ? F->adi[d] : AdiShape{0, 0, 0};
   A.fuse = sizeof(T) == 4 && F->adi_fuse;
+  A.any = F->adi_any;
   return A;
 }
 
@@ -143,6 +149,10 @@ void adi_sweep(int dim, const AdiLaunch& A, const FilmDev<T>& D, const FieldRef&
 // One Douglas ADI step (three sweeps) of `chains` chains.
 template <typename T>
 void adi_step(const AdiLaunch& A, const FilmDev<T>& D, const FieldRef& fr, int st, int chains, cudaStream_t s) {
+  if (A.any) {
+    adi_any_step<T>(D, fr, st, chains, s);
+    return;
+  }
   if constexpr (sizeof(T) == 4) {
     if (A.fuse) {
       adi_fused_sweep(A.sh[0], D, st, chains, s);
@@ -172,7 +182,7 @@ struct AdiTuneKey {
 };
 struct AdiTuneVal {
   AdiShape sh[3];
-  bool fuse = false;
+  bool fuse = false, any = false;
   std::string report;
 };
 std::mutex g_adi_mu;
@@ -181,6 +191,8 @@ std::map<AdiTuneKey, AdiTuneVal> g_adi_tune;
 void adi_defaults(FilmState* F, const FilmDev<float>& D) {
   for (int d = 0; d < 3; ++d) F->adi[d] = adi_default_shape(d, D);
   F->adi_fuse = false;
+  // a line length with no warp shape would run one thread per line
+  F->adi_any = F->any_ok && !(F->adi[0].g && F->adi[1].g && F->adi[2].g);
   F->adi_set = true;
 }
 
@@ -192,8 +204,9 @@ int adi_tune(adscf_ctx* ctx, FilmState* F, const FilmDev<float>& D, const FieldR
     if (it != g_adi_tune.end()) {
       for (int d = 0; d < 3; ++d) F->adi[d] = it->second.sh[d];
       F->adi_fuse = it->second.fuse;
+      F->adi_any = it->second.any;
       F->adi_set = true;
-      ctx->film_launches = 1 + (F->adi_fuse ? 2 : 3) * ctx->ns;
+      ctx->film_launches = 1 + (F->adi_fuse || F->adi_any ? 2 : 3) * ctx->ns;
       ctx->tune_report = it->second.report + " (cached)";
       return ADSCF_OK;
     }
@@ -273,11 +286,26 @@ int adi_tune(adscf_ctx* ctx, FilmState* F, const FilmDev<float>& D, const FieldR
       rep += line;
     }
   }
+  // the sweeps on lines of any length, against the chosen ones, as whole steps
+  if (F->any_ok) {
+    float us[2] = {1e30f, 1e30f};
+    A.fuse = val.fuse;
+    for (int k = 0; k < 2; ++k) {
+      A.any = k == 1;
+      const int rc = time_graph([&] { adi_step<float>(A, D, fr, 1, 2, s); }, &us[k]);
+      if (rc) return rc;
+    }
+    val.any = us[1] < us[0];
+    char line[96];
+    std::snprintf(line, sizeof(line), " any=%s [any %.2f us against %.2f us];", val.any ? "yes" : "no", us[1], us[0]);
+    rep += line;
+  }
   CK(cudaGetLastError());
   for (int d = 0; d < 3; ++d) F->adi[d] = val.sh[d];
   F->adi_fuse = val.fuse;
+  F->adi_any = val.any;
   F->adi_set = true;
-  ctx->film_launches = 1 + (F->adi_fuse ? 2 : 3) * ctx->ns;
+  ctx->film_launches = 1 + (F->adi_fuse || F->adi_any ? 2 : 3) * ctx->ns;
   val.report = rep;
   ctx->tune_report = rep;
   std::lock_guard<std::mutex> lk(g_adi_mu);
@@ -440,6 +468,8 @@ void fill_dev(adscf_ctx* ctx, FilmState* F, const adscf_params* p) {
   D.err = F->d_err;
   D.dx = p->sizex / p->gx;
   D.dy = p->sizey / p->gy;
+  D.hx2 = 0.5 / D.dx / D.dx;
+  D.hy2 = 0.5 / D.dy / D.dy;
   D.w1 = static_cast<T*>(F->d_w1);
   const size_t n1 = (size_t)ctx->gz + 1;
   D.alf = F->d_alf;
@@ -539,12 +569,18 @@ int film_create(adscf_ctx* ctx, const adscf_params* p) {
   if (rc) return rc;
   if (F->t64) fill_dev<double>(ctx, F, p);
   else fill_dev<float>(ctx, F, p);
-  ctx->film_launches = ctx->geometry == ADSCF_FILM_3D ? 1 + 3 * ctx->ns : 1;
+  if (ctx->geometry == ADSCF_FILM_3D) {
+    F->any_ok = F->t64 ? adi_any_ok(F->f64, F->optin) : adi_any_ok(F->f32, F->optin);
+    // FP64 sweeps: one thread per line only where the lines are too long
+    F->adi_any = F->t64 && F->any_ok;
+  }
+  ctx->film_launches = ctx->geometry == ADSCF_FILM_3D ? 1 + (F->adi_any ? 2 : 3) * ctx->ns : 1;
   ctx->film_contour_launches = 1;
   if (ctx->geometry == ADSCF_FILM_3D && !F->t64) {   // FP32 ADI sweeps: pick their shapes
     FilmDev<float>& D = F->f32;
     if (!ctx->autotune) {
       adi_defaults(F, D);
+      ctx->film_launches = 1 + (F->adi_any ? 2 : 3) * ctx->ns;
       return ADSCF_OK;
     }
     const size_t n = (size_t)ctx->ntypes * D.npts;
@@ -579,6 +615,7 @@ int film_set_adi_plan(adscf_ctx* ctx, const int lanes[3], int staged) {
   if (fuse && !adi_fused_ok(sh[0], sh[1], F->f32)) return ADSCF_E_ARG;
   for (int d = 0; d < 3; ++d) F->adi[d] = sh[d];
   F->adi_fuse = fuse;
+  F->adi_any = false;
   F->adi_set = true;
   ctx->film_launches = 1 + (fuse ? 2 : 3) * ctx->ns;
   return ADSCF_OK;

@@ -1,5 +1,7 @@
-// film_adi.cu -- launches of the warp-cooperative FP32 Douglas ADI sweeps
-// (film_warp.cuh) for Film_3D contexts in split precision.
+// film_adi.cu -- launches of the cooperative Douglas ADI sweeps of Film_3D
+// contexts: the FP32 warp shapes (film_warp.cuh) and the sweeps on lines of
+// any length in either precision (film_any.cuh).
+#include "film_any.cuh"
 #include "film_warp.cuh"
 #include "internal.h"
 
@@ -169,3 +171,44 @@ void adi_warp_sweep(int dim, AdiShape sh, const FilmDev<float>& D, int step, int
     }
   }
 }
+
+// ---- lines of any length (film_any.cuh) --------------------------------------
+namespace {
+
+template <typename T>
+size_t any_smem_xy(const FilmDev<T>& D) { return 2 * (size_t)D.gy * (D.gx | 1) * sizeof(T); }
+template <typename T>
+size_t any_smem_z(const FilmDev<T>& D, int tl) { return ((size_t)(D.gz + 1) * (2 * (tl + 1) + 3) + 1) * sizeof(T); }
+// lines of a z tile: 16 (128-byte rows in FP64, 64 in FP32), fewer while the
+// tiles do not cover the SMs
+template <typename T>
+int any_tile(const FilmDev<T>& D, int chains) {
+  int tl = 16;
+  while (tl > 4 && (D.nlines + tl - 1) / tl * chains < 152) tl /= 2;
+  return tl;
+}
+int any_threads(int lines, int lanes, int cap) { return std::min(cap, std::max(64, (lines * lanes + 31) / 32 * 32)); }
+
+}  // namespace
+
+// whether the sweeps take the film's lines, and the kernels' shared memory
+// limits (per function and device); `optin`: opt-in shared memory per block
+template <typename T>
+bool adi_any_ok(const FilmDev<T>& D, int optin) {
+  if (!adiany::lanes(D.gx) || !adiany::lanes(D.gy) || !adiany::lanes(D.gz + 1)) return false;
+  if (any_smem_xy(D) > (size_t)optin || any_smem_z(D, 16) > (size_t)optin) return false;
+  return cudaFuncSetAttribute(k_adi_xy_any<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin) == cudaSuccess &&
+         cudaFuncSetAttribute(k_adi_z_any<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin) == cudaSuccess;
+}
+template <typename T>
+void adi_any_step(const FilmDev<T>& D, const FieldRef& fr, int step, int chains, cudaStream_t s) {
+  const int tx = any_threads(std::max(D.gy * adiany::lanes(D.gx), D.gx * adiany::lanes(D.gy)), 1, 512);
+  k_adi_xy_any<T><<<dim3(D.gz - 1, chains), tx, any_smem_xy(D), s>>>(D, fr, step);
+  const int tl = any_tile(D, chains);
+  k_adi_z_any<T><<<dim3((D.nlines + tl - 1) / tl, chains), any_threads(tl, adiany::lanes(D.gz + 1), 512),
+                   any_smem_z(D, tl), s>>>(D, fr, step, tl);
+}
+template bool adi_any_ok<float>(const FilmDev<float>&, int);
+template bool adi_any_ok<double>(const FilmDev<double>&, int);
+template void adi_any_step<float>(const FilmDev<float>&, const FieldRef&, int, int, cudaStream_t);
+template void adi_any_step<double>(const FilmDev<double>&, const FieldRef&, int, int, cudaStream_t);

@@ -58,6 +58,7 @@ struct FilmDev {
   int* err;              // pivot / non-finite flags
   // ADI (Film_3D) only
   double dx, dy;
+  double hx2, hy2;       // 1 / (2 dx dx), 1 / (2 dy dy)
   T* w1;                 // [2][npts] intermediate q*, q** of the ADI sweeps
   // FP32 sweeps: FP32 copies of the mesh factors and, for the ADI sweeps, of
   // the field ([ntypes][npts], filled per propagation)

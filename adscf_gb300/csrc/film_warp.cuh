@@ -73,10 +73,12 @@ __device__ __forceinline__ void eliminate(const T (&a)[K], const T (&d)[K], cons
 // place of r.  `periodic`: row 0 of lane 0 couples to the last lane's
 // separator through a, and that separator to row 0 through c (all G lanes
 // own rows).  K is a compile-time constant so that every row stays in
-// registers.  All G lanes of the group must call it together.
+// registers.  i0 = 1: the lane has K - 1 rows, entries 1 .. K - 1, and entry 0
+// repeats its left neighbour (a = -1, d = 1, c = 0, r = 0); K >= 3 then.  All
+// G lanes of the group must call it together.
 template <int G, int K, typename T>
 __device__ __forceinline__ void solve(const T (&a)[K], const T (&d)[K], const T (&c)[K],
-                                      T (&r)[K], bool periodic, int* err) {
+                                      T (&r)[K], bool periodic, int* err, int i0 = 0) {
   static_assert(K >= 2, "a lane needs an interior row and a separator");
   const int lane = threadIdx.x & 31;
   const int gl = lane & (G - 1);          // lane within the group
@@ -88,7 +90,9 @@ __device__ __forceinline__ void solve(const T (&a)[K], const T (&d)[K], const T 
   // lane and the first interior row of the next lane
   constexpr int S = K - 1, Li = K - 2;
   const int nx = base + ((gl + 1) & (G - 1));
-  T xn = __shfl_sync(mask, x[0], nx), yn = __shfl_sync(mask, y[0], nx), zn = __shfl_sync(mask, z[0], nx);
+  constexpr int F1 = K > 2 ? 1 : 0;        // a short lane's first row
+  T xn = __shfl_sync(mask, i0 ? x[F1] : x[0], nx), yn = __shfl_sync(mask, i0 ? y[F1] : y[0], nx),
+    zn = __shfl_sync(mask, i0 ? z[F1] : z[0], nx);
   if (!periodic && gl == G - 1) { xn = (T)0; yn = (T)0; zn = (T)0; }
   T A = r_mul(a[S], y[Li]);
   T B = r_fma(c[S], yn, r_fma(a[S], z[Li], d[S]));
