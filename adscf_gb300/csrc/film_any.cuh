@@ -20,8 +20,13 @@
 // z lines whose systems are not diagonally dominant (ds w / 2 below -0.99)
 // run the reference's serial recurrence, with its pivots and their checks.
 //
-// Bound: FP64 the FP64 pipe (about 110 FP64 instructions a point and step),
-// FP32 latency.
+// The x and y matrices are the same for every line of a sweep: each warp makes
+// their factors once and applies them line after line.
+//
+// Bound: FP64 the FP64 pipe and the wave of 99 planes on 152 SMs, FP32 latency.
+// A step of both chains, thread per line -> here: 20x35x100 FP64 220 -> 52 us
+// (69 without the factors), FP32 43.5 -> 12.5; 48^3 FP64 57 us, FP32 69.5 ->
+// 12.1; 96x96x64 FP32 175 -> 26.
 #pragma once
 #include "film_warp.cuh"
 
@@ -75,6 +80,89 @@ __device__ __forceinline__ T pair(T a, T c, T qm, T q0, T qp) {
   return r_fma(a, r_sub(qm, q0), r_mul(c, r_sub(qp, q0)));
 }
 
+// Factors of the periodic matrix (a, d, a) of the x and y lines, the same for
+// every line of a sweep: made once per warp, applied line after line (solve:
+// fw::solve's operations on the right-hand side alone, about 5 a row where
+// the whole solve takes 30).
+template <typename T, int G, int K>
+struct Factors {
+  static constexpr int LG = G == 4 ? 2 : G == 8 ? 3 : G == 16 ? 4 : 5;
+  T bet[K - 1], m[K - 1], g[K - 1], y[K - 1], z[K - 1];
+  T kl[LG], kr[LG], iden, a;
+  int i0;
+
+  __device__ __forceinline__ Factors(T a_, T d_, int i0_, int* err) : a(a_), i0(i0_) {
+    const unsigned mask = 0xffffffffu;
+    const int lane = threadIdx.x & 31, gl = lane & (G - 1), base = lane - gl;
+    T b = (T)1;
+#pragma unroll
+    for (int i = 0; i < K - 1; ++i) {
+      const bool pad = i < i0;
+      const T ai = pad ? (T)-1 : a, di = pad ? (T)1 : d_;
+      const T cm = i > 0 && !(i - 1 < i0) ? a : (T)0;       // super-diagonal of the row above
+      g[i] = i == 0 ? (T)0 : r_mul(cm, b);
+      const T piv = i == 0 ? di : r_fma(-ai, g[i], di);
+      if (piv == (T)0) atomicOr(err, 1);
+      b = fw::rcp(piv);
+      bet[i] = b;
+      m[i] = r_mul(-ai, b);
+      y[i] = i == 0 ? m[0] : r_mul(m[i], y[i > 0 ? i - 1 : 0]);
+      z[i] = i == K - 2 ? r_mul(-a, b) : (T)0;
+    }
+#pragma unroll
+    for (int i = K - 3; i >= 0; --i) {
+      y[i] = r_fma(-g[i + 1], y[i + 1], y[i]);
+      z[i] = r_mul(-g[i + 1], z[i + 1]);
+    }
+    const int nx = base + ((gl + 1) & (G - 1));
+    const T yn = __shfl_sync(mask, i0 ? y[1] : y[0], nx), zn = __shfl_sync(mask, i0 ? z[1] : z[0], nx);
+    T A = r_mul(a, y[K - 2]), B = r_fma(a, yn, r_fma(a, z[K - 2], d_)), C = r_mul(a, zn);
+#pragma unroll
+    for (int s = 0; s < LG; ++s) {
+      const int st = 1 << s, su = base + ((gl - st) & (G - 1)), sd = base + ((gl + st) & (G - 1));
+      if (B == (T)0) atomicOr(err, 1);
+      const T i1 = fw::rcp(B);
+      kl[s] = r_mul(A, __shfl_sync(mask, i1, su));
+      kr[s] = r_mul(C, __shfl_sync(mask, i1, sd));
+      const T Au = __shfl_sync(mask, A, su), Cu = __shfl_sync(mask, C, su);
+      const T Ad = __shfl_sync(mask, A, sd), Cd = __shfl_sync(mask, C, sd);
+      B = r_fma(-kr[s], Ad, r_fma(-kl[s], Cu, B));
+      A = r_mul(-kl[s], Au);
+      C = r_mul(-kr[s], Cd);
+    }
+    const T den = r_add(r_add(A, C), B);
+    if (den == (T)0) atomicOr(err, 1);
+    iden = fw::rcp(den);
+  }
+
+  // r: right-hand side of the lane's entries (0 in a pad entry); the solution
+  // on return
+  __device__ __forceinline__ void solve(T (&r)[K]) const {
+    const unsigned mask = 0xffffffffu;
+    const int lane = threadIdx.x & 31, gl = lane & (G - 1), base = lane - gl;
+    T x[K - 1];
+#pragma unroll
+    for (int i = 0; i < K - 1; ++i)
+      x[i] = i == 0 ? r_mul(r[0], bet[0]) : r_fma(m[i], x[i > 0 ? i - 1 : 0], r_mul(r[i], bet[i]));
+#pragma unroll
+    for (int i = K - 3; i >= 0; --i) x[i] = r_fma(-g[i + 1], x[i + 1], x[i]);
+    const T xn = __shfl_sync(mask, i0 ? x[1] : x[0], base + ((gl + 1) & (G - 1)));
+    T R = r_fma(-a, xn, r_fma(-a, x[K - 2], r[K - 1]));
+#pragma unroll
+    for (int s = 0; s < LG; ++s) {
+      const int st = 1 << s;
+      const T Ru = __shfl_sync(mask, R, base + ((gl - st) & (G - 1)));
+      const T Rd = __shfl_sync(mask, R, base + ((gl + st) & (G - 1)));
+      R = r_fma(-kr[s], Rd, r_fma(-kl[s], Ru, R));
+    }
+    const T v = r_mul(R, iden);
+    const T vl = __shfl_sync(mask, v, base + ((gl - 1) & (G - 1)));
+#pragma unroll
+    for (int i = 0; i < K - 1; ++i) r[i] = r_fma(z[i], v, r_fma(y[i], vl, x[i]));
+    r[K - 1] = v;
+  }
+};
+
 // x sweep of the plane P ([y][x], pitch pt) into D
 template <typename T, int G, int K>
 __device__ __forceinline__ void x_lines(const FilmDev<T>& F, const Coef<T>& cf, const T* P, T* D, int pt, const T* p0,
@@ -83,16 +171,17 @@ __device__ __forceinline__ void x_lines(const FilmDev<T>& F, const Coef<T>& cf, 
   const int gl = threadIdx.x & (G - 1), ng = blockDim.x / G;
   const Rows R = rows_of<G, K>(gx, gl);
   const T az = r_mul(-cf.ds, mesh(F, z, 0)), cz = r_mul(-cf.ds, mesh(F, z, 1));
-  const T dg = r_fma((T)-2, cf.ax, (T)1);
-  for (int y0 = 0; y0 < gy; y0 += ng) {
-    const int yl = y0 + threadIdx.x / G;
+  const Factors<T, G, K> fac(cf.ax, r_fma((T)-2, cf.ax, (T)1), R.i0, F.err);
+  // a warp leaves when its lines are done (its lanes stay together)
+  for (int y0 = (threadIdx.x & ~31) / G; y0 < gy; y0 += ng) {
+    const int yl = y0 + (threadIdx.x & 31) / G;
     const bool live = yl < gy;
     const int y = live ? yl : 0;
     const int ym = (y == 0 ? gy : y) - 1, yp = y == gy - 1 ? 0 : y + 1;
-    T a[K], d[K], c[K], r[K];
+    T r[K];
 #pragma unroll
     for (int i = 0; i < K; ++i) {
-      a[i] = (T)-1; d[i] = (T)1; c[i] = (T)0; r[i] = (T)0;
+      r[i] = (T)0;
       if (i >= R.i0) {
         const int x = R.start + i - R.i0;
         const int xm = (x == 0 ? gx : x) - 1, xp = x == gx - 1 ? 0 : x + 1;
@@ -102,11 +191,10 @@ __device__ __forceinline__ void x_lines(const FilmDev<T>& F, const Coef<T>& cf, 
         t = r_add(t, pair(cf.ay, cf.ay, P[ym * pt + x], q0, P[yp * pt + x]));
         t = r_add(t, pair(az, cz, __ldg(p0 + g - L), q0, __ldg(p0 + g + L)));
         t = r_fma(r_mul(cf.hds, fieldv(F, w, ty, g)), q0, t);
-        a[i] = cf.ax; c[i] = cf.ax; d[i] = dg;
         r[i] = r_mul((T)-2, t);
       }
     }
-    fw::solve<G, K>(a, d, c, r, true, F.err, R.i0);
+    fac.solve(r);
     if (live) {
 #pragma unroll
       for (int i = 0; i < K; ++i)
@@ -121,21 +209,15 @@ __device__ __forceinline__ void y_lines(const FilmDev<T>& F, const Coef<T>& cf, 
   const int gx = F.gx, gy = F.gy;
   const int gl = threadIdx.x & (G - 1), ng = blockDim.x / G;
   const Rows R = rows_of<G, K>(gy, gl);
-  const T dg = r_fma((T)-2, cf.ay, (T)1);
-  for (int x0 = 0; x0 < gx; x0 += ng) {
-    const int xl = x0 + threadIdx.x / G;
+  const Factors<T, G, K> fac(cf.ay, r_fma((T)-2, cf.ay, (T)1), R.i0, F.err);
+  for (int x0 = (threadIdx.x & ~31) / G; x0 < gx; x0 += ng) {
+    const int xl = x0 + (threadIdx.x & 31) / G;
     const bool live = xl < gx;
     const int x = live ? xl : 0;
-    T a[K], d[K], c[K], r[K];
+    T r[K];
 #pragma unroll
-    for (int i = 0; i < K; ++i) {
-      const bool in = i >= R.i0;
-      a[i] = in ? cf.ay : (T)-1;
-      c[i] = in ? cf.ay : (T)0;
-      d[i] = in ? dg : (T)1;
-      r[i] = in ? D[(R.start + i - R.i0) * pt + x] : (T)0;
-    }
-    fw::solve<G, K>(a, d, c, r, true, F.err, R.i0);
+    for (int i = 0; i < K; ++i) r[i] = i >= R.i0 ? D[(R.start + i - R.i0) * pt + x] : (T)0;
+    fac.solve(r);
     if (live) {
 #pragma unroll
       for (int i = 0; i < K; ++i)
@@ -155,13 +237,13 @@ __device__ __forceinline__ bool far_below(double hw) {
 // at pitch pt; tab: alpha, gamma, beta; lines [0, cnt) of the tile exist
 template <typename T, int G, int K>
 __device__ __forceinline__ void z_lines(const FilmDev<T>& F, const Coef<T>& cf, T* D, T* W, const T* tab, int pt,
-                                        int tl, int cnt, int* dummy) {
+                                        int cnt, int* dummy) {
   const int n = F.gz + 1;
   const int gl = threadIdx.x & (G - 1), ng = blockDim.x / G;
   const Rows R = rows_of<G, K>(n, gl);
   const T *al = tab, *ga = tab + n, *be = tab + 2 * n;
-  for (int l0 = 0; l0 < tl; l0 += ng) {
-    const int ll = l0 + threadIdx.x / G;
+  for (int l0 = (threadIdx.x & ~31) / G; l0 < cnt; l0 += ng) {
+    const int ll = l0 + (threadIdx.x & 31) / G;
     const bool live = ll < cnt;
     const int l = live ? ll : 0;
     T a[K], d[K], c[K], r[K];
@@ -300,7 +382,7 @@ k_adi_z_any(FilmDev<T> F, FieldRef fr, int s, int tl) {
     W[j * pt + lx] = v;
   }
   __syncthreads();
-#define ADSCF_ANY_CALL(G, K) adiany::z_lines<T, G, K>(F, cf, D, W, tab, pt, tl, cnt, dummy)
+#define ADSCF_ANY_CALL(G, K) adiany::z_lines<T, G, K>(F, cf, D, W, tab, pt, cnt, dummy)
   ADSCF_ANY_SHAPE(n, ADSCF_ANY_CALL)
 #undef ADSCF_ANY_CALL
   __syncthreads();

@@ -32,9 +32,17 @@
 
 namespace fw {
 
-// pivots: the hardware reciprocal in FP32 (see rcp_hw), correctly rounded in FP64
+// Reciprocal pivots.  FP32: the hardware reciprocal (see rcp_hw).  FP64: the
+// hardware's approximation y (about 20 bits) and two Newton-Raphson steps y +=
+// y (1 - x y): four FP64 instructions (each 64 cycles on its SM quarter) and
+// no branch for the range ends, which a pivot of 1 + O(ds) does not come near.
 __device__ __forceinline__ float rcp(float x) { return rcp_hw(x); }
-__device__ __forceinline__ double rcp(double x) { return __drcp_rn(x); }
+__device__ __forceinline__ double rcp(double x) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  y = __fma_rn(y, __fma_rn(-x, y, 1.0), y);
+  return __fma_rn(y, __fma_rn(-x, y, 1.0), y);
+}
 
 // Local elimination of the interior rows 0..K-2 of a lane with three
 // right-hand sides -- r, -a_0 at the first row, -c_{K-2} at the last row: on
@@ -107,11 +115,22 @@ __device__ __forceinline__ void solve(const T (&a)[K], const T (&d)[K], const T 
     T Cu = __shfl_sync(mask, C, su), Ru = __shfl_sync(mask, R, su);
     T Ad = __shfl_sync(mask, A, sd), Bd = __shfl_sync(mask, B, sd);
     T Cd = __shfl_sync(mask, C, sd), Rd = __shfl_sync(mask, R, sd);
-    if (!periodic && gl - st < 0) { Au = (T)0; Bu = (T)1; Cu = (T)0; Ru = (T)0; }
-    if (!periodic && gl + st >= G) { Ad = (T)0; Bd = (T)1; Cd = (T)0; Rd = (T)0; }
-    if (Bu == (T)0 || Bd == (T)0) atomicOr(err, 1);
-    const T kl = r_mul(A, rcp(Bu));
-    const T kr = r_mul(C, rcp(Bd));
+    T iu = (T)0, id = (T)0;
+    if constexpr (sizeof(T) == 8) {   // one reciprocal a lane, shuffled
+      if (B == (T)0) atomicOr(err, 1);
+      const T i0 = rcp(B);
+      iu = __shfl_sync(mask, i0, su);
+      id = __shfl_sync(mask, i0, sd);
+    }
+    if (!periodic && gl - st < 0) { Au = (T)0; Bu = (T)1; iu = (T)1; Cu = (T)0; Ru = (T)0; }
+    if (!periodic && gl + st >= G) { Ad = (T)0; Bd = (T)1; id = (T)1; Cd = (T)0; Rd = (T)0; }
+    if constexpr (sizeof(T) == 4) {
+      if (Bu == (T)0 || Bd == (T)0) atomicOr(err, 1);
+      iu = rcp(Bu);
+      id = rcp(Bd);
+    }
+    const T kl = r_mul(A, iu);
+    const T kr = r_mul(C, id);
     const T nB = r_fma(-kr, Ad, r_fma(-kl, Cu, B));
     const T nR = r_fma(-kr, Rd, r_fma(-kl, Ru, R));
     A = r_mul(-kl, Au);
