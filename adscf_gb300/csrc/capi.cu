@@ -179,9 +179,11 @@ int enqueue_iteration(adscf_ctx* ctx) {
 
 int build_iteration_graph(adscf_ctx* ctx) {
   if (ctx->g_iter) return ADSCF_OK;
+  int rc = film_prepare(ctx);
+  if (rc) return rc;
   cudaGraph_t g;
   CK(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
-  int rc = enqueue_iteration(ctx);
+  rc = enqueue_iteration(ctx);
   cudaError_t e = cudaStreamEndCapture(ctx->stream, &g);
   if (rc) return rc;
   if (e != cudaSuccess) return set_err(ctx, ADSCF_E_CUDA, std::string("capture: ") + cudaGetErrorString(e));
@@ -193,9 +195,11 @@ int build_iteration_graph(adscf_ctx* ctx) {
 
 int build_prop_graph(adscf_ctx* ctx) {
   if (ctx->g_prop) return ADSCF_OK;
+  int rc = film_prepare(ctx);
+  if (rc) return rc;
   cudaGraph_t g;
   CK(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
-  int rc = enqueue_propagate(ctx, ctx->d_tmp);
+  rc = enqueue_propagate(ctx, ctx->d_tmp);
   cudaError_t e = cudaStreamEndCapture(ctx->stream, &g);
   if (rc) return rc;
   if (e != cudaSuccess) return set_err(ctx, ADSCF_E_CUDA, std::string("capture: ") + cudaGetErrorString(e));

@@ -12,6 +12,7 @@
 #include "film_host.h"
 #include "film_kernels.cuh"
 #include "film_warp.cuh"
+#include "film_line.cuh"
 #include "internal.h"
 
 struct FilmState {
@@ -33,6 +34,8 @@ struct FilmState {
   void* d_gam = nullptr;
   void* d_w1 = nullptr;
   int* d_err = nullptr;
+  double2* d_fac = nullptr;     // factors of every step (film_line.cuh), from the first propagation on
+  bool fac_tried = false;
   double max_ratio = 1.0;       // largest neighbour spacing ratio of the mesh
   int optin = 0;                // opt-in shared memory per block
   // free energy at fixed fields and its wall-potential gradient
@@ -329,6 +332,38 @@ void field_f32(const FilmDev<float>& D, const FieldRef& fr, size_t n, cudaStream
 // FP64 lines whose warps find enough idle SMs spread them over a cluster
 // (one FP64 pipe per SM); with more (line, chain) pairs than that the SMs
 // are busy anyway and a line's warps share a CTA, whose barrier is cheaper.
+// FP64 lines of up to 1024 rows whose chains find an SM each apply factors made
+// ahead (film_line.cuh) in both chains of a propagation.  More lines keep the
+// SMs busy as they are, and the factors (27 to 56 KB a line and step) are kept
+// under 1 GB; without them the chains eliminate as they go.
+bool line_factors_ok(const adscf_ctx* ctx) {
+  const FilmState* F = ctx->film;
+  const FilmDev<double>& D = F->f64;
+  if (!F->t64 || ctx->geometry == ADSCF_FILM_3D || D.gz + 1 > fl::kMaxRows || 2 * D.nlines > 152) return false;
+  const size_t step = fl::step_bytes(fl::rows_per_lane(D.gz + 1));
+  return fl::kStages * step <= (size_t)F->optin - 1024 && step * D.ns * D.nlines <= ((size_t)1 << 30);
+}
+template <int K>
+int launch_line_t(adscf_ctx* ctx, const FilmDev<double>& D, const FieldRef& fr, cudaStream_t s) {
+  const size_t sm = fl::kStages * fl::step_bytes(K);
+  double2* fac = ctx->film->d_fac;
+  CK(cudaFuncSetAttribute(k_line_chain<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+  k_line_factors<K><<<dim3(D.ns, D.nlines), fl::kThreads, 0, s>>>(D, fr, fac);
+  k_line_chain<K><<<dim3(D.nlines, 2), fl::kThreads, sm, s>>>(D, fr, fac);
+  return ADSCF_OK;
+}
+int launch_line(adscf_ctx* ctx, const FilmDev<double>& D, const FieldRef& fr, cudaStream_t s) {
+  switch (fl::rows_per_lane(D.gz + 1)) {
+    case 2: return launch_line_t<2>(ctx, D, fr, s);
+    case 3: return launch_line_t<3>(ctx, D, fr, s);
+    case 4: return launch_line_t<4>(ctx, D, fr, s);
+    case 5: return launch_line_t<5>(ctx, D, fr, s);
+    case 6: return launch_line_t<6>(ctx, D, fr, s);
+    case 7: return launch_line_t<7>(ctx, D, fr, s);
+    default: return launch_line_t<8>(ctx, D, fr, s);
+  }
+}
+
 template <typename T>
 int launch_chains_1d(adscf_ctx* ctx, const FilmDev<T>& D, const FieldRef& fr, int chains, cudaStream_t s) {
   const int n = D.gz + 1;
@@ -374,7 +409,10 @@ int chains_t(adscf_ctx* ctx, const double* d_w) {
     const AdiLaunch A = adi_launch<T>(F, D, 2);
     for (int st = 1; st <= D.ns; ++st) adi_step<T>(A, D, fr, st, 2, s);
   } else {
-    const int rc = launch_chains_1d<T>(ctx, D, fr, 2, s);
+    int rc = film_prepare(ctx);
+    if (rc) return rc;
+    if constexpr (sizeof(T) == 8) rc = F->d_fac ? launch_line(ctx, D, fr, s) : launch_chains_1d<T>(ctx, D, fr, 2, s);
+    else rc = launch_chains_1d<T>(ctx, D, fr, 2, s);
     if (rc) return rc;
   }
   CK(cudaGetLastError());
@@ -574,7 +612,9 @@ int film_create(adscf_ctx* ctx, const adscf_params* p) {
     // FP64 sweeps: one thread per line only where the lines are too long
     F->adi_any = F->t64 && F->any_ok;
   }
-  ctx->film_launches = ctx->geometry == ADSCF_FILM_3D ? 1 + (F->adi_any ? 2 : 3) * ctx->ns : 1;
+  ctx->film_launches = ctx->geometry == ADSCF_FILM_3D ? 1 + (F->adi_any ? 2 : 3) * ctx->ns
+                       : line_factors_ok(ctx)            ? 2
+                                                         : 1;
   ctx->film_contour_launches = 1;
   if (ctx->geometry == ADSCF_FILM_3D && !F->t64) {   // FP32 ADI sweeps: pick their shapes
     FilmDev<float>& D = F->f32;
@@ -674,9 +714,28 @@ void film_destroy(adscf_ctx* ctx) {
   cudaFree(F->d_dss); cudaFree(F->d_adicf); cudaFree(F->d_wA); cudaFree(F->d_wB); cudaFree(F->d_graft);
   cudaFree(F->d_alf); cudaFree(F->d_wf);
   cudaFree(F->d_q); cudaFree(F->d_qd); cudaFree(F->d_gam); cudaFree(F->d_w1);
-  cudaFree(F->d_err); cudaFree(ctx->d_qpart);
+  cudaFree(F->d_err); cudaFree(ctx->d_qpart); cudaFree(F->d_fac);
   delete F;
   ctx->film = nullptr;
+}
+
+// The factor workspace of FP64 lines, on the first propagation of this context
+// by itself (a film of a batch is swept with the batch, and needs none); not
+// inside a stream capture.
+int film_prepare(adscf_ctx* ctx) {
+  FilmState* F = ctx->film;
+  if (!F || F->fac_tried || !line_factors_ok(ctx)) return ADSCF_OK;
+  cudaStreamCaptureStatus st;
+  CK(cudaStreamIsCapturing(ctx->stream, &st));
+  if (st != cudaStreamCaptureStatusNone) return ADSCF_OK;
+  F->fac_tried = true;
+  const FilmDev<double>& D = F->f64;
+  if (cudaMalloc(&F->d_fac, fl::step_bytes(fl::rows_per_lane(D.gz + 1)) * D.ns * D.nlines) != cudaSuccess) {
+    cudaGetLastError();
+    F->d_fac = nullptr;
+  }
+  ctx->film_launches = F->d_fac ? 2 : 1;
+  return ADSCF_OK;
 }
 
 int film_enqueue_chains(adscf_ctx* ctx, const double* d_w) {

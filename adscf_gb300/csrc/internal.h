@@ -190,6 +190,7 @@ void adj_destroy(adscf_ctx* ctx);
 int film_create(adscf_ctx* ctx, const adscf_params* p);
 int film_check_pivot(adscf_ctx* ctx);
 void film_destroy(adscf_ctx* ctx);
+int film_prepare(adscf_ctx* ctx);               // workspace of the chains, before a capture of them
 int film_enqueue_propagate(adscf_ctx* ctx, const double* d_w);
 int film_enqueue_chains(adscf_ctx* ctx, const double* d_w);
 int film_enqueue_contour(adscf_ctx* ctx);
