@@ -340,14 +340,18 @@ int create_t(adscf_ctx* ctx) {
   CK(cudaMalloc(&ctx->d_inst, sizeof(BulkDev<T>)));
   CK(cudaMemcpy(ctx->d_inst, &I, sizeof(I), cudaMemcpyHostToDevice));
   hb<T>(ctx) = I;
-  // Mixed-radix passes where a line length has no register FFT.  Of the
-  // shapes that have one on every axis, FP64 takes them too unless the axes
-  // are equal (one_reg; its FP32 passes at 64 x 32 x 128 take 18.8 us a double
-  // step against 20.7), and at 32^3, whose 1024 lines are 16 register-FFT
-  // blocks on 152 SMs (23 against 60 us).
+  // Mixed-radix passes where a line length has no register FFT, and of the
+  // shapes that have one on every axis
+  //  - FP32 with a line of 256 points, whose register passes leave L2 four
+  //    times a double step (256^3 542 us a double step with them, 405 here;
+  //    64 x 64 x 256 44.8 and 30.3, 256 x 64 x 64 31.6 and 27.3; without one
+  //    the register passes are ahead: 64 x 32 x 128 18.8 and 20.7);
+  //  - FP64 but 256^3, where HBM bounds both (4641 and 4704 us): the cut takes
+  //    two passes for four (64^3 73.4 and 69.6 us, 128^3 609 and 531, 32^3 60
+  //    and 23).
   const bool all_reg = ctx->regx && ctx->regy && ctx->regz;
-  const bool one_reg = all_reg && ctx->regx == ctx->regy && ctx->regx == ctx->regz;
-  const bool mixed = sizeof(T) == 8 ? !one_reg || ctx->regx == 32 : !all_reg;
+  const int n256 = (ctx->regx == 256) + (ctx->regy == 256) + (ctx->regz == 256);
+  const bool mixed = !all_reg || (sizeof(T) == 8 ? n256 < 3 : n256 > 0);
   if (mixed && !ctx->use_generic) {
     if ((rc = mx_setup<T>(ctx, I, fk, g64))) return rc;
   }
@@ -434,9 +438,11 @@ void step_nn(adscf_ctx* ctx, int t) {
   }
 }
 
+bool mx_runs(const adscf_ctx* ctx) { return ctx->mx && !ctx->mx_off; }
+
 template <typename T>
 void step_t(adscf_ctx* ctx, int t) {
-  if (ctx->mx) {
+  if (mx_runs(ctx)) {
     mx_step(ctx, t);
     return;
   }
@@ -460,7 +466,7 @@ void step_t(adscf_ctx* ctx, int t) {
 template <typename T>
 int chains_t(adscf_ctx* ctx) {
   const XAux none{nullptr, nullptr, nullptr};
-  if (ctx->mx) {
+  if (mx_runs(ctx)) {
     mx_real(ctx, 0);
   } else if (sizeof(T) == 4 && ctx->plan_x == PK_FUSED) {
     // the initial plane pass also does Yf of step 1
@@ -795,7 +801,7 @@ int bulk_hold_slices(adscf_ctx* ctx, bool full) {
 }
 // kernel launches of a propagation's contour steps and its first pass
 int bulk_chain_launches(const adscf_ctx* ctx) {
-  const bool two = ctx->mx || ctx->plan_x == PK_FUSED;
+  const bool two = mx_runs(ctx) || ctx->plan_x == PK_FUSED;
   return 1 + (two ? 2 : 4) * ctx->ns;
 }
 // bound of the TMA passes' pipeline waits (0: every wait gives up at once)

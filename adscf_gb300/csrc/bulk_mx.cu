@@ -346,11 +346,16 @@ int mx_factors(adscf_ctx* ctx, const std::vector<T>& fk, const std::vector<doubl
   const int gx = ctx->gx, gy = ctx->gy, gz = ctx->gz;
   const size_t nxy = (size_t)gx * gy;
   std::vector<T> out(2 * nxy + 2 * (size_t)gz);
+  std::vector<int> f[3];
+  for (int d = 0; d < 3; ++d)
+    for (int p = 0; p < M->a[d].n; ++p) f[d].push_back(mx_freq(M->a[d], p));
   for (int h = 0; h < 2; ++h) {
-    for (int y = 0; y < gy; ++y)
-      for (int x = 0; x < gx; ++x)
-        out[h * nxy + (size_t)y * gx + x] = fk[h * nxy + (size_t)mx_freq(M->a[1], y) * gx + mx_freq(M->a[0], x)];
-    for (int z = 0; z < gz; ++z) out[2 * nxy + (size_t)h * gz + z] = fk[2 * nxy + (size_t)h * gz + mx_freq(M->a[2], z)];
+    for (int y = 0; y < gy; ++y) {
+      const T* from = fk.data() + h * nxy + (size_t)f[1][y] * gx;
+      T* to = out.data() + h * nxy + (size_t)y * gx;
+      for (int x = 0; x < gx; ++x) to[x] = from[f[0][x]];
+    }
+    for (int z = 0; z < gz; ++z) out[2 * nxy + (size_t)h * gz + z] = fk[2 * nxy + (size_t)h * gz + f[2][z]];
   }
   if (sizeof(T) == 4) out[0] = out[nxy] = (T)0;
   CK(cudaMemcpy(M->d_fk, out.data(), out.size() * sizeof(T), cudaMemcpyHostToDevice));

@@ -799,6 +799,7 @@ int adscf_set_pass_plan(adscf_ctx* ctx, int y, int z, int x) {
                     (x == ADSCF_PASS_FUSED && ctx->tma && ctx->xy_grid);
   if (!ok_yz(y) || !ok_yz(z) || !ok_x) return set_err(ctx, ADSCF_E_ARG, "pass kernel not available for this shape");
   ctx->plan_y = y; ctx->plan_z = z; ctx->plan_x = x;
+  ctx->mx_off = true;
   if (ctx->g_iter) { cudaGraphExecDestroy(ctx->g_iter); ctx->g_iter = nullptr; }
   if (ctx->g_prop) { cudaGraphExecDestroy(ctx->g_prop); ctx->g_prop = nullptr; }
   return ADSCF_OK;

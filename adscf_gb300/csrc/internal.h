@@ -70,6 +70,7 @@ struct adscf_ctx {
   int* d_flags = nullptr;             // device error flags (bounded-wait expiry)
   float2* d_dcin = nullptr;           // fused XY plan: [2][gz] (0,0) pencils entering the z pass, [gz] convolved
   struct BulkMx* mx = nullptr;        // mixed-radix passes (bulk_mx.cuh), null where the register FFT runs
+  bool mx_off = false;                // a pinned pass plan runs the line passes instead
   // kernel per pass of a double step (PK_*), chosen by the autotuner
   int plan_y = PK_PLAIN, plan_z = PK_PLAIN, plan_x = PK_PLAIN;
   int autotune = 1;

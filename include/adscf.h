@@ -258,8 +258,12 @@ ADSCF_API int adscf_set_wait_limit(adscf_ctx *ctx, int polls);
  * the TMA-fed Y and Z passes with the fused plane pass where they exist,
  * else the persistent, else the plain kernels).
  * All plans compute the same arithmetic: results do not depend on the choice.
+ * Grids that run the mixed-radix passes (FP64 but 256^3; FP32 with a line of
+ * 256 points or one that has no register FFT) tune their launch geometry
+ * instead, which changes no operation either.
  * adscf_tuning writes the plan and the per-candidate timings as text;
- * adscf_set_pass_plan pins a plan (ADSCF_E_ARG if unavailable).           */
+ * adscf_set_pass_plan pins a plan of line passes (ADSCF_E_ARG if
+ * unavailable; equal to the mixed-radix passes to rounding).              */
 enum { ADSCF_PASS_PLAIN = 0, ADSCF_PASS_PERSISTENT = 1, ADSCF_PASS_TMA = 2,
        ADSCF_PASS_FUSED = 3 /* x only: one plane pass for Yi + X + Yf */ };
 ADSCF_API int adscf_tuning(const adscf_ctx *ctx, char *buf, int len);

@@ -61,3 +61,20 @@ def test_default_plan_without_the_tuner_agrees(rng, monkeypatch):
             with Context(BULK, grid=grid, size=size, ds=ds, block_length=f, precision=prec) as c:
                 out.append(c.propagate_diblock(w)[0])
     assert np.array_equal(out[0], out[2]) and np.array_equal(out[1], out[3])
+
+
+# FP64 1e-16 and FP32 6e-8 (random over the transforms' operations) per step, 20 steps
+@pytest.mark.parametrize("grid,prec,tol", [((64, 64, 64), FP64, 1e-12), ((128, 64, 32), FP64, 1e-12),
+                                           ((256, 32, 64), FP64, 1e-12), ((256, 32, 32), SPLIT, 2e-6),
+                                           ((32, 256, 64), SPLIT, 2e-6), ((64, 32, 256), SPLIT, 2e-6),
+                                           ((30, 36, 40), SPLIT, 2e-6)])
+def test_against_the_line_passes(rng, grid, prec, tol):
+    """Grids with a register FFT on every axis that run the mixed-radix
+    passes; a pinned plan runs the line passes."""
+    w = rng.standard_normal((2,) + grid[::-1])
+    with Context(BULK, grid=grid, size=(3.7, 4.1, 3.9), ds=0.05, block_length=(0.4, 0.6), precision=prec) as c:
+        a, ra = c.propagate_diblock(w)
+        c.set_pass_plan(0, 0, 0)
+        b, rb = c.propagate_diblock(w)
+    assert abs(ra.Qsum / rb.Qsum - 1.0) < tol
+    assert np.max(np.abs(a - b)) < 5 * tol * np.max(np.abs(b))
