@@ -87,6 +87,11 @@ int mx_freq(const mxk::Axis& A, int p) {
   return k;
 }
 
+// Row pitch of k_mx_b's tile: an odd number of columns, so that the rows of a z
+// stage's lines lie in different banks (256^3 split 409 -> 362 us a double step,
+// 128 x 128 x 256 106 -> 92, 60 x 72 x 100 18.7 -> 17.9).
+int pitch_b(int gz, int mi, int cols) { return (mi > 1 ? gz | 1 : gz) * cols; }
+
 template <typename T>
 size_t bytes_a(const BulkMx* M, int ro) {
   return ((size_t)ro * (M->a[0].n | 1) + M->a[0].n + M->a[1].n) * sizeof(cplx<T>);
@@ -94,7 +99,7 @@ size_t bytes_a(const BulkMx* M, int ro) {
 template <typename T>
 size_t bytes_b(const BulkMx* M, int mi, int cols) {
   const size_t gy = M->a[1].n, gz = M->a[2].n;
-  const size_t tile = (mi * gz * cols + gy + gz) * sizeof(cplx<T>) + 2 * gz * sizeof(T);
+  const size_t tile = (mi * pitch_b((int)gz, mi, cols) + gy + gz) * sizeof(cplx<T>) + 2 * gz * sizeof(T);
   return sizeof(T) == 4 ? std::max(tile, 2 * (gz + 1) * sizeof(float2) + 8 * gz * sizeof(float4)) : tile;
 }
 int outer_rows(const BulkMx* M, int cut) {
@@ -116,6 +121,7 @@ bool geometry(BulkMx* M, int cut, int cols, int cap_a, int cap_b) {
   D.pitch = pitch;
   D.cols = cols;
   for (D.lc = 0; (1 << D.lc) < cols;) ++D.lc;
+  D.pb = pitch_b(gz, mi, cols);
   D.ctiles = (gx + cols - 1) / cols;
   D.ntiles = D.ctiles * ro;
   D.rx = X.nst ? X.rad[0] : 1;
@@ -152,11 +158,11 @@ bool geometry(BulkMx* M, int cut, int cols, int cap_a, int cap_b) {
     S.tw = ro * pitch + gx;
     D.a.s[D.a.n++] = S;
   }
-  const int pts = (mi * gz) << D.lc;          // k_mx_b: tile [y'][z][c]
+  const int pts = mi * D.pb;                  // k_mx_b: tile [y'][z][c]
   for (int s = cut; s < Y.nst; ++s) {         // inner y stages: lines (z, c)
     mxk::Step S = step(Y, s, 1, mi, gz << D.lc);
     S.lmask = cols - 1; S.lsh = D.lc;
-    S.ls = 1; S.ls2 = cols; S.es = gz << D.lc;
+    S.ls = 1; S.ls2 = cols; S.es = D.pb;
     S.gls = 1; S.gls2 = gx * gy; S.ges = gx;
     S.tw = pts;
     D.b.s[D.b.n++] = S;
@@ -164,7 +170,7 @@ bool geometry(BulkMx* M, int cut, int cols, int cap_a, int cap_b) {
   for (int s = 0; s + 1 < Z.nst; ++s) {       // z stages: lines (y', c)
     mxk::Step S = step(Z, s, 1, gz, mi << D.lc);
     S.lmask = cols - 1; S.lsh = D.lc;
-    S.ls = 1; S.ls2 = gz << D.lc; S.es = cols;
+    S.ls = 1; S.ls2 = D.pb; S.es = cols;
     S.gls = 1; S.gls2 = gx; S.ges = gx * gy;
     S.tw = pts + gy;
     D.b.s[D.b.n++] = S;
@@ -390,6 +396,12 @@ int mx_setup(adscf_ctx* ctx, const BulkDev<T>& I, const std::vector<T>& fk, cons
                   cudaDeviceGetAttribute(&M->optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->dev) == cudaSuccess;
   mxk::Dev<T>& D = M->dev<T>();
   D.gx = gx; D.gy = gy; D.gz = gz;
+  // Where the factors, spectrum and node (32 bytes a point) exceed L2, factors
+  // and nodes stream so that the spectrum stays: 256^3 362 -> 352 us a double
+  // step, 160^3 98 -> 93, 128 x 128 x 256 92 -> 85; below, the factors stay too
+  // (64 x 64 x 256 27.7 us, 29.3 streamed).
+  int l2 = 0;
+  if (cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, ctx->dev) == cudaSuccess) D.stream = (size_t)ctx->npts * 32 > (size_t)l2;
   if (!ok || !default_geometry<T>(M, G)) {
     delete M;
     return ADSCF_OK;

@@ -67,6 +67,8 @@ struct Dev {
   int ro, mi;                   // outer rows of a tile (R_o), rows of an inner block (M')
   int pitch;                    // row pitch of k_mx_a's tile (odd)
   int cols, lc, ctiles;         // columns of k_mx_b's tile (a power of two, its log), tiles along x
+  int pb;                       // pitch of its rows, [y'][z][column]
+  int stream;                   // FP32: factors and slices past L2's eviction order
   int ntiles;                   // blocks of columns of k_mx_b (the rest convolve the pencil)
   Prog a, b;                    // steps around the real-space visit / the diffusion factor
   int rx, rz;                   // radices of those visits (1: none)
@@ -234,7 +236,7 @@ __device__ __forceinline__ void mid_r(const Dev<T>& D, cplx<T>* sm, const T* fz,
     const int u = fdiv(t, D.mgz), l = t - u * lines;
     const int c = l & (D.cols - 1), yy = l >> D.lc;
     if (c >= nl) continue;
-    cplx<T>* p = sm + ((yy * gz + u * R) << D.lc) + c;
+    cplx<T>* p = sm + yy * D.pb + ((u * R) << D.lc) + c;
     const T ah = __ldg(fxy + (size_t)yy * D.gx + c);
     T al = (T)0;
     if constexpr (sizeof(T) == 4) al = __ldg(fxy + nxy + (size_t)yy * D.gx + c);
@@ -259,6 +261,17 @@ __device__ __forceinline__ void mid_r(const Dev<T>& D, cplx<T>* sm, const T* fz,
 #pragma unroll
     for (int r = 0; r < R; ++r) p[r << D.lc] = v[r];
   }
+}
+
+// Boltzmann factors of a point
+template <typename T>
+__device__ __forceinline__ EPt<T> load_e(const Dev<T>& D, const T* E, size_t p) {
+  if constexpr (sizeof(T) == 4)
+    if (D.stream) {
+      const float4 v = __ldcs(reinterpret_cast<const float4*>(E) + p);
+      return {v.x, v.y, v.z, v.w};
+    }
+  return load_ept(E, p);
 }
 
 // Last inverse stage of the x rows, node t of both chains and the first
@@ -297,14 +310,15 @@ __device__ __forceinline__ void real_r(const Dev<T>& D, cplx<T>* sm, const T* E,
     }
 #pragma unroll
     for (int r = 0; r < R; ++r) {
-      const EPt<T> ev = load_ept(E, gp + r * Mp);
+      const EPt<T> ev = load_e(D, E, gp + r * Mp);
       if (init) {
         v[r] = mk<T>(fA ? ev.a : ev.b, bA ? ev.a : ev.b);
         sl[gp + r * Mp] = mk<T>((T)1, (T)1);
       } else {
         const cplx<T> q = mk<T>(emul(v[r].x, fA ? ev.a : ev.b, fA ? ev.al : ev.bl),
                                 emul(v[r].y, bA ? ev.a : ev.b, bA ? ev.al : ev.bl));
-        sl[gp + r * Mp] = q;
+        if (sizeof(T) == 4 && D.stream) __stcs(sl + gp + r * Mp, q);
+        else sl[gp + r * Mp] = q;
         v[r] = mk<T>(emul(q.x, fA2 ? ev.a : ev.b, fA2 ? ev.al : ev.bl),
                      emul(q.y, bA2 ? ev.a : ev.b, bA2 ? ev.al : ev.bl));
       }
@@ -461,7 +475,7 @@ k_mx_b(const __grid_constant__ mxk::Dev<T> D) {
   }
   const int k = blockIdx.x / D.ctiles, c0 = (blockIdx.x - k * D.ctiles) << D.lc;
   const int nl = min(D.cols, gx - c0);
-  const int pts = (mi * gz) << D.lc;
+  const int pts = mi * D.pb;
   T* fz = reinterpret_cast<T*>(sm + pts + D.gy + gz);
   if (mi > 1)
     for (int i = threadIdx.x; i < D.gy; i += blockDim.x) sm[pts + i] = D.tw[D.tw_y + i];
@@ -475,7 +489,7 @@ k_mx_b(const __grid_constant__ mxk::Dev<T> D) {
   tmak::pdl_wait();
   __syncthreads();
   if (D.b.n == 0) {
-    for (int e = threadIdx.x; e < pts; e += blockDim.x) {
+    for (int e = threadIdx.x; e < gz << D.lc; e += blockDim.x) {
       const int c = e & (D.cols - 1), zz = e >> D.lc;
       if (c < nl) sm[e] = g[(size_t)zz * nxy + c];
     }
@@ -506,7 +520,7 @@ k_mx_b(const __grid_constant__ mxk::Dev<T> D) {
     if (!dst) __syncthreads();
   }
   if (D.b.n == 0) {
-    for (int e = threadIdx.x; e < pts; e += blockDim.x) {
+    for (int e = threadIdx.x; e < gz << D.lc; e += blockDim.x) {
       const int c = e & (D.cols - 1), zz = e >> D.lc;
       if (c < nl) g[(size_t)zz * nxy + c] = sm[e];
     }
