@@ -14,6 +14,7 @@
 
 #include "internal.h"
 #include "adjoint_kernels.cuh"
+#include "adjoint_mx_host.h"
 
 struct AdjState {
   AdjDev A{};
@@ -34,6 +35,7 @@ struct AdjState {
   double2* seg_spec = nullptr;          // spectrum of the segment runs
   BulkDev<double>* d_seg = nullptr;
   size_t smz2 = 0;                      // generic z pass (two line buffers)
+  AdjMx mx;                             // mixed-radix passes
 };
 
 namespace {
@@ -143,6 +145,7 @@ void adj_destroy(adscf_ctx* ctx) {
   cudaFree(s->ck); cudaFree(s->bufA); cudaFree(s->bufB); cudaFree(s->seg_spec); cudaFree(s->d_seg);
   cudaFree(s->A.sf); cudaFree(s->A.b); cudaFree(s->d_w); cudaFree(s->A.part);
   cudaFree(s->A.sc); cudaFree(s->A.gpart); cudaFree(s->d_inst2);
+  adj_mx_free(&s->mx);
   cudaFree(s->wx); cudaFree(s->wy2); cudaFree(s->wy1); cudaFree(s->wz);
   delete s;
   ctx->adj = nullptr;
@@ -231,13 +234,18 @@ int propagate_ckpt(adscf_ctx* ctx, AdjState* s) {
   return ADSCF_OK;
 }
 
-// the forward pass from the fields already in the adjoint buffer
-int forward_core(adscf_ctx* ctx, double* free_energy, double* sc_out) {
+// the forward pass from the fields already in the adjoint buffer; grad: keep
+// what a backward pass on the mixed-radix passes needs
+int forward_core(adscf_ctx* ctx, double* free_energy, double* sc_out, bool grad) {
   int rc;
   AdjState* s = ctx->adj;
   if ((rc = bulk_enqueue_expfield(ctx, s->d_w))) return rc;
+  if (grad && !ctx->adj_ckpt && (rc = adj_mx_setup(ctx, &s->mx))) return rc;
+  s->mx.kept = grad && !ctx->adj_ckpt && s->mx.keep;
   if (ctx->adj_ckpt) {
     if ((rc = propagate_ckpt(ctx, s))) return rc;
+  } else if (s->mx.kept) {
+    if ((rc = adj_mx_forward(ctx, &s->mx))) return rc;
   } else {
     if ((rc = bulk_enqueue_propagate(ctx))) return rc;
   }
@@ -251,6 +259,22 @@ int forward_core(adscf_ctx* ctx, double* free_energy, double* sc_out) {
   s->gen = ++ctx->prop_gen;
   if (free_energy) *free_energy = sc[ADJ_F];
   if (sc_out) std::memcpy(sc_out, sc, sizeof(sc));
+  return ADSCF_OK;
+}
+
+// the gradient from the stress partials of A
+int read_gradient(adscf_ctx* ctx, const AdjDev& A, double* grad) {
+  k_adj_grad<<<1, 32, 0, ctx->stream>>>(A);
+  CK(cudaGetLastError());
+  double sc[ADJ_NSC];
+  int rc;
+  if ((rc = read_scalars(ctx, sc))) return rc;
+  grad[0] = sc[ADJ_DLX];
+  grad[1] = sc[ADJ_DLY];
+  grad[2] = sc[ADJ_DLZ];
+  grad[3] = sc[ADJ_DCHI];
+  for (int i = 0; i < 4; ++i)
+    if (!std::isfinite(grad[i])) return set_err(ctx, ADSCF_E_NONFINITE, "non-finite adjoint gradient");
   return ADSCF_OK;
 }
 }  // namespace
@@ -271,7 +295,7 @@ int adscf_forward(adscf_ctx* ctx, const double* field, double* free_energy) {
   if ((rc = check_ctx(ctx)) || (rc = adj_setup(ctx))) return rc;
   const size_t nv = 2 * (size_t)ctx->npts;
   if ((rc = h2d(ctx, ctx->adj->d_w, field, nv))) return rc;
-  return forward_core(ctx, free_energy, nullptr);
+  return forward_core(ctx, free_energy, nullptr, true);
 }
 
 int adscf_forward_dev(adscf_ctx* ctx, const double* d_field, double* free_energy) {
@@ -281,7 +305,7 @@ int adscf_forward_dev(adscf_ctx* ctx, const double* d_field, double* free_energy
   if ((rc = check_ctx(ctx)) || (rc = adj_setup(ctx))) return rc;
   const size_t nv = 2 * (size_t)ctx->npts;
   CK(cudaMemcpyAsync(ctx->adj->d_w, d_field, nv * sizeof(double), cudaMemcpyDeviceToDevice, ctx->stream));
-  return forward_core(ctx, free_energy, nullptr);
+  return forward_core(ctx, free_energy, nullptr, true);
 }
 
 // FP64 free energy at the context's current (device-resident) SCF field.  A
@@ -311,7 +335,7 @@ int adscf_free_energy_fp64(adscf_ctx* ctx, adscf_iter_result* out) {
   CK(cudaMemcpyAsync(c64->adj->d_w, field, nv * sizeof(double), cudaMemcpyDeviceToDevice, ctx->stream));
   double sc[ADJ_NSC];
   double F = 0.0;
-  if ((rc = forward_core(c64, &F, sc))) return set_err(ctx, rc, c64->err);
+  if ((rc = forward_core(c64, &F, sc, false))) return set_err(ctx, rc, c64->err);
   *out = adscf_iter_result{};
   out->free_energy = F;
   out->Qsum = c64->dvol * sc[ADJ_S];
@@ -329,6 +353,7 @@ int adscf_set_adjoint_checkpoint(adscf_ctx* ctx, int every) {
   // checkpointed passes never read the context's slices: release them
   if ((rc = bulk_hold_slices(ctx, every == 0))) return rc;
   AdjState* s = ctx->adj;
+  if (every) adj_mx_free(&s->mx);
   s->A.I.slices = ctx->hb64.slices;
   s->A.slA = s->A.slB = ctx->hb64.slices;
   BulkDev<double> two[2] = {s->A.I, s->A.I};
@@ -358,6 +383,12 @@ int adscf_backward(adscf_ctx* ctx, double* grad) {
     return set_err(ctx, ADSCF_E_STATE, "adscf_backward needs the state of an immediately preceding adscf_forward");
   AdjDev A = s->A;
   cudaStream_t st = ctx->stream;
+  if (s->mx.kept) {
+    if ((rc = adj_mx_backward(ctx, &s->mx, A.b, A.sc))) return rc;
+    A.gpart = s->mx.gpart;
+    A.nztiles = s->mx.ntiles;
+    return read_gradient(ctx, A, grad);
+  }
   const double2* tw = static_cast<const double2*>(ctx->d_tw);
   const double* fk = static_cast<const double*>(ctx->d_fk);
   const double2* tw64 = static_cast<const double2*>(ctx->d_tw64);
@@ -389,17 +420,7 @@ int adscf_backward(adscf_ctx* ctx, double* grad) {
       k_bulk_strided<double><<<s->nwy1, BULK_THREADS, s->smy, st>>>(s->d_inst2, s->wy1, tw, fk, tw64,
                                                                      ctx->d_g64, t, 1);
   }
-  k_adj_grad<<<1, 32, 0, st>>>(A);
-  CK(cudaGetLastError());
-  double sc[ADJ_NSC];
-  if ((rc = read_scalars(ctx, sc))) return rc;
-  grad[0] = sc[ADJ_DLX];
-  grad[1] = sc[ADJ_DLY];
-  grad[2] = sc[ADJ_DLZ];
-  grad[3] = sc[ADJ_DCHI];
-  for (int i = 0; i < 4; ++i)
-    if (!std::isfinite(grad[i])) return set_err(ctx, ADSCF_E_NONFINITE, "non-finite adjoint gradient");
-  return ADSCF_OK;
+  return read_gradient(ctx, A, grad);
 }
 
 }  // extern "C"

@@ -454,3 +454,17 @@ void mx_step(adscf_ctx* ctx, int t) {
   else step_t<double>(ctx, t);
 }
 int mx_tune(adscf_ctx* ctx) { return ctx->prec == ADSCF_SPLIT ? tune_t<float>(ctx) : tune_t<double>(ctx); }
+
+bool mx_launch64(const adscf_ctx* ctx, MxLaunch64& L) {
+  const BulkMx* M = ctx->mx;
+  if (!M || ctx->mx_off || ctx->prec != ADSCF_FP64) return false;
+  L = MxLaunch64{M->d64, M->thr_a, M->thr_b, M->grid_a, M->grid_b, M->sm_a, M->sm_b, M->optin};
+  L.D.slices = ctx->hb64.slices;
+  L.D.I = static_cast<const BulkDev<double>*>(ctx->d_inst);
+  return true;
+}
+void mx_freqs(const adscf_ctx* ctx, std::vector<int>& f) {
+  f.clear();
+  for (const mxk::Axis& A : ctx->mx->a)
+    for (int p = 0; p < A.n; ++p) f.push_back(mx_freq(A, p));
+}

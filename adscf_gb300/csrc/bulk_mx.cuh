@@ -35,7 +35,11 @@
 // fewer points than lanes take small radices, which leave every quarter a
 // short program.
 #pragma once
+#include <vector>
+
 #include "bulk_tma.cuh"
+
+struct adscf_ctx;
 
 namespace mxk {
 
@@ -224,12 +228,24 @@ __device__ __forceinline__ void stage_r(const Step& S, cplx<T>* sm, int tile_j, 
   }
 }
 
+// What the visit of the diffusion factor does besides, for the adjoint: the
+// forward pass keeps its spectra (kStore), the reverse pass adds Re(conj(kept)
+// spectrum) up per frequency (kDot).  Both lie in tile order: point (row yy,
+// position zp, column c) of a block at ((zp M' + yy) cols + c).
+enum { kPlain = 0, kStore = 1, kDot = 2 };
+template <typename T>
+struct Side {
+  cplx<T>* keep;                // the block's part of the kept spectrum
+  double* dot;                  // and of the sums
+};
+
 // Last forward stage, diffusion factor and first inverse stage of the z lines
 // in one visit of the points (both stages have M = R, no twiddles).  Lines
 // (row yy of the block, column c); fz: the g_z / N factors by position (hi
 // [n], lo [n]); fxy: the tile's g_xy (rows gx apart, lo parts at + nxy).
-template <typename T, int R>
-__device__ __forceinline__ void mid_r(const Dev<T>& D, cplx<T>* sm, const T* fz, const T* fxy, int nl) {
+template <typename T, int R, int MODE = kPlain>
+__device__ __forceinline__ void mid_r(const Dev<T>& D, cplx<T>* sm, const T* fz, const T* fxy, int nl,
+                                      const Side<T>& sd = Side<T>{}) {
   const int gz = D.gz, lines = D.mi << D.lc, nxy = D.gx * D.gy;
   const int total = gz / R * lines;
   for (int t = threadIdx.x; t < total; t += blockDim.x) {
@@ -244,6 +260,18 @@ __device__ __forceinline__ void mid_r(const Dev<T>& D, cplx<T>* sm, const T* fz,
 #pragma unroll
     for (int r = 0; r < R; ++r) v[r] = p[r << D.lc];
     if constexpr (R > 1) dft<T, R>(v, +1);
+    if constexpr (MODE != kPlain) {
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        const size_t at = (size_t)(((u * R + r) * D.mi + yy) << D.lc) + c;
+        if constexpr (MODE == kStore) {
+          sd.keep[at] = v[r];
+        } else {
+          const cplx<T> f = sd.keep[at];
+          sd.dot[at] += f.x * v[r].x + f.y * v[r].y;
+        }
+      }
+    }
 #pragma unroll
     for (int r = 0; r < R; ++r) {
       const T bh = fz[u * R + r];
@@ -425,9 +453,8 @@ k_mx_a(const __grid_constant__ mxk::Dev<T> D, int t) {
 // output of the FP32 (0, 0) pencil per warp.  Shared memory: M' gz cols + gy
 // + gz points and 2 gz factors.
 // ---------------------------------------------------------------------------
-template <typename T, int BT>
-__global__ void __launch_bounds__(BT, BT == 512 ? 1 : sizeof(T) == 4 ? 3 : 2)
-k_mx_b(const __grid_constant__ mxk::Dev<T> D) {
+template <typename T, int MODE>
+__device__ __forceinline__ void mx_b_body(const mxk::Dev<T>& D, const mxk::Side<T>& sd) {
   extern __shared__ __align__(16) unsigned char smraw[];
   cplx<T>* sm = reinterpret_cast<cplx<T>*>(smraw);
   const int gx = D.gx, gz = D.gz, mi = D.mi, nxy = gx * D.gy;
@@ -504,9 +531,9 @@ k_mx_b(const __grid_constant__ mxk::Dev<T> D) {
     __syncthreads();
   }
   if (D.rz == 1) {
-    mxk::mid_r<T, 1>(D, sm, fz, fxy, nl);
+    mxk::mid_r<T, 1, MODE>(D, sm, fz, fxy, nl, sd);
   } else {
-#define ADSCF_MX_CALL(R_) mxk::mid_r<T, R_>(D, sm, fz, fxy, nl)
+#define ADSCF_MX_CALL(R_) mxk::mid_r<T, R_, MODE>(D, sm, fz, fxy, nl, sd)
     ADSCF_MX_SWITCH(D.rz, ADSCF_MX_CALL)
 #undef ADSCF_MX_CALL
   }
@@ -526,3 +553,18 @@ k_mx_b(const __grid_constant__ mxk::Dev<T> D) {
     }
   }
 }
+template <typename T, int BT>
+__global__ void __launch_bounds__(BT, BT == 512 ? 1 : sizeof(T) == 4 ? 3 : 2)
+k_mx_b(const __grid_constant__ mxk::Dev<T> D) {
+  mx_b_body<T, mxk::kPlain>(D, mxk::Side<T>{});
+}
+
+// Plan of a context for launches from another file
+struct MxLaunch64 {
+  mxk::Dev<double> D;
+  int thr_a, thr_b, grid_a, grid_b;
+  size_t sm_a, sm_b;
+  int optin;
+};
+bool mx_launch64(const adscf_ctx* ctx, MxLaunch64& L);   // false: the context does not run these passes
+void mx_freqs(const adscf_ctx* ctx, std::vector<int>& f);   // frequency by position, x then y then z
