@@ -88,7 +88,7 @@ k_mx_adj_a(const __grid_constant__ mxk::Dev<double> D, const double* __restrict_
            int t) {
   extern __shared__ __align__(16) unsigned char smraw[];
   double2* sm = reinterpret_cast<double2*>(smraw);
-  const BulkDev<double>& I = *D.I;
+  const BulkDev<double>& I = *D.io.I;
   const int gx = D.gx, ro = D.ro, mi = D.mi;
   const int z = blockIdx.x / mi, j = blockIdx.x - z * mi;
   const size_t base = ((size_t)z * D.gy + j) * gx, rs = (size_t)mi * gx;
@@ -105,9 +105,9 @@ k_mx_adj_a(const __grid_constant__ mxk::Dev<double> D, const double* __restrict_
   const float2 wt = node_weights(I, t), wu = node_weights(I, u);
   const mxk::Seeds c{I.ds * (double)wt.x, I.ds * (double)wt.y, I.ds * (double)wu.x, I.ds * (double)wu.y,
                      first ? sc[ADJ_AS] : 0.0};
-  const double2* sl = D.slices + (size_t)u * (size_t)I.npts + base;
-  const double* E = D.E + base * 2;
-  double2* g = D.spec + base;
+  const double2* sl = D.io.slices + (size_t)u * (size_t)I.npts + base;
+  const double* E = D.io.E + base * 2;
+  double2* g = D.io.spec + base;
   __syncthreads();
   if (!first) {
     for (int r = 0; r < ro; ++r) {   // the tile's factors on their way to L1
@@ -152,7 +152,7 @@ template <int BT, int MODE>
 __global__ void __launch_bounds__(BT, BT == 512 ? 1 : 2)
 k_mx_b_side(const __grid_constant__ mxk::Dev<double> D, double2* keep, double* dot, int tile) {
   const size_t at = (size_t)blockIdx.x * tile;
-  mx_b_body<double, MODE>(D, mxk::Side<double>{keep + at, dot ? dot + at : nullptr});
+  mx_b_body<double, MODE>(D, D.io, mxk::Side<double>{keep + at, dot ? dot + at : nullptr});
 }
 
 // Block sums of k_c^2 G(k) / M W(k) for c = x, y, z into gpart[block][3];
@@ -168,7 +168,7 @@ k_mx_adj_sum(const __grid_constant__ mxk::Dev<double> D, const double* __restric
   for (int e = threadIdx.x; e < tile; e += blockDim.x) {
     const int x = c0 + (e & (D.cols - 1)), r = e >> D.lc, zp = r / mi, y = k * mi + r - zp * mi;
     if (x >= gx) continue;
-    const double v = w[e] * (D.fk[(size_t)y * gx + x] * D.fk[2 * (size_t)gx * gy + zp]);
+    const double v = w[e] * (D.io.fk[(size_t)y * gx + x] * D.io.fk[2 * (size_t)gx * gy + zp]);
     acc[0] += v * adj_k2(frq[x], gx, lx);
     acc[1] += v * adj_k2(frq[gx + y], gy, ly);
     acc[2] += v * adj_k2(frq[gx + gy + zp], D.gz, lz);

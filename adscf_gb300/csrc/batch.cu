@@ -9,10 +9,13 @@
 // on its contour (work lists sorted by Ns, so the active tiles of step t are
 // a prefix), one contour launch, and batched closure / Anderson solve / mix
 // launches with each instance's mixing history on the device.  One batch
-// iteration is one CUDA graph.  Instances are grouped by pass kernel: cubic
-// grids of 32..256 points run the register-FFT passes of bulk_reg.cuh, every
-// other grid of 2, 3 and 5 factors the generic mixed-radix passes of
-// bulk_kernels.cuh; each group has its own Ns-sorted work lists and launches.
+// iteration is one CUDA graph.  The chains run the mixed-radix passes grid by
+// grid (batch_mx.cu); ADSCF_BATCH_SWEEP=1, more than 64 different grids and
+// lines past 1024 points take the persistent sweep of the line passes, and
+// ADSCF_BATCH_SWEEP=0 those passes launch by launch: there instances are
+// grouped by pass kernel, cubic grids of 24..256 points on the register-FFT
+// passes of bulk_reg.cuh, every other grid of 2, 3 and 5 factors on the generic
+// passes of bulk_kernels.cuh, each group with its own Ns-sorted work lists.
 //
 // Film batches (Film_CK_AD/Film_1D, Brush_CK_AD: one z line per film with its
 // own graded mesh, adaptive contour and wall potential) sweep every film's
@@ -32,6 +35,7 @@
 #include <vector>
 
 #include "internal.h"
+#include "batch_mx.h"
 #include "bulk_host.h"
 #include "bulk_reg.cuh"
 #include "film_host.h"
@@ -81,6 +85,7 @@ struct adscf_batch {
   int sweep_grid = 0;
   int sweep_help = 0;                   // class with the most point-steps (finished CTAs help it)
   size_t sweep_smem = 0;
+  struct BatchMx* mx = nullptr;         // mixed-radix passes (batch_mx.cu), null where the sweep runs
   bool sweep = true;                    // persistent sweeps (ADSCF_BATCH_SWEEP=0: one launch per pass)
   int sweep_tiles = 8;                  // tiles per sweep item (ADSCF_SWEEP_TILES)
   cudaGraphExec_t g_iter = nullptr;
@@ -519,7 +524,17 @@ int build(adscf_batch* b) {
   // as the work lists
   {
     if (const char* e = std::getenv("ADSCF_SWEEP_TILES")) b->sweep_tiles = std::max(1, std::min(64, std::atoi(e)));
-    if (const char* e = std::getenv("ADSCF_BATCH_SWEEP")) b->sweep = std::atoi(e) != 0;
+    const char* pin = std::getenv("ADSCF_BATCH_SWEEP");
+    if (pin) b->sweep = std::atoi(pin) != 0;
+    if (!pin) {   // a batch of any size: one 64^3 split grid 3.3 ms an iteration, 19 in the sweep
+      std::vector<BatchMxInst> in(n);
+      for (int i = 0; i < n; ++i) {
+        const BulkDev<T>& d = I[i];
+        in[i] = BatchMxInst{d.gx, d.gy, d.gz, d.ns, static_cast<const BulkDev<T>*>(b->d_inst) + i, d.spec, d.slices, d.E,
+                            fk.data() + d.gxy_off, g64.data() + d.g64_off};
+      }
+      b->mx = batch_mx_create<T>(b->dev, in);
+    }
     std::vector<int> tx(n), ty(n), tz(n), before(n, 0);
     for (int i = 0; i < n; ++i) {
       const BulkDev<T>& d = I[i];
@@ -932,6 +947,13 @@ int enqueue_propagation(adscf_batch* b) {
   cudaStream_t s = b->stream;
   const XAux none{nullptr, nullptr, nullptr};
   const double* g64 = b->d_g64;
+  if (b->mx) {
+    std::string why;
+    if (batch_mx_enqueue(b->mx, s, why)) return berr(b, ADSCF_E_CUDA, "batch passes: " + why);
+    k_bulk_contour<T><<<dim3(b->cont_blocks, b->n), BULK_THREADS, 0, s>>>(d);
+    BK(cudaGetLastError());
+    return ADSCF_OK;
+  }
   // one launch per kernel class and pass; a class with no instance left on
   // its contour at step t launches nothing
   auto xpass = [&](const adscf_batch::PassClass& C, int grid, int t, int mode) {
@@ -1437,6 +1459,7 @@ int adscf_batch_destroy(adscf_batch* b) {
   if (!b) return ADSCF_OK;
   if (b->stream) cudaStreamSynchronize(b->stream);
   batch_adj_destroy(b);
+  batch_mx_destroy(b->mx);
   if (b->g_iter) cudaGraphExecDestroy(b->g_iter);
   cudaFree(b->pool); cudaFree(b->d_inst); cudaFree(b->d_S);
   cudaFree(b->d_tw); cudaFree(b->d_fk); cudaFree(b->d_g64);
@@ -1528,6 +1551,7 @@ int adscf_batch_launches(const adscf_batch* b) {
     }
     return k;
   }
+  if (b->mx) return 4 + batch_mx_launches(b->mx);
   if (b->sweep) return 5;   // sweep, contour, closure, solve, mix (and a memset of the counters)
   int k = 4;   // contour, closure, solve, mix
   for (const auto& C : b->cls) {

@@ -65,6 +65,19 @@ struct Prog {
   Step s[kMaxSteps];            // in forward order
 };
 
+// Arrays of one context
+template <typename T>
+struct Io {
+  const T* fk;                  // by position: g_xy hi, lo [gy gx] each, g_z / N hi, lo [gz] each
+  const BulkDev<T>* I;
+  cplx<T>* spec;
+  cplx<T>* slices;
+  const T* E;
+  float2* dcin;                 // [gz][gy] FP32 kx = 0 entries of the rows before the y and z transforms
+  float2* dcout;                // [gz] the pencil convolved by the z pass
+  const float2* dcc;            // [gz] its kernel, (hi, lo)
+};
+
 template <typename T>
 struct Dev {
   int gx, gy, gz;
@@ -80,14 +93,7 @@ struct Dev {
   unsigned mgj, mgz;            // divisions by gx / rx, and by the z lines of a tile
   int tw_x, tw_y, tw_z;         // twiddle tables in `tw`
   const cplx<T>* tw;
-  const T* fk;                  // by position: g_xy hi, lo [gy gx] each, g_z / N hi, lo [gz] each
-  const BulkDev<T>* I;
-  cplx<T>* spec;
-  cplx<T>* slices;
-  const T* E;
-  float2* dcin;                 // [gz][gy] FP32 kx = 0 entries of the rows before the y and z transforms
-  float2* dcout;                // [gz] the pencil convolved by the z pass
-  const float2* dcc;            // [gz] its kernel, (hi, lo)
+  Io<T> io;
 };
 
 __host__ __device__ __forceinline__ unsigned div_magic(int d) {
@@ -373,11 +379,10 @@ __device__ __forceinline__ void real_r(const Dev<T>& D, cplx<T>* sm, const T* E,
 // chains: slice 0 = (1, 1).  Shared memory: R_o pitch + gx + gy points.
 // ---------------------------------------------------------------------------
 template <typename T>
-__global__ void __launch_bounds__(128, sizeof(T) == 4 ? 6 : 4)
-k_mx_a(const __grid_constant__ mxk::Dev<T> D, int t) {
+__device__ __forceinline__ void mx_a_body(const mxk::Dev<T>& D, const mxk::Io<T>& io, int t) {
   extern __shared__ __align__(16) unsigned char smraw[];
   cplx<T>* sm = reinterpret_cast<cplx<T>*>(smraw);
-  const BulkDev<T>& I = *D.I;
+  const BulkDev<T>& I = *io.I;
   const int gx = D.gx, ro = D.ro, mi = D.mi;
   const int z = blockIdx.x / mi, j = blockIdx.x - z * mi;
   const size_t base = ((size_t)z * D.gy + j) * gx;
@@ -395,13 +400,13 @@ k_mx_a(const __grid_constant__ mxk::Dev<T> D, int t) {
   const unsigned f = (chain_type_fwd(I, tt) == 0 ? 1u : 0u) | (chain_type_bwd(I, tt) == 0 ? 2u : 0u) |
                      (chain_type_fwd(I, t + 1) == 0 ? 4u : 0u) | (chain_type_bwd(I, t + 1) == 0 ? 8u : 0u) |
                      (more ? 16u : 0u);
-  cplx<T>* sl = D.slices + (size_t)t * (size_t)I.npts + base;
-  const T* E = D.E + base * (sizeof(T) == 4 ? 4 : 2);
-  cplx<T>* g = D.spec + base;
+  cplx<T>* sl = io.slices + (size_t)t * (size_t)I.npts + base;
+  const T* E = io.E + base * (sizeof(T) == 4 ? 4 : 2);
+  cplx<T>* g = io.spec + base;
   // the x step where a row's kx = 0 entry is complete (none: the real visit)
   const int xs = sizeof(T) == 4 ? D.nxs - 1 : -2;
-  float2* dci = sizeof(T) == 4 ? D.dcin + (size_t)z * D.gy + j : nullptr;
-  float2* dco = sizeof(T) == 4 ? D.dcout + z : nullptr;
+  float2* dci = sizeof(T) == 4 ? io.dcin + (size_t)z * D.gy + j : nullptr;
+  float2* dco = sizeof(T) == 4 ? io.dcout + z : nullptr;
   tmak::pdl_wait();
   __syncthreads();
   if (t > 0) {
@@ -447,6 +452,18 @@ k_mx_a(const __grid_constant__ mxk::Dev<T> D, int t) {
   }
 }
 
+template <typename T>
+__global__ void __launch_bounds__(128, sizeof(T) == 4 ? 6 : 4)
+k_mx_a(const __grid_constant__ mxk::Dev<T> D, int t) {
+  mx_a_body<T>(D, D.io, t);
+}
+// contexts blockIdx.y of a batch that share D's grid
+template <typename T>
+__global__ void __launch_bounds__(128, sizeof(T) == 4 ? 6 : 4)
+k_mx_a_b(const __grid_constant__ mxk::Dev<T> D, const mxk::Io<T>* __restrict__ ios, int t) {
+  mx_a_body<T>(D, ios[blockIdx.y], t);
+}
+
 // ---------------------------------------------------------------------------
 // Diffusion pass of the row block k (positions [k M', (k + 1) M') of y) and a
 // tile of `cols` columns: block k ctiles + tile.  Blocks from ntiles on: one
@@ -454,7 +471,7 @@ k_mx_a(const __grid_constant__ mxk::Dev<T> D, int t) {
 // + gz points and 2 gz factors.
 // ---------------------------------------------------------------------------
 template <typename T, int MODE>
-__device__ __forceinline__ void mx_b_body(const mxk::Dev<T>& D, const mxk::Side<T>& sd) {
+__device__ __forceinline__ void mx_b_body(const mxk::Dev<T>& D, const mxk::Io<T>& io, const mxk::Side<T>& sd) {
   extern __shared__ __align__(16) unsigned char smraw[];
   cplx<T>* sm = reinterpret_cast<cplx<T>*>(smraw);
   const int gx = D.gx, gz = D.gz, mi = D.mi, nxy = gx * D.gy;
@@ -463,7 +480,7 @@ __device__ __forceinline__ void mx_b_body(const mxk::Dev<T>& D, const mxk::Side<
     if ((int)blockIdx.x >= D.ntiles) {
       float2* in = reinterpret_cast<float2*>(smraw);
       float2* c = in + ((gz + 1) & ~1);
-      for (int i = threadIdx.x; i < gz; i += blockDim.x) c[i] = D.dcc[i];
+      for (int i = threadIdx.x; i < gz; i += blockDim.x) c[i] = io.dcc[i];
       tmak::pdl_wait();
       // row sums in float-float, eight threads per plane (rows y = k, k + 8,
       // ... each, then over k): many loads are in flight
@@ -471,7 +488,7 @@ __device__ __forceinline__ void mx_b_body(const mxk::Dev<T>& D, const mxk::Side<
       float4* part = reinterpret_cast<float4*>(c + ((gz + 1) & ~1));
       for (int i = threadIdx.x; i < gz * kParts; i += blockDim.x) {
         float xh = 0.f, xl = 0.f, yh = 0.f, yl = 0.f;
-        const float2* row = D.dcin + (size_t)(i / kParts) * D.gy;
+        const float2* row = io.dcin + (size_t)(i / kParts) * D.gy;
 #pragma unroll 4
         for (int y = i % kParts; y < D.gy; y += kParts) {
           const float2 v = row[y];
@@ -495,7 +512,7 @@ __device__ __forceinline__ void mx_b_body(const mxk::Dev<T>& D, const mxk::Side<
       const int z = ((int)blockIdx.x - D.ntiles) * (blockDim.x >> 5) + (threadIdx.x >> 5);
       if (z < gz) {
         const float2 o = tmak::dc_point(in, c, gz, z);
-        if ((threadIdx.x & 31) == 0) D.dcout[z] = o;
+        if ((threadIdx.x & 31) == 0) io.dcout[z] = o;
       }
       return;
     }
@@ -508,11 +525,11 @@ __device__ __forceinline__ void mx_b_body(const mxk::Dev<T>& D, const mxk::Side<
     for (int i = threadIdx.x; i < D.gy; i += blockDim.x) sm[pts + i] = D.tw[D.tw_y + i];
   for (int i = threadIdx.x; i < gz; i += blockDim.x) sm[pts + D.gy + i] = D.tw[D.tw_z + i];
   {
-    const T* gzt = D.fk + 2 * (size_t)nxy;
+    const T* gzt = io.fk + 2 * (size_t)nxy;
     for (int i = threadIdx.x; i < 2 * gz; i += blockDim.x) fz[i] = gzt[i];
   }
-  cplx<T>* g = D.spec + (size_t)k * mi * gx + c0;
-  const T* fxy = D.fk + (size_t)k * mi * gx + c0;
+  cplx<T>* g = io.spec + (size_t)k * mi * gx + c0;
+  const T* fxy = io.fk + (size_t)k * mi * gx + c0;
   tmak::pdl_wait();
   __syncthreads();
   if (D.b.n == 0) {
@@ -556,7 +573,12 @@ __device__ __forceinline__ void mx_b_body(const mxk::Dev<T>& D, const mxk::Side<
 template <typename T, int BT>
 __global__ void __launch_bounds__(BT, BT == 512 ? 1 : sizeof(T) == 4 ? 3 : 2)
 k_mx_b(const __grid_constant__ mxk::Dev<T> D) {
-  mx_b_body<T, mxk::kPlain>(D, mxk::Side<T>{});
+  mx_b_body<T, mxk::kPlain>(D, D.io, mxk::Side<T>{});
+}
+template <typename T, int BT>
+__global__ void __launch_bounds__(BT, BT == 512 ? 1 : sizeof(T) == 4 ? 3 : 2)
+k_mx_b_b(const __grid_constant__ mxk::Dev<T> D, const mxk::Io<T>* __restrict__ ios) {
+  mx_b_body<T, mxk::kPlain>(D, ios[blockIdx.y], mxk::Side<T>{});
 }
 
 // Plan of a context for launches from another file

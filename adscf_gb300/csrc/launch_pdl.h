@@ -8,10 +8,10 @@
 // the previous kernel on the stream finishes; the TMA passes wait for it
 // (griddepcontrol.wait) before they touch its output.
 template <typename... KArgs, typename... Args>
-inline void launch_pdl(void (*kern)(KArgs...), int grid, int block, size_t smem, cudaStream_t s,
+inline void launch_pdl(void (*kern)(KArgs...), dim3 grid, int block, size_t smem, cudaStream_t s,
                 Args&&... args) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
+  cfg.gridDim = grid;
   cfg.blockDim = dim3(block);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
