@@ -78,7 +78,8 @@ int adj_mx_backward(adscf_ctx* ctx, AdjMx* X, const double* b, const double* sc)
     k_mx_adj_a<<<L.grid_a, L.thr_a, L.sm_a, s>>>(L.D, b, sc, t);
     step_b<mxk::kDot>(L, X->keep + (size_t)(t - 1) * X->pts, X->dot, X->tile, s);
   }
-  k_mx_adj_sum<<<X->ntiles, 256, 0, s>>>(L.D, X->dot, X->frq, X->tile, ctx->p.sizex, ctx->p.sizey, ctx->p.sizez,
+  k_mx_adj_sum<<<X->ntiles, 256, 0, s>>>(L.D, X->dot, X->frq, X->tile, L.yz, ctx->p.sizex,
+                                         L.yz ? ctx->p.sizez : ctx->p.sizey, L.yz ? ctx->p.sizey : ctx->p.sizez,
                                          X->gpart);
   CK(cudaGetLastError());
   return ADSCF_OK;

@@ -156,10 +156,11 @@ k_mx_b_side(const __grid_constant__ mxk::Dev<double> D, double2* keep, double* d
 }
 
 // Block sums of k_c^2 G(k) / M W(k) for c = x, y, z into gpart[block][3];
-// frq: frequency by position (x, then y, then z)
+// frq: frequency by position (x, then y, then z); yz: D's y axis is the grid's z
+// axis, lx, ly, lz are D's
 static __global__ void __launch_bounds__(256)
 k_mx_adj_sum(const __grid_constant__ mxk::Dev<double> D, const double* __restrict__ dot, const int* __restrict__ frq,
-             int tile, double lx, double ly, double lz, double* __restrict__ gpart) {
+             int tile, bool yz, double lx, double ly, double lz, double* __restrict__ gpart) {
   __shared__ double red[3 * 32];
   const int gx = D.gx, gy = D.gy, mi = D.mi;
   const int k = blockIdx.x / D.ctiles, c0 = (blockIdx.x - k * D.ctiles) << D.lc;
@@ -174,5 +175,5 @@ k_mx_adj_sum(const __grid_constant__ mxk::Dev<double> D, const double* __restric
     acc[2] += v * adj_k2(frq[gx + gy + zp], D.gz, lz);
   }
   const double s = block_reduce_k<3>(acc, red);
-  if (threadIdx.x < 3) gpart[blockIdx.x * 3 + threadIdx.x] = s;
+  if (threadIdx.x < 3) gpart[blockIdx.x * 3 + (yz && threadIdx.x ? 3 - threadIdx.x : threadIdx.x)] = s;
 }

@@ -144,7 +144,17 @@ template <typename T>
 int mx_factors(adscf_ctx* ctx, const std::vector<T>& fk, const std::vector<double>& g64) {
   BulkMx* M = ctx->mx;
   const int gz = ctx->gz;
-  const std::vector<T> out = mx_table<T>(M, fk.data());
+  std::vector<T> out;
+  if (M->yz) {   // g_xy g_z of the rows, and a z axis of one point
+    const size_t gx = ctx->gx, nxy = gx * gz;
+    std::vector<T> f(2 * nxy + 2, (T)0);
+    for (size_t z = 0; z < (size_t)gz; ++z)
+      for (size_t x = 0; x < gx; ++x) f[z * gx + x] = fk[x] * fk[2 * gx + z];
+    f[2 * nxy] = (T)1;
+    out = mx_table<T>(M, f.data());
+  } else {
+    out = mx_table<T>(M, fk.data());
+  }
   CK(cudaMemcpy(M->d_fk, out.data(), out.size() * sizeof(T), cudaMemcpyHostToDevice));
   if (sizeof(T) == 4) {
     std::vector<float2> c(gz);
@@ -169,21 +179,29 @@ template <typename T>
 int mx_setup(adscf_ctx* ctx, const BulkDev<T>& I, const std::vector<T>& fk, const std::vector<double>& g64) {
   BulkMx* M = new (std::nothrow) BulkMx();
   if (!M) return set_err(ctx, ADSCF_E_OOM, "mixed-radix plan");
-  const int gx = ctx->gx, gy = ctx->gy, gz = ctx->gz;
   const int rmax = sizeof(T) == 4 ? 16 : std::max(5, std::min(16, ctx->npts / 19456));
   Geom G;
-  const bool ok = mx_axis(gx, rmax, M->a[0]) && mx_axis(gy, rmax, M->a[1]) && mx_axis(gz, rmax, M->a[2]) &&
-                  M->a[0].nst + M->a[1].nst <= mxk::kMaxSteps && M->a[1].nst + M->a[2].nst <= mxk::kMaxSteps &&
-                  cudaDeviceGetAttribute(&M->optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->dev) == cudaSuccess;
   mxk::Dev<T>& D = M->dev<T>();
-  D.gx = gx; D.gy = gy; D.gz = gz;
+  auto plan = [&](int gx, int gy, int gz) {
+    D.gx = gx; D.gy = gy; D.gz = gz;
+    return mx_axis(gx, rmax, M->a[0]) && mx_axis(gy, rmax, M->a[1]) && mx_axis(gz, rmax, M->a[2]) &&
+           M->a[0].nst + M->a[1].nst <= mxk::kMaxSteps && M->a[1].nst + M->a[2].nst <= mxk::kMaxSteps &&
+           default_geometry<T>(M, G);
+  };
+  bool ok = cudaDeviceGetAttribute(&M->optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->dev) == cudaSuccess;
+  // FP64 grids of one y row take z for y, the axis that is cut between the
+  // passes: one block of rows and one of columns would each hold whole lines (64
+  // x 1 x 300 27 us a double step).  FP32 keeps its (0, 0) pencil along z.
+  M->yz = sizeof(T) == 8 && ctx->gy == 1 && ctx->gz > 1 && ok && plan(ctx->gx, ctx->gz, 1);
+  if (!M->yz) ok = ok && plan(ctx->gx, ctx->gy, ctx->gz);
+  const int gx = D.gx, gy = D.gy, gz = D.gz;
   // Where the factors, spectrum and node (32 bytes a point) exceed L2, factors
   // and nodes stream so that the spectrum stays: 256^3 362 -> 352 us a double
   // step, 160^3 98 -> 93, 128 x 128 x 256 92 -> 85; below, the factors stay too
   // (64 x 64 x 256 27.7 us, 29.3 streamed).
   int l2 = 0;
   if (cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, ctx->dev) == cudaSuccess) D.stream = (size_t)ctx->npts * 32 > (size_t)l2;
-  if (!ok || !default_geometry<T>(M, G)) {
+  if (!ok) {
     delete M;
     return ADSCF_OK;
   }
@@ -239,7 +257,7 @@ int mx_tune(adscf_ctx* ctx) { return ctx->prec == ADSCF_SPLIT ? tune_t<float>(ct
 bool mx_launch64(const adscf_ctx* ctx, MxLaunch64& L) {
   const BulkMx* M = ctx->mx;
   if (!M || ctx->mx_off || ctx->prec != ADSCF_FP64) return false;
-  L = MxLaunch64{M->d64, M->thr_a, M->thr_b, M->grid_a, M->grid_b, M->sm_a, M->sm_b, M->optin};
+  L = MxLaunch64{M->d64, M->yz, M->thr_a, M->thr_b, M->grid_a, M->grid_b, M->sm_a, M->sm_b, M->optin};
   L.D.io.slices = ctx->hb64.slices;
   L.D.io.I = static_cast<const BulkDev<double>*>(ctx->d_inst);
   return true;

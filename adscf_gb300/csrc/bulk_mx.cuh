@@ -584,6 +584,7 @@ k_mx_b_b(const __grid_constant__ mxk::Dev<T> D, const mxk::Io<T>* __restrict__ i
 // Plan of a context for launches from another file
 struct MxLaunch64 {
   mxk::Dev<double> D;
+  bool yz;                      // D's y axis is the grid's z axis
   int thr_a, thr_b, grid_a, grid_b;
   size_t sm_a, sm_b;
   int optin;

@@ -17,6 +17,7 @@ struct BulkMx {
   void* d_fk = nullptr;         // diffusion factors by position (T)
   float2* d_dc = nullptr;       // dcin [gz][gy], dcout [gz], kernel [gz]
   int optin = 0;                // opt-in shared memory per block
+  bool yz = false;              // the grid's z axis is the passes' y axis
   template <typename T> mxk::Dev<T>& dev();
   mxk::Dev<float> d32{};
   mxk::Dev<double> d64{};
