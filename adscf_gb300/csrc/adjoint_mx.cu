@@ -59,10 +59,10 @@ void adj_mx_free(AdjMx* X) {
 int adj_mx_forward(adscf_ctx* ctx, AdjMx* X) {
   MxLaunch64 L;
   if (!mx_launch64(ctx, L)) return set_err(ctx, ADSCF_E_STATE, "adjoint passes");
-  mx_real(ctx, 0);
+  mx_real_plain(ctx, 0);
   for (int t = 1; t <= ctx->ns; ++t) {
     step_b<mxk::kStore>(L, X->keep + (size_t)(t - 1) * X->pts, nullptr, X->tile, ctx->stream);
-    mx_real(ctx, t);
+    mx_real_plain(ctx, t);
   }
   CK(cudaGetLastError());
   return bulk_enqueue_contour(ctx);

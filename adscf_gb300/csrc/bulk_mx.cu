@@ -12,25 +12,35 @@
 
 #include "bulk_host.h"
 #include "bulk_mx_plan.h"
+#include "bulk_mx_spread.cuh"
 #include "internal.h"
 
 namespace {
 
 template <typename T>
-void real_t(adscf_ctx* ctx, int t) {
+void real_t(adscf_ctx* ctx, int t, bool spread) {
   const BulkMx* M = ctx->mx;
   mxk::Dev<T> D = ctx->mx->dev<T>();
   if constexpr (sizeof(T) == 4) D.io.slices = ctx->hb32.slices;
   else D.io.slices = ctx->hb64.slices;
   D.io.I = static_cast<const BulkDev<T>*>(ctx->d_inst);
+  if constexpr (sizeof(T) == 8)
+    if (spread) {
+      k_mx_a_spread<<<M->grid_a, M->thr_as, M->sm_a, ctx->stream>>>(D, t);
+      return;
+    }
   launch<T>(k_mx_a<T>, M->grid_a, M->thr_a, M->sm_a, ctx->stream, D, t);
 }
 template <typename T>
 void step_t(adscf_ctx* ctx, int t) {
   const BulkMx* M = ctx->mx;
   const mxk::Dev<T>& D = ctx->mx->dev<T>();
-  launch<T>(M->thr_b > 256 ? k_mx_b<T, 512> : k_mx_b<T, 256>, M->grid_b, M->thr_b, M->sm_b, ctx->stream, D);
-  real_t<T>(ctx, t);
+  if (M->spread) {
+    if constexpr (sizeof(T) == 8) k_mx_b_spread<<<M->grid_b, M->thr_bs, M->sm_b, ctx->stream>>>(D);
+  } else {
+    launch<T>(M->thr_b > 256 ? k_mx_b<T, 512> : k_mx_b<T, 256>, M->grid_b, M->thr_b, M->sm_b, ctx->stream, D);
+  }
+  real_t<T>(ctx, t, M->spread);
 }
 
 // Geometry tuner, run at context creation on the context's buffers (unit
@@ -69,7 +79,7 @@ int tune_t(adscf_ctx* ctx) {
   auto time = [&](const Geom& G, float* us) -> int {
     *us = 1e30f;
     if (!geometry<T>(M, G.cut, G.cols, G.cap_a, G.cap_b)) return ADSCF_OK;
-    real_t<T>(ctx, 0);
+    real_t<T>(ctx, 0, M->spread);
     cudaGraph_t g = nullptr;
     cudaGraphExec_t ge = nullptr;
     CK(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
@@ -124,13 +134,14 @@ int tune_t(adscf_ctx* ctx) {
       if ((rc = consider(Geom{cut, cols, start.cap_a, cap}))) return rc;
     }
   if ((rc = consider(Geom{best.cut, best.cols, 64, best.cap_b}))) return rc;
+  if (M->spread && (rc = consider(Geom{best.cut, best.cols, 32, best.cap_b}))) return rc;
   CK(cudaGetLastError());
   geometry<T>(M, best.cut, best.cols, best.cap_a, best.cap_b);
   const mxk::Dev<T>& D = M->dev<T>();
   char line[160];
   std::snprintf(line, sizeof(line),
                 "mixed radix %.2f us/double step: row sets of %d, row blocks of %d x %d columns, threads %d and %d", us,
-                D.ro, D.mi, D.cols, M->thr_a, M->thr_b);
+                D.ro, D.mi, D.cols, M->spread ? M->thr_as : M->thr_a, M->spread ? M->thr_bs : M->thr_b);
   ctx->tune_report = line;
   std::lock_guard<std::mutex> lk(g_geom_mu);
   g_geom[key] = {best, line};
@@ -190,8 +201,9 @@ int mx_setup(adscf_ctx* ctx, const BulkDev<T>& I, const std::vector<T>& fk, cons
   };
   bool ok = cudaDeviceGetAttribute(&M->optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->dev) == cudaSuccess;
   // FP64 grids of one y row take z for y, the axis that is cut between the
-  // passes: one block of rows and one of columns would each hold whole lines (64
-  // x 1 x 300 27 us a double step).  FP32 keeps its (0, 0) pencil along z.
+  // passes: a block then holds 100 of the 300 points of a z line of 64 x 1 x 300
+  // (27.0 and 26.4 us a double step, 21.2 with an output per lane).  FP32 keeps
+  // its (0, 0) pencil along z.
   M->yz = sizeof(T) == 8 && ctx->gy == 1 && ctx->gz > 1 && ok && plan(ctx->gx, ctx->gz, 1);
   if (!M->yz) ok = ok && plan(ctx->gx, ctx->gy, ctx->gz);
   const int gx = D.gx, gy = D.gy, gz = D.gz;
@@ -206,6 +218,18 @@ int mx_setup(adscf_ctx* ctx, const BulkDev<T>& I, const std::vector<T>& fk, cons
     return ADSCF_OK;
   }
   ctx->mx = M;
+  if (sizeof(T) == 8) {
+    // An output per lane up to 32768 points, whose radix-4 stages are 256 warps
+    // of butterflies on 608 SM quarters: us a double step without and with,
+    // 16^3 20.1 and 12.8, 32 x 1 x 64 18.6 and 13.4, 64 x 1 x 300 27.1 and 21.2,
+    // 24^3 21.0 and 18.0, 32^3 23.2 and 21.5; above, the quarters have work
+    // enough and the repeated additions cost more (40^3 37.3 and 51.2).
+    M->spread = ctx->npts <= 32768;
+    for (const mxk::Axis& A : M->a)
+      for (int i = 0; i < A.nst; ++i) M->spread = M->spread && A.rad[i] <= 5;
+    CK(cudaFuncSetAttribute(k_mx_a_spread, cudaFuncAttributeMaxDynamicSharedMemorySize, M->optin));
+    CK(cudaFuncSetAttribute(k_mx_b_spread, cudaFuncAttributeMaxDynamicSharedMemorySize, M->optin));
+  }
   CK(cudaFuncSetAttribute(k_mx_a<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, M->optin));
   CK(cudaFuncSetAttribute(k_mx_b<T, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, M->optin));
   CK(cudaFuncSetAttribute(k_mx_b<T, 512>, cudaFuncAttributeMaxDynamicSharedMemorySize, M->optin));
@@ -245,9 +269,11 @@ void mx_destroy(adscf_ctx* ctx) {
 
 // real-space pass of node t, and a whole double step
 void mx_real(adscf_ctx* ctx, int t) {
-  if (ctx->prec == ADSCF_SPLIT) real_t<float>(ctx, t);
-  else real_t<double>(ctx, t);
+  if (ctx->prec == ADSCF_SPLIT) real_t<float>(ctx, t, false);
+  else real_t<double>(ctx, t, ctx->mx->spread);
 }
+// the same beside passes of bulk_mx.cuh
+void mx_real_plain(adscf_ctx* ctx, int t) { real_t<double>(ctx, t, false); }
 void mx_step(adscf_ctx* ctx, int t) {
   if (ctx->prec == ADSCF_SPLIT) step_t<float>(ctx, t);
   else step_t<double>(ctx, t);

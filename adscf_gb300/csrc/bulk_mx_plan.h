@@ -12,6 +12,8 @@
 struct BulkMx {
   mxk::Axis a[3];               // x, y, z
   int thr_a = 32, thr_b = 32, grid_a = 0, grid_b = 0;
+  int thr_as = 32, thr_bs = 32; // threads of the kernels with an output per lane
+  bool spread = false;          // those run the chains
   size_t sm_a = 0, sm_b = 0;
   void* d_tw = nullptr;         // twiddles (cplx<T>)
   void* d_fk = nullptr;         // diffusion factors by position (T)
@@ -142,6 +144,8 @@ bool geometry(BulkMx* M, int cut, int cols, int cap_a, int cap_b) {
   D.rx = X.nst ? X.rad[0] : 1;
   D.rz = Z.nst ? Z.rad[Z.nst - 1] : 1;
   D.nxs = X.nst > 1 ? X.nst - 1 : 0;
+  D.zrp = Z.nst > 1 ? Z.rad[Z.nst - 2] : 0;
+  D.ztwp = Z.nst > 1 ? gz / Z.m[Z.nst - 2] : 0;
   D.mgj = mxk::div_magic(gx / D.rx);
   D.mgz = mxk::div_magic(mi << D.lc);
   D.a.n = D.b.n = 0;
@@ -157,6 +161,9 @@ bool geometry(BulkMx* M, int cut, int cols, int cap_a, int cap_b) {
     S.lmask = 0x7fffffff; S.lsh = 31;
     S.tws = A.n / A.m[s];
     S.jmul = scale; S.jin = scale > 1 ? 1 : 0;
+    S.rp = s > 0 ? A.rad[s - 1] : 0;
+    S.twp = s > 0 ? A.n / A.m[s - 1] : 0;
+    S.nb = npts / S.m;
     return S;
   };
   for (int s = 1; s < X.nst; ++s) {           // k_mx_a: lines are the tile's rows
@@ -196,6 +203,13 @@ bool geometry(BulkMx* M, int cut, int cols, int cap_a, int cap_b) {
   auto threads = [](int tasks, int cap) { return std::min(cap, std::max(32, (tasks + 31) / 32 * 32)); };
   M->thr_a = threads(max_a, cap_a);
   M->thr_b = threads(max_b, cap_b);
+  // a lane per output: 32 / R butterflies a warp
+  auto warps = [](int tasks, int R) { return (tasks + 32 / R - 1) / (32 / R); };
+  int wa = X.nst ? warps(gx / D.rx * ro, D.rx) : 1, wb = Z.nst ? warps(gz / D.rz * (mi << D.lc), D.rz) : 1;
+  for (int i = 0; i < D.a.n; ++i) wa = std::max(wa, warps(D.a.s[i].total, D.a.s[i].R));
+  for (int i = 0; i < D.b.n; ++i) wb = std::max(wb, warps(D.b.s[i].total, D.b.s[i].R));
+  M->thr_as = std::min(2 * cap_a, 32 * wa);
+  M->thr_bs = std::min(std::min(256, cap_b), 32 * wb);
   M->grid_a = mi * gz;
   M->grid_b = D.ntiles;
   if (sizeof(T) == 4) M->grid_b += (gz + M->thr_b / 32 - 1) / (M->thr_b / 32);

@@ -78,3 +78,22 @@ def test_against_the_line_passes(rng, grid, prec, tol):
         b, rb = c.propagate_diblock(w)
     assert abs(ra.Qsum / rb.Qsum - 1.0) < tol
     assert np.max(np.abs(a - b)) < 5 * tol * np.max(np.abs(b))
+
+
+@pytest.mark.parametrize("grid", [(2, 1, 1), (1, 5, 1), (1, 1, 3), (3, 4, 5), (25, 1, 1), (1, 1, 125), (6, 1, 50),
+                                  (30, 9, 8), (27, 20, 16), (10, 75, 12), (16, 45, 40), (32, 32, 32), (36, 30, 32)])
+def test_small_fp64_grids(rng, grid):
+    """One output of a butterfly per lane up to 32768 points (the last grid is
+    past it): radices 2 to 5, one-point axes, butterflies that do not fill a
+    warp, and columns that do not fill a tile."""
+    size, ds, f = (3.7, 4.1, 3.9), 0.05, (0.4, 0.6)
+    w = rng.standard_normal((2,) + grid[::-1])
+    ref = ob.propagate_diblock(w, grid, size, ds, f)
+    want = ob.density_by_type(ref["density"])
+    with Context(BULK, grid=grid, size=size, ds=ds, block_length=f, precision=FP64) as c:
+        dens, res = c.propagate_diblock(w)
+        c.set_field(w)
+        r = c.scf_run(1)
+    # FP64 rounding of 20 steps
+    assert abs(res.Qsum / ref["Qsum"] - 1.0) < 1e-12 and abs(r.Qsum / res.Qsum - 1.0) < 1e-12
+    assert np.max(np.abs(dens - want)) < 5e-12 * np.max(want)
