@@ -96,6 +96,16 @@ __device__ __forceinline__ void store_boltzmann(float* E, size_t p, int c, doubl
 __device__ __forceinline__ void store_boltzmann(double* E, size_t p, int c, double a) {
   E[2 * p + c] = exp_boltzmann(a);
 }
+// both species of a point in one store
+__device__ __forceinline__ void store_boltzmann2(float* E, size_t p, double a, double b) {
+  float4 v;
+  exp_ff(a, v.x, v.z);
+  exp_ff(b, v.y, v.w);
+  reinterpret_cast<float4*>(E)[p] = v;
+}
+__device__ __forceinline__ void store_boltzmann2(double* E, size_t p, double a, double b) {
+  reinterpret_cast<double2*>(E)[p] = make_double2(exp_boltzmann(a), exp_boltzmann(b));
+}
 
 template <typename T>
 __device__ __forceinline__ int seq_type(const BulkDev<T>& I, int t) {
@@ -598,8 +608,7 @@ k_bulk_contour(const BulkDev<T>* __restrict__ insts) {
 template <typename T>
 __global__ void k_expfield(const double* __restrict__ w, T* __restrict__ E, size_t npts, double ds) {
   for (size_t p = blockIdx.x * (size_t)blockDim.x + threadIdx.x; p < npts; p += (size_t)gridDim.x * blockDim.x) {
-    store_boltzmann(E, p, 0, -0.5 * ds * w[p]);
-    store_boltzmann(E, p, 1, -0.5 * ds * w[npts + p]);
+    store_boltzmann2(E, p, -0.5 * ds * w[p], -0.5 * ds * w[npts + p]);
   }
 }
 

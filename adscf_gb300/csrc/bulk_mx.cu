@@ -238,15 +238,18 @@ int mx_setup(adscf_ctx* ctx, const BulkDev<T>& I, const std::vector<T>& fk, cons
   D.tw_x = bulkhost::twiddle_offset<T>(gx, tw, seen);
   D.tw_y = bulkhost::twiddle_offset<T>(gy, tw, seen);
   D.tw_z = bulkhost::twiddle_offset<T>(gz, tw, seen);
-  CK(cudaMalloc(&M->d_tw, tw.size() * sizeof(cplx<T>)));
+  // one allocation: twiddles, factors, the pencil's rows
+  const size_t twb = (tw.size() * sizeof(cplx<T>) + 255) / 256 * 256;
+  const size_t fkb = ((2 * (size_t)gx * gy + 2 * (size_t)gz) * sizeof(T) + 255) / 256 * 256;
+  const size_t dcb = sizeof(T) == 4 ? (size_t)gz * (gy + 2) * sizeof(float2) : 0;
+  CK(cudaMalloc(&M->d_tw, twb + fkb + dcb));
   CK(cudaMemcpy(M->d_tw, tw.data(), tw.size() * sizeof(cplx<T>), cudaMemcpyHostToDevice));
-  CK(cudaMalloc(&M->d_fk, (2 * (size_t)gx * gy + 2 * (size_t)gz) * sizeof(T)));
+  M->d_fk = static_cast<unsigned char*>(M->d_tw) + twb;
   if (sizeof(T) == 4) {
-    const size_t n = (size_t)gz * (gy + 2);
-    CK(cudaMalloc(&M->d_dc, n * sizeof(float2)));
-    CK(cudaMemset(M->d_dc, 0, n * sizeof(float2)));
-    D.io.dcin = M->d_dc;
-    D.io.dcout = M->d_dc + (size_t)gz * gy;
+    float2* dc = reinterpret_cast<float2*>(static_cast<unsigned char*>(M->d_fk) + fkb);
+    CK(cudaMemset(dc, 0, dcb));
+    D.io.dcin = dc;
+    D.io.dcout = dc + (size_t)gz * gy;
     D.io.dcc = D.io.dcout + gz;
   }
   D.tw = static_cast<const cplx<T>*>(M->d_tw);
@@ -261,8 +264,6 @@ template int mx_setup<double>(adscf_ctx*, const BulkDev<double>&, const std::vec
 void mx_destroy(adscf_ctx* ctx) {
   if (!ctx->mx) return;
   cudaFree(ctx->mx->d_tw);
-  cudaFree(ctx->mx->d_fk);
-  cudaFree(ctx->mx->d_dc);
   delete ctx->mx;
   ctx->mx = nullptr;
 }

@@ -15,9 +15,8 @@ struct BulkMx {
   int thr_as = 32, thr_bs = 32; // threads of the kernels with an output per lane
   bool spread = false;          // those run the chains
   size_t sm_a = 0, sm_b = 0;
-  void* d_tw = nullptr;         // twiddles (cplx<T>)
+  void* d_tw = nullptr;         // twiddles (cplx<T>), the allocation that holds d_fk too
   void* d_fk = nullptr;         // diffusion factors by position (T)
-  float2* d_dc = nullptr;       // dcin [gz][gy], dcout [gz], kernel [gz]
   int optin = 0;                // opt-in shared memory per block
   bool yz = false;              // the grid's z axis is the passes' y axis
   template <typename T> mxk::Dev<T>& dev();

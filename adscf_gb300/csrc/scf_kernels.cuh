@@ -130,6 +130,37 @@ __global__ void k_solve_b(const ScfDev* __restrict__ Ss, int have_closure, int d
 __global__ void k_meanfield_only(ScfDev S, const double* __restrict__ dens, double* __restrict__ field);
 
 #ifdef ADSCF_SCF_IMPL
+// Sums of N values over a warp, each lane left with at most one: every exchange
+// halves the values a lane holds, so N = 18 takes 20 additions where a tree per
+// value takes 90 (an FP64 instruction holds its SM quarter for 64 cycles, and
+// a closure thread has one to a few points).  Returns the index of the lane's
+// value, left in v[0], or -1.
+template <int N, int O = 16>
+__device__ __forceinline__ int warp_sum_each(double (&v)[N], int at, int n) {
+  const int lane = threadIdx.x & 31;
+  constexpr int H = (N + 1) / 2;
+  const bool up = lane & O;
+  double w[H];
+#pragma unroll
+  for (int i = 0; i < H; ++i) {
+    const double hi = i + H < N ? v[i + H < N ? i + H : 0] : 0.0;
+    const double other = __shfl_xor_sync(0xffffffffu, up ? v[i] : hi, O);
+    w[i] = (up ? hi : v[i]) + other;
+  }
+  // the upper half of n values holds n - H of them
+  at += up ? H : 0;
+  n = up ? n - H : min(n, H);
+  if constexpr (O > 1) {
+    const int r = warp_sum_each<H, O / 2>(w, at, n);
+    v[0] = w[0];
+    return r;
+  } else {
+    static_assert(H == 1 || N > 32, "at most 32 values");
+    v[0] = w[0];
+    return n > 0 ? at : -1;
+  }
+}
+
 // Per point: phi_new = scale*dist; accuracy; mean field; residual into the
 // history slot of iteration k; energy and mixing partial sums.  Block `bid`
 // of `nb` blocks working on this instance.
@@ -150,8 +181,9 @@ __device__ __forceinline__ void closure_body(const ScfDev& S, int flags, int bid
   double acc[NA];
 #pragma unroll
   for (int i = 0; i < NA; ++i) acc[i] = 0.0;
+  const bool planes = S.wz || S.ext || S.wall_mask;
   for (int p = bid * blockDim.x + threadIdx.x; p < S.npts; p += nb * blockDim.x) {
-    const int z = p / S.plane;
+    const int z = planes ? p / S.plane : 0;
     const double wgt = S.wz ? S.wz[z] : S.dvol;
     const bool interior = !S.wall_mask || (z > 0 && z < S.nplanes - 1);
     double phi[2], wn[2];
@@ -226,16 +258,13 @@ __device__ __forceinline__ void closure_body(const ScfDev& S, int flags, int bid
   }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const bool amax = flags & CL_CONJ;   // P_ACC holds a maximum
+  double amx = acc[P_ACC];
+  if (amax) {
 #pragma unroll
-  for (int i = 0; i < NA; ++i) {
-    double x = acc[i];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const double y = __shfl_down_sync(0xffffffffu, x, o);
-      x = (amax && i == P_ACC) ? fmax(x, y) : x + y;
-    }
-    if (lane == 0) red[i * 32 + warp] = x;
+    for (int o = 16; o > 0; o >>= 1) amx = fmax(amx, __shfl_xor_sync(0xffffffffu, amx, o));
   }
+  const int own = warp_sum_each<NA>(acc, 0, NA);
+  if (own >= 0) red[own * 32 + warp] = amax && own == P_ACC ? amx : acc[0];
   __syncthreads();
   if (threadIdx.x < NPART) {   // entries past NA (slots this closure does not hold) are 0
     double r = 0.0;
@@ -535,30 +564,37 @@ __device__ __forceinline__ void mix_body(const ScfDev& S, T* E, double ds, int b
   __syncthreads();
   const size_t nv = (size_t)S.ntypes * S.npts;
   const bool use_y = S.hy && S.mixing_type == 3 && kn - 1 > S.warm;
-  for (size_t i = bid * (size_t)blockDim.x + threadIdx.x; i < nv; i += (size_t)nb * blockDim.x) {
-    double x;
-    const int z = (int)((i % S.npts) / S.plane);
-    const bool interior = !S.wall_mask || (z > 0 && z < S.nplanes - 1);
-    if (!interior) {
-      x = S.hx[(size_t)cur * nv + i];
-    } else if (use_y) {
-      x = 0.0;
+  auto mixed = [&](size_t i) {
+    double x = 0.0;
+    if (use_y) {
       for (int k = 0; k < nnz; ++k) {
         const int j = nzj[k];
         x += ca[j] * S.hy[(size_t)j * nv + i];
       }
     } else {
-      x = 0.0;
       for (int j = 0; j < S.slots; ++j) {
         if (ca[j] != 0.0) x += ca[j] * S.hx[(size_t)j * nv + i];
         if (cb[j] != 0.0) x += cb[j] * S.hr[(size_t)j * nv + i];
       }
     }
-    S.hx[(size_t)nxt * nv + i] = x;
-    if (E) {  // interleaved Boltzmann factors of the next propagation (two species)
-      const int c = i >= (size_t)S.npts;
-      store_boltzmann(E, i - (size_t)c * S.npts, c, -0.5 * ds * x);
+    return x;
+  };
+  if (E) {   // bulk, two species: with the interleaved Boltzmann factors of the next propagation
+    for (size_t p = bid * (size_t)blockDim.x + threadIdx.x; p < (size_t)S.npts; p += (size_t)nb * blockDim.x) {
+      const double x0 = mixed(p), x1 = mixed(S.npts + p);
+      S.hx[(size_t)nxt * nv + p] = x0;
+      S.hx[(size_t)nxt * nv + S.npts + p] = x1;
+      store_boltzmann2(E, p, -0.5 * ds * x0, -0.5 * ds * x1);
     }
+    return;
+  }
+  for (size_t i = bid * (size_t)blockDim.x + threadIdx.x; i < nv; i += (size_t)nb * blockDim.x) {
+    bool interior = true;
+    if (S.wall_mask) {
+      const int z = (int)(i % S.npts) / S.plane;
+      interior = z > 0 && z < S.nplanes - 1;
+    }
+    S.hx[(size_t)nxt * nv + i] = interior ? mixed(i) : S.hx[(size_t)cur * nv + i];
   }
 }
 
