@@ -12,7 +12,6 @@
 
 #include "bulk_host.h"
 #include "bulk_mx_plan.h"
-#include "bulk_mx_spread.cuh"
 #include "internal.h"
 
 namespace {
@@ -26,7 +25,7 @@ void real_t(adscf_ctx* ctx, int t, bool spread) {
   D.io.I = static_cast<const BulkDev<T>*>(ctx->d_inst);
   if constexpr (sizeof(T) == 8)
     if (spread) {
-      k_mx_a_spread<<<M->grid_a, M->thr_as, M->sm_a, ctx->stream>>>(D, t);
+      mx_spread_a(D, M->sp, M->grid_a, M->thr_as, M->sm_a, ctx->stream, t);
       return;
     }
   launch<T>(k_mx_a<T>, M->grid_a, M->thr_a, M->sm_a, ctx->stream, D, t);
@@ -36,7 +35,7 @@ void step_t(adscf_ctx* ctx, int t) {
   const BulkMx* M = ctx->mx;
   const mxk::Dev<T>& D = ctx->mx->dev<T>();
   if (M->spread) {
-    if constexpr (sizeof(T) == 8) k_mx_b_spread<<<M->grid_b, M->thr_bs, M->sm_b, ctx->stream>>>(D);
+    if constexpr (sizeof(T) == 8) mx_spread_b(D, M->sp, M->grid_b, M->thr_bs, M->sm_b, ctx->stream);
   } else {
     launch<T>(M->thr_b > 256 ? k_mx_b<T, 512> : k_mx_b<T, 256>, M->grid_b, M->thr_b, M->sm_b, ctx->stream, D);
   }
@@ -202,7 +201,7 @@ int mx_setup(adscf_ctx* ctx, const BulkDev<T>& I, const std::vector<T>& fk, cons
   bool ok = cudaDeviceGetAttribute(&M->optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->dev) == cudaSuccess;
   // FP64 grids of one y row take z for y, the axis that is cut between the
   // passes: a block then holds 100 of the 300 points of a z line of 64 x 1 x 300
-  // (27.0 and 26.4 us a double step, 21.2 with an output per lane).  FP32 keeps
+  // (27.0 and 26.4 us a double step, 21.7 with an output per lane).  FP32 keeps
   // its (0, 0) pencil along z.
   M->yz = sizeof(T) == 8 && ctx->gy == 1 && ctx->gz > 1 && ok && plan(ctx->gx, ctx->gz, 1);
   if (!M->yz) ok = ok && plan(ctx->gx, ctx->gy, ctx->gz);
@@ -221,14 +220,13 @@ int mx_setup(adscf_ctx* ctx, const BulkDev<T>& I, const std::vector<T>& fk, cons
   if (sizeof(T) == 8) {
     // An output per lane up to 32768 points, whose radix-4 stages are 256 warps
     // of butterflies on 608 SM quarters: us a double step without and with,
-    // 16^3 20.1 and 12.8, 32 x 1 x 64 18.6 and 13.4, 64 x 1 x 300 27.1 and 21.2,
-    // 24^3 21.0 and 18.0, 32^3 23.2 and 21.5; above, the quarters have work
+    // 16^3 20.1 and 12.8, 32 x 1 x 64 18.6 and 13.4, 64 x 1 x 300 26.8 and 21.7,
+    // 24^3 21.0 and 18.0, 32^3 22.8 and 21.8; above, the quarters have work
     // enough and the repeated additions cost more (40^3 37.3 and 51.2).
     M->spread = ctx->npts <= 32768;
     for (const mxk::Axis& A : M->a)
       for (int i = 0; i < A.nst; ++i) M->spread = M->spread && A.rad[i] <= 5;
-    CK(cudaFuncSetAttribute(k_mx_a_spread, cudaFuncAttributeMaxDynamicSharedMemorySize, M->optin));
-    CK(cudaFuncSetAttribute(k_mx_b_spread, cudaFuncAttributeMaxDynamicSharedMemorySize, M->optin));
+    CK(mx_spread_setup(M->optin));
   }
   CK(cudaFuncSetAttribute(k_mx_a<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, M->optin));
   CK(cudaFuncSetAttribute(k_mx_b<T, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, M->optin));

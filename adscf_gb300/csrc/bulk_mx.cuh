@@ -58,9 +58,18 @@ struct Step {
   int ls, ls2, es;              // pitches in shared memory
   int gls, gls2, ges;           // pitches in global memory (first and last steps)
   int tw, tws, jmul, jin;       // twiddle table, W index = (jmul j + jin tile j) tws k
-  int rp, twp, nb;              // stage before: its radix (0: none) and twiddle step; blocks of M in a tile
 };
 constexpr int kMaxSteps = 8;
+// stage before a step's one on its axis: radix (0: none) and twiddle step, and
+// the blocks of the step's length in a tile; for the steps of both programs and
+// the z visit (bulk_mx_spread.cuh)
+struct Prev {
+  int rp, twp, nb;
+};
+struct Spread {
+  Prev a[kMaxSteps], b[kMaxSteps];
+  int zrp, ztwp;
+};
 struct Prog {
   int n;
   Step s[kMaxSteps];            // in forward order
@@ -90,7 +99,6 @@ struct Dev {
   int ntiles;                   // blocks of columns of k_mx_b (the rest convolve the pencil)
   Prog a, b;                    // steps around the real-space visit / the diffusion factor
   int rx, rz;                   // radices of those visits (1: none)
-  int zrp, ztwp;                // z stage before the visit's: radix (0: none), twiddle step
   int nxs;                      // x steps of program a (its first ones)
   unsigned mgj, mgz;            // divisions by gx / rx, and by the z lines of a tile
   int tw_x, tw_y, tw_z;         // twiddle tables in `tw`

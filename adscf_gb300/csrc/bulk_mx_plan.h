@@ -14,6 +14,7 @@ struct BulkMx {
   int thr_a = 32, thr_b = 32, grid_a = 0, grid_b = 0;
   int thr_as = 32, thr_bs = 32; // threads of the kernels with an output per lane
   bool spread = false;          // those run the chains
+  mxk::Spread sp{};             // and what their inverse stages need
   size_t sm_a = 0, sm_b = 0;
   void* d_tw = nullptr;         // twiddles (cplx<T>), the allocation that holds d_fk too
   void* d_fk = nullptr;         // diffusion factors by position (T)
@@ -25,6 +26,14 @@ struct BulkMx {
 };
 template <> inline mxk::Dev<float>& BulkMx::dev<float>() { return d32; }
 template <> inline mxk::Dev<double>& BulkMx::dev<double>() { return d64; }
+
+// kernels with an output per lane (bulk_mx_spread.cu), in a file of their own:
+// beside those of bulk_mx.cuh they cost the latter 3 % (60 x 72 x 100 split 18.4
+// us a double step, 17.9 without)
+cudaError_t mx_spread_setup(int optin);
+void mx_spread_a(const mxk::Dev<double>& D, const mxk::Spread& W, int grid, int threads, size_t smem, cudaStream_t s,
+                 int t);
+void mx_spread_b(const mxk::Dev<double>& D, const mxk::Spread& W, int grid, int threads, size_t smem, cudaStream_t s);
 
 namespace {
 
@@ -143,8 +152,12 @@ bool geometry(BulkMx* M, int cut, int cols, int cap_a, int cap_b) {
   D.rx = X.nst ? X.rad[0] : 1;
   D.rz = Z.nst ? Z.rad[Z.nst - 1] : 1;
   D.nxs = X.nst > 1 ? X.nst - 1 : 0;
-  D.zrp = Z.nst > 1 ? Z.rad[Z.nst - 2] : 0;
-  D.ztwp = Z.nst > 1 ? gz / Z.m[Z.nst - 2] : 0;
+  mxk::Spread& W = M->sp;
+  W.zrp = Z.nst > 1 ? Z.rad[Z.nst - 2] : 0;
+  W.ztwp = Z.nst > 1 ? gz / Z.m[Z.nst - 2] : 0;
+  auto prev = [](const mxk::Axis& A, int s, int npts, int m) {
+    return s > 0 ? mxk::Prev{A.rad[s - 1], A.n / A.m[s - 1], npts / m} : mxk::Prev{0, 0, 0};
+  };
   D.mgj = mxk::div_magic(gx / D.rx);
   D.mgz = mxk::div_magic(mi << D.lc);
   D.a.n = D.b.n = 0;
@@ -160,9 +173,6 @@ bool geometry(BulkMx* M, int cut, int cols, int cap_a, int cap_b) {
     S.lmask = 0x7fffffff; S.lsh = 31;
     S.tws = A.n / A.m[s];
     S.jmul = scale; S.jin = scale > 1 ? 1 : 0;
-    S.rp = s > 0 ? A.rad[s - 1] : 0;
-    S.twp = s > 0 ? A.n / A.m[s - 1] : 0;
-    S.nb = npts / S.m;
     return S;
   };
   for (int s = 1; s < X.nst; ++s) {           // k_mx_a: lines are the tile's rows
@@ -170,6 +180,7 @@ bool geometry(BulkMx* M, int cut, int cols, int cap_a, int cap_b) {
     S.ls = pitch; S.es = 1;
     S.gls = 0; S.ges = 1;                     // in or out directly only where a tile is one row
     S.tw = ro * pitch;
+    W.a[D.a.n] = prev(X, s, gx, S.m);
     D.a.s[D.a.n++] = S;
   }
   for (int s = 0; s < cut; ++s) {             // outer y stages: lines x, rows M' apart
@@ -177,6 +188,7 @@ bool geometry(BulkMx* M, int cut, int cols, int cap_a, int cap_b) {
     S.ls = 1; S.es = pitch;
     S.gls = 1; S.ges = mi * gx;
     S.tw = ro * pitch + gx;
+    W.a[D.a.n] = prev(Y, s, ro, S.m);
     D.a.s[D.a.n++] = S;
   }
   const int pts = mi * D.pb;                  // k_mx_b: tile [y'][z][c]
@@ -186,6 +198,7 @@ bool geometry(BulkMx* M, int cut, int cols, int cap_a, int cap_b) {
     S.ls = 1; S.ls2 = cols; S.es = D.pb;
     S.gls = 1; S.gls2 = gx * gy; S.ges = gx;
     S.tw = pts;
+    W.b[D.b.n] = prev(Y, s, mi, S.m);
     D.b.s[D.b.n++] = S;
   }
   for (int s = 0; s + 1 < Z.nst; ++s) {       // z stages: lines (y', c)
@@ -194,6 +207,7 @@ bool geometry(BulkMx* M, int cut, int cols, int cap_a, int cap_b) {
     S.ls = 1; S.ls2 = D.pb; S.es = cols;
     S.gls = 1; S.gls2 = gx; S.ges = gx * gy;
     S.tw = pts + gy;
+    W.b[D.b.n] = prev(Z, s, gz, S.m);
     D.b.s[D.b.n++] = S;
   }
   int max_a = gx / D.rx * ro, max_b = gz / D.rz * (mi << D.lc);

@@ -86,10 +86,10 @@ struct Lane {
   }
 };
 
-// One stage (as stage_r); b0: blocks of the axis before the tile's first one,
+// One stage (as stage_r); V: the stage before, b0: blocks of the axis before the tile's first one,
 // in stages of S's length per row block
 template <int SG, bool SRC, int R>
-__device__ __forceinline__ void spread_r(const Step& S, double2* sm, int tile_j, int b0, double2* g, int nl) {
+__device__ __forceinline__ void spread_r(const Step& S, const Prev& V, double2* sm, int tile_j, int b0, double2* g, int nl) {
   const Lane<R> ln;
   const double2* w = sm + S.tw;
   for (int t0 = ln.first; t0 < S.total; t0 += ln.step) {
@@ -117,7 +117,7 @@ __device__ __forceinline__ void spread_r(const Step& S, double2* sm, int tile_j,
       }
       int wi;
       if (SG > 0) wi = (S.jmul * j + S.jin * tile_j) * S.tws * ln.k;
-      else wi = S.rp ? (S.jmul * (j + ln.k * S.mp) + S.jin * tile_j) * ((b + b0 * S.nb) % S.rp) * S.twp : 0;
+      else wi = V.rp ? (S.jmul * (j + ln.k * S.mp) + S.jin * tile_j) * ((b + b0 * V.nb) % V.rp) * V.twp : 0;
       const double2 wv = w[wi];
       o = dft_out<R, SG>(v, ln.k);
       if (wi) o = SG > 0 ? cmul<double>(o, wv) : cmulc<double>(o, wv);
@@ -240,7 +240,7 @@ __device__ __forceinline__ void spread_real_1(const Dev<double>& D, double2* sm,
 
 // k_mx_a
 static __global__ void __launch_bounds__(256, 2)
-k_mx_a_spread(const __grid_constant__ mxk::Dev<double> D, int t) {
+k_mx_a_spread(const __grid_constant__ mxk::Dev<double> D, const __grid_constant__ mxk::Spread W, int t) {
   extern __shared__ __align__(16) unsigned char smraw[];
   double2* sm = reinterpret_cast<double2*>(smraw);
   const BulkDev<double>& I = *D.io.I;
@@ -271,7 +271,7 @@ k_mx_a_spread(const __grid_constant__ mxk::Dev<double> D, int t) {
     for (int i = D.a.n - 1; i >= 0; --i) {
       const mxk::Step& S = D.a.s[i];
       double2* src = i == D.a.n - 1 ? g : nullptr;
-#define ADSCF_MX_CALL(R_) mxk::spread_r<-1, true, R_>(S, sm, j, 0, src, gx)
+#define ADSCF_MX_CALL(R_) mxk::spread_r<-1, true, R_>(S, W.a[i], sm, j, 0, src, gx)
       ADSCF_MXS_SWITCH(S.R, ADSCF_MX_CALL)
 #undef ADSCF_MX_CALL
       __syncthreads();
@@ -289,7 +289,7 @@ k_mx_a_spread(const __grid_constant__ mxk::Dev<double> D, int t) {
   for (int i = 0; i < D.a.n; ++i) {
     const mxk::Step& S = D.a.s[i];
     double2* dst = i == D.a.n - 1 ? g : nullptr;
-#define ADSCF_MX_CALL(R_) mxk::spread_r<+1, false, R_>(S, sm, j, 0, dst, gx)
+#define ADSCF_MX_CALL(R_) mxk::spread_r<+1, false, R_>(S, W.a[i], sm, j, 0, dst, gx)
     ADSCF_MXS_SWITCH(S.R, ADSCF_MX_CALL)
 #undef ADSCF_MX_CALL
     if (!dst) __syncthreads();
@@ -300,7 +300,7 @@ k_mx_a_spread(const __grid_constant__ mxk::Dev<double> D, int t) {
 
 // k_mx_b
 static __global__ void __launch_bounds__(256, 2)
-k_mx_b_spread(const __grid_constant__ mxk::Dev<double> D) {
+k_mx_b_spread(const __grid_constant__ mxk::Dev<double> D, const __grid_constant__ mxk::Spread W) {
   extern __shared__ __align__(16) unsigned char smraw[];
   double2* sm = reinterpret_cast<double2*>(smraw);
   const int gx = D.gx, gz = D.gz, mi = D.mi, nxy = gx * D.gy;
@@ -325,7 +325,7 @@ k_mx_b_spread(const __grid_constant__ mxk::Dev<double> D) {
   for (int i = 0; i < D.b.n; ++i) {
     const mxk::Step& S = D.b.s[i];
     double2* src = i == 0 ? g : nullptr;
-#define ADSCF_MX_CALL(R_) mxk::spread_r<+1, true, R_>(S, sm, 0, 0, src, nl)
+#define ADSCF_MX_CALL(R_) mxk::spread_r<+1, true, R_>(S, W.b[i], sm, 0, 0, src, nl)
     ADSCF_MXS_SWITCH(S.R, ADSCF_MX_CALL)
 #undef ADSCF_MX_CALL
     __syncthreads();
@@ -333,7 +333,7 @@ k_mx_b_spread(const __grid_constant__ mxk::Dev<double> D) {
   if (D.rz == 1) {
     mxk::mid_r<double, 1>(D, sm, fz, fxy, nl);
   } else {
-#define ADSCF_MX_CALL(R_) mxk::spread_mid_r<R_>(D, sm, fz, fxy, nl, D.zrp, D.ztwp, sm + pts + D.gy)
+#define ADSCF_MX_CALL(R_) mxk::spread_mid_r<R_>(D, sm, fz, fxy, nl, W.zrp, W.ztwp, sm + pts + D.gy)
     ADSCF_MXS_SWITCH(D.rz, ADSCF_MX_CALL)
 #undef ADSCF_MX_CALL
   }
@@ -341,7 +341,7 @@ k_mx_b_spread(const __grid_constant__ mxk::Dev<double> D) {
   for (int i = D.b.n - 1; i >= 0; --i) {
     const mxk::Step& S = D.b.s[i];
     double2* dst = i == 0 ? g : nullptr;
-#define ADSCF_MX_CALL(R_) mxk::spread_r<-1, false, R_>(S, sm, 0, k, dst, nl)
+#define ADSCF_MX_CALL(R_) mxk::spread_r<-1, false, R_>(S, W.b[i], sm, 0, k, dst, nl)
     ADSCF_MXS_SWITCH(S.R, ADSCF_MX_CALL)
 #undef ADSCF_MX_CALL
     if (!dst) __syncthreads();
