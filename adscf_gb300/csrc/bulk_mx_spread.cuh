@@ -248,6 +248,7 @@ k_mx_a_spread(const __grid_constant__ mxk::Dev<double> D, const __grid_constant_
   const int z = blockIdx.x / mi, j = blockIdx.x - z * mi;
   const size_t base = ((size_t)z * D.gy + j) * gx;
   const int ns = I.ns;
+  tmak::pdl_launch_dependents();
   {
     double2* tw = sm + ro * D.pitch;
     for (int i = threadIdx.x; i < gx; i += blockDim.x) tw[i] = D.tw[D.tw_x + i];
@@ -262,6 +263,7 @@ k_mx_a_spread(const __grid_constant__ mxk::Dev<double> D, const __grid_constant_
   double2* sl = D.io.slices + (size_t)t * (size_t)I.npts + base;
   const double* E = D.io.E + base * 2;
   double2* g = D.io.spec + base;
+  tmak::pdl_wait();
   __syncthreads();
   if (t > 0) {
     if (D.a.n == 0) {
@@ -308,12 +310,14 @@ k_mx_b_spread(const __grid_constant__ mxk::Dev<double> D, const __grid_constant_
   const int nl = min(D.cols, gx - c0);
   const int pts = mi * D.pb;
   double* fz = reinterpret_cast<double*>(sm + pts + D.gy + gz);
+  tmak::pdl_launch_dependents();
   if (mi > 1)
     for (int i = threadIdx.x; i < D.gy; i += blockDim.x) sm[pts + i] = D.tw[D.tw_y + i];
   for (int i = threadIdx.x; i < gz; i += blockDim.x) sm[pts + D.gy + i] = D.tw[D.tw_z + i];
   for (int i = threadIdx.x; i < gz; i += blockDim.x) fz[i] = D.io.fk[2 * (size_t)nxy + i];
   double2* g = D.io.spec + (size_t)k * mi * gx + c0;
   const double* fxy = D.io.fk + (size_t)k * mi * gx + c0;
+  tmak::pdl_wait();
   __syncthreads();
   if (D.b.n == 0) {
     for (int e = threadIdx.x; e < gz << D.lc; e += blockDim.x) {
