@@ -21,7 +21,7 @@ void step_b(const MxLaunch64& L, double2* keep, double* dot, int tile, cudaStrea
 // generic passes (adjoint.cu).
 int adj_mx_setup(adscf_ctx* ctx, AdjMx* X) {
   MxLaunch64 L;
-  if (!mx_launch64(ctx, L)) {
+  if (ctx->mx_off || !mx_launch64(ctx, L)) {   // a pinned plan runs the generic sweep
     adj_mx_free(X);
     return ADSCF_OK;
   }

@@ -281,7 +281,7 @@ int mx_tune(adscf_ctx* ctx) { return ctx->prec == ADSCF_SPLIT ? tune_t<float>(ct
 
 bool mx_launch64(const adscf_ctx* ctx, MxLaunch64& L) {
   const BulkMx* M = ctx->mx;
-  if (!M || ctx->mx_off || ctx->prec != ADSCF_FP64) return false;
+  if (!M || ctx->prec != ADSCF_FP64) return false;
   L = MxLaunch64{M->d64, M->yz, M->thr_a, M->thr_b, M->grid_a, M->grid_b, M->sm_a, M->sm_b, M->optin};
   L.D.io.slices = ctx->hb64.slices;
   L.D.io.I = static_cast<const BulkDev<double>*>(ctx->d_inst);

@@ -599,5 +599,5 @@ struct MxLaunch64 {
   size_t sm_a, sm_b;
   int optin;
 };
-bool mx_launch64(const adscf_ctx* ctx, MxLaunch64& L);   // false: the context does not run these passes
+bool mx_launch64(const adscf_ctx* ctx, MxLaunch64& L);   // false: the context has no such plan
 void mx_freqs(const adscf_ctx* ctx, std::vector<int>& f);   // frequency by position, x then y then z

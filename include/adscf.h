@@ -258,8 +258,8 @@ ADSCF_API int adscf_set_wait_limit(adscf_ctx *ctx, int polls);
  * the TMA-fed Y and Z passes with the fused plane pass where they exist,
  * else the persistent, else the plain kernels).
  * All plans compute the same arithmetic: results do not depend on the choice.
- * Grids that run the mixed-radix passes (FP64 but 256^3; FP32 with a line of
- * 256 points or one that has no register FFT) tune their launch geometry
+ * Grids that run the mixed-radix passes (FP64 but 256^3; FP32 32^3, with a line
+ * of 256 points or with one that has no register FFT) tune their launch geometry
  * instead, which changes no operation either.
  * adscf_tuning writes the plan and the per-candidate timings as text;
  * adscf_set_pass_plan pins a plan of line passes (ADSCF_E_ARG if
@@ -281,7 +281,9 @@ ADSCF_API int adscf_set_pass_plan(adscf_ctx *ctx, int y, int z, int x);
  * bit for bit.  On a square plane whose x and y sweeps chose one unstaged
  * shape (16 or 8 lanes, 2 or 4 points each), the two sweeps as one kernel
  * per plane and chain (the plane held in shared memory, the same arithmetic)
- * are timed too and kept if faster ("xy=fused").  adscf_tuning reports the
+ * are timed too and kept if faster ("xy=fused"), and so are the sweeps on
+ * lines of any length, 9 to 160 rows each ("any=yes"), which FP64 sweeps and
+ * lines without a warp shape always take.  adscf_tuning reports the
  * choice and the timings ("GxK", "s" for staged); adscf_set_adi_plan pins
  * lanes per line for each sweep (0: one thread per line), staging (mask: 2 y,
  * 4 z) and the fused x + y kernel (mask 8); ADSCF_E_ARG if no shape matches,
@@ -296,7 +298,9 @@ ADSCF_API int adscf_set_adi_plan(adscf_ctx *ctx, int x_lanes, int y_lanes, int z
  * without mixing -- chain term log(rho V/Q) - 1 minus dvol sum(phi w) plus
  * Interaction_Energy (mod_FloryHuggins.f90:74-96), over rho V, with phi
  * from Propagate_Diblock (mod_diblock.f90:100-173) -- keeping every
- * propagator slice on the device.
+ * propagator slice on the device, and every step's spectrum too while those
+ * take at most a quarter of the free memory (the gradient then transforms
+ * the adjoint chains alone).
  * adscf_backward: reverse-mode adjoint of that discrete free energy at the
  * same fields: grad[0..2] = dF/dL_x, dF/dL_y, dF/dL_z (cell stress),
  * grad[3] = dF/dchi.  Exact for the discretisation (pseudo-spectral steps,
