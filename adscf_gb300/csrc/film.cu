@@ -47,6 +47,7 @@ struct FilmState {
   // per line), from the autotuner or the defaults
   AdiShape adi[3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
   bool adi_fuse = false;        // x and y sweeps as one plane kernel (shape adi[0])
+  void* d_anyfac = nullptr;     // their factors by schedule entry [ns + 3]
   bool any_ok = false;          // the sweeps on lines of any length (film_any.cuh) take this film
   bool adi_any = false;         // and run it
   bool adi_set = false;
@@ -59,6 +60,8 @@ void adi_warp_sweep(int dim, AdiShape sh, const FilmDev<float>& D, int step, int
 bool adi_fused_ok(AdiShape x, AdiShape y, const FilmDev<float>& D);
 void adi_fused_sweep(AdiShape sh, const FilmDev<float>& D, int step, int chains, cudaStream_t s);
 template <typename T> bool adi_any_ok(const FilmDev<T>& D, int optin);
+template <typename T> void adi_any_factors(const FilmDev<T>& D, cudaStream_t s);
+size_t adi_any_factor_vals(int entries);
 template <typename T> void adi_any_step(const FilmDev<T>& D, const FieldRef& fr, int step, int chains, cudaStream_t s);
 
 namespace {
@@ -209,7 +212,7 @@ int adi_tune(adscf_ctx* ctx, FilmState* F, const FilmDev<float>& D, const FieldR
       F->adi_fuse = it->second.fuse;
       F->adi_any = it->second.any;
       F->adi_set = true;
-      ctx->film_launches = 1 + (F->adi_fuse || F->adi_any ? 2 : 3) * ctx->ns;
+      ctx->film_launches = 1 + F->adi_any + (F->adi_fuse || F->adi_any ? 2 : 3) * ctx->ns;
       ctx->tune_report = it->second.report + " (cached)";
       return ADSCF_OK;
     }
@@ -292,6 +295,7 @@ int adi_tune(adscf_ctx* ctx, FilmState* F, const FilmDev<float>& D, const FieldR
   // the sweeps on lines of any length, against the chosen ones, as whole steps
   if (F->any_ok) {
     float us[2] = {1e30f, 1e30f};
+    adi_any_factors(D, s);
     A.fuse = val.fuse;
     for (int k = 0; k < 2; ++k) {
       A.any = k == 1;
@@ -308,7 +312,7 @@ int adi_tune(adscf_ctx* ctx, FilmState* F, const FilmDev<float>& D, const FieldR
   F->adi_fuse = val.fuse;
   F->adi_any = val.any;
   F->adi_set = true;
-  ctx->film_launches = 1 + (F->adi_fuse || F->adi_any ? 2 : 3) * ctx->ns;
+  ctx->film_launches = 1 + F->adi_any + (F->adi_fuse || F->adi_any ? 2 : 3) * ctx->ns;
   val.report = rep;
   ctx->tune_report = rep;
   std::lock_guard<std::mutex> lk(g_adi_mu);
@@ -407,6 +411,7 @@ int chains_t(adscf_ctx* ctx, const double* d_w) {
       if (!F->adi_set) adi_defaults(F, D);
     }
     const AdiLaunch A = adi_launch<T>(F, D, 2);
+    if (A.any) adi_any_factors(D, s);
     for (int st = 1; st <= D.ns; ++st) adi_step<T>(A, D, fr, st, 2, s);
   } else {
     int rc = film_prepare(ctx);
@@ -444,6 +449,7 @@ int step_single_t(adscf_ctx* ctx, double* d_prop, const double* d_w, double ds) 
     CK(cudaMemcpyAsync(F->d_adicf + 6 * (D.ns + 1), h_cf, sizeof(h_cf), cudaMemcpyHostToDevice, s));
     D.adicf = F->d_adicf + 6 * (D.ns + 1);
   }
+  if (D.fac) D.fac += adi_any_factor_vals(D.ns + 1);
   D.dss = F->d_dss + D.ns + 1;
   D.ns = 1;
   D.na = 1;
@@ -459,6 +465,7 @@ int step_single_t(adscf_ctx* ctx, double* d_prop, const double* d_w, double ds) 
       if (!F->adi_set) adi_defaults(F, fdev<float>(F));
     }
     const AdiLaunch A = adi_launch<T>(F, D, 1);
+    if (A.any) adi_any_factors(D, s);
     adi_step<T>(A, D, fr, 1, 1, s);
   } else {
     const int rc = launch_chains_1d<T>(ctx, D, fr, 1, s);
@@ -609,10 +616,15 @@ int film_create(adscf_ctx* ctx, const adscf_params* p) {
   else fill_dev<float>(ctx, F, p);
   if (ctx->geometry == ADSCF_FILM_3D) {
     F->any_ok = F->t64 ? adi_any_ok(F->f64, F->optin) : adi_any_ok(F->f32, F->optin);
+    if (F->any_ok) {
+      CK(cudaMalloc(&F->d_anyfac, adi_any_factor_vals(ctx->ns + 3) * (F->t64 ? sizeof(double) : sizeof(float))));
+      F->f64.fac = static_cast<double*>(F->d_anyfac);
+      F->f32.fac = static_cast<float*>(F->d_anyfac);
+    }
     // FP64 sweeps: one thread per line only where the lines are too long
     F->adi_any = F->t64 && F->any_ok;
   }
-  ctx->film_launches = ctx->geometry == ADSCF_FILM_3D ? 1 + (F->adi_any ? 2 : 3) * ctx->ns
+  ctx->film_launches = ctx->geometry == ADSCF_FILM_3D ? 1 + F->adi_any + (F->adi_any ? 2 : 3) * ctx->ns
                        : line_factors_ok(ctx)            ? 2
                                                          : 1;
   ctx->film_contour_launches = 1;
@@ -620,7 +632,7 @@ int film_create(adscf_ctx* ctx, const adscf_params* p) {
     FilmDev<float>& D = F->f32;
     if (!ctx->autotune) {
       adi_defaults(F, D);
-      ctx->film_launches = 1 + (F->adi_any ? 2 : 3) * ctx->ns;
+      ctx->film_launches = 1 + F->adi_any + (F->adi_any ? 2 : 3) * ctx->ns;
       return ADSCF_OK;
     }
     const size_t n = (size_t)ctx->ntypes * D.npts;
@@ -714,7 +726,7 @@ void film_destroy(adscf_ctx* ctx) {
   cudaFree(F->d_dss); cudaFree(F->d_adicf); cudaFree(F->d_wA); cudaFree(F->d_wB); cudaFree(F->d_graft);
   cudaFree(F->d_alf); cudaFree(F->d_wf);
   cudaFree(F->d_q); cudaFree(F->d_qd); cudaFree(F->d_gam); cudaFree(F->d_w1);
-  cudaFree(F->d_err); cudaFree(ctx->d_qpart); cudaFree(F->d_fac);
+  cudaFree(F->d_err); cudaFree(ctx->d_qpart); cudaFree(F->d_fac); cudaFree(F->d_anyfac);
   delete F;
   ctx->film = nullptr;
 }

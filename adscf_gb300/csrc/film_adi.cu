@@ -213,6 +213,12 @@ void adi_any_step(const FilmDev<T>& D, const FieldRef& fr, int step, int chains,
   k_adi_z_any<T><<<dim3((D.nlines + tl - 1) / tl, chains), any_threads(tl, adiany::lanes(D.gz + 1), 512),
                    any_smem_z(D, tl), s>>>(D, fr, step, tl);
 }
+// the x and y factors of D.ns schedule entries, before the first step
+template <typename T>
+void adi_any_factors(const FilmDev<T>& D, cudaStream_t s) { k_adi_any_factors<T><<<D.ns, 64, 0, s>>>(D); }
+size_t adi_any_factor_vals(int entries) { return (size_t)entries * 2 * adiany::kFacAxis; }
+template void adi_any_factors<float>(const FilmDev<float>&, cudaStream_t);
+template void adi_any_factors<double>(const FilmDev<double>&, cudaStream_t);
 template bool adi_any_ok<float>(const FilmDev<float>&, int);
 template bool adi_any_ok<double>(const FilmDev<double>&, int);
 template void adi_any_step<float>(const FilmDev<float>&, const FieldRef&, int, int, cudaStream_t);

@@ -20,8 +20,8 @@
 // z lines whose systems are not diagonally dominant (ds w / 2 below -0.99)
 // run the reference's serial recurrence, with its pivots and their checks.
 //
-// The x and y matrices are the same for every line of a sweep: each warp makes
-// their factors once and applies them line after line.
+// The x and y matrices are the same for every line of a sweep: their factors
+// are made once a propagation and applied line after line.
 //
 // Bound: FP64 the FP64 pipe and the wave of 99 planes on 152 SMs, FP32 latency.
 // A step of both chains, thread per line -> here: 20x35x100 FP64 220 -> 52 us
@@ -81,9 +81,12 @@ __device__ __forceinline__ T pair(T a, T c, T qm, T q0, T qp) {
 }
 
 // Factors of the periodic matrix (a, d, a) of the x and y lines, the same for
-// every line of a sweep: made once per warp, applied line after line (solve:
-// fw::solve's operations on the right-hand side alone, about 5 a row where
-// the whole solve takes 30).
+// every line and plane of a step: made once a propagation for every schedule
+// entry (k_adi_any_factors), applied line after line (solve: fw::solve's
+// operations on the right-hand side alone, about 5 a row where the whole
+// solve takes 30).  Stored by value, then lane of the line.
+constexpr int kFacVals = 5 * 4 + 2 * 5 + 1;   // K = 5, 32 lanes
+constexpr int kFacAxis = kFacVals * 32;
 template <typename T, int G, int K>
 struct Factors {
   static constexpr int LG = G == 4 ? 2 : G == 8 ? 3 : G == 16 ? 4 : 5;
@@ -135,6 +138,24 @@ struct Factors {
     iden = fw::rcp(den);
   }
 
+  template <typename Op>
+  __device__ __forceinline__ void each(Op op) {
+    int k = 0;
+#pragma unroll
+    for (int i = 0; i < K - 1; ++i) {
+      op(bet[i], k++); op(m[i], k++); op(g[i], k++); op(y[i], k++); op(z[i], k++);
+    }
+#pragma unroll
+    for (int i = 0; i < LG; ++i) { op(kl[i], k++); op(kr[i], k++); }
+    op(iden, k);
+  }
+  __device__ __forceinline__ void store(T* tab, int gl) {
+    each([&](T v, int k) { tab[k * G + gl] = v; });
+  }
+  __device__ __forceinline__ Factors(T a_, int i0_, const T* tab, int gl) : a(a_), i0(i0_) {
+    each([&](T& v, int k) { v = __ldg(tab + k * G + gl); });
+  }
+
   // r: right-hand side of the lane's entries (0 in a pad entry); the solution
   // on return
   __device__ __forceinline__ void solve(T (&r)[K]) const {
@@ -166,12 +187,12 @@ struct Factors {
 // x sweep of the plane P ([y][x], pitch pt) into D
 template <typename T, int G, int K>
 __device__ __forceinline__ void x_lines(const FilmDev<T>& F, const Coef<T>& cf, const T* P, T* D, int pt, const T* p0,
-                                        const double* w, int ty, int z) {
+                                        const double* w, int ty, int z, const T* tab) {
   const int gx = F.gx, gy = F.gy, L = F.nlines;
   const int gl = threadIdx.x & (G - 1), ng = blockDim.x / G;
   const Rows R = rows_of<G, K>(gx, gl);
   const T az = r_mul(-cf.ds, mesh(F, z, 0)), cz = r_mul(-cf.ds, mesh(F, z, 1));
-  const Factors<T, G, K> fac(cf.ax, r_fma((T)-2, cf.ax, (T)1), R.i0, F.err);
+  const Factors<T, G, K> fac(cf.ax, R.i0, tab, gl);
   // a warp leaves when its lines are done (its lanes stay together)
   for (int y0 = (threadIdx.x & ~31) / G; y0 < gy; y0 += ng) {
     const int yl = y0 + (threadIdx.x & 31) / G;
@@ -205,11 +226,11 @@ __device__ __forceinline__ void x_lines(const FilmDev<T>& F, const Coef<T>& cf, 
 
 // y sweep of the increments D in place
 template <typename T, int G, int K>
-__device__ __forceinline__ void y_lines(const FilmDev<T>& F, const Coef<T>& cf, T* D, int pt) {
+__device__ __forceinline__ void y_lines(const FilmDev<T>& F, const Coef<T>& cf, T* D, int pt, const T* tab) {
   const int gx = F.gx, gy = F.gy;
   const int gl = threadIdx.x & (G - 1), ng = blockDim.x / G;
   const Rows R = rows_of<G, K>(gy, gl);
-  const Factors<T, G, K> fac(cf.ay, r_fma((T)-2, cf.ay, (T)1), R.i0, F.err);
+  const Factors<T, G, K> fac(cf.ay, R.i0, tab, gl);
   for (int x0 = (threadIdx.x & ~31) / G; x0 < gx; x0 += ng) {
     const int xl = x0 + (threadIdx.x & 31) / G;
     const bool live = xl < gx;
@@ -314,6 +335,26 @@ __device__ __forceinline__ void z_lines(const FilmDev<T>& F, const Coef<T>& cf, 
 
 }  // namespace adiany
 
+// Factors of schedule entry 1 + blockIdx.x: x lines by warp 0, y lines by warp 1
+template <typename T>
+__global__ void __launch_bounds__(64)
+k_adi_any_factors(FilmDev<T> F) {
+  const int k = 1 + blockIdx.x, lane = threadIdx.x & 31;
+  const adiany::Coef<T> cf = adiany::coef(F, 0, k);
+  T* tab = F.fac + (size_t)k * (2 * adiany::kFacAxis);
+  const bool x = threadIdx.x < 32;
+  const T a = x ? cf.ax : cf.ay, d = r_fma((T)-2, a, (T)1);
+  const int n = x ? F.gx : F.gy;
+  if (!x) tab += adiany::kFacAxis;
+#define ADSCF_ANY_CALL(G, K)                                                                        \
+  {                                                                                                 \
+    adiany::Factors<T, G, K> f(a, d, adiany::rows_of<G, K>(n, lane & (G - 1)).i0, F.err);           \
+    if (lane < G) f.store(tab, lane);                                                               \
+  }
+  ADSCF_ANY_SHAPE(n, ADSCF_ANY_CALL)
+#undef ADSCF_ANY_CALL
+}
+
 // x and y sweeps of interior plane 1 + blockIdx.x, chain blockIdx.y.  Shared
 // memory: two planes of gy rows at pitch gx | 1.
 template <typename T>
@@ -327,17 +368,18 @@ k_adi_xy_any(FilmDev<T> F, FieldRef fr, int s) {
   const adiany::Coef<T> cf = adiany::coef(F, dir, s);
   const int ty = (F.brush || F.single) ? 0 : film_type(dir, s, F.ns, F.na);
   const double* w = sizeof(T) == 4 ? nullptr : fr.get();
+  const T* tab = F.fac + (size_t)(dir == 0 ? s : F.ns + 1 - s) * (2 * adiany::kFacAxis);
   const T* p0 = (dir == 0 ? F.q : F.qd) + (size_t)(s - 1) * F.npts;
   T* out = F.w1 + (size_t)dir * F.npts + (size_t)z * L;
   const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
   for (int y = threadIdx.x >> 5; y < gy; y += nw)
     for (int x = lane; x < gx; x += 32) P[y * pt + x] = __ldg(p0 + (size_t)z * L + (size_t)y * gx + x);
   __syncthreads();
-#define ADSCF_ANY_CALL(G, K) adiany::x_lines<T, G, K>(F, cf, P, D, pt, p0, w, ty, z)
+#define ADSCF_ANY_CALL(G, K) adiany::x_lines<T, G, K>(F, cf, P, D, pt, p0, w, ty, z, tab)
   ADSCF_ANY_SHAPE(gx, ADSCF_ANY_CALL)
 #undef ADSCF_ANY_CALL
   __syncthreads();
-#define ADSCF_ANY_CALL(G, K) adiany::y_lines<T, G, K>(F, cf, D, pt)
+#define ADSCF_ANY_CALL(G, K) adiany::y_lines<T, G, K>(F, cf, D, pt, tab + adiany::kFacAxis)
   ADSCF_ANY_SHAPE(gy, ADSCF_ANY_CALL)
 #undef ADSCF_ANY_CALL
   __syncthreads();

@@ -60,6 +60,7 @@ struct FilmDev {
   double dx, dy;
   double hx2, hy2;       // 1 / (2 dx dx), 1 / (2 dy dy)
   T* w1;                 // [2][npts] intermediate q*, q** of the ADI sweeps
+  T* fac;                // x and y factors by schedule entry (film_any.cuh), from entry 1
   // FP32 sweeps: FP32 copies of the mesh factors and, for the ADI sweeps, of
   // the field ([ntypes][npts], filled per propagation)
   const float* alf;
