@@ -182,8 +182,8 @@ size_t any_smem_z(const FilmDev<T>& D, int tl) { return ((size_t)(D.gz + 1) * (2
 // lines of a z block.  FP32: 16 (whole sectors and few blocks), 8 where that
 // leaves less than 64 blocks (16x12x83: 10.7 against 11.0 us a step; 20x35x100
 // at 88 blocks 12.5 with 16, 12.9 with 8).  FP64: 4, so that the FP64 work
-// reaches every SM quarter (17x12x83: 25.3 us a step against 36.2 with 16,
-// 20x35x100 51.6 against 55.3, 96x96x64 the same).
+// reaches every SM quarter (17x12x83: 20.2 us a step against 23.4 with 8,
+// 20x35x100 40.1 against 44.7, 48^3 and 96x96x64 the same).
 template <typename T>
 int any_tile(const FilmDev<T>& D, int chains) {
   if (sizeof(T) == 8) return 4;
@@ -204,10 +204,9 @@ bool adi_any_ok(const FilmDev<T>& D, int optin) {
 }
 template <typename T>
 void adi_any_step(const FilmDev<T>& D, const FieldRef& fr, int step, int chains, cudaStream_t s) {
-  // FP64: 256 threads, two blocks an SM with fewer table set-ups (48^3 57 against
-  // 65 us a step); FP32: 512 (48^3 12.1 against 13.6 us)
-  const int tx = any_threads(std::max(D.gy * adiany::lanes(D.gx), D.gx * adiany::lanes(D.gy)), 1,
-                             sizeof(T) == 8 ? 256 : 512);
+  // every line of a plane at once, up to 512 threads (48^3 FP64 48.6 us a step,
+  // 54.3 with 128; FP32 12.1, 13.6 with 256)
+  const int tx = any_threads(std::max(D.gy * adiany::lanes(D.gx), D.gx * adiany::lanes(D.gy)), 1, 512);
   k_adi_xy_any<T><<<dim3(D.gz - 1, chains), tx, any_smem_xy(D), s>>>(D, fr, step);
   const int tl = any_tile(D, chains);
   k_adi_z_any<T><<<dim3((D.nlines + tl - 1) / tl, chains), any_threads(tl, adiany::lanes(D.gz + 1), 512),

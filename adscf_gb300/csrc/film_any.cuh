@@ -24,9 +24,9 @@
 // are made once a propagation and applied line after line.
 //
 // Bound: FP64 the FP64 pipe and the wave of 99 planes on 152 SMs, FP32 latency.
-// A step of both chains, thread per line -> here: 20x35x100 FP64 220 -> 52 us
-// (69 without the factors), FP32 43.5 -> 12.5; 48^3 FP64 57 us, FP32 69.5 ->
-// 12.1; 96x96x64 FP32 175 -> 26.
+// A step of both chains, thread per line -> here: 20x35x100 FP64 220 -> 40 us
+// (53 with factors made by every warp, 69 line by line), FP32 43.5 -> 12.5;
+// 48^3 FP64 49 us, FP32 69.5 -> 11.9; 96x96x64 FP32 175 -> 25.
 #pragma once
 #include "film_warp.cuh"
 
