@@ -343,13 +343,13 @@ int create_t(adscf_ctx* ctx) {
   // Mixed-radix passes where a line length has no register FFT, and of the
   // shapes that have one on every axis
   //  - FP32 with a line of 256 points, whose register passes leave L2 four
-  //    times a double step (256^3 542 us a double step with them, 405 here;
-  //    64 x 64 x 256 44.8 and 30.3, 256 x 64 x 64 31.6 and 27.3; without one
+  //    times a double step (256^3 542 us a double step with them, 348 here;
+  //    64 x 64 x 256 44.8 and 27.4, 256 x 64 x 64 31.6 and 27.3; without one
   //    the register passes are ahead: 64 x 32 x 128 18.8 and 20.7), and 32^3,
   //    whose 1024 lines are 16 register-FFT blocks (14.6 and 12.1);
   //  - FP64 but 256^3, where HBM bounds both (4641 and 4704 us): the cut takes
-  //    two passes for four (64^3 73.4 and 69.6 us, 128^3 609 and 531, 32^3 60
-  //    and 23).
+  //    two passes for four (64^3 73.4 and 69.5 us, 128^3 609 and 530, 32^3 60
+  //    and 22).
   const bool all_reg = ctx->regx && ctx->regy && ctx->regz;
   const bool cube32 = all_reg && ctx->regx == 32 && ctx->regy == 32 && ctx->regz == 32;
   const int n256 = (ctx->regx == 256) + (ctx->regy == 256) + (ctx->regz == 256);

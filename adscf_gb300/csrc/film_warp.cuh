@@ -401,8 +401,9 @@ k_film1d_warp_b(const FilmDev<T>* __restrict__ Fs, const ScfDev* __restrict__ Ss
 // arithmetic is the same either way: K and W depend on the line length alone.
 // Bound: FP64 issue, one warp instruction per 64 cycles on each SM quarter.
 // Measured (GB300, FP64, against one thread per line and chain): brush of
-// 1001 rows and 1200 steps 1368 -> 11.6 ms; an SCF iteration of a 501-row
-// film with 100 steps 56.8 -> 0.95 ms.
+// 1001 rows and 1200 steps 1368 -> 11.1 ms; an SCF iteration of a 501-row
+// film with 100 steps 56.8 -> 0.91 ms (with the factors made ahead, where
+// film_line.cuh takes the line, 4.2 and 0.27).
 // ---------------------------------------------------------------------------
 constexpr int kFilmGroupK = 4;
 constexpr int kFilmGroupMaxW = 32;
