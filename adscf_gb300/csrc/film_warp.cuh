@@ -388,7 +388,7 @@ k_film1d_warp_b(const FilmDev<T>* __restrict__ Fs, const ScfDev* __restrict__ Ss
 //    unknowns as extra right-hand sides, so every row of the warp is
 //    x + y U(previous warp) + z U(this warp), U = solution at a warp's last row;
 //  - the warps exchange seven numbers each (their last row's equation and
-//    their first row's x, y, z) and every warp solves the W equations in U
+//    their first row's x, y, z; ten in FP32, see FilmGroupSm) and every warp solves the W equations in U
 //    itself, one lane per equation: one barrier per contour step.
 // The exchange slots are double buffered by step parity: a warp writes the
 // slots of step s + 2 only after the barrier of step s + 1, which every warp
@@ -433,9 +433,17 @@ __device__ __forceinline__ void cluster_barrier() {
 
 }  // namespace fw
 
+// What the warps exchange a step, by step parity: A, B, R, c of their last
+// row's equation and x0, y0, z0 of their first row.  FP32 forms the next
+// step's right-hand side from differences of q, with its own copy of the next
+// warp's first q: it takes the six numbers that row is made of there (x, y, z of
+// the row, X, Y, Z of its separator), so that the copy never differs from the
+// row.  A copy that rounds on its own drifts, and ds / dz^2 times the drift is
+// a source at every warp's edge (1501 rows, 1200 steps: density 1e-5 off).
 template <typename T>
 struct FilmGroupSm {
-  T ex[2][7][kFilmGroupMaxW];           // by step parity: A, B, R, c, x0, y0, z0 of every warp
+  static constexpr int kN = sizeof(T) == 4 ? 10 : 7;
+  T ex[2][kN][kFilmGroupMaxW];
 };
 
 // `chain`, `stride`, `field`, `wstride` as film1d_chain_warp / film_warp_tables;
@@ -546,14 +554,22 @@ __device__ __forceinline__ void film1d_chain_group(const FilmDev<T>& F, int dir,
     const T X30 = __shfl_sync(mask, X, 30), Y30 = __shfl_sync(mask, Y, 30), Z30 = __shfl_sync(mask, Z, 30);
     const T eA = __shfl_sync(mask, r_mul(As, Y30), 31), eB = __shfl_sync(mask, r_fma(As, Z30, Bs), 31);
     const T eR = __shfl_sync(mask, r_fma(-As, X30, Rs), 31), eC = __shfl_sync(mask, c[S], 31);
-    const T fx = __shfl_sync(mask, r_fma(z[0], X, x[0]), 0), fy = __shfl_sync(mask, r_fma(z[0], Y, y[0]), 0);
-    const T fz = __shfl_sync(mask, r_mul(z[0], Z), 0);
     T (*ex)[kFilmGroupMaxW] = sm.ex[s & 1];
-    for (int k = lane; k < 7 * csize; k += 32) {
-      const int which = k % 7, to = k / 7;
-      const T v = which == 0 ? eA : which == 1 ? eB : which == 2 ? eR : which == 3 ? eC : which == 4 ? fx : which == 5 ? fy : fz;
-      if (csize == 1) ex[which][w] = v;
-      else fw::cluster_store(fw::cluster_map(&ex[which][w], to), v);
+    if constexpr (sizeof(T) == 4) {       // one CTA
+      if (lane == 0) {
+        ex[0][w] = eA; ex[1][w] = eB; ex[2][w] = eR; ex[3][w] = eC;
+        ex[4][w] = x[0]; ex[5][w] = y[0]; ex[6][w] = z[0];
+        ex[7][w] = X; ex[8][w] = Y; ex[9][w] = Z;
+      }
+    } else {
+      const T fx = __shfl_sync(mask, r_fma(z[0], X, x[0]), 0), fy = __shfl_sync(mask, r_fma(z[0], Y, y[0]), 0);
+      const T fz = __shfl_sync(mask, r_mul(z[0], Z), 0);
+      for (int k = lane; k < 7 * csize; k += 32) {
+        const int which = k % 7, to = k / 7;
+        const T v = which == 0 ? eA : which == 1 ? eB : which == 2 ? eR : which == 3 ? eC : which == 4 ? fx : which == 5 ? fy : fz;
+        if (csize == 1) ex[which][w] = v;
+        else fw::cluster_store(fw::cluster_map(&ex[which][w], to), v);
+      }
     }
     if (csize == 1) __syncthreads();
     else fw::cluster_barrier();
@@ -561,7 +577,14 @@ __device__ __forceinline__ void film1d_chain_group(const FilmDev<T>& F, int dir,
     T gA = (T)0, gB = (T)1, gC = (T)0, gR = (T)0, hx = (T)0, hy = (T)0, hz = (T)0;
     if (lane < W) {
       gA = ex[0][lane]; gB = ex[1][lane]; gR = ex[2][lane];
-      if (lane + 1 < W) { hx = ex[4][lane + 1]; hy = ex[5][lane + 1]; hz = ex[6][lane + 1]; }
+      if (lane + 1 < W) {
+        hx = ex[4][lane + 1]; hy = ex[5][lane + 1]; hz = ex[6][lane + 1];
+        if constexpr (sizeof(T) == 4) {
+          hx = r_fma(hz, ex[7][lane + 1], hx);
+          hy = r_fma(hz, ex[8][lane + 1], hy);
+          hz = r_mul(hz, ex[9][lane + 1]);
+        }
+      }
       const T cc = ex[3][lane];
       gB = r_fma(cc, hy, gB);
       gR = r_fma(-cc, hx, gR);
@@ -597,11 +620,13 @@ __device__ __forceinline__ void film1d_chain_group(const FilmDev<T>& F, int dir,
       q[i] = cn_new_q(q[i], u);
       if (s0 + i < n) qn[(size_t)(s0 + i) * stride] = q[i];
     }
-    if constexpr (sizeof(T) == 4) {   // the neighbouring warps' edge rows
-      const T UN = __shfl_sync(mask, U, w + 1 < W ? w + 1 : w);
-      const T nx_ = __shfl_sync(mask, hx, w), ny_ = __shfl_sync(mask, hy, w), nz_ = __shfl_sync(mask, hz, w);
+    if constexpr (sizeof(T) == 4) {   // the neighbouring warps' edge rows, by those warps' own operations
       qlo = cn_new_q(qlo, UL);
-      if (w + 1 < W) qhi = cn_new_q(qhi, r_fma(nz_, UN, r_fma(ny_, UR, nx_)));
+      if (w + 1 < W) {
+        const T UN = __shfl_sync(mask, U, w + 1);
+        const T vn = r_fma(ex[9][w + 1], UN, r_fma(ex[8][w + 1], UR, ex[7][w + 1]));
+        qhi = cn_new_q(qhi, r_fma(ex[6][w + 1], vn, r_fma(ex[5][w + 1], UR, ex[4][w + 1])));
+      }
     }
   }
 }
