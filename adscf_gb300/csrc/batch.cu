@@ -1176,7 +1176,7 @@ template <typename T>
 int set_fields_t(adscf_batch* b, const double* fields) {
   int rc = pack_buffer(b);
   if (rc) return rc;
-  const bool pin = host_pinned(fields);
+  const bool pin = host_pinned(fields, b->foff[b->n] * sizeof(double));
   if (!pin && (rc = pinned(b, b->pack_cap * sizeof(double)))) return rc;
   dim3 g = pack_grid(b);
   for (int i0 = 0, i1; i0 < b->n; i0 = i1) {
@@ -1196,7 +1196,7 @@ int set_fields_t(adscf_batch* b, const double* fields) {
 int get_t(adscf_batch* b, double* out, bool fields) {
   int rc = pack_buffer(b);
   if (rc) return rc;
-  const bool pin = host_pinned(out);
+  const bool pin = host_pinned(out, b->foff[b->n] * sizeof(double));
   if (!pin && (rc = pinned(b, b->pack_cap * sizeof(double)))) return rc;
   dim3 g = pack_grid(b);
   for (int i0 = 0, i1; i0 < b->n; i0 = i1) {
@@ -1355,7 +1355,7 @@ int adscf_batch_forward(adscf_batch* b, const double* fields, double* free_energ
   BatchAdj* a = b->adj;
   const int n = b->n;
   const size_t bytes = b->foff[n] * sizeof(double);
-  if (host_pinned(fields)) {
+  if (host_pinned(fields, bytes)) {
     BK(cudaMemcpyAsync(a->d_w, fields, bytes, cudaMemcpyHostToDevice, b->stream));
   } else {
     if ((rc = pinned(b, bytes))) return rc;

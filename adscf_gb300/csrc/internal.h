@@ -144,7 +144,7 @@ struct EventPair {
 // memory through the context's page-locked staging buffer
 int grid_blocks(size_t n, int per, int cap);
 int ensure_pinned(adscf_ctx* ctx, size_t bytes);
-bool host_pinned(const void* p);
+bool host_pinned(const void* p, size_t bytes);
 // copies of `bytes` through the page-locked buffer `pin` of that size, in
 // chunks, so that the DMA of one chunk runs beside the memcpy of the next;
 // staged_h2d returns with the copies enqueued, staged_d2h when all is in h
