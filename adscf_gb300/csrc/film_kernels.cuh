@@ -788,13 +788,33 @@ static __global__ void __launch_bounds__(256) k_film_fe(ScfDev S, const double* 
   if (threadIdx.x < FE_N) part[z * FE_N + threadIdx.x] = r;
 }
 
-// out: [0] F, [1] dF/dchi (brush: dF/dww), [2 + c*nplanes + z] dF/dU_c(z)
+// s + lo += v, exactly but for the rounding of lo
+__device__ __forceinline__ void sum_pair(double& s, double& lo, double v) {
+  const double t = __dadd_rn(s, v), b = __dsub_rn(t, s);
+  lo = __dadd_rn(lo, __dadd_rn(__dsub_rn(s, __dsub_rn(t, b)), __dsub_rn(v, b)));
+  s = t;
+}
+// out: [0] F, [1] dF/dchi (brush: dF/dww), [2 + c*nplanes + z] dF/dU_c(z).  One
+// warp: lane k adds up term k over the planes.  The sums are carried in pairs
+// and F is rounded once: the sums of some ten each left F two units off in the
+// last place, which a difference of two F for a step of 1e-5 shows.
 static __global__ void k_film_fe_sc(ScfDev S, const double* __restrict__ part, double* __restrict__ out) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  const double Q = q_total_serial(S);
-  double t[FE_N] = {0, 0, 0, 0, 0, 0, 0};
-  for (int z = 0; z < S.nplanes; ++z)
-    for (int k = 0; k < FE_N; ++k) t[k] += S.wz[z] * part[z * FE_N + k];
+  const int k = threadIdx.x;
+  double s = 0.0, lo = 0.0;
+  if (k < FE_N)
+    for (int z = 0; z < S.nplanes; ++z) {
+      const double w = S.wz[z], v = part[z * FE_N + k], p = __dmul_rn(w, v);
+      sum_pair(s, lo, p);
+      lo = __dadd_rn(lo, __fma_rn(w, v, -p));
+    }
+  double t[FE_N], tl[FE_N];
+#pragma unroll
+  for (int i = 0; i < FE_N; ++i) {
+    t[i] = __shfl_sync(0xffffffffu, s, i);
+    tl[i] = __shfl_sync(0xffffffffu, lo, i);
+  }
+  const double Q = q_total(S);
+  if (threadIdx.x != 0) return;
   double rho, energy;
   if (S.ensemble == 1) {
     rho = S.rho;
@@ -804,7 +824,12 @@ static __global__ void k_film_fe_sc(ScfDev S, const double* __restrict__ part, d
     energy = -rho * S.volume;
   }
   const double rv = rho * S.volume;
-  out[0] = (energy - t[FE_PHIW] + t[FE_EINT] + t[FE_EEXT]) / rv;
+  double el = __dsub_rn(__dadd_rn(tl[FE_EINT], tl[FE_EEXT]), tl[FE_PHIW]);
+  sum_pair(energy, el, -t[FE_PHIW]);
+  sum_pair(energy, el, t[FE_EINT]);
+  sum_pair(energy, el, t[FE_EEXT]);
+  const double f = energy / rv;
+  out[0] = __dadd_rn(f, __dadd_rn(__fma_rn(-f, rv, energy), el) / rv);
   out[1] = t[FE_X01] / rv;
   for (int z = 0; z < S.nplanes; ++z) {
     out[2 + z] = S.wz[z] * part[z * FE_N + FE_S0] / rv;

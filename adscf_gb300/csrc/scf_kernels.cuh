@@ -74,9 +74,8 @@ struct ScfDev {
 // Q = qscale * (sum of the contour kernel's per-block partials) in one fixed
 // order: lane-strided partial sums s_l (blocks b = l mod 32, increasing b),
 // then a butterfly over the 32 lanes.  Floating-point addition commutes
-// exactly, so every lane of the butterfly ends with the same bits, and
-// q_total_serial replays the same additions in one thread: every caller sees
-// the same Q.  All 32 lanes of a warp must call q_total.
+// exactly, so every lane of the butterfly ends with the same bits: every caller
+// sees the same Q.  All 32 lanes of a warp must call q_total.
 __device__ __forceinline__ double warp_sum_fixed(const double* v, int n, size_t stride) {
   const int lane = threadIdx.x & 31;
   double s = 0.0;
@@ -87,19 +86,6 @@ __device__ __forceinline__ double warp_sum_fixed(const double* v, int n, size_t 
 }
 __device__ __forceinline__ double q_total(const ScfDev& S) {
   return warp_sum_fixed(S.qpart, S.nqpart, 1) * S.qscale;
-}
-__device__ __forceinline__ double q_total_serial(const ScfDev& S) {
-  double s[32];
-  for (int l = 0; l < 32; ++l) {
-    s[l] = 0.0;
-    for (int b = l; b < S.nqpart; b += 32) s[l] += S.qpart[b];
-  }
-  for (int o = 16; o > 0; o >>= 1) {
-    double t[32];
-    for (int l = 0; l < 32; ++l) t[l] = s[l] + s[l ^ o];
-    for (int l = 0; l < 32; ++l) s[l] = t[l];
-  }
-  return s[0] * S.qscale;
 }
 
 __device__ __forceinline__ double density_scale(const ScfDev& S, double Q) {
