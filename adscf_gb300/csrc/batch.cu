@@ -40,7 +40,7 @@
 #include "bulk_reg.cuh"
 #include "film_host.h"
 #include "film_kernels.cuh"
-#include "film_warp.cuh"
+#include "film_line.cuh"
 #include "adjoint_kernels.cuh"
 
 struct adscf_batch {
@@ -101,9 +101,10 @@ struct adscf_batch {
   void* d_f64 = nullptr;                // FilmDev<double>[n]
   int* d_list32 = nullptr;              // films sweeping in FP32 / FP64, by contour length
   int* d_list64 = nullptr;
-  // line sweeps by precision (0 FP32, 1 FP64) and warps per line (0: one warp
-  // per line; 1..4: 4, 8, 16, 32 warps): (film << 1) | chain, longest
-  // contours first; lines past 4096 rows are in d_long
+  // line sweeps by precision (0 FP32, 1 FP64) and class: (film << 1) | chain,
+  // longest contours first.  Class 0: one warp per line; 1..4: 4, 8, 16, 32 warps
+  // (FP64: class 1 has all of 257 to 1024 rows); lines past 4096 rows are in
+  // d_long
   int* d_fsweep[2][5] = {};
   int n_fsweep[2][5] = {};
   int* d_long[2] = {};                  // films of more than 4096 rows
@@ -828,7 +829,8 @@ int build_film(adscf_batch* b) {
       const int rows = b->npts[f];
       int k = 0;
       if (rows > kFilmGroupRows) { longl[f64p].push_back(f); continue; }
-      if (rows > kFilmWarpRows)
+      if (f64p && rows <= fl::kMaxRows) k = rows > kFilmWarpRows;
+      else if (rows > kFilmWarpRows)
         for (k = 1; (2 << k) < film_group_warps(rows);) ++k;
       sweep[f64p][k].push_back(f << 1);
       sweep[f64p][k].push_back((f << 1) | 1);
@@ -897,18 +899,33 @@ int build_film(adscf_batch* b) {
 }
 
 // chains of a batch's films of one precision: a warp per (film, chain) up to
-// 256 rows, 4 to 32 warps up to 4096, a thread per (film, chain) beyond
+// 256 rows, 4 to 32 warps up to 4096, a thread per (film, chain) beyond, with the
+// operations of the films' single contexts (film.cu)
 template <typename T>
 void film_sweeps(adscf_batch* b) {
   cudaStream_t s = b->stream;
   constexpr int p = sizeof(T) == 8;
   const FilmDev<T>* F = static_cast<const FilmDev<T>*>(p ? b->d_f64 : b->d_f32);
-  if (const int n = b->n_fsweep[p][0]) k_film1d_warp_b<T><<<(n + 3) / 4, 128, 0, s>>>(F, b->d_S, b->d_fsweep[p][0], n);
-  for (int k = 1; k < 5; ++k) {
+  int k = 1;
+  if (const int n = b->n_fsweep[p][0]) {
+    if constexpr (p) k_line_elim_b<1><<<(n + 3) / 4, fl::kThreads, fl::elim_bytes(fl::kMaxK), s>>>(F, b->d_S, b->d_fsweep[p][0], n);
+    else k_film1d_warp_b<<<(n + 3) / 4, 128, 0, s>>>(F, b->d_S, b->d_fsweep[p][0], n);
+  }
+  if constexpr (p) {
+    if (const int n = b->n_fsweep[p][1])
+      k_line_elim_b<4><<<n, fl::kThreads, fl::elim_bytes(fl::kMaxK), s>>>(F, b->d_S, b->d_fsweep[p][1], n);
+    k = 2;
+  }
+  for (; k < 5; ++k) {
     const int n = b->n_fsweep[p][k], threads = 32 * (2 << k);
     if (!n) continue;
-    if (threads <= 256) k_film1d_group_b<T, 256><<<n, threads, 0, s>>>(F, b->d_S, b->d_fsweep[p][k]);
-    else k_film1d_group_b<T, 1024><<<n, threads, 0, s>>>(F, b->d_S, b->d_fsweep[p][k]);
+    if constexpr (!p) {
+      if (threads <= 256) {
+        k_film1d_group_b<T, 256><<<n, threads, 0, s>>>(F, b->d_S, b->d_fsweep[p][k]);
+        continue;
+      }
+    }
+    k_film1d_group_b<T, 1024><<<n, threads, 0, s>>>(F, b->d_S, b->d_fsweep[p][k]);
   }
   if (const int n = b->n_long[p]) {
     const int W = p ? b->lanes64 : b->lanes32, zcap = p ? b->zcap64 : b->zcap32, pw = b->film_per_warp;
@@ -929,8 +946,8 @@ int enqueue_film(adscf_batch* b) {
   film_sweeps<double>(b);
   // one-line films: blocks of 128 points, twice as many resident films as
   // with 256 (a longer line takes its points in passes)
-  if (b->n32) k_film_contour_b<float><<<b->n32, 128, 0, s>>>(f32, b->d_list32);
-  if (b->n64) k_film_contour_b<double><<<b->n64, 256, 0, s>>>(f64, b->d_list64);
+  if (b->n32) k_film_contour_b<float><<<b->n32, kFilmContourB32, 0, s>>>(f32, b->d_list32);
+  if (b->n64) k_film_contour_b<double><<<b->n64, kFilmContourB64, 0, s>>>(f64, b->d_list64);
   launch_closure_b(b->d_S, b->max_slots, CL_MEANFIELD | CL_MIXDOTS, dim3(1, b->n), s, b->film_cl_threads);
   // each partial is summed by one warp whatever the block size
   k_solve_b<<<b->n, b->film_cl_threads, 0, s>>>(b->d_S, 1, 1);

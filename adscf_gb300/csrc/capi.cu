@@ -426,7 +426,7 @@ int adscf_ctx_create(const adscf_params* p, adscf_ctx** out) {
   S.lambda = p->lambda;
   S.lam_warm = p->lam_warm > 0 ? p->lam_warm : 1.0e-3;
   S.qpart = ctx->d_qpart;
-  S.nqpart = ctx->contour_blocks;
+  S.nqpart = ctx->qparts ? ctx->qparts : ctx->contour_blocks;
   S.qscale = ctx->geometry == ADSCF_BULK ? ctx->dvol : 1.0;
   S.part = ctx->d_part;
   S.npart_blocks = ctx->closure_blocks;

@@ -320,8 +320,8 @@ int adi_tune(adscf_ctx* ctx, FilmState* F, const FilmDev<float>& D, const FieldR
   return ADSCF_OK;
 }
 
-// Contour kernel of a film: 32 points a block with the nodes dealt to its
-// warps while those blocks fit the SMs in one wave (two of 1024 threads on
+// Contour kernel of a film: 32 points a block with the nodes' terms dealt to
+// its warps while those blocks fit the SMs in one wave (two of 1024 threads on
 // each of 152), one thread per point beyond, where the points alone fill them.
 constexpr int kFewPoints = 32 * 2 * 152;
 bool film_few_points(int npts) { return npts <= kFewPoints; }
@@ -331,49 +331,57 @@ void field_f32(const FilmDev<float>& D, const FieldRef& fr, size_t n, cudaStream
   k_film_wconv<<<(int)std::min<size_t>((n + 255) / 256, 152 * 4), 256, 0, s>>>(fr, D.wf, n);
 }
 
-// 1D chains of every line (film_warp.cuh): one warp per (line, chain) up to
-// 256 rows, several warps up to 4096, one thread per (line, chain) beyond.
-// FP64 lines whose warps find enough idle SMs spread them over a cluster
-// (one FP64 pipe per SM); with more (line, chain) pairs than that the SMs
-// are busy anyway and a line's warps share a CTA, whose barrier is cheaper.
-// FP64 lines of up to 1024 rows whose chains find an SM each apply factors made
-// ahead (film_line.cuh) in both chains of a propagation.  More lines keep the
-// SMs busy as they are, and the factors (27 to 56 KB a line and step) are kept
-// under 1 GB; without them the chains eliminate as they go.
+// 1D chains of every line.  FP64 lines of up to 1024 rows: film_line.cuh, whose
+// chains apply factors made ahead where they find an SM each (the factors, 9 to
+// 56 KB a line and step, are kept under 1 GB), else make them as they go: more
+// lines keep the SMs busy as they are, and the results are the same bits.
+bool line_ok(const FilmDev<double>& D) { return D.gz + 1 <= fl::kMaxRows; }
 bool line_factors_ok(const adscf_ctx* ctx) {
   const FilmState* F = ctx->film;
   const FilmDev<double>& D = F->f64;
-  if (!F->t64 || ctx->geometry == ADSCF_FILM_3D || D.gz + 1 > fl::kMaxRows || 2 * D.nlines > 152) return false;
-  const size_t step = fl::step_bytes(fl::rows_per_lane(D.gz + 1));
+  if (!F->t64 || ctx->geometry == ADSCF_FILM_3D || !line_ok(D) || 2 * D.nlines > 152) return false;
+  const size_t step = fl::step_bytes(D.gz + 1);
   return fl::kStages * step <= (size_t)F->optin - 1024 && step * D.ns * D.nlines <= ((size_t)1 << 30);
 }
-template <int K>
-int launch_line_t(adscf_ctx* ctx, const FilmDev<double>& D, const FieldRef& fr, cudaStream_t s) {
-  const size_t sm = fl::kStages * fl::step_bytes(K);
-  double2* fac = ctx->film->d_fac;
-  CK(cudaFuncSetAttribute(k_line_chain<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-  k_line_factors<K><<<dim3(D.ns, D.nlines), fl::kThreads, 0, s>>>(D, fr, fac);
-  k_line_chain<K><<<dim3(D.nlines, 2), fl::kThreads, sm, s>>>(D, fr, fac);
+template <int K, int W>
+int launch_line_t(const FilmDev<double>& D, const FieldRef& fr, double2* fac, int chains, cudaStream_t s) {
+  constexpr int per = fl::kThreads / (32 * W);   // lines or steps a block
+  if (!fac) {
+    k_line_elim<K, W><<<dim3((D.nlines + per - 1) / per, chains), fl::kThreads, fl::elim_bytes(K), s>>>(D, fr);
+    return ADSCF_OK;
+  }
+  const size_t sm = fl::kStages * fl::step_bytes(D.gz + 1);
+  if (cudaFuncSetAttribute(k_line_chain<K, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) != cudaSuccess)
+    return ADSCF_E_CUDA;
+  k_line_factors<K, W><<<dim3((D.ns + per - 1) / per, D.nlines), fl::kThreads, 0, s>>>(D, fr, fac);
+  k_line_chain<K, W><<<dim3(D.nlines, chains), 32 * W, sm, s>>>(D, fr, fac);
   return ADSCF_OK;
 }
-int launch_line(adscf_ctx* ctx, const FilmDev<double>& D, const FieldRef& fr, cudaStream_t s) {
-  switch (fl::rows_per_lane(D.gz + 1)) {
-    case 2: return launch_line_t<2>(ctx, D, fr, s);
-    case 3: return launch_line_t<3>(ctx, D, fr, s);
-    case 4: return launch_line_t<4>(ctx, D, fr, s);
-    case 5: return launch_line_t<5>(ctx, D, fr, s);
-    case 6: return launch_line_t<6>(ctx, D, fr, s);
-    case 7: return launch_line_t<7>(ctx, D, fr, s);
-    default: return launch_line_t<8>(ctx, D, fr, s);
-  }
+int launch_line(const FilmDev<double>& D, const FieldRef& fr, double2* fac, int chains, cudaStream_t s) {
+#define ADSCF_LINE_CALL(K, W) return launch_line_t<K, W>(D, fr, fac, chains, s)
+  ADSCF_LINE_SHAPE(D.gz + 1, ADSCF_LINE_CALL)
+#undef ADSCF_LINE_CALL
 }
 
+// The other lines (film_warp.cuh): FP32 one warp per (line, chain) up to 256
+// rows; several warps up to 4096, one thread per (line, chain) beyond.  FP64
+// lines whose warps find enough idle SMs spread them over a cluster
+// (one FP64 pipe per SM); with more (line, chain) pairs than that the SMs
+// are busy anyway and a line's warps share a CTA, whose barrier is cheaper.
 template <typename T>
 int launch_chains_1d(adscf_ctx* ctx, const FilmDev<T>& D, const FieldRef& fr, int chains, cudaStream_t s) {
   const int n = D.gz + 1;
-  if (n <= kFilmWarpRows) {
-    k_film1d_warp<T><<<dim3((D.nlines + 3) / 4, chains), 128, 0, s>>>(D, fr);
-  } else if (n <= kFilmGroupRows) {
+  if constexpr (sizeof(T) == 8) {
+    // a single step has no other to share factors with
+    if (line_ok(D)) {
+      const int rc = launch_line(D, fr, D.single ? nullptr : ctx->film->d_fac, chains, s);
+      return rc ? set_err(ctx, rc, "line chain attributes") : rc;
+    }
+  } else if (n <= kFilmWarpRows) {
+    k_film1d_warp<<<dim3((D.nlines + 3) / 4, chains), 128, 0, s>>>(D, fr);
+    return ADSCF_OK;
+  }
+  if (n <= kFilmGroupRows) {
     const int W = film_group_warps(n);
     const bool spread = sizeof(T) == 8 && (long long)D.nlines * chains * std::min(W, 8) <= 152;
     const int csize = spread ? std::min(W, 8) : 1;
@@ -416,9 +424,7 @@ int chains_t(adscf_ctx* ctx, const double* d_w) {
   } else {
     int rc = film_prepare(ctx);
     if (rc) return rc;
-    if constexpr (sizeof(T) == 8) rc = F->d_fac ? launch_line(ctx, D, fr, s) : launch_chains_1d<T>(ctx, D, fr, 2, s);
-    else rc = launch_chains_1d<T>(ctx, D, fr, 2, s);
-    if (rc) return rc;
+    if ((rc = launch_chains_1d<T>(ctx, D, fr, 2, s))) return rc;
   }
   CK(cudaGetLastError());
   return ADSCF_OK;
@@ -609,6 +615,7 @@ int film_create(adscf_ctx* ctx, const adscf_params* p) {
   }
   ctx->contour_blocks = film_few_points(ctx->npts) ? (ctx->npts + 31) / 32
                                                    : (int)std::min<size_t>(((size_t)ctx->npts + 255) / 256, 152 * 4);
+  if (film_few_points(ctx->npts) && ctx->gx * ctx->gy == 1) ctx->qparts = 1;   // block 0 has all of a line's Q
   CK(cudaMalloc(&ctx->d_qpart, ctx->contour_blocks * sizeof(double)));
   int rc = F->t64 ? alloc_t<double>(ctx, F, gam_elems) : alloc_t<float>(ctx, F, gam_elems);
   if (rc) return rc;
@@ -742,7 +749,7 @@ int film_prepare(adscf_ctx* ctx) {
   if (st != cudaStreamCaptureStatusNone) return ADSCF_OK;
   F->fac_tried = true;
   const FilmDev<double>& D = F->f64;
-  if (cudaMalloc(&F->d_fac, fl::step_bytes(fl::rows_per_lane(D.gz + 1)) * D.ns * D.nlines) != cudaSuccess) {
+  if (cudaMalloc(&F->d_fac, fl::step_bytes(D.gz + 1) * D.ns * D.nlines) != cudaSuccess) {
     cudaGetLastError();
     F->d_fac = nullptr;
   }

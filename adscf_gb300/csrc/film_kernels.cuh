@@ -489,17 +489,40 @@ __global__ void k_film_fill(T* __restrict__ q, T* __restrict__ qd, int n) {
 // would wait on.  FP64 slices keep plain FP64 accumulation.
 constexpr int kFilmContourChunk = 256;   // contour nodes per staged weight chunk
 
-__device__ __forceinline__ void ffw_add(float& sh, float& sl, float x, float y, float2 w) {
-  const float p = x * y;
-  const float e = fmaf(x, y, -p);                // x y = p + e exactly
-  const float t = p * w.x;
-  const float te = fmaf(p, w.x, -t);             // p wh = t + te exactly
-  const float lo = fmaf(e, w.x, fmaf(p, w.y, te));
-  const float s = sh + t;                        // TwoSum(sh, t)
-  const float bp = s - sh;
-  const float err = (sh - (s - bp)) + (t - bp);
-  sl += err + lo;
+// The term of one node and the sum it goes to, every operation rounded
+// explicitly: a film's densities are the same bits whatever kernel sums them.
+struct FfTerm {
+  float t, lo;           // x y w = t + lo
+};
+__device__ __forceinline__ FfTerm ffw_term(float x, float y, float2 w) {
+  const float p = __fmul_rn(x, y);
+  const float e = __fmaf_rn(x, y, -p);           // x y = p + e exactly
+  const float t = __fmul_rn(p, w.x);
+  const float te = __fmaf_rn(p, w.x, -t);        // p wh = t + te exactly
+  return FfTerm{t, __fmaf_rn(e, w.x, __fmaf_rn(p, w.y, te))};
+}
+__device__ __forceinline__ void ffw_add(float& sh, float& sl, FfTerm v) {
+  const float s = __fadd_rn(sh, v.t);            // TwoSum(sh, t)
+  const float bp = __fsub_rn(s, sh);
+  const float err = __fadd_rn(__fsub_rn(sh, __fsub_rn(s, bp)), __fsub_rn(v.t, bp));
+  sl = __fadd_rn(sl, __fadd_rn(err, v.lo));
   sh = s;
+}
+__device__ __forceinline__ float2 split_weight(double w) {
+  const float h = (float)w;
+  return make_float2(h, (float)(w - (double)h));
+}
+// thread k of n: its points' part of Q
+template <typename T>
+__device__ __forceinline__ double film_q_part(const FilmDev<T>& F, int k, int n) {
+  const size_t np = F.npts;
+  double qs = 0.0;
+  for (int p = k; p < F.npts; p += n) {
+    double qn = (double)F.q[(size_t)F.ns * np + p];
+    if (F.brush) qn = r_mul(qn, (double)F.qd[p]);
+    qs = r_fma(F.wz[p / F.nlines], qn, qs);
+  }
+  return qs;
 }
 
 template <typename T>
@@ -507,7 +530,6 @@ __device__ __forceinline__ void film_contour_body(const FilmDev<T>& F, int bid, 
   __shared__ double red[32];
   const int N = F.ns;
   const size_t np = F.npts;
-  double qs = 0.0;
   if constexpr (sizeof(T) == 4) {
     __shared__ float2 wsh[2][kFilmContourChunk];
     for (int pb = bid * blockDim.x; pb < F.npts; pb += nb * blockDim.x) {   // uniform per block
@@ -518,12 +540,8 @@ __device__ __forceinline__ void film_contour_body(const FilmDev<T>& F, int bid, 
         const int cn = min(kFilmContourChunk, N + 1 - s0);
         __syncthreads();
         for (int k = threadIdx.x; k < cn; k += blockDim.x) {
-          const double wa = F.wA[s0 + k];
-          const float wah = (float)wa;
-          wsh[0][k] = make_float2(wah, (float)(wa - (double)wah));
-          const double wb = F.ntypes == 2 ? F.wB[s0 + k] : 0.0;
-          const float wbh = (float)wb;
-          wsh[1][k] = make_float2(wbh, (float)(wb - (double)wbh));
+          wsh[0][k] = split_weight(F.wA[s0 + k]);
+          wsh[1][k] = split_weight(F.ntypes == 2 ? F.wB[s0 + k] : 0.0);
         }
         __syncthreads();
         if (ok) {
@@ -531,18 +549,14 @@ __device__ __forceinline__ void film_contour_body(const FilmDev<T>& F, int bid, 
           for (int k = 0; k < cn; ++k) {
             const int s = s0 + k;
             const float x = F.q[(size_t)s * np + p], y = F.qd[(size_t)(N - s) * np + p];
-            ffw_add(ah, al, x, y, wsh[0][k]);
-            if (F.ntypes == 2) ffw_add(bh, bl, x, y, wsh[1][k]);
+            ffw_add(ah, al, ffw_term(x, y, wsh[0][k]));
+            if (F.ntypes == 2) ffw_add(bh, bl, ffw_term(x, y, wsh[1][k]));
           }
         }
       }
       if (ok) {
         F.dist[p] = (double)ah + (double)al;
         if (F.ntypes == 2) F.dist[np + p] = (double)bh + (double)bl;
-        const int z = p / F.nlines;
-        double qn = (double)F.q[(size_t)N * np + p];
-        if (F.brush) qn *= (double)F.qd[p];
-        qs += F.wz[z] * qn;
       }
     }
   } else {
@@ -550,19 +564,15 @@ __device__ __forceinline__ void film_contour_body(const FilmDev<T>& F, int bid, 
       double a0 = 0.0, a1 = 0.0;
 #pragma unroll 4
       for (int s = 0; s <= N; ++s) {
-        const double pr = (double)F.q[(size_t)s * np + p] * (double)F.qd[(size_t)(N - s) * np + p];
-        a0 += F.wA[s] * pr;
-        if (F.ntypes == 2) a1 += F.wB[s] * pr;
+        const double pr = r_mul(F.q[(size_t)s * np + p], F.qd[(size_t)(N - s) * np + p]);
+        a0 = r_fma(F.wA[s], pr, a0);
+        if (F.ntypes == 2) a1 = r_fma(F.wB[s], pr, a1);
       }
       F.dist[p] = a0;
       if (F.ntypes == 2) F.dist[np + p] = a1;
-      const int z = p / F.nlines;
-      double qn = (double)F.q[(size_t)N * np + p];
-      if (F.brush) qn *= (double)F.qd[p];
-      qs += F.wz[z] * qn;
     }
   }
-  const double tot = block_reduce_1(qs, red);
+  const double tot = block_reduce_1(film_q_part(F, bid * blockDim.x + threadIdx.x, nb * blockDim.x), red);
   if (threadIdx.x == 0) F.qpart[bid] = tot;
 }
 
@@ -572,60 +582,60 @@ k_film_contour(FilmDev<T> F) { film_contour_body<T>(F, blockIdx.x, gridDim.x); }
 
 // The same for a film of few points: with one thread per point a 1001-point
 // line has four blocks, each thread waiting on Ns + 1 slice loads in turn.
-// Here a block takes 32 points and deals the nodes to its 32 warps (node s to
-// warp s mod 32), each summing as above; the 32 partial sums of a point are
-// added in FP64 in the order of the warps.
+// Here a block takes 32 points: warps 2 to 31 form the terms of 30 nodes at a
+// time, and warp 0 (block A or the homopolymer) and warp 1 (block B) add them
+// up in the order of the nodes, as the thread of film_contour_body does, while
+// the next 30 load.  Q of a one-line film is block 0's, by as many threads as
+// k_film_contour_b has: a batched film's Q and densities are those of its
+// context.  Bound: FP64 the additions, 64 cycles a node (101 nodes 3 us).
+constexpr int kFilmContourB32 = 128, kFilmContourB64 = 256;   // threads of k_film_contour_b
 template <typename T>
 __global__ void __launch_bounds__(1024)
 k_film_contour_s(FilmDev<T> F) {
-  __shared__ double part[2][32][33];
+  constexpr int NB = 30;
+  using Term = typename std::conditional<sizeof(T) == 4, FfTerm, double>::type;
+  __shared__ Term term[2][sizeof(T) == 4 ? 2 : 1][NB][32];
+  __shared__ double red[32];
   const int lane = threadIdx.x & 31, g = threadIdx.x >> 5;
   const int p = blockIdx.x * 32 + lane;
-  const int N = F.ns;
+  const int N = F.ns, types = F.ntypes;
   const size_t np = F.npts;
-  double a0 = 0.0, a1 = 0.0;
-  if (p < F.npts) {
-    if constexpr (sizeof(T) == 4) {
-      float ah = 0.f, al = 0.f, bh = 0.f, bl = 0.f;
-#pragma unroll 4
-      for (int s = g; s <= N; s += 32) {
-        const float x = F.q[(size_t)s * np + p], y = F.qd[(size_t)(N - s) * np + p];
-        const double wa = F.wA[s], wb = F.ntypes == 2 ? F.wB[s] : 0.0;
-        const float wah = (float)wa, wbh = (float)wb;
-        ffw_add(ah, al, x, y, make_float2(wah, (float)(wa - (double)wah)));
-        if (F.ntypes == 2) ffw_add(bh, bl, x, y, make_float2(wbh, (float)(wb - (double)wbh)));
+  const bool live = p < F.npts;
+  float sh = 0.f, sl = 0.f;
+  double a = 0.0;
+  for (int s0 = 0, buf = 0; s0 <= N; s0 += NB, buf ^= 1) {
+    const int s = s0 + g - 2;
+    if (g >= 2 && s <= N && live) {
+      const T x = F.q[(size_t)s * np + p], y = F.qd[(size_t)(N - s) * np + p];
+      if constexpr (sizeof(T) == 4) {
+        term[buf][0][g - 2][lane] = ffw_term(x, y, split_weight(F.wA[s]));
+        if (types == 2) term[buf][1][g - 2][lane] = ffw_term(x, y, split_weight(F.wB[s]));
+      } else {
+        term[buf][0][g - 2][lane] = r_mul(x, y);
       }
-      a0 = (double)ah + (double)al;
-      a1 = (double)bh + (double)bl;
-    } else {
-#pragma unroll 4
-      for (int s = g; s <= N; s += 32) {
-        const double pr = (double)F.q[(size_t)s * np + p] * (double)F.qd[(size_t)(N - s) * np + p];
-        a0 += F.wA[s] * pr;
-        if (F.ntypes == 2) a1 += F.wB[s] * pr;
+    }
+    __syncthreads();   // the other buffer's terms were added before this barrier
+    if (g < types && live) {
+      const double* w = (g == 0 ? F.wA : F.wB) + s0;
+      const int cn = min(NB, N + 1 - s0);
+#pragma unroll 10
+      for (int k = 0; k < cn; ++k) {
+        if constexpr (sizeof(T) == 4) ffw_add(sh, sl, term[buf][g][k][lane]);
+        else a = r_fma(w[k], term[buf][0][k][lane], a);
       }
     }
   }
-  part[0][g][lane] = a0;
-  part[1][g][lane] = a1;
-  __syncthreads();
-  if (g < F.ntypes && p < F.npts) {   // warp 0: block A (or homopolymer), warp 1: block B
-    double t = 0.0;
-#pragma unroll
-    for (int k = 0; k < 32; ++k) t += part[g][k][lane];
-    F.dist[(size_t)g * np + p] = t;
+  if (g < types && live) F.dist[(size_t)g * np + p] = sizeof(T) == 4 ? (double)sh + (double)sl : a;
+  double qs = 0.0;
+  if (F.nlines == 1) {
+    if (blockIdx.x > 0) return;
+    constexpr int n = sizeof(T) == 4 ? kFilmContourB32 : kFilmContourB64;
+    if (threadIdx.x < n) qs = film_q_part(F, threadIdx.x, n);
+  } else if (g == 0 && live) {
+    qs = film_q_part(F, p, F.npts);
   }
-  if (g == 0) {
-    double qn = 0.0;
-    if (p < F.npts) {
-      qn = (double)F.q[(size_t)N * np + p];
-      if (F.brush) qn *= (double)F.qd[p];
-      qn *= F.wz[p / F.nlines];
-    }
-#pragma unroll
-    for (int o = 16; o; o >>= 1) qn += __shfl_xor_sync(0xffffffffu, qn, o);
-    if (lane == 0) F.qpart[blockIdx.x] = qn;
-  }
+  const double tot = block_reduce_1(qs, red);
+  if (threadIdx.x == 0) F.qpart[blockIdx.x] = tot;
 }
 
 // ---------------------------------------------------------------------------

@@ -153,37 +153,29 @@ __device__ __forceinline__ void solve(const T (&a)[K], const T (&d)[K], const T 
 }  // namespace fw
 
 // ---------------------------------------------------------------------------
-// 1D CN chain (Film_1D / brush) with one warp per (line, chain): lane l owns
-// rows [l K, l K + K - 1] of the line's gz + 1 rows (K = film_warp_rows; rows
-// past the wall are identity padding), keeps their q in registers for the
-// whole contour, and solves each step with fw::solve.  `chain`: slices
+// 1D CN chain (Film_1D / brush, FP32 increment form, see cn_rhs) with one warp
+// per (line, chain): lane l owns rows [l K, l K + K - 1] of the line's gz + 1
+// rows (K = film_warp_rows; rows past the wall are identity padding), keeps
+// their q in registers for the whole contour, exchanges edge values by
+// shuffles, and solves each step with fw::solve.  `chain`: slices
 // [(ns+1)][npts] of the chain, rows of this line at stride `stride`.
-//
-// FP32 solves for the increment u = q' - q (see cn_rhs).  FP64 writes the
-// step (1 + ds M) q' = (1 - ds M) q as (1 + ds M) v = q, q' = 2 v - q (on the
-// walls v = q / 2, so q' = 0): the right-hand side is q itself, which spares
-// five FP64 operations a row and the neighbours' values on GB300's narrow
-// FP64 pipe.  The matrix is the reference's; the elimination order is not,
-// so results equal the serial Thomas solve to rounding.
-//
-// Bound: FP64 issue (a warp instruction per 64 cycles on each SM quarter), in
-// FP32 the latency of the solve's dependent operations.
-//
-// Per-warp shared memory `sm` holds, by row: the mesh factors alpha, gamma,
-// the term of types 0 and 1 that multiplies the step (FP32: the field, FP64:
-// beta + w / 2), and a staging row through which each finished slice goes to
-// global memory (coalesced for one-line films).
+// Per-warp shared memory `sm` holds, by row: the mesh factors alpha, gamma, the
+// field of types 0 and 1, and a staging row through which each finished
+// slice goes to global memory (coalesced for one-line films).
+// Bound: the latency of the solve's dependent operations.
 // ---------------------------------------------------------------------------
 constexpr int kFilmWarpM = 8;                 // rows per lane at most: lines up to 32 * 8 planes
 constexpr int kFilmWarpRows = 32 * kFilmWarpM;
-template <typename T>
 struct FilmWarpSm {
-  T al[kFilmWarpRows], ga[kFilmWarpRows], w0[kFilmWarpRows], w1[kFilmWarpRows], stage[kFilmWarpRows];
+  float al[kFilmWarpRows], ga[kFilmWarpRows], w0[kFilmWarpRows], w1[kFilmWarpRows], stage[kFilmWarpRows];
 };
 
 // One CN row of a step: matrix and right-hand side from the mesh factors al,
 // ga and the step's term w (FP32: field, FP64: beta + w / 2); qm, q0, qp: q
-// of the row and its neighbours (FP64 reads q0 only)
+// of the row and its neighbours (FP64 reads q0 only).  FP64 writes the step
+// (1 + ds M) q' = (1 - ds M) q as (1 + ds M) v = q, q' = 2 v - q (on the walls v
+// = q / 2, so q' = 0): the right-hand side is q itself, which spares five FP64
+// operations a row and the neighbours' values on GB300's narrow FP64 pipe.
 template <typename T>
 __device__ __forceinline__ void cn_line_row(const CnStep& st, T al, T ga, T w, T qm, T q0, T qp,
                                             T& a, T& d, T& c, T& r) {
@@ -207,18 +199,18 @@ __device__ __forceinline__ double cn_wall_rhs(double q) { return r_mul(0.5, q); 
 __device__ __forceinline__ float cn_new_q(float q, float u) { return __fadd_rn(q, u); }
 __device__ __forceinline__ double cn_new_q(double q, double u) { return r_fma(2.0, u, -q); }
 
-template <int K, typename T>
-__device__ __forceinline__ void film1d_chain_warp(const FilmDev<T>& F, int dir, T* chain,
-                                                  size_t stride, FilmWarpSm<T>& sm) {
+template <int K>
+__device__ __forceinline__ void film1d_chain_warp(const FilmDev<float>& F, int dir, float* chain,
+                                                  size_t stride, FilmWarpSm& sm) {
   const int lane = threadIdx.x & 31;
   const int n = F.gz + 1;
   const int s0 = lane * K;                    // this lane's rows s0 .. s0 + K - 1
-  T q[K];
+  float q[K];
 #pragma unroll
   for (int i = 0; i < K; ++i) {
     const int j = s0 + i;
-    T v = (T)0;
-    if (j < n) v = F.single ? chain[(size_t)j * stride] : (dir == 1 && F.brush) ? (T)F.graft[j] : (T)1;
+    float v = 0.f;
+    if (j < n) v = F.single ? chain[(size_t)j * stride] : (dir == 1 && F.brush) ? (float)F.graft[j] : 1.f;
     q[i] = v;
   }
   if (!F.single) {
@@ -232,30 +224,27 @@ __device__ __forceinline__ void film1d_chain_warp(const FilmDev<T>& F, int dir, 
   for (int s = 1; s <= F.ns; ++s) {
     const CnStep st = cn_step(film_ds(F.dss, dir, s, F.ns));
     const int ty = (F.brush || F.single) ? 0 : film_type(dir, s, F.ns, F.na);
-    const T* wl = ty == 0 ? sm.w0 : sm.w1;
-    // FP32: edge values of the neighbouring lanes' rows
-    T qprev = (T)0, qnext = (T)0;
-    if constexpr (sizeof(T) == 4) {
-      qprev = __shfl_up_sync(0xffffffffu, q[K - 1], 1);
-      qnext = __shfl_down_sync(0xffffffffu, q[0], 1);
-    }
-    T a[K], d[K], c[K], r[K];
+    const float* wl = ty == 0 ? sm.w0 : sm.w1;
+    // edge values of the neighbouring lanes' rows
+    const float qprev = __shfl_up_sync(0xffffffffu, q[K - 1], 1);
+    const float qnext = __shfl_down_sync(0xffffffffu, q[0], 1);
+    float a[K], d[K], c[K], r[K];
 #pragma unroll
     for (int i = 0; i < K; ++i) {
       const int j = s0 + i;
-      a[i] = (T)0; d[i] = (T)1; c[i] = (T)0; r[i] = (T)0;
+      a[i] = 0.f; d[i] = 1.f; c[i] = 0.f; r[i] = 0.f;
       if (j < n) {
         if (j == 0 || j == n - 1) {
           r[i] = cn_wall_rhs(q[i]);            // Dirichlet wall: q' = 0
         } else {
-          const T qm = i == 0 ? qprev : q[i > 0 ? i - 1 : 0];
-          const T qp = i == K - 1 ? qnext : q[i + 1 < K ? i + 1 : i];
-          cn_line_row<T>(st, sm.al[j], sm.ga[j], wl[j], qm, q[i], qp, a[i], d[i], c[i], r[i]);
+          const float qm = i == 0 ? qprev : q[i > 0 ? i - 1 : 0];
+          const float qp = i == K - 1 ? qnext : q[i + 1 < K ? i + 1 : i];
+          cn_line_row<float>(st, sm.al[j], sm.ga[j], wl[j], qm, q[i], qp, a[i], d[i], c[i], r[i]);
         }
       }
     }
     fw::solve<32, K>(a, d, c, r, false, F.err);
-    T* qn = chain + (size_t)s * F.npts;
+    float* qn = chain + (size_t)s * F.npts;
 #pragma unroll
     for (int i = 0; i < K; ++i) {
       q[i] = cn_new_q(q[i], r[i]);
@@ -270,9 +259,8 @@ __device__ __forceinline__ void film1d_chain_warp(const FilmDev<T>& F, int dir, 
 // rows per lane of an n-row line: the smallest K >= 2 with 32 K >= n
 __host__ __device__ __forceinline__ int film_warp_rows(int n) { return n <= 64 ? 2 : (n + 31) / 32; }
 
-template <typename T>
-__device__ __forceinline__ void film1d_chain_warp_any(const FilmDev<T>& F, int dir, T* chain,
-                                                      size_t stride, FilmWarpSm<T>& sm) {
+__device__ __forceinline__ void film1d_chain_warp_any(const FilmDev<float>& F, int dir, float* chain,
+                                                      size_t stride, FilmWarpSm& sm) {
   switch (film_warp_rows(F.gz + 1)) {
     case 2: film1d_chain_warp<2>(F, dir, chain, stride, sm); break;
     case 3: film1d_chain_warp<3>(F, dir, chain, stride, sm); break;
@@ -297,18 +285,16 @@ __device__ __forceinline__ T cn_term(const FilmDev<T>& F, int j, double w) {
   else return r_fma(0.5, w, F.beta[j]);
 }
 
-// mesh factors and field terms of one line into the warp's shared memory;
-// `field`: [ntypes][npts], rows of the line at stride `wstride` (FP32: the
-// rounding to FP32 that k_film_wconv makes)
-template <typename T>
-__device__ __forceinline__ void film_warp_tables(const FilmDev<T>& F, const double* field, size_t wstride,
-                                                 FilmWarpSm<T>& sm) {
+// mesh factors and FP32 field of one line into the warp's shared memory;
+// `field`: [ntypes][npts], rows of the line at stride `wstride`
+__device__ __forceinline__ void film_warp_tables(const FilmDev<float>& F, const double* field, size_t wstride,
+                                                 FilmWarpSm& sm) {
   const int lane = threadIdx.x & 31;
   for (int j = lane; j <= F.gz; j += 32) {
-    sm.al[j] = cn_mesh<T>(F, j, false);
-    sm.ga[j] = cn_mesh<T>(F, j, true);
-    sm.w0[j] = cn_term<T>(F, j, field[(size_t)j * wstride]);
-    sm.w1[j] = F.ntypes == 2 && !F.single ? cn_term<T>(F, j, field[F.npts + (size_t)j * wstride]) : (T)0;
+    sm.al[j] = F.alf[j];
+    sm.ga[j] = F.gaf[j];
+    sm.w0[j] = (float)field[(size_t)j * wstride];
+    sm.w1[j] = F.ntypes == 2 && !F.single ? (float)field[F.npts + (size_t)j * wstride] : 0.f;
   }
   __syncwarp();
 }
@@ -338,50 +324,40 @@ __device__ __forceinline__ bool film_line_dominant(const FilmDev<T>& F, const do
 
 // Single context (Film_1D / brush lines of one film): one warp per (line,
 // chain); blockIdx.y = chain.
-template <typename T>
-__global__ void __launch_bounds__(128)
-k_film1d_warp(FilmDev<T> F, FieldRef fr) {
-  __shared__ FilmWarpSm<T> sm_all[4];
+static __global__ void __launch_bounds__(128)
+k_film1d_warp(FilmDev<float> F, FieldRef fr) {
+  __shared__ FilmWarpSm sm_all[4];
   const int wib = threadIdx.x >> 5;
   const int line = blockIdx.x * 4 + wib;
   if (line >= F.nlines) return;
   const int dir = blockIdx.y;
   const size_t L = F.nlines;
-  FilmWarpSm<T>& sm = sm_all[wib];
-  if (sizeof(T) == 8 && !film_line_dominant<T>(F, fr.get() + line, L)) {
-    if ((threadIdx.x & 31) == 0) film1d_chain<T>(F, fr.get(), line, dir);
-    return;
-  }
-  film_warp_tables<T>(F, fr.get() + line, L, sm);
-  film1d_chain_warp_any<T>(F, dir, (dir == 0 ? F.q : F.qd) + line, L, sm);
+  FilmWarpSm& sm = sm_all[wib];
+  film_warp_tables(F, fr.get() + line, L, sm);
+  film1d_chain_warp_any(F, dir, (dir == 0 ? F.q : F.qd) + line, L, sm);
 }
 
 // Batch: one warp per (film, chain) of `items` ((film << 1) | chain, longest
 // contours first), the field from the film's current SCF history slot.
-template <typename T>
-__global__ void __launch_bounds__(128)
-k_film1d_warp_b(const FilmDev<T>* __restrict__ Fs, const ScfDev* __restrict__ Ss,
+static __global__ void __launch_bounds__(128)
+k_film1d_warp_b(const FilmDev<float>* __restrict__ Fs, const ScfDev* __restrict__ Ss,
                 const int* __restrict__ items, int nitems) {
-  __shared__ FilmWarpSm<T> sm_all[4];
+  __shared__ FilmWarpSm sm_all[4];
   const int wib = threadIdx.x >> 5;
   const int it = blockIdx.x * 4 + wib;
   if (it >= nitems) return;
   const int f = items[it] >> 1, dir = items[it] & 1;
-  const FilmDev<T> F = Fs[f];
+  const FilmDev<float> F = Fs[f];
   const ScfDev& S = Ss[f];
   const double* field = S.hx + (size_t)((*S.iter) % S.slots) * ((size_t)S.ntypes * S.npts);
-  FilmWarpSm<T>& sm = sm_all[wib];
-  if (sizeof(T) == 8 && !film_line_dominant<T>(F, field, 1)) {
-    if ((threadIdx.x & 31) == 0) film1d_chain<T>(F, field, 0, dir);
-    return;
-  }
-  film_warp_tables<T>(F, field, 1, sm);
-  film1d_chain_warp_any<T>(F, dir, dir == 0 ? F.q : F.qd, 1, sm);
+  FilmWarpSm& sm = sm_all[wib];
+  film_warp_tables(F, field, 1, sm);
+  film1d_chain_warp_any(F, dir, dir == 0 ? F.q : F.qd, 1, sm);
 }
 
 // ---------------------------------------------------------------------------
-// Longer lines (257 .. 4096 rows): W warps per (line, chain), K = 4 rows per
-// lane, W the power of two >= rows / 128.  Each warp reduces its 128 rows to
+// Longer lines (FP32 257 .. 4096 rows, FP64 1025 .. 4096, film_line.cuh has the
+// shorter ones): W warps per (line, chain), K = 4 rows per lane, W the power of two >= rows / 128.  Each warp reduces its 128 rows to
 // one equation in the last rows of itself and its neighbours:
 //  - lanes eliminate their interior rows (fw::eliminate), then the warp's 31
 //    first separators by cyclic reduction with the warp's two boundary
@@ -400,10 +376,9 @@ k_film1d_warp_b(const FilmDev<T>* __restrict__ Fs, const ScfDev* __restrict__ Ss
 // cluster's.  Many lines keep their warps in one CTA (clusters of one).  The
 // arithmetic is the same either way: K and W depend on the line length alone.
 // Bound: FP64 issue, one warp instruction per 64 cycles on each SM quarter.
-// Measured (GB300, FP64, against one thread per line and chain): brush of
-// 1001 rows and 1200 steps 1368 -> 11.1 ms; an SCF iteration of a 501-row
-// film with 100 steps 56.8 -> 0.91 ms (with the factors made ahead, where
-// film_line.cuh takes the line, 4.2 and 0.27).
+// Measured (GB300, one line, against one thread per line and chain; a step of
+// both chains): FP64 2001 rows 2290 -> 17 us; FP32 301 rows 52 -> 8.6 us, 1001
+// rows 157 -> 9.6.
 // ---------------------------------------------------------------------------
 constexpr int kFilmGroupK = 4;
 constexpr int kFilmGroupMaxW = 32;

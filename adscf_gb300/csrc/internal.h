@@ -76,6 +76,7 @@ struct adscf_ctx {
   int autotune = 1;
   std::string tune_report;
   int contour_blocks = 0;
+  int qparts = 0;                     // partial sums of Q they leave (0: one each)
 
   // ---- SCF state (FP64)
   ScfDev S{};
