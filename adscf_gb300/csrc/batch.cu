@@ -103,12 +103,14 @@ struct adscf_batch {
   int* d_list64 = nullptr;
   // line sweeps by precision (0 FP32, 1 FP64) and class: (film << 1) | chain,
   // longest contours first.  Class 0: one warp per line; 1..4: 4, 8, 16, 32 warps
-  // (FP64: class 1 has all of 257 to 1024 rows); lines past 4096 rows are in
-  // d_long
+  // (FP64: class 1 has all of 257 to 1024 rows)
   int* d_fsweep[2][5] = {};
   int n_fsweep[2][5] = {};
-  int* d_long[2] = {};                  // films of more than 4096 rows
-  int n_long[2] = {};
+  // films that may run the recurrence, a thread per chain, and which of them do:
+  // always past 4096 rows, else as their sweep finds (film_line_serial)
+  int* d_ser[2] = {};
+  int n_ser[2] = {};
+  int* d_serial = nullptr;              // [n]
   int n32 = 0, n64 = 0;
   // shared-memory line sweeps: rows per line (max gz + 1 of the list) and
   // lanes per block (0: the list sweeps on global memory)
@@ -823,12 +825,13 @@ int build_film(adscf_batch* b) {
   };
   std::stable_sort(l32.begin(), l32.end(), by_work);
   std::stable_sort(l64.begin(), l64.end(), by_work);
-  std::vector<int> sweep[2][5], longl[2];
+  std::vector<int> sweep[2][5], ser[2], serial(n, 0);
   for (int f64p = 0; f64p < 2; ++f64p)
     for (int f : f64p ? l64 : l32) {
       const int rows = b->npts[f];
       int k = 0;
-      if (rows > kFilmGroupRows) { longl[f64p].push_back(f); continue; }
+      if (f64p || rows > kFilmWarpRows) ser[f64p].push_back(f);
+      if (rows > kFilmGroupRows) { serial[f] = 1; continue; }
       if (f64p && rows <= fl::kMaxRows) k = rows > kFilmWarpRows;
       else if (rows > kFilmWarpRows)
         for (k = 1; (2 << k) < film_group_warps(rows);) ++k;
@@ -840,8 +843,8 @@ int build_film(adscf_batch* b) {
   b->film_cl_threads = closure_threads(max_npts);
   b->n32 = (int)l32.size();
   b->n64 = (int)l64.size();
-  // layout of the shared-memory sweeps of lines past 4096 rows: one thread
-  // per (film, chain) runs a serial recurrence, so the first `per_warp` lanes of each warp work and
+  // layout of the shared-memory sweeps: one thread per (film, chain) runs a
+  // serial recurrence, so the first `per_warp` lanes of each warp work and
   // a block holds `warps` warps: W = warps * per_warp lines share the
   // block's shared memory.  ADSCF_FILM_LANES / ADSCF_FILM_WARPS override.
   {
@@ -861,8 +864,8 @@ int build_film(adscf_batch* b) {
       W = warps * b->film_per_warp;
       if (warps == 0) W = 0;
     };
-    lanes(longl[0], sizeof(float), b->zcap32, b->lanes32);
-    lanes(longl[1], sizeof(double), b->zcap64, b->lanes64);
+    lanes(ser[0], sizeof(float), b->zcap32, b->lanes32);
+    lanes(ser[1], sizeof(double), b->zcap64, b->lanes64);
     BK(cudaFuncSetAttribute(k_film1d_chains_sm<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
     BK(cudaFuncSetAttribute(k_film1d_chains_sm<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
   }
@@ -882,10 +885,12 @@ int build_film(adscf_batch* b) {
     return ADSCF_OK;
   };
   for (int p = 0; p < 2; ++p) {
-    int rc = up(longl[p], b->d_long[p], b->n_long[p]);
+    int rc = up(ser[p], b->d_ser[p], b->n_ser[p]);
     for (int k = 0; k < 5 && !rc; ++k) rc = up(sweep[p][k], b->d_fsweep[p][k], b->n_fsweep[p][k]);
     if (rc) return rc;
   }
+  BK(cudaMalloc(&b->d_serial, n * sizeof(int)));
+  BK(cudaMemcpyAsync(b->d_serial, serial.data(), n * sizeof(int), cudaMemcpyHostToDevice, b->stream));
   if (!l64.empty())
     BK(cudaMemcpyAsync(b->d_list64, l64.data(), l64.size() * sizeof(int), cudaMemcpyHostToDevice, b->stream));
   BK(cudaMalloc(&b->d_S, n * sizeof(ScfDev)));
@@ -899,8 +904,9 @@ int build_film(adscf_batch* b) {
 }
 
 // chains of a batch's films of one precision: a warp per (film, chain) up to
-// 256 rows, 4 to 32 warps up to 4096, a thread per (film, chain) beyond, with the
-// operations of the films' single contexts (film.cu)
+// 256 rows, 4 to 32 warps up to 4096, with the operations of the films' single
+// contexts (film.cu), then a thread per (film, chain) for the films of more rows
+// and those whose systems are not diagonally dominant
 template <typename T>
 void film_sweeps(adscf_batch* b) {
   cudaStream_t s = b->stream;
@@ -908,12 +914,12 @@ void film_sweeps(adscf_batch* b) {
   const FilmDev<T>* F = static_cast<const FilmDev<T>*>(p ? b->d_f64 : b->d_f32);
   int k = 1;
   if (const int n = b->n_fsweep[p][0]) {
-    if constexpr (p) k_line_elim_b<1><<<(n + 3) / 4, fl::kThreads, fl::elim_bytes(fl::kMaxK), s>>>(F, b->d_S, b->d_fsweep[p][0], n);
+    if constexpr (p) k_line_elim_b<1><<<(n + 3) / 4, fl::kThreads, fl::elim_bytes(fl::kMaxK), s>>>(F, b->d_S, b->d_fsweep[p][0], n, b->d_serial);
     else k_film1d_warp_b<<<(n + 3) / 4, 128, 0, s>>>(F, b->d_S, b->d_fsweep[p][0], n);
   }
   if constexpr (p) {
     if (const int n = b->n_fsweep[p][1])
-      k_line_elim_b<4><<<n, fl::kThreads, fl::elim_bytes(fl::kMaxK), s>>>(F, b->d_S, b->d_fsweep[p][1], n);
+      k_line_elim_b<4><<<n, fl::kThreads, fl::elim_bytes(fl::kMaxK), s>>>(F, b->d_S, b->d_fsweep[p][1], n, b->d_serial);
     k = 2;
   }
   for (; k < 5; ++k) {
@@ -921,20 +927,20 @@ void film_sweeps(adscf_batch* b) {
     if (!n) continue;
     if constexpr (!p) {
       if (threads <= 256) {
-        k_film1d_group_b<T, 256><<<n, threads, 0, s>>>(F, b->d_S, b->d_fsweep[p][k]);
+        k_film1d_group_b<T, 256><<<n, threads, 0, s>>>(F, b->d_S, b->d_fsweep[p][k], b->d_serial);
         continue;
       }
     }
-    k_film1d_group_b<T, 1024><<<n, threads, 0, s>>>(F, b->d_S, b->d_fsweep[p][k]);
+    k_film1d_group_b<T, 1024><<<n, threads, 0, s>>>(F, b->d_S, b->d_fsweep[p][k], b->d_serial);
   }
-  if (const int n = b->n_long[p]) {
+  if (const int n = b->n_ser[p]) {
     const int W = p ? b->lanes64 : b->lanes32, zcap = p ? b->zcap64 : b->zcap32, pw = b->film_per_warp;
     if (W)
       k_film1d_chains_sm<T><<<dim3((n + W - 1) / W, 2), 32 * (W / pw), film_sweep_smem(zcap, W, sizeof(T)), s>>>(
-          F, b->d_S, b->d_long[p], n, zcap, pw);
+          F, b->d_S, b->d_ser[p], n, zcap, pw, b->d_serial);
     else
       k_film1d_chains_b<T><<<dim3((n + FILM_THREADS - 1) / FILM_THREADS, 2), FILM_THREADS, 0, s>>>(
-          F, b->d_S, b->d_long[p], n);
+          F, b->d_S, b->d_ser[p], n, b->d_serial);
   }
 }
 
@@ -1483,11 +1489,12 @@ int adscf_batch_destroy(adscf_batch* b) {
   for (auto& C : b->cls) { cudaFree(C.wx); cudaFree(C.wy); cudaFree(C.wz); }
   cudaFree(b->d_f32); cudaFree(b->d_f64); cudaFree(b->d_list32); cudaFree(b->d_list64);
   for (int p = 0; p < 2; ++p) {
-    cudaFree(b->d_long[p]);
+    cudaFree(b->d_ser[p]);
     for (int* d : b->d_fsweep[p]) cudaFree(d);
   }
   cudaFree(b->d_items); cudaFree(b->d_ctl); cudaFree(b->d_ranges);
   cudaFree(b->d_tabf);
+  cudaFree(b->d_serial);
   cudaFree(b->d_foff);
   cudaFree(b->d_pack);
   if (b->h_pinned) cudaFreeHost(b->h_pinned);
@@ -1563,7 +1570,7 @@ int adscf_batch_launches(const adscf_batch* b) {
   if (b->film) {
     int k = (b->n32 > 0) + (b->n64 > 0) + 3;   // contours, closure, solve, mix
     for (int p = 0; p < 2; ++p) {
-      k += b->n_long[p] > 0;
+      k += b->n_ser[p] > 0;
       for (int c : b->n_fsweep[p]) k += c > 0;
     }
     return k;

@@ -36,6 +36,7 @@ struct FilmState {
   int* d_err = nullptr;
   double2* d_fac = nullptr;     // factors of every step (film_line.cuh), from the first propagation on
   bool fac_tried = false;
+  int* d_serial = nullptr;      // contexts of several lines: those that run the recurrence (film_line_serial)
   double max_ratio = 1.0;       // largest neighbour spacing ratio of the mesh
   int optin = 0;                // opt-in shared memory per block
   // free energy at fixed fields and its wall-potential gradient
@@ -344,23 +345,43 @@ bool line_factors_ok(const adscf_ctx* ctx) {
   return fl::kStages * step <= (size_t)F->optin - 1024 && step * D.ns * D.nlines <= ((size_t)1 << 30);
 }
 template <int K, int W>
-int launch_line_t(const FilmDev<double>& D, const FieldRef& fr, double2* fac, int chains, cudaStream_t s) {
+int launch_line_t(const FilmDev<double>& D, const FieldRef& fr, double2* fac, int* serial, int chains, cudaStream_t s) {
   constexpr int per = fl::kThreads / (32 * W);   // lines or steps a block
   if (!fac) {
-    k_line_elim<K, W><<<dim3((D.nlines + per - 1) / per, chains), fl::kThreads, fl::elim_bytes(K), s>>>(D, fr);
+    k_line_elim<K, W><<<dim3((D.nlines + per - 1) / per, chains), fl::kThreads, fl::elim_bytes(K), s>>>(D, fr, serial);
     return ADSCF_OK;
   }
   const size_t sm = fl::kStages * fl::step_bytes(D.gz + 1);
   if (cudaFuncSetAttribute(k_line_chain<K, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) != cudaSuccess)
     return ADSCF_E_CUDA;
   k_line_factors<K, W><<<dim3((D.ns + per - 1) / per, D.nlines), fl::kThreads, 0, s>>>(D, fr, fac);
-  k_line_chain<K, W><<<dim3(D.nlines, chains), 32 * W, sm, s>>>(D, fr, fac);
+  k_line_chain<K, W><<<dim3(D.nlines, chains), 32 * W, sm, s>>>(D, fr, fac, serial);
   return ADSCF_OK;
 }
-int launch_line(const FilmDev<double>& D, const FieldRef& fr, double2* fac, int chains, cudaStream_t s) {
-#define ADSCF_LINE_CALL(K, W) return launch_line_t<K, W>(D, fr, fac, chains, s)
+int launch_line(const FilmDev<double>& D, const FieldRef& fr, double2* fac, int* serial, int chains, cudaStream_t s) {
+#define ADSCF_LINE_CALL(K, W) return launch_line_t<K, W>(D, fr, fac, serial, chains, s)
   ADSCF_LINE_SHAPE(D.gz + 1, ADSCF_LINE_CALL)
 #undef ADSCF_LINE_CALL
+}
+
+// FP64 lines so many that a thread each keeps the FP64 pipes busy, with fewer
+// instructions than the cooperative solves where those have few rows a lane or
+// spill.  us a step of both chains, cooperative and a thread each: 64 rows 157 and
+// 168 at 12288 lines, 201 and 171 at 16384; 128 rows 416 and 495 at 24576, 1075 and
+// 1083 at 65536; 256 rows 1774 and 2178 there; 301 rows 358 and 484 at 4096, 698 and
+// 609 at 8192; 501 rows 1216 and 1359 at 12288, 1612 and 1401 at 16384; 640 rows
+// 1763 and 1791 at 16384, 768 rows 3843 and 3810 at 32768, 1024 rows 4584 and 5090
+// there; 1101 rows 1920 and 2226 at 4096, 3820 and 2331 at 8192; 4001 rows 5173 and
+// 8280 at 4096, 10323 and 8538 at 8192.  FP32 lines of several warps are ahead at
+// any number (301 rows, 32768 lines: 373 and 414).
+template <typename T>
+bool film_line_crowd(int rows, int lines) {
+  if (sizeof(T) == 4) return false;
+  if (rows <= 112) return lines > 12288;
+  if (rows <= kFilmWarpRows) return false;
+  if (rows <= 352) return lines > 6144;
+  if (rows <= 704) return lines > 12288;
+  return rows > fl::kMaxRows && lines > 4096;
 }
 
 // The other lines (film_warp.cuh): FP32 one warp per (line, chain) up to 256
@@ -371,17 +392,27 @@ int launch_line(const FilmDev<double>& D, const FieldRef& fr, double2* fac, int 
 template <typename T>
 int launch_chains_1d(adscf_ctx* ctx, const FilmDev<T>& D, const FieldRef& fr, int chains, cudaStream_t s) {
   const int n = D.gz + 1;
-  if constexpr (sizeof(T) == 8) {
-    // a single step has no other to share factors with
-    if (line_ok(D)) {
-      const int rc = launch_line(D, fr, D.single ? nullptr : ctx->film->d_fac, chains, s);
-      return rc ? set_err(ctx, rc, "line chain attributes") : rc;
+  const dim3 g((D.nlines + FILM_THREADS - 1) / FILM_THREADS, chains);
+  int* serial = ctx->film->d_serial;
+  if constexpr (sizeof(T) == 4) {
+    if (n <= kFilmWarpRows) {
+      k_film1d_warp<<<dim3((D.nlines + 3) / 4, chains), 128, 0, s>>>(D, fr);
+      return ADSCF_OK;
     }
-  } else if (n <= kFilmWarpRows) {
-    k_film1d_warp<<<dim3((D.nlines + 3) / 4, chains), 128, 0, s>>>(D, fr);
+  }
+  if (n > kFilmGroupRows || film_line_crowd<T>(n, D.nlines)) {
+    if constexpr (sizeof(T) == 4) field_f32(D, fr, (size_t)(D.single ? 1 : D.ntypes) * D.npts, s);
+    k_film1d_chains<T><<<g, FILM_THREADS, 0, s>>>(D, fr, nullptr);
     return ADSCF_OK;
   }
-  if (n <= kFilmGroupRows) {
+  bool line = false;
+  if constexpr (sizeof(T) == 8) {
+    line = line_ok(D);
+    // a single step has no other to share factors with
+    const int rc = line ? launch_line(D, fr, D.single ? nullptr : ctx->film->d_fac, serial, chains, s) : ADSCF_OK;
+    if (rc) return set_err(ctx, rc, "line chain attributes");
+  }
+  if (!line) {
     const int W = film_group_warps(n);
     const bool spread = sizeof(T) == 8 && (long long)D.nlines * chains * std::min(W, 8) <= 152;
     const int csize = spread ? std::min(W, 8) : 1;
@@ -396,12 +427,10 @@ int launch_chains_1d(adscf_ctx* ctx, const FilmDev<T>& D, const FieldRef& fr, in
     at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = csize > 1 ? 1 : 0;
-    if (cfg.blockDim.x <= 256) CK(cudaLaunchKernelEx(&cfg, k_film1d_group<T, 256>, D, fr, csize));
-    else CK(cudaLaunchKernelEx(&cfg, k_film1d_group<T, 1024>, D, fr, csize));
-  } else {
-    const dim3 g((D.nlines + FILM_THREADS - 1) / FILM_THREADS, chains);
-    k_film1d_chains<T><<<g, FILM_THREADS, 0, s>>>(D, fr);
+    if (cfg.blockDim.x <= 256) CK(cudaLaunchKernelEx(&cfg, k_film1d_group<T, 256>, D, fr, csize, serial));
+    else CK(cudaLaunchKernelEx(&cfg, k_film1d_group<T, 1024>, D, fr, csize, serial));
   }
+  if (serial) k_film1d_chains<T><<<g, FILM_THREADS, 0, s>>>(D, fr, serial);
   return ADSCF_OK;
 }
 
@@ -611,7 +640,9 @@ int film_create(adscf_ctx* ctx, const adscf_params* p) {
     }
     CK(cudaMalloc(&F->d_alf, f3.size() * sizeof(float)));
     CK(cudaMemcpy(F->d_alf, f3.data(), f3.size() * sizeof(float), cudaMemcpyHostToDevice));
-    if (ctx->geometry == ADSCF_FILM_3D) CK(cudaMalloc(&F->d_wf, (size_t)ctx->ntypes * ctx->npts * sizeof(float)));
+    const int rows = ctx->gz + 1, lines = ctx->gx * ctx->gy;
+    const int copies = ctx->geometry == ADSCF_FILM_3D || rows > kFilmGroupRows ? 1 : rows > kFilmWarpRows && lines > 1 ? 2 : 0;
+    if (copies) CK(cudaMalloc(&F->d_wf, (size_t)copies * ctx->ntypes * ctx->npts * sizeof(float)));
   }
   ctx->contour_blocks = film_few_points(ctx->npts) ? (ctx->npts + 31) / 32
                                                    : (int)std::min<size_t>(((size_t)ctx->npts + 255) / 256, 152 * 4);
@@ -631,9 +662,12 @@ int film_create(adscf_ctx* ctx, const adscf_params* p) {
     // FP64 sweeps: one thread per line only where the lines are too long
     F->adi_any = F->t64 && F->any_ok;
   }
+  const int rows = ctx->gz + 1;
+  if (ctx->geometry != ADSCF_FILM_3D && ctx->gx * ctx->gy > 1 && rows <= kFilmGroupRows && (F->t64 || rows > kFilmWarpRows) &&
+      !(F->t64 && film_line_crowd<double>(rows, ctx->gx * ctx->gy)))
+    CK(cudaMalloc(&F->d_serial, ctx->gx * ctx->gy * sizeof(int)));
   ctx->film_launches = ctx->geometry == ADSCF_FILM_3D ? 1 + F->adi_any + (F->adi_any ? 2 : 3) * ctx->ns
-                       : line_factors_ok(ctx)            ? 2
-                                                         : 1;
+                                                      : (line_factors_ok(ctx) ? 2 : 1) + (F->d_serial != nullptr);
   ctx->film_contour_launches = 1;
   if (ctx->geometry == ADSCF_FILM_3D && !F->t64) {   // FP32 ADI sweeps: pick their shapes
     FilmDev<float>& D = F->f32;
@@ -734,6 +768,7 @@ void film_destroy(adscf_ctx* ctx) {
   cudaFree(F->d_alf); cudaFree(F->d_wf);
   cudaFree(F->d_q); cudaFree(F->d_qd); cudaFree(F->d_gam); cudaFree(F->d_w1);
   cudaFree(F->d_err); cudaFree(ctx->d_qpart); cudaFree(F->d_fac); cudaFree(F->d_anyfac);
+  cudaFree(F->d_serial);
   delete F;
   ctx->film = nullptr;
 }
@@ -753,7 +788,7 @@ int film_prepare(adscf_ctx* ctx) {
     cudaGetLastError();
     F->d_fac = nullptr;
   }
-  ctx->film_launches = F->d_fac ? 2 : 1;
+  ctx->film_launches = (F->d_fac ? 2 : 1) + (F->d_serial != nullptr);
   return ADSCF_OK;
 }
 

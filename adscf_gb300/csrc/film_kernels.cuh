@@ -61,8 +61,9 @@ struct FilmDev {
   double hx2, hy2;       // 1 / (2 dx dx), 1 / (2 dy dy)
   T* w1;                 // [2][npts] intermediate q*, q** of the ADI sweeps
   T* fac;                // x and y factors by schedule entry (film_any.cuh), from entry 1
-  // FP32 sweeps: FP32 copies of the mesh factors and, for the ADI sweeps, of
-  // the field ([ntypes][npts], filled per propagation)
+  // FP32 sweeps: FP32 copies of the mesh factors and of the field, filled per
+  // propagation (ADI sweeps, chains of more than 4096 rows: [ntypes][npts]; contexts
+  // of several lines: [chain][ntypes][npts], of those that run the recurrence)
   const float* alf;
   const float* bef;
   const float* gaf;
@@ -198,7 +199,8 @@ __device__ __forceinline__ double film_ds(const double* dss, int dir, int s, int
 // blockIdx.y = chain (0 forward, 1 backward).
 // ---------------------------------------------------------------------------
 template <typename T>
-__device__ __forceinline__ void film1d_chain(const FilmDev<T>& F, const double* field, int line, int dir) {
+__device__ __forceinline__ void film1d_chain(const FilmDev<T>& F, const double* field, int line, int dir,
+                                             bool own_copy = true) {
   const int L = F.nlines, gz = F.gz;
   T* chain = dir == 0 ? F.q : F.qd;
   T* gam = F.gam + (size_t)dir * (gz + 1) * L;
@@ -206,10 +208,27 @@ __device__ __forceinline__ void film1d_chain(const FilmDev<T>& F, const double* 
   if (!F.single)
     for (int j = 0; j <= gz; ++j)
       chain[(size_t)j * L + line] = (dir == 1 && F.brush) ? (T)F.graft[j] : (T)1;
+  // FP32, where the film has the memory: the field in FP32, half the traffic of
+  // every step; own_copy: this chain makes a copy of its line's here
+  float* wl = nullptr;
+  if constexpr (sizeof(T) == 4) {
+    wl = F.wf;
+    if (wl && own_copy) {
+      const int types = F.single ? 1 : F.ntypes;
+      wl += (size_t)dir * F.ntypes * F.npts;
+      for (int ty = 0; ty < types; ++ty)
+#pragma unroll 16
+        for (int j = 0; j <= gz; ++j) {
+          const size_t i = (size_t)ty * F.npts + (size_t)j * L + line;
+          wl[i] = (float)field[i];
+        }
+    }
+  }
   for (int s = 1; s <= F.ns; ++s) {
     const CnStep st = cn_step(film_ds(F.dss, dir, s, F.ns));
     const int ty = (F.brush || F.single) ? 0 : film_type(dir, s, F.ns, F.na);
     const double* w = field + (size_t)ty * F.npts;
+    const float* ws = wl ? wl + (size_t)ty * F.npts : nullptr;
     const T* qp = chain + (size_t)(s - 1) * F.npts;
     T* qn = chain + (size_t)s * F.npts;
     // forward elimination (increment form for FP32 sweeps, see cn_rhs)
@@ -225,7 +244,8 @@ __device__ __forceinline__ void film1d_chain(const FilmDev<T>& F, const double* 
         const T q_jp1 = qp[(size_t)(j + 1) * L + line];
         const size_t i = (size_t)j * L + line;
         T b, hw;
-        cn_row<T>(F, st, j, w[i], (float)w[i], a, c, b, hw);
+        if constexpr (sizeof(T) == 4) cn_row<T>(F, st, j, 0.0, ws ? ws[i] : (float)w[i], a, c, b, hw);
+        else cn_row<T>(F, st, j, w[i], 0.f, a, c, b, hw);
         diag = r_add(r_add((T)1, b), hw);
         rhs = cn_rhs<T>(a, b, c, hw, q_jm1, q_j, q_jp1);
         q_jm1 = q_j;
@@ -257,10 +277,10 @@ static __global__ void k_film_wconv(FieldRef fr, float* __restrict__ wf, size_t 
 
 template <typename T>
 __global__ void __launch_bounds__(FILM_THREADS)
-k_film1d_chains(FilmDev<T> F, FieldRef fr) {
+k_film1d_chains(FilmDev<T> F, FieldRef fr, const int* __restrict__ only) {   // only: the marked lines, or null (all)
   const int line = blockIdx.x * blockDim.x + threadIdx.x;
-  if (line >= F.nlines) return;
-  film1d_chain<T>(F, fr.get(), line, blockIdx.y);
+  if (line >= F.nlines || (only && !only[line])) return;
+  film1d_chain<T>(F, fr.get(), line, blockIdx.y, only != nullptr);
 }
 
 // ---------------------------------------------------------------------------
@@ -648,10 +668,11 @@ k_film_contour_s(FilmDev<T> F) {
 template <typename T>
 __global__ void __launch_bounds__(FILM_THREADS)
 k_film1d_chains_b(const FilmDev<T>* __restrict__ Fs, const ScfDev* __restrict__ Ss,
-                  const int* __restrict__ films, int nf) {
+                  const int* __restrict__ films, int nf, const int* __restrict__ serial) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= nf) return;
   const int f = films[k];
+  if (!serial[f]) return;
   // by value: the sweep's stores could alias a struct read through a pointer,
   // which would force a reload of every field pointer per point
   const FilmDev<T> F = Fs[f];
@@ -674,7 +695,7 @@ k_film1d_chains_b(const FilmDev<T>* __restrict__ Fs, const ScfDev* __restrict__ 
 template <typename T>
 __global__ void __launch_bounds__(256)
 k_film1d_chains_sm(const FilmDev<T>* __restrict__ Fs, const ScfDev* __restrict__ Ss,
-                   const int* __restrict__ films, int nf, int zcap, int per_warp) {
+                   const int* __restrict__ films, int nf, int zcap, int per_warp, const int* __restrict__ serial) {
   extern __shared__ __align__(16) unsigned char smraw[];
   constexpr bool inc = sizeof(T) == 4;
   // the first per_warp lanes of each warp work (a warp's instruction stream
@@ -685,6 +706,7 @@ k_film1d_chains_sm(const FilmDev<T>* __restrict__ Fs, const ScfDev* __restrict__
   const int k = blockIdx.x * W + lane;
   if (k >= nf) return;
   const int f = films[k];
+  if (!serial[f]) return;
   const FilmDev<T> F = Fs[f];
   const double* field = Ss[f].hx + (size_t)((*Ss[f].iter) % Ss[f].slots) * ((size_t)Ss[f].ntypes * Ss[f].npts);
   T* qv = reinterpret_cast<T*>(smraw) + lane;

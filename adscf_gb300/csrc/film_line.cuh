@@ -377,16 +377,13 @@ k_line_factors(FilmDev<double> F, FieldRef fr, double2* __restrict__ fac) {
 // 2.2 ms, 1001 rows and 1200 steps 11.1 -> 4.1 ms against factors in the chain.
 template <int K, int W>
 __global__ void __launch_bounds__(32 * W)
-k_line_chain(FilmDev<double> F, FieldRef fr, const double2* __restrict__ fac) {
+k_line_chain(FilmDev<double> F, FieldRef fr, const double2* __restrict__ fac, int* __restrict__ serial) {
   using S = fl::Slot<K, W>;
   constexpr int T = 32 * W, P = S::pairs * T;
   extern __shared__ __align__(16) unsigned char smraw[];
   __shared__ fl::Exchange ex;
   const int n = F.gz + 1, L = F.nlines, ns = F.ns, line = blockIdx.x, dir = blockIdx.y;
-  if (!film_line_dominant<double>(F, fr.get() + line, L)) {
-    if (threadIdx.x == 0) film1d_chain<double>(F, fr.get(), line, dir);
-    return;
-  }
+  if (film_line_serial<double>(F, fr.get(), line, dir, threadIdx.x == 0, serial)) return;
   double2* ring = reinterpret_cast<double2*>(smraw) + threadIdx.x;
   const double2* src = fac + (size_t)line * ns * P + threadIdx.x;
   auto fetch = [&](int s) {
@@ -424,16 +421,13 @@ k_line_chain(FilmDev<double> F, FieldRef fr, const double2* __restrict__ fac) {
 // Chain blockIdx.y of lines (128 / 32 W a block) of one context
 template <int K, int W>
 __global__ void __launch_bounds__(fl::kThreads)
-k_line_elim(FilmDev<double> F, FieldRef fr) {
+k_line_elim(FilmDev<double> F, FieldRef fr, int* __restrict__ serial) {
   extern __shared__ __align__(16) unsigned char smraw[];
   __shared__ fl::Exchange ex;
   constexpr int T = 32 * W;
   const int sub = threadIdx.x / T, line = blockIdx.x * (fl::kThreads / T) + sub, dir = blockIdx.y;
   if (line >= F.nlines) return;
-  if (!film_line_dominant<double>(F, fr.get() + line, F.nlines)) {
-    if ((threadIdx.x & (T - 1)) == 0) film1d_chain<double>(F, fr.get(), line, dir);
-    return;
-  }
+  if (film_line_serial<double>(F, fr.get(), line, dir, (threadIdx.x & (T - 1)) == 0, serial)) return;
   fl::chain_elim<K, W>(F, dir, (dir == 0 ? F.q : F.qd) + line, fr.get() + line,
                        reinterpret_cast<double*>(smraw) + sub * 4 * K * T, &ex);
 }
@@ -441,7 +435,8 @@ k_line_elim(FilmDev<double> F, FieldRef fr) {
 // for all lengths, so that short lines and long ones run beside each other
 template <int W>
 __global__ void __launch_bounds__(fl::kThreads)
-k_line_elim_b(const FilmDev<double>* __restrict__ Fs, const ScfDev* __restrict__ Ss, const int* __restrict__ items, int nitems) {
+k_line_elim_b(const FilmDev<double>* __restrict__ Fs, const ScfDev* __restrict__ Ss, const int* __restrict__ items, int nitems,
+              int* __restrict__ serial) {
   extern __shared__ __align__(16) unsigned char smraw[];
   __shared__ fl::Exchange ex;
   constexpr int T = 32 * W;
@@ -451,10 +446,7 @@ k_line_elim_b(const FilmDev<double>* __restrict__ Fs, const ScfDev* __restrict__
   const FilmDev<double> F = Fs[f];
   const ScfDev& S = Ss[f];
   const double* field = S.hx + (size_t)((*S.iter) % S.slots) * ((size_t)S.ntypes * S.npts);
-  if (!film_line_dominant<double>(F, field, 1)) {
-    if ((threadIdx.x & (T - 1)) == 0) film1d_chain<double>(F, field, 0, dir);
-    return;
-  }
+  if (film_line_serial<double>(F, field, 0, dir, (threadIdx.x & (T - 1)) == 0, serial + f)) return;
   double* chain = dir == 0 ? F.q : F.qd;
   double* sm = reinterpret_cast<double*>(smraw) + sub * 4 * fl::kMaxK * T;
   switch (fl::rows_per_lane(F.gz + 1)) {

@@ -304,7 +304,7 @@ __device__ __forceinline__ void film_warp_tables(const FilmDev<float>& F, const 
 // are, b = |a| + |c|).  Then no elimination order meets a zero pivot.  Where
 // it is not, the order decides which pivots vanish and how far rounding
 // grows, and the chain runs the reference's serial recurrence instead
-// (film1d_chain).  Every lane of a warp calls it; the answer is uniform over
+// (film_line_serial).  Every lane of a warp calls it; the answer is uniform over
 // the warps of a line.
 template <typename T>
 __device__ __forceinline__ bool film_line_dominant(const FilmDev<T>& F, const double* field, size_t wstride) {
@@ -320,6 +320,26 @@ __device__ __forceinline__ bool film_line_dominant(const FilmDev<T>& F, const do
 #pragma unroll
   for (int o = 16; o; o >>= 1) ds = fmax(ds, __shfl_xor_sync(0xffffffffu, ds, o));
   return 1.0 + 0.5 * ds * lo >= 0.01;
+}
+
+// Whether line `line` is not for the cooperative solve.  Its chains then run the
+// recurrence: here, by the thread with `lead`, where `serial` is null (a context
+// of one line), else in k_film1d_chains or k_film1d_chains_sm behind this kernel,
+// which take the lines that are marked in `serial` a thread each, neighbouring
+// lines in neighbouring threads (2048 lines of 101 rows, a step of both chains:
+// 766 us with a lane of every warp at work).
+template <typename T>
+__device__ __forceinline__ bool film_line_serial(const FilmDev<T>& F, const double* field, int line, int dir, bool lead,
+                                                 int* __restrict__ serial) {
+  const bool yes = !film_line_dominant<T>(F, field + line, F.nlines);
+  if (lead) {
+    if (serial) {
+      if (dir == 0) serial[line] = yes;
+    } else if (yes) {
+      film1d_chain<T>(F, field, line, dir);
+    }
+  }
+  return yes;
 }
 
 // Single context (Film_1D / brush lines of one film): one warp per (line,
@@ -611,15 +631,12 @@ __device__ __forceinline__ void film1d_chain_group(const FilmDev<T>& F, int dir,
 // 1024 (lines of more than 1024 rows in one CTA) spill some.
 template <typename T, int MAXT>
 __global__ void __launch_bounds__(MAXT)
-k_film1d_group(FilmDev<T> F, FieldRef fr, int csize) {
+k_film1d_group(FilmDev<T> F, FieldRef fr, int csize, int* __restrict__ serial) {
   __shared__ FilmGroupSm<T> sm;
   if (csize > 1) fw::cluster_barrier();   // every CTA of the cluster runs before its memory is written
   const int line = blockIdx.x / csize, dir = blockIdx.y;
   const size_t L = F.nlines;
-  if (!film_line_dominant<T>(F, fr.get() + line, L)) {
-    if (threadIdx.x == 0 && blockIdx.x % csize == 0) film1d_chain<T>(F, fr.get(), line, dir);
-    return;
-  }
+  if (film_line_serial<T>(F, fr.get(), line, dir, threadIdx.x == 0 && blockIdx.x % csize == 0, serial)) return;
   film1d_chain_group<T>(F, dir, (dir == 0 ? F.q : F.qd) + line, L, fr.get() + line, L, blockIdx.x % csize, csize, sm);
 }
 
@@ -627,16 +644,14 @@ k_film1d_group(FilmDev<T> F, FieldRef fr, int csize) {
 // per line.
 template <typename T, int MAXT>
 __global__ void __launch_bounds__(MAXT)
-k_film1d_group_b(const FilmDev<T>* __restrict__ Fs, const ScfDev* __restrict__ Ss, const int* __restrict__ items) {
+k_film1d_group_b(const FilmDev<T>* __restrict__ Fs, const ScfDev* __restrict__ Ss, const int* __restrict__ items,
+                 int* __restrict__ serial) {
   __shared__ FilmGroupSm<T> sm;
   const int f = items[blockIdx.x] >> 1, dir = items[blockIdx.x] & 1;
   const FilmDev<T> F = Fs[f];
   const ScfDev& S = Ss[f];
   const double* field = S.hx + (size_t)((*S.iter) % S.slots) * ((size_t)S.ntypes * S.npts);
-  if (!film_line_dominant<T>(F, field, 1)) {
-    if (threadIdx.x == 0) film1d_chain<T>(F, field, 0, dir);
-    return;
-  }
+  if (film_line_serial<T>(F, field, 0, dir, threadIdx.x == 0, serial + f)) return;
   film1d_chain_group<T>(F, dir, dir == 0 ? F.q : F.qd, 1, field, 1, 0, 1, sm);
 }
 
