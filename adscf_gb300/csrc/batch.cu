@@ -10,8 +10,8 @@
 // a prefix), one contour launch, and batched closure / Anderson solve / mix
 // launches with each instance's mixing history on the device.  One batch
 // iteration is one CUDA graph.  The chains run the mixed-radix passes grid by
-// grid (batch_mx.cu); ADSCF_BATCH_SWEEP=1, more than 64 different grids and
-// lines past 1024 points take the persistent sweep of the line passes, and
+// grid (batch_mx.cu); instances with lines past 1024 points, and all of them past 64
+// different grids or with ADSCF_BATCH_SWEEP=1, take the persistent sweep of the line passes, with
 // ADSCF_BATCH_SWEEP=0 those passes launch by launch: there instances are
 // grouped by pass kernel, cubic grids of 24..256 points on the register-FFT
 // passes of bulk_reg.cuh, every other grid of 2, 3 and 5 factors on the generic
@@ -85,7 +85,8 @@ struct adscf_batch {
   int sweep_grid = 0;
   int sweep_help = 0;                   // class with the most point-steps (finished CTAs help it)
   size_t sweep_smem = 0;
-  struct BatchMx* mx = nullptr;         // mixed-radix passes (batch_mx.cu), null where the sweep runs
+  struct BatchMx* mx = nullptr;         // mixed-radix passes (batch_mx.cu)
+  int n_line = 0;                       // instances that run the line passes instead
   bool sweep = true;                    // persistent sweeps (ADSCF_BATCH_SWEEP=0: one launch per pass)
   int sweep_tiles = 8;                  // tiles per sweep item (ADSCF_SWEEP_TILES)
   cudaGraphExec_t g_iter = nullptr;
@@ -474,12 +475,32 @@ int build(adscf_batch* b) {
   std::vector<int> ones(n, 1);
   BK(cudaMemcpyAsync(b->d_iterall, ones.data(), n * sizeof(int), cudaMemcpyHostToDevice, b->stream));
 
+  // The chains of every grid with a mixed-radix plan: one 64^3 split grid takes 3.3
+  // ms an iteration there, 19 in the sweep.  What follows is for the others alone.
+  const char* pin = std::getenv("ADSCF_BATCH_SWEEP");
+  if (pin) b->sweep = std::atoi(pin) != 0;
+  std::vector<char> on_mx(n, 0);
+  if (!pin) {
+    std::vector<BatchMxInst> in(n);
+    for (int i = 0; i < n; ++i) {
+      const BulkDev<T>& d = I[i];
+      in[i] = BatchMxInst{d.gx, d.gy, d.gz, d.ns, static_cast<const BulkDev<T>*>(b->d_inst) + i, d.spec, d.slices, d.E,
+                          fk.data() + d.gxy_off, g64.data() + d.g64_off};
+    }
+    std::string why;
+    b->mx = batch_mx_create<T>(b->dev, in, on_mx, why);
+    if (!b->mx) return berr(b, ADSCF_E_OOM, "batch passes: " + why);
+  }
+  b->n_line = n - (int)std::count(on_mx.begin(), on_mx.end(), 1);
+
   // work lists per kernel class, instances by descending Ns: the tiles of the
   // instances still on their contour at step t are a prefix
-  std::vector<int> ord(n);
-  for (int i = 0; i < n; ++i) ord[i] = i;
+  std::vector<int> ord;
+  for (int i = 0; i < n; ++i)
+    if (!on_mx[i]) ord.push_back(i);
   std::stable_sort(ord.begin(), ord.end(), [&](int a, int c2) { return b->ns[a] > b->ns[c2]; });
   auto class_of = [&](int i) {
+    if (on_mx[i]) return -1;
     const BulkDev<T>& d = I[i];
     const int g = d.gx;
     return (d.gy == g && d.gz == g && batch_reg_size(g)) ? g : 0;
@@ -525,21 +546,10 @@ int build(adscf_batch* b) {
   // items of the persistent sweeps (k_batch_sweep), class by class: per step
   // and pass, the class's instances still on their contour in the same order
   // as the work lists
-  {
+  if (b->n_line) {
     if (const char* e = std::getenv("ADSCF_SWEEP_TILES")) b->sweep_tiles = std::max(1, std::min(64, std::atoi(e)));
-    const char* pin = std::getenv("ADSCF_BATCH_SWEEP");
-    if (pin) b->sweep = std::atoi(pin) != 0;
-    if (!pin) {   // a batch of any size: one 64^3 split grid 3.3 ms an iteration, 19 in the sweep
-      std::vector<BatchMxInst> in(n);
-      for (int i = 0; i < n; ++i) {
-        const BulkDev<T>& d = I[i];
-        in[i] = BatchMxInst{d.gx, d.gy, d.gz, d.ns, static_cast<const BulkDev<T>*>(b->d_inst) + i, d.spec, d.slices, d.E,
-                            fk.data() + d.gxy_off, g64.data() + d.g64_off};
-      }
-      b->mx = batch_mx_create<T>(b->dev, in);
-    }
     std::vector<int> tx(n), ty(n), tz(n), before(n, 0);
-    for (int i = 0; i < n; ++i) {
+    for (int i : ord) {
       const BulkDev<T>& d = I[i];
       const int cn = class_of(i);
       const int lx = cn ? BULK_THREADS / reg_tpl(cn) : d.px.lpc;
@@ -594,7 +604,7 @@ int build(adscf_batch* b) {
   ADSCF_BATTR(24) ADSCF_BATTR(32) ADSCF_BATTR(40) ADSCF_BATTR(48) ADSCF_BATTR(64) ADSCF_BATTR(128)
   ADSCF_BATTR(256)
 #undef ADSCF_BATTR
-  {  // persistent sweep: each class's share of the resident CTAs in proportion
+  if (b->n_line) {  // persistent sweep: each class's share of the resident CTAs in proportion
      // to its point-steps (at least one CTA); the kernel's static shared
      // memory counts against the opt-in limit
     const int ncls = (int)b->sw.size();
@@ -973,9 +983,11 @@ int enqueue_propagation(adscf_batch* b) {
   if (b->mx) {
     std::string why;
     if (batch_mx_enqueue(b->mx, s, why)) return berr(b, ADSCF_E_CUDA, "batch passes: " + why);
-    k_bulk_contour<T><<<dim3(b->cont_blocks, b->n), BULK_THREADS, 0, s>>>(d);
-    BK(cudaGetLastError());
-    return ADSCF_OK;
+    if (!b->n_line) {
+      k_bulk_contour<T><<<dim3(b->cont_blocks, b->n), BULK_THREADS, 0, s>>>(d);
+      BK(cudaGetLastError());
+      return ADSCF_OK;
+    }
   }
   // one launch per kernel class and pass; a class with no instance left on
   // its contour at step t launches nothing
@@ -1575,9 +1587,9 @@ int adscf_batch_launches(const adscf_batch* b) {
     }
     return k;
   }
-  if (b->mx) return 4 + batch_mx_launches(b->mx);
-  if (b->sweep) return 5;   // sweep, contour, closure, solve, mix (and a memset of the counters)
-  int k = 4;   // contour, closure, solve, mix
+  int k = 4 + (b->mx ? batch_mx_launches(b->mx) : 0);   // contour, closure, solve, mix
+  if (!b->n_line) return k;
+  if (b->sweep) return k + 1;   // (and a memset of the counters)
   for (const auto& C : b->cls) {
     k += C.px[0] > 0;
     for (int t = 1; t <= b->maxns; ++t) k += 2 * (C.py[t] > 0) + (C.pz[t] > 0) + (C.px[t] > 0);

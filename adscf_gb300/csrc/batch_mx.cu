@@ -24,7 +24,8 @@ namespace {
 
 // Grids of one batch: each adds a stream and two graph nodes a step, captured on
 // the first pass (64 instances of 16^3 to 30^3, 100 steps: 4 grids 4.7 ms an
-// iteration and 12.7 ms the first, 64 grids 6.8 and 49; the sweep 68 to 76).
+// iteration and 12.7 ms the first, 64 grids 6.8 and 49; the sweep 68 to 76).  A
+// batch of more runs the sweep, whose results differ at rounding.
 constexpr size_t kMaxGrids = 64;
 
 struct Class {
@@ -46,16 +47,19 @@ struct BatchMx {
 
 namespace {
 
+// Plan of a grid, from its sizes alone: an instance's result does not depend on
+// what else is in the batch.  FP64 radices as in mx_setup, up to npts / 19456; the
+// number of instances with the grid in its place spared large classes a stage
+// (64 grids of 32^3 447 us a double step, 466 with this rule) but cost others more
+// (64 of 48^3 1926 and 1699, 64 of 24^3 to 64^3 1362 and 1322).  false: lines or
+// tiles the passes do not take.
 template <typename T>
-bool build_class(Class& C, int dev, bool stream, const std::vector<BatchMxInst>& in, const std::vector<int>& ids) {
+bool plan_class(Class& C, int optin, int gx, int gy, int gz) {
   BulkMx* M = &C.M;
-  const BatchMxInst& f = in[ids[0]];
-  const int gx = f.gx, gy = f.gy, gz = f.gz;
-  const size_t np = (size_t)gx * gy * gz, nxy = (size_t)gx * gy;
-  const int rmax = sizeof(T) == 4 ? 16 : (int)std::max<size_t>(5, std::min<size_t>(16, np * ids.size() / 19456));
+  const int rmax = sizeof(T) == 4 ? 16 : std::max(5, std::min(16, gx * gy * gz / 19456));
   if (!mx_axis(gx, rmax, M->a[0]) || !mx_axis(gy, rmax, M->a[1]) || !mx_axis(gz, rmax, M->a[2])) return false;
   if (M->a[0].nst + M->a[1].nst > mxk::kMaxSteps || M->a[1].nst + M->a[2].nst > mxk::kMaxSteps) return false;
-  if (cudaDeviceGetAttribute(&M->optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) return false;
+  M->optin = optin;
   mxk::Dev<T>& D = M->dev<T>();
   D.gx = gx; D.gy = gy; D.gz = gz;
   // 64-byte column runs: 64 grids of 24^3 to 64^3 split 23.9 ms an iteration, 26.7
@@ -63,6 +67,16 @@ bool build_class(Class& C, int dev, bool stream, const std::vector<BatchMxInst>&
   Geom G;
   if (!default_geometry<T>(M, G)) return false;
   if (!geometry<T>(M, G.cut, 2 * G.cols, G.cap_a, G.cap_b)) geometry<T>(M, G.cut, G.cols, G.cap_a, G.cap_b);
+  return true;
+}
+
+// Tables and lists of the instances `ids` of one grid, by descending Ns
+template <typename T>
+bool fill_class(Class& C, bool stream, const std::vector<BatchMxInst>& in, const std::vector<int>& ids) {
+  BulkMx* M = &C.M;
+  mxk::Dev<T>& D = M->dev<T>();
+  const int gx = D.gx, gy = D.gy, gz = D.gz;
+  const size_t nxy = (size_t)gx * gy;
   D.stream = stream;
   std::vector<cplx<T>> tw;
   std::vector<std::pair<int, int>> seen;
@@ -74,10 +88,8 @@ bool build_class(Class& C, int dev, bool stream, const std::vector<BatchMxInst>&
   if (cudaMalloc(&M->d_tw, tw.size() * sizeof(cplx<T>)) || cudaMalloc(&C.d_tab, each * ids.size()) ||
       cudaMalloc(&C.d_ios, ids.size() * sizeof(mxk::Io<T>)) ||
       cudaStreamCreateWithFlags(&C.st, cudaStreamNonBlocking) ||
-      cudaEventCreateWithFlags(&C.done, cudaEventDisableTiming)) {
-    cudaGetLastError();
+      cudaEventCreateWithFlags(&C.done, cudaEventDisableTiming))
     return false;
-  }
   std::vector<unsigned char> tab(each * ids.size(), 0);
   std::vector<mxk::Io<T>> ios(ids.size());
   int maxns = 0;
@@ -133,39 +145,47 @@ void chains(Class& C) {
 }  // namespace
 
 template <typename T>
-BatchMx* batch_mx_create(int dev, const std::vector<BatchMxInst>& in) {
+BatchMx* batch_mx_create(int dev, const std::vector<BatchMxInst>& in, std::vector<char>& taken, std::string& err) {
   BatchMx* B = new (std::nothrow) BatchMx();
-  if (!B) return nullptr;
-  B->f64 = sizeof(T) == 8;
-  std::map<std::tuple<int, int, int>, std::vector<int>> groups;
-  for (int i = 0; i < (int)in.size(); ++i) groups[{in[i].gx, in[i].gy, in[i].gz}].push_back(i);
-  if (groups.size() > kMaxGrids) {
-    delete B;
+  if (!B) {
+    err = "host memory";
     return nullptr;
   }
+  B->f64 = sizeof(T) == 8;
+  taken.assign(in.size(), 0);
+  std::map<std::tuple<int, int, int>, std::vector<int>> groups;
+  for (int i = 0; i < (int)in.size(); ++i) groups[{in[i].gx, in[i].gy, in[i].gz}].push_back(i);
+  if (groups.size() > kMaxGrids) return B;
   // factors, spectra and nodes of the batch past L2: stream (as for one large
   // grid: 24.0 against 25.2 ms an iteration of 64 grids)
   size_t pts = 0;
   for (const BatchMxInst& q : in) pts += (size_t)q.gx * q.gy * q.gz;
-  int l2 = 0;
+  int l2 = 0, optin = 0;
   cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev);
-  const bool stream = pts * 32 > (size_t)l2;
-  bool ok = cudaEventCreateWithFlags(&B->fork, cudaEventDisableTiming) == cudaSuccess;
+  bool ok = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) == cudaSuccess &&
+            cudaEventCreateWithFlags(&B->fork, cudaEventDisableTiming) == cudaSuccess;
   for (auto& g : groups) {
-    if (!ok) break;
-    std::stable_sort(g.second.begin(), g.second.end(), [&](int a, int b) { return in[a].ns > in[b].ns; });
-    B->cls.emplace_back();
-    ok = g.second.size() <= 65535 && build_class<T>(B->cls.back(), dev, stream, in, g.second);
+    Class plan;
+    if (!plan_class<T>(plan, optin, std::get<0>(g.first), std::get<1>(g.first), std::get<2>(g.first))) continue;
+    std::vector<int>& ids = g.second;
+    std::stable_sort(ids.begin(), ids.end(), [&](int a, int b) { return in[a].ns > in[b].ns; });
+    for (int i : ids) taken[i] = 1;
+    // at most 65535 instances a launch (gridDim.y)
+    for (size_t at = 0; at < ids.size() && ok; at += 65535) {
+      B->cls.push_back(plan);
+      ok = fill_class<T>(B->cls.back(), pts * 32 > (size_t)l2, in,
+                         std::vector<int>(ids.begin() + at, ids.begin() + std::min(ids.size(), at + 65535)));
+    }
   }
   if (!ok) {
-    cudaGetLastError();
+    err = cudaGetErrorString(cudaGetLastError());
     batch_mx_destroy(B);
     return nullptr;
   }
   return B;
 }
-template BatchMx* batch_mx_create<float>(int, const std::vector<BatchMxInst>&);
-template BatchMx* batch_mx_create<double>(int, const std::vector<BatchMxInst>&);
+template BatchMx* batch_mx_create<float>(int, const std::vector<BatchMxInst>&, std::vector<char>&, std::string&);
+template BatchMx* batch_mx_create<double>(int, const std::vector<BatchMxInst>&, std::vector<char>&, std::string&);
 
 void batch_mx_destroy(BatchMx* B) {
   if (!B) return;
@@ -179,6 +199,7 @@ void batch_mx_destroy(BatchMx* B) {
 }
 
 int batch_mx_enqueue(BatchMx* B, cudaStream_t s, std::string& err) {
+  if (B->cls.empty()) return 0;
   cudaError_t e = cudaEventRecord(B->fork, s);
   for (Class& C : B->cls) {
     if (e == cudaSuccess) e = cudaStreamWaitEvent(C.st, B->fork, 0);

@@ -19,10 +19,11 @@ struct BatchMxInst {
   const double* g64;
 };
 
-// null: a grid without a plan, or no memory
+// Passes of the instances whose grid has a plan (taken; none in a batch of more
+// than 64 grids); null: no memory, err
 template <typename T>
-BatchMx* batch_mx_create(int dev, const std::vector<BatchMxInst>& in);
+BatchMx* batch_mx_create(int dev, const std::vector<BatchMxInst>& in, std::vector<char>& taken, std::string& err);
 void batch_mx_destroy(BatchMx* B);
-// both chains of every instance, on s and the batch's own streams beside it
+// both chains of every instance taken, on s and the batch's own streams beside it
 int batch_mx_enqueue(BatchMx* B, cudaStream_t s, std::string& err);
 int batch_mx_launches(const BatchMx* B);
