@@ -234,17 +234,18 @@ int propagate_ckpt(adscf_ctx* ctx, AdjState* s) {
   return ADSCF_OK;
 }
 
-// the forward pass from the fields already in the adjoint buffer; grad: keep
-// what a backward pass on the mixed-radix passes needs
+// the forward pass from the fields already in the adjoint buffer; grad: a backward
+// pass may follow
 int forward_core(adscf_ctx* ctx, double* free_energy, double* sc_out, bool grad) {
   int rc;
   AdjState* s = ctx->adj;
   if ((rc = bulk_enqueue_expfield(ctx, s->d_w))) return rc;
-  if (grad && !ctx->adj_ckpt && (rc = adj_mx_setup(ctx, &s->mx))) return rc;
-  s->mx.kept = grad && !ctx->adj_ckpt && s->mx.keep;
+  if (ctx->mx_off) adj_mx_free(&s->mx);   // a pinned plan runs the generic sweep
+  s->mx.on = ctx->mx && !ctx->mx_off && !ctx->adj_ckpt;
+  s->mx.kept = false;
   if (ctx->adj_ckpt) {
     if ((rc = propagate_ckpt(ctx, s))) return rc;
-  } else if (s->mx.kept) {
+  } else if (grad && s->mx.on) {
     if ((rc = adj_mx_forward(ctx, &s->mx))) return rc;
   } else {
     if ((rc = bulk_enqueue_propagate(ctx))) return rc;
@@ -383,8 +384,8 @@ int adscf_backward(adscf_ctx* ctx, double* grad) {
     return set_err(ctx, ADSCF_E_STATE, "adscf_backward needs the state of an immediately preceding adscf_forward");
   AdjDev A = s->A;
   cudaStream_t st = ctx->stream;
-  if (s->mx.kept) {
-    if ((rc = adj_mx_backward(ctx, &s->mx, A.b, A.sc))) return rc;
+  if (s->mx.on) {
+    if ((rc = adj_mx_backward(ctx, &s->mx, A.b, A.sc, A.sf))) return rc;
     A.gpart = s->mx.gpart;
     A.nztiles = s->mx.ntiles;
     return read_gradient(ctx, A, grad);

@@ -1,11 +1,14 @@
 // adjoint_mx.cuh -- the reverse sweep of adjoint_kernels.cuh on the mixed-radix
 // passes (bulk_mx.cuh).
 //
-// A forward pass for a gradient keeps the spectrum of every step after its
-// forward transform, Xf(t) = FFT(E(t) z_{t-1}), in the order in which the
-// diffusion pass holds it.  The reverse sweep then transforms the adjoint pair
-// alone, six line transforms a step for nine, in two passes like a forward
-// step:
+// The gradient needs the spectrum of every step after its forward transform,
+// Xf(t) = FFT(E(t) z_{t-1}), in the order in which the diffusion pass holds it.
+// Forward passes for a gradient keep them where they take little of the memory
+// (adj_mx_keep), and the reverse sweep transforms the adjoint pair alone, six line
+// transforms a step for nine.  A sweep behind a forward pass that kept none makes
+// them again from the slices, with the forward
+// pass's own operations (k_mx_a_from, or its counterpart with an output per lane, and
+// kSpec), so that the gradient is the same bits.  Two passes like a forward step:
 //   k_mx_adj_a(t): inverse y and x of the adjoint spectrum -> E(t+1) -> + seeds
 //                  -> E(t) -> forward x and y;
 //   k_mx_b, kDot : forward y and z, W(k) += Re(conj(Xf(t, k)) Ya(t, k)), G / M,
@@ -145,6 +148,11 @@ k_mx_adj_a(const __grid_constant__ mxk::Dev<double> D, const double* __restrict_
   }
   if (D.a.n == 0)
     for (int x = threadIdx.x; x < gx; x += blockDim.x) g[x] = sm[x];
+}
+
+// Real-space pass after node t of the chains, from its slice, into D.io.spec
+static __global__ void __launch_bounds__(128, 4) k_mx_a_from(const __grid_constant__ mxk::Dev<double> D, int t) {
+  mx_a_body<double, true>(D, D.io, t);
 }
 
 // Diffusion pass with side data of `tile` points a block

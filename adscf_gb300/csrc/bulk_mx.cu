@@ -271,8 +271,6 @@ void mx_real(adscf_ctx* ctx, int t) {
   if (ctx->prec == ADSCF_SPLIT) real_t<float>(ctx, t, false);
   else real_t<double>(ctx, t, ctx->mx->spread);
 }
-// the same beside passes of bulk_mx.cuh
-void mx_real_plain(adscf_ctx* ctx, int t) { real_t<double>(ctx, t, false); }
 void mx_step(adscf_ctx* ctx, int t) {
   if (ctx->prec == ADSCF_SPLIT) step_t<float>(ctx, t);
   else step_t<double>(ctx, t);
@@ -282,7 +280,8 @@ int mx_tune(adscf_ctx* ctx) { return ctx->prec == ADSCF_SPLIT ? tune_t<float>(ct
 bool mx_launch64(const adscf_ctx* ctx, MxLaunch64& L) {
   const BulkMx* M = ctx->mx;
   if (!M || ctx->prec != ADSCF_FP64) return false;
-  L = MxLaunch64{M->d64, M->yz, M->thr_a, M->thr_b, M->grid_a, M->grid_b, M->sm_a, M->sm_b, M->optin};
+  L = MxLaunch64{M->d64, M->yz, M->thr_a, M->thr_b, M->grid_a, M->grid_b, M->sm_a, M->sm_b, M->optin,
+                 M->spread, M->sp, M->thr_as, M->thr_bs};
   L.D.io.slices = ctx->hb64.slices;
   L.D.io.I = static_cast<const BulkDev<double>*>(ctx->d_inst);
   return true;

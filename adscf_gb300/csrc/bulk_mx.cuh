@@ -246,9 +246,10 @@ __device__ __forceinline__ void stage_r(const Step& S, cplx<T>* sm, int tile_j, 
 
 // What the visit of the diffusion factor does besides, for the adjoint: the
 // forward pass keeps its spectra (kStore), the reverse pass adds Re(conj(kept)
-// spectrum) up per frequency (kDot).  Both lie in tile order: point (row yy,
-// position zp, column c) of a block at ((zp M' + yy) cols + c).
-enum { kPlain = 0, kStore = 1, kDot = 2 };
+// spectrum) up per frequency (kDot), from spectra that were kept or are made again
+// from the slices (kSpec: the spectrum alone, nothing after it).  All lie in tile
+// order: point (row yy, position zp, column c) of a block at ((zp M' + yy) cols + c).
+enum { kPlain = 0, kStore = 1, kDot = 2, kSpec = 3 };
 template <typename T>
 struct Side {
   cplx<T>* keep;                // the block's part of the kept spectrum
@@ -280,7 +281,7 @@ __device__ __forceinline__ void mid_r(const Dev<T>& D, cplx<T>* sm, const T* fz,
 #pragma unroll
       for (int r = 0; r < R; ++r) {
         const size_t at = (size_t)(((u * R + r) * D.mi + yy) << D.lc) + c;
-        if constexpr (MODE == kStore) {
+        if constexpr (MODE != kDot) {
           sd.keep[at] = v[r];
         } else {
           const cplx<T> f = sd.keep[at];
@@ -288,6 +289,7 @@ __device__ __forceinline__ void mid_r(const Dev<T>& D, cplx<T>* sm, const T* fz,
         }
       }
     }
+    if constexpr (MODE == kSpec) continue;
 #pragma unroll
     for (int r = 0; r < R; ++r) {
       const T bh = fz[u * R + r];
@@ -325,8 +327,9 @@ __device__ __forceinline__ EPt<T> load_e(const Dev<T>& D, const T* E, size_t p) 
 // slice at the tile's first row, its rows M' gx apart; f: bits 0-3 = forward /
 // backward chain takes the A factor at node t, at node t + 1; bit 4: t <
 // Ns, the forward stage follows; init: no inverse, slice = (1, 1); dco, dci:
-// as dc of stage_r where this is the rows' only stage, else null.
-template <typename T, int R>
+// as dc of stage_r where this is the rows' only stage, else null.  FROM: no
+// inverse, node t is the slice.
+template <typename T, int R, bool FROM = false>
 __device__ __forceinline__ void real_r(const Dev<T>& D, cplx<T>* sm, const T* E, cplx<T>* sl, unsigned f, bool init,
                                        float2* dco, float2* dci) {
   const int Mp = D.gx / R;
@@ -339,7 +342,7 @@ __device__ __forceinline__ void real_r(const Dev<T>& D, cplx<T>* sm, const T* E,
     cplx<T>* p = sm + l * D.pitch + j;
     const size_t gp = l * rs + j;
     cplx<T> v[R];
-    if (!init) {
+    if (!FROM && !init) {
 #pragma unroll
       for (int r = 0; r < R; ++r) v[r] = p[r * Mp];
       if constexpr (sizeof(T) == 4)
@@ -355,7 +358,11 @@ __device__ __forceinline__ void real_r(const Dev<T>& D, cplx<T>* sm, const T* E,
 #pragma unroll
     for (int r = 0; r < R; ++r) {
       const EPt<T> ev = load_e(D, E, gp + r * Mp);
-      if (init) {
+      if constexpr (FROM) {
+        const cplx<T> q = sl[gp + r * Mp];
+        v[r] = mk<T>(emul(q.x, fA2 ? ev.a : ev.b, fA2 ? ev.al : ev.bl),
+                     emul(q.y, bA2 ? ev.a : ev.b, bA2 ? ev.al : ev.bl));
+      } else if (init) {
         v[r] = mk<T>(fA ? ev.a : ev.b, bA ? ev.a : ev.b);
         sl[gp + r * Mp] = mk<T>((T)1, (T)1);
       } else {
@@ -386,9 +393,10 @@ __device__ __forceinline__ void real_r(const Dev<T>& D, cplx<T>* sm, const T* E,
 
 // ---------------------------------------------------------------------------
 // Real-space pass of the row set (j, z): block j + M' z.  t = 0 starts the
-// chains: slice 0 = (1, 1).  Shared memory: R_o pitch + gx + gy points.
+// chains: slice 0 = (1, 1).  FROM: the pass after node t, from its slice.  Shared
+// memory: R_o pitch + gx + gy points.
 // ---------------------------------------------------------------------------
-template <typename T>
+template <typename T, bool FROM = false>
 __device__ __forceinline__ void mx_a_body(const mxk::Dev<T>& D, const mxk::Io<T>& io, int t) {
   extern __shared__ __align__(16) unsigned char smraw[];
   cplx<T>* sm = reinterpret_cast<cplx<T>*>(smraw);
@@ -419,7 +427,7 @@ __device__ __forceinline__ void mx_a_body(const mxk::Dev<T>& D, const mxk::Io<T>
   float2* dco = sizeof(T) == 4 ? io.dcout + z : nullptr;
   tmak::pdl_wait();
   __syncthreads();
-  if (t > 0) {
+  if (!FROM && t > 0) {
     // the tile's Boltzmann factors on their way to L1 while it is transformed
     for (int r = 0; r < ro; ++r) {
       const char* e0 = reinterpret_cast<const char*>(E) + r * rs * 16;
@@ -439,10 +447,10 @@ __device__ __forceinline__ void mx_a_body(const mxk::Dev<T>& D, const mxk::Io<T>
     }
   }
   if (D.rx == 1) {
-    mxk::real_r<T, 1>(D, sm, E, sl, f, t == 0, xs == -1 ? dco : nullptr, xs == -1 ? dci : nullptr);
+    mxk::real_r<T, 1, FROM>(D, sm, E, sl, f, t == 0, xs == -1 ? dco : nullptr, xs == -1 ? dci : nullptr);
   } else {
 #define ADSCF_MX_CALL(R_) \
-  mxk::real_r<T, R_>(D, sm, E, sl, f, t == 0, xs == -1 ? dco : nullptr, xs == -1 ? dci : nullptr)
+  mxk::real_r<T, R_, FROM>(D, sm, E, sl, f, t == 0, xs == -1 ? dco : nullptr, xs == -1 ? dci : nullptr)
     ADSCF_MX_SWITCH(D.rx, ADSCF_MX_CALL)
 #undef ADSCF_MX_CALL
   }
@@ -564,6 +572,7 @@ __device__ __forceinline__ void mx_b_body(const mxk::Dev<T>& D, const mxk::Io<T>
     ADSCF_MX_SWITCH(D.rz, ADSCF_MX_CALL)
 #undef ADSCF_MX_CALL
   }
+  if constexpr (MODE == mxk::kSpec) return;
   __syncthreads();
   for (int i = D.b.n - 1; i >= 0; --i) {
     const mxk::Step& S = D.b.s[i];
@@ -598,6 +607,13 @@ struct MxLaunch64 {
   int thr_a, thr_b, grid_a, grid_b;
   size_t sm_a, sm_b;
   int optin;
+  bool spread;                  // its chains run the kernels with an output per lane
+  mxk::Spread sp;
+  int thr_as, thr_bs;
 };
 bool mx_launch64(const adscf_ctx* ctx, MxLaunch64& L);   // false: the context has no such plan
+// those kernels with side data (mode kStore or kSpec), and the real-space pass after
+// node t from its slice
+void mx_spread_b_side(const MxLaunch64& L, int mode, double2* keep, int tile, cudaStream_t s);
+void mx_spread_a_from(const MxLaunch64& L, int t, cudaStream_t s);
 void mx_freqs(const adscf_ctx* ctx, std::vector<int>& f);   // frequency by position, x then y then z

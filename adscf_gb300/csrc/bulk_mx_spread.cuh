@@ -137,9 +137,9 @@ __device__ __forceinline__ void spread_r(const Step& S, const Prev& V, double2* 
 
 // the z lines' last forward stage, diffusion factor and first inverse stage
 // (as mid_r); rp, twp: radix and twiddle step of the stage before, w: z twiddles
-template <int R>
+template <int R, int MODE>
 __device__ __forceinline__ void spread_mid_r(const Dev<double>& D, double2* sm, const double* fz, const double* fxy,
-                                             int nl, int rp, int twp, const double2* w) {
+                                             int nl, int rp, int twp, const double2* w, const Side<double>& sd) {
   const Lane<R> ln;
   const int lines = D.mi << D.lc, total = D.gz / R * lines;
   for (int t0 = ln.first; t0 < total; t0 += ln.step) {
@@ -155,8 +155,10 @@ __device__ __forceinline__ void spread_mid_r(const Dev<double>& D, double2* sm, 
 #pragma unroll
       for (int r = 0; r < R; ++r) v[r] = p[r << D.lc];
       o = dft_out<R, 1>(v, ln.k);
+      if constexpr (MODE != kPlain) sd.keep[(size_t)(((u * R + ln.k) * D.mi + yy) << D.lc) + c] = o;
       o = make_double2(o.x * f, o.y * f);
     }
+    if constexpr (MODE == kSpec) continue;
     __syncwarp();
     if (live) p[ln.k << D.lc] = o;
     __syncwarp();
@@ -174,7 +176,7 @@ __device__ __forceinline__ void spread_mid_r(const Dev<double>& D, double2* sm, 
 }
 
 // the x rows' last inverse stage, node t and first forward stage (as real_r)
-template <int R>
+template <int R, bool FROM>
 __device__ __forceinline__ void spread_real_r(const Dev<double>& D, double2* sm, const double* E, double2* sl, unsigned f,
                                               bool init) {
   const Lane<R> ln;
@@ -191,7 +193,10 @@ __device__ __forceinline__ void spread_real_r(const Dev<double>& D, double2* sm,
     if (live) {
       const size_t g = l * rs + j + ln.k * Mp;
       const EPt<double> ev = load_ept(E, g);
-      if (init) {
+      if constexpr (FROM) {
+        const double2 q = sl[g];
+        o = make_double2(q.x * (fA2 ? ev.a : ev.b), q.y * (bA2 ? ev.a : ev.b));
+      } else if (init) {
         sl[g] = make_double2(1.0, 1.0);
         o = make_double2(fA ? ev.a : ev.b, bA ? ev.a : ev.b);
       } else {
@@ -221,6 +226,7 @@ __device__ __forceinline__ void spread_real_r(const Dev<double>& D, double2* sm,
 }
 
 // a one-point x axis: node t of row l in lane l
+template <bool FROM>
 __device__ __forceinline__ void spread_real_1(const Dev<double>& D, double2* sm, const double* E, double2* sl, unsigned f,
                                               bool init) {
   const size_t rs = (size_t)D.mi * D.gx;
@@ -228,6 +234,11 @@ __device__ __forceinline__ void spread_real_1(const Dev<double>& D, double2* sm,
   for (int l = threadIdx.x; l < D.ro; l += blockDim.x) {
     double2* p = sm + l * D.pitch;
     const EPt<double> ev = load_ept(E, l * rs);
+    if constexpr (FROM) {
+      const double2 q = sl[l * rs];
+      *p = make_double2(q.x * (fA2 ? ev.a : ev.b), q.y * (bA2 ? ev.a : ev.b));
+      continue;
+    }
     double2 q = make_double2(1.0, 1.0);
     if (!init) q = make_double2(p->x * (fA ? ev.a : ev.b), p->y * (bA ? ev.a : ev.b));
     sl[l * rs] = q;
@@ -239,8 +250,8 @@ __device__ __forceinline__ void spread_real_1(const Dev<double>& D, double2* sm,
 }  // namespace mxk
 
 // k_mx_a
-static __global__ void __launch_bounds__(256, 2)
-k_mx_a_spread(const __grid_constant__ mxk::Dev<double> D, const __grid_constant__ mxk::Spread W, int t) {
+template <bool FROM>
+__device__ __forceinline__ void spread_a_body(const mxk::Dev<double>& D, const mxk::Spread& W, int t) {
   extern __shared__ __align__(16) unsigned char smraw[];
   double2* sm = reinterpret_cast<double2*>(smraw);
   const BulkDev<double>& I = *D.io.I;
@@ -265,7 +276,7 @@ k_mx_a_spread(const __grid_constant__ mxk::Dev<double> D, const __grid_constant_
   double2* g = D.io.spec + base;
   tmak::pdl_wait();
   __syncthreads();
-  if (t > 0) {
+  if (!FROM && t > 0) {
     if (D.a.n == 0) {
       for (int x = threadIdx.x; x < gx; x += blockDim.x) sm[x] = g[x];
       __syncthreads();
@@ -280,9 +291,9 @@ k_mx_a_spread(const __grid_constant__ mxk::Dev<double> D, const __grid_constant_
     }
   }
   if (D.rx == 1) {
-    mxk::spread_real_1(D, sm, E, sl, f, t == 0);
+    mxk::spread_real_1<FROM>(D, sm, E, sl, f, t == 0);
   } else {
-#define ADSCF_MX_CALL(R_) mxk::spread_real_r<R_>(D, sm, E, sl, f, t == 0)
+#define ADSCF_MX_CALL(R_) mxk::spread_real_r<R_, FROM>(D, sm, E, sl, f, t == 0)
     ADSCF_MXS_SWITCH(D.rx, ADSCF_MX_CALL)
 #undef ADSCF_MX_CALL
   }
@@ -300,9 +311,18 @@ k_mx_a_spread(const __grid_constant__ mxk::Dev<double> D, const __grid_constant_
     for (int x = threadIdx.x; x < gx; x += blockDim.x) g[x] = sm[x];
 }
 
-// k_mx_b
 static __global__ void __launch_bounds__(256, 2)
-k_mx_b_spread(const __grid_constant__ mxk::Dev<double> D, const __grid_constant__ mxk::Spread W) {
+k_mx_a_spread(const __grid_constant__ mxk::Dev<double> D, const __grid_constant__ mxk::Spread W, int t) {
+  spread_a_body<false>(D, W, t);
+}
+static __global__ void __launch_bounds__(256, 2)
+k_mx_a_spread_from(const __grid_constant__ mxk::Dev<double> D, const __grid_constant__ mxk::Spread W, int t) {
+  spread_a_body<true>(D, W, t);
+}
+
+// k_mx_b
+template <int MODE>
+__device__ __forceinline__ void spread_b_body(const mxk::Dev<double>& D, const mxk::Spread& W, const mxk::Side<double>& sd) {
   extern __shared__ __align__(16) unsigned char smraw[];
   double2* sm = reinterpret_cast<double2*>(smraw);
   const int gx = D.gx, gz = D.gz, mi = D.mi, nxy = gx * D.gy;
@@ -335,12 +355,13 @@ k_mx_b_spread(const __grid_constant__ mxk::Dev<double> D, const __grid_constant_
     __syncthreads();
   }
   if (D.rz == 1) {
-    mxk::mid_r<double, 1>(D, sm, fz, fxy, nl);
+    mxk::mid_r<double, 1, MODE>(D, sm, fz, fxy, nl, sd);
   } else {
-#define ADSCF_MX_CALL(R_) mxk::spread_mid_r<R_>(D, sm, fz, fxy, nl, W.zrp, W.ztwp, sm + pts + D.gy)
+#define ADSCF_MX_CALL(R_) mxk::spread_mid_r<R_, MODE>(D, sm, fz, fxy, nl, W.zrp, W.ztwp, sm + pts + D.gy, sd)
     ADSCF_MXS_SWITCH(D.rz, ADSCF_MX_CALL)
 #undef ADSCF_MX_CALL
   }
+  if constexpr (MODE == mxk::kSpec) return;
   __syncthreads();
   for (int i = D.b.n - 1; i >= 0; --i) {
     const mxk::Step& S = D.b.s[i];
@@ -356,4 +377,14 @@ k_mx_b_spread(const __grid_constant__ mxk::Dev<double> D, const __grid_constant_
       if (c < nl) g[(size_t)zz * nxy + c] = sm[e];
     }
   }
+}
+static __global__ void __launch_bounds__(256, 2)
+k_mx_b_spread(const __grid_constant__ mxk::Dev<double> D, const __grid_constant__ mxk::Spread W) {
+  spread_b_body<mxk::kPlain>(D, W, mxk::Side<double>{});
+}
+// with side data of `tile` points a block
+template <int MODE>
+__global__ void __launch_bounds__(256, 2)
+k_mx_b_spread_side(const __grid_constant__ mxk::Dev<double> D, const __grid_constant__ mxk::Spread W, double2* keep, int tile) {
+  spread_b_body<MODE>(D, W, mxk::Side<double>{keep + (size_t)blockIdx.x * tile, nullptr});
 }

@@ -173,7 +173,6 @@ template <typename T>
 int mx_factors(adscf_ctx* ctx, const std::vector<T>& fk, const std::vector<double>& g64);
 int mx_tune(adscf_ctx* ctx);
 void mx_real(adscf_ctx* ctx, int t);
-void mx_real_plain(adscf_ctx* ctx, int t);
 void mx_step(adscf_ctx* ctx, int t);
 void mx_destroy(adscf_ctx* ctx);
 int bulk_enqueue_chains(adscf_ctx* ctx);        // both chains, all steps

@@ -298,9 +298,12 @@ ADSCF_API int adscf_set_adi_plan(adscf_ctx *ctx, int x_lanes, int y_lanes, int z
  * without mixing -- chain term log(rho V/Q) - 1 minus dvol sum(phi w) plus
  * Interaction_Energy (mod_FloryHuggins.f90:74-96), over rho V, with phi
  * from Propagate_Diblock (mod_diblock.f90:100-173) -- keeping every
- * propagator slice on the device, and every step's spectrum too while those
- * take at most a quarter of the free memory (the gradient then transforms
- * the adjoint chains alone).
+ * propagator slice on the device, and every step's spectrum too (the gradient
+ * then transforms the adjoint chains alone): up to 1 GB of spectra from the
+ * first forward pass on, more from the first backward pass on and while they
+ * take at most a quarter of the free memory and a sixteenth of the GPU's.  A
+ * backward pass without them makes them again, with the same result bit for
+ * bit; adscf_set_adjoint_checkpoint gives them back.
  * adscf_backward: reverse-mode adjoint of that discrete free energy at the
  * same fields: grad[0..2] = dF/dL_x, dF/dL_y, dF/dL_z (cell stress),
  * grad[3] = dF/dchi.  Exact for the discretisation (pseudo-spectral steps,
