@@ -774,8 +774,8 @@ void film_destroy(adscf_ctx* ctx) {
 }
 
 // The factor workspace of FP64 lines, on the first propagation of this context
-// by itself (a film of a batch is swept with the batch, and needs none); not
-// inside a stream capture.
+// by itself (a film of a batch is swept with the batch, and needs none), where it
+// takes at most a quarter of the free memory; not inside a stream capture.
 int film_prepare(adscf_ctx* ctx) {
   FilmState* F = ctx->film;
   if (!F || F->fac_tried || !line_factors_ok(ctx)) return ADSCF_OK;
@@ -784,7 +784,10 @@ int film_prepare(adscf_ctx* ctx) {
   if (st != cudaStreamCaptureStatusNone) return ADSCF_OK;
   F->fac_tried = true;
   const FilmDev<double>& D = F->f64;
-  if (cudaMalloc(&F->d_fac, fl::step_bytes(D.gz + 1) * D.ns * D.nlines) != cudaSuccess) {
+  const size_t bytes = fl::step_bytes(D.gz + 1) * D.ns * D.nlines;
+  size_t avail = 0, total = 0;
+  CK(cudaMemGetInfo(&avail, &total));
+  if (bytes <= avail / 4 && cudaMalloc(&F->d_fac, bytes) != cudaSuccess) {
     cudaGetLastError();
     F->d_fac = nullptr;
   }
