@@ -1171,8 +1171,10 @@ k_batch_pack(const ScfDev* __restrict__ Ss, double* __restrict__ pack, const lon
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < nv; e += gridDim.x * blockDim.x) dst[e] = src[e];
 }
 
-// Device side of the packed copies, allocated by the first of them: the whole
-// batch, or, where memory is short, as much as fits (at least an instance).
+// Device side of the packed copies, allocated by the first of them: the batch, or
+// its instances in turns of 128 MB (2 ms of a copy; a copy and a launch each), or,
+// where memory is short, what fits; at least an instance.
+constexpr size_t kPackDoubles = (size_t(128) << 20) / sizeof(double);
 int pack_buffer(adscf_batch* b) {
   if (b->d_pack) return ADSCF_OK;
   if (!b->d_foff) {
@@ -1183,7 +1185,7 @@ int pack_buffer(adscf_batch* b) {
   }
   size_t least = 1;
   for (int i = 0; i < b->n; ++i) least = std::max(least, b->foff[i + 1] - b->foff[i]);
-  for (size_t cap = std::max(least, b->foff[b->n]);; cap = std::max(least, cap / 2)) {
+  for (size_t cap = std::max(least, std::min(kPackDoubles, b->foff[b->n]));; cap = std::max(least, cap / 2)) {
     if (cudaMalloc(&b->d_pack, cap * sizeof(double)) == cudaSuccess) {
       b->pack_cap = cap;
       return ADSCF_OK;
