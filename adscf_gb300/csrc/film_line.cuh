@@ -376,7 +376,7 @@ k_line_factors(FilmDev<double> F, FieldRef fr, double2* __restrict__ fac) {
 // memory: kStages steps of factors.  501 rows, 8 iterations of 100 steps 7.2 ->
 // 2.2 ms, 1001 rows and 1200 steps 11.1 -> 4.1 ms against factors in the chain.
 template <int K, int W>
-__global__ void __launch_bounds__(32 * W)
+__global__ void __launch_bounds__(32 * W, 1)
 k_line_chain(FilmDev<double> F, FieldRef fr, const double2* __restrict__ fac, int* __restrict__ serial) {
   using S = fl::Slot<K, W>;
   constexpr int T = 32 * W, P = S::pairs * T;

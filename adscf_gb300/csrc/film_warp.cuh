@@ -328,6 +328,12 @@ __device__ __forceinline__ bool film_line_dominant(const FilmDev<T>& F, const do
 // which take the lines that are marked in `serial` a thread each, neighbouring
 // lines in neighbouring threads (2048 lines of 101 rows, a step of both chains:
 // 766 us with a lane of every warp at work).
+// film1d_chain as a call: inlined into the cooperative kernels it takes registers
+// from their loops
+template <typename T>
+__device__ __noinline__ void film1d_chain_call(const FilmDev<T>& F, const double* field, int line, int dir) {
+  film1d_chain<T>(F, field, line, dir);
+}
 template <typename T>
 __device__ __forceinline__ bool film_line_serial(const FilmDev<T>& F, const double* field, int line, int dir, bool lead,
                                                  int* __restrict__ serial) {
@@ -336,7 +342,7 @@ __device__ __forceinline__ bool film_line_serial(const FilmDev<T>& F, const doub
     if (serial) {
       if (dir == 0) serial[line] = yes;
     } else if (yes) {
-      film1d_chain<T>(F, field, line, dir);
+      film1d_chain_call<T>(F, field, line, dir);
     }
   }
   return yes;
