@@ -780,6 +780,7 @@ int build_film(adscf_batch* b) {
       D.ns = b->ns[i]; D.na = na[i];
       D.ntypes = nt; D.brush = brush; D.single = 0; D.span = q.int_span;
       D.alpha = dtab + to[i].al; D.beta = dtab + to[i].be; D.gamma = dtab + to[i].ga;
+      D.ds_max = tb[i].ds_max; D.backwards = tb[i].backwards;
       D.dss = dtab + to[i].dss; D.wA = dtab + to[i].wA; D.wB = dtab + to[i].wB;
       D.wz = dtab + to[i].wz;
       D.graft = brush ? dtab + to[i].graft : nullptr;

@@ -38,6 +38,8 @@ struct FilmState {
   bool fac_tried = false;
   int* d_serial = nullptr;      // contexts of several lines: those that run the recurrence (film_line_serial)
   double max_ratio = 1.0;       // largest neighbour spacing ratio of the mesh
+  double ds_max = 0.0;          // longest contour step
+  bool backwards = false;       // a step is negative
   int optin = 0;                // opt-in shared memory per block
   // free energy at fixed fields and its wall-potential gradient
   double* d_fe_w = nullptr;     // [ntypes][npts] field copy
@@ -486,6 +488,8 @@ int step_single_t(adscf_ctx* ctx, double* d_prop, const double* d_w, double ds) 
   }
   if (D.fac) D.fac += adi_any_factor_vals(D.ns + 1);
   D.dss = F->d_dss + D.ns + 1;
+  D.ds_max = ds;
+  D.backwards = false;
   D.ns = 1;
   D.na = 1;
   D.single = 1;
@@ -536,6 +540,7 @@ void fill_dev(adscf_ctx* ctx, FilmState* F, const adscf_params* p) {
   D.single = 0;
   D.span = p->int_span;
   D.alpha = F->d_alpha; D.beta = F->d_beta; D.gamma = F->d_gamma;
+  D.ds_max = F->ds_max; D.backwards = F->backwards;
   D.dss = F->d_dss; D.wA = F->d_wA; D.wB = F->d_wB;
   D.adicf = F->d_adicf;
   D.wz = ctx->d_wz;
@@ -571,6 +576,7 @@ int film_create(adscf_ctx* ctx, const adscf_params* p) {
   std::string why;
   if (film_tables(*p, ctx->ns, ctx->na, tb, why)) return set_err(ctx, ADSCF_E_ARG, why);
   F->max_ratio = tb.max_ratio;
+  F->ds_max = tb.ds_max; F->backwards = tb.backwards;
   ctx->S.chain_len = tb.chain_len;
   const std::vector<double>& al = tb.al;
   const std::vector<double>& be = tb.be;
@@ -653,7 +659,8 @@ int film_create(adscf_ctx* ctx, const adscf_params* p) {
   if (F->t64) fill_dev<double>(ctx, F, p);
   else fill_dev<float>(ctx, F, p);
   if (ctx->geometry == ADSCF_FILM_3D) {
-    F->any_ok = F->t64 ? adi_any_ok(F->f64, F->optin) : adi_any_ok(F->f32, F->optin);
+    // (a step backwards leaves systems that are not dominant on every axis)
+    F->any_ok = !tb.backwards && (F->t64 ? adi_any_ok(F->f64, F->optin) : adi_any_ok(F->f32, F->optin));
     if (F->any_ok) {
       CK(cudaMalloc(&F->d_anyfac, adi_any_factor_vals(ctx->ns + 3) * (F->t64 ? sizeof(double) : sizeof(float))));
       F->f64.fac = static_cast<double*>(F->d_anyfac);

@@ -15,6 +15,8 @@ struct FilmTables {
   std::vector<double> wA, wB;       // [ns+1] contour weights per block
   double max_ratio = 1.0;           // largest neighbour spacing ratio of the mesh
   double chain_len = 0.0;           // sum of the contour steps
+  double ds_max = 0.0;              // the longest of them
+  bool backwards = false;           // one is negative
 };
 
 // geometry, grid (gz intervals), dz[0..gz], box (dx = sizex/gx, dy = sizey/gy),
@@ -58,7 +60,13 @@ inline int film_tables(const adscf_params& p, int ns, int na, FilmTables& T, std
     for (int s = 1; s <= ns; ++s) T.dss[s] = p.ds;
   }
   T.chain_len = 0.0;
-  for (int s = 1; s <= ns; ++s) T.chain_len += T.dss[s];
+  T.ds_max = 0.0;
+  T.backwards = false;
+  for (int s = 1; s <= ns; ++s) {
+    T.chain_len += T.dss[s];
+    T.ds_max = std::max(T.ds_max, T.dss[s]);
+    T.backwards |= T.dss[s] < 0;
+  }
   // contour weights: diblock = trapezoid per block with the step sizes
   // (mod_diblock.f90:143-154 for uniform steps); brush = the
   // 1/2 (dss_s + dss_{s+1}) rule of mod_homopolymer.f90:231-239

@@ -45,6 +45,8 @@ struct FilmDev {
   const double* alpha;   // [gz+1] 1/(h1 (h1+h2))  (a_z = -ds alpha)
   const double* beta;    // [gz+1] b_z / ds
   const double* gamma;   // [gz+1] 1/(h2 (h1+h2))  (c_z = -ds gamma)
+  double ds_max;         // longest contour step, and whether one is negative
+  bool backwards;
   const double* dss;     // [ns+1] contour steps, dss[0] = 0
   const double* wA;      // [ns+1] contour weights of block A (or homopolymer)
   const double* wB;      // [ns+1] contour weights of block B

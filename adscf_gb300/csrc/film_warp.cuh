@@ -301,25 +301,22 @@ __device__ __forceinline__ void film_warp_tables(const FilmDev<float>& F, const 
 
 // Whether every system of a line's chains is diagonally dominant: 1 + ds w / 2
 // >= 0.01 for the largest step and the lowest field value (the mesh terms
-// are, b = |a| + |c|).  Then no elimination order meets a zero pivot.  Where
+// are, b = |a| + |c|, unless a step goes backwards).  Then no elimination order meets a zero pivot.  Where
 // it is not, the order decides which pivots vanish and how far rounding
 // grows, and the chain runs the reference's serial recurrence instead
 // (film_line_serial).  Every lane of a warp calls it; the answer is uniform over
 // the warps of a line.
 template <typename T>
 __device__ __forceinline__ bool film_line_dominant(const FilmDev<T>& F, const double* field, size_t wstride) {
+  if (F.backwards) return false;
   double lo = 0.0;
   const int types = F.single ? 1 : F.ntypes;
   for (int t = 0; t < types; ++t)
+#pragma unroll 4
     for (int j = threadIdx.x & 31; j <= F.gz; j += 32) lo = fmin(lo, field[(size_t)t * F.npts + (size_t)j * wstride]);
 #pragma unroll
   for (int o = 16; o; o >>= 1) lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
-  if (lo >= 0.0) return true;
-  double ds = 0.0;
-  for (int s = 1 + (threadIdx.x & 31); s <= F.ns; s += 32) ds = fmax(ds, F.dss[s]);
-#pragma unroll
-  for (int o = 16; o; o >>= 1) ds = fmax(ds, __shfl_xor_sync(0xffffffffu, ds, o));
-  return 1.0 + 0.5 * ds * lo >= 0.01;
+  return 1.0 + 0.5 * F.ds_max * lo >= 0.01;
 }
 
 // Whether line `line` is not for the cooperative solve.  Its chains then run the
