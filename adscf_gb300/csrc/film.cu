@@ -666,7 +666,7 @@ int film_create(adscf_ctx* ctx, const adscf_params* p) {
       F->f64.fac = static_cast<double*>(F->d_anyfac);
       F->f32.fac = static_cast<float*>(F->d_anyfac);
     }
-    // FP64 sweeps: one thread per line only where the lines are too long
+    // FP64 sweeps: one thread per line where a line is too short or too long or the plane too large
     F->adi_any = F->t64 && F->any_ok;
   }
   const int rows = ctx->gz + 1;

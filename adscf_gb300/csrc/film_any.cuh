@@ -23,7 +23,10 @@
 // The x and y matrices are the same for every line of a sweep: their factors
 // are made once a propagation and applied line after line.
 //
-// Bound: FP64 the FP64 pipe and the wave of 99 planes on 152 SMs, FP32 latency.
+// Two planes have to fit a block's shared memory: in FP64 up to 120 x 120 points.
+//
+// Bound: FP64 the FP64 pipe and a last wave of planes (two chains of gz - 1 on 152
+// SMs) that is not full, FP32 latency.
 // A step of both chains, thread per line -> here: 20x35x100 FP64 220 -> 40 us
 // (53 with factors made by every warp, 69 line by line), FP32 43.5 -> 12.5;
 // 48^3 FP64 49 us, FP32 69.5 -> 11.9; 96x96x64 FP32 175 -> 25.

@@ -283,7 +283,9 @@ ADSCF_API int adscf_set_pass_plan(adscf_ctx *ctx, int y, int z, int x);
  * per plane and chain (the plane held in shared memory, the same arithmetic)
  * are timed too and kept if faster ("xy=fused"), and so are the sweeps on
  * lines of any length, 9 to 160 rows each ("any=yes"), which FP64 sweeps and
- * lines without a warp shape always take.  adscf_tuning reports the
+ * lines without a warp shape take where two planes fit a block's shared memory
+ * (FP64: gy (gx | 1) at most 14528, 120 x 120 or 112 x 128) and no contour step
+ * is negative; else a thread solves a line.  adscf_tuning reports the
  * choice and the timings ("GxK", "s" for staged); adscf_set_adi_plan pins
  * lanes per line for each sweep (0: one thread per line), staging (mask: 2 y,
  * 4 z) and the fused x + y kernel (mask 8); ADSCF_E_ARG if no shape matches,
