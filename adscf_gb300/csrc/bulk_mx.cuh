@@ -1,6 +1,7 @@
-// bulk_mx.cuh -- mixed-radix passes of the bulk propagator for grids the
-// register FFT does not cover (lines of 2, 3 and 5 factors, unequal axes,
-// two-dimensional grids), and for FP64 grids too small to fill the GPU there.
+// bulk_mx.cuh -- mixed-radix passes of the bulk propagator: grids with a line that
+// has no register FFT (lengths of 2, 3 and 5 factors up to 1024), and of the others
+// those where they are ahead (create_t in bulk.cu: FP64 but 256^3, FP32 with a line
+// of 256 points, and 32^3).
 //
 // Same double step as bulk_kernels.cuh in two passes over the spectrum.  A
 // line of n = R_1 R_2 ... R_S points is transformed in place in shared
@@ -475,7 +476,10 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 6 : 4)
 k_mx_a(const __grid_constant__ mxk::Dev<T> D, int t) {
   mx_a_body<T>(D, D.io, t);
 }
-// contexts blockIdx.y of a batch that share D's grid
+// Contexts blockIdx.y of a batch that share D's grid.  Their arrays come from a
+// struct in memory where k_mx_a has kernel parameters, and at the same registers
+// (blocks an SM) the pointers spill: 140 bytes here, 392 in k_mx_b_b<float, 256>, of
+// k_mx_a's 0 and k_mx_b's 20.
 template <typename T>
 __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 6 : 4)
 k_mx_a_b(const __grid_constant__ mxk::Dev<T> D, const mxk::Io<T>* __restrict__ ios, int t) {
