@@ -112,6 +112,7 @@ struct adscf_batch {
   int* d_ser[2] = {};
   int n_ser[2] = {};
   int* d_serial = nullptr;              // [n]
+  bool short64 = true;                  // no FP64 line of one warp has more than 128 rows
   int n32 = 0, n64 = 0;
   // shared-memory line sweeps: rows per line (max gz + 1 of the list) and
   // lanes per block (0: the list sweeps on global memory)
@@ -842,6 +843,7 @@ int build_film(adscf_batch* b) {
       const int rows = b->npts[f];
       int k = 0;
       if (f64p || rows > kFilmWarpRows) ser[f64p].push_back(f);
+      if (f64p && rows <= kFilmWarpRows && fl::rows_per_lane(rows) > 4) b->short64 = false;
       if (rows > kFilmGroupRows) { serial[f] = 1; continue; }
       if (f64p && rows <= fl::kMaxRows) k = rows > kFilmWarpRows;
       else if (rows > kFilmWarpRows)
@@ -925,12 +927,15 @@ void film_sweeps(adscf_batch* b) {
   const FilmDev<T>* F = static_cast<const FilmDev<T>*>(p ? b->d_f64 : b->d_f32);
   int k = 1;
   if (const int n = b->n_fsweep[p][0]) {
-    if constexpr (p) k_line_elim_b<1><<<(n + 3) / 4, fl::kThreads, fl::elim_bytes(fl::kMaxK), s>>>(F, b->d_S, b->d_fsweep[p][0], n, b->d_serial);
+    if constexpr (p) {
+      if (b->short64) k_line_elim_b<1, 4><<<(n + 3) / 4, fl::kThreads, fl::elim_bytes(4), s>>>(F, b->d_S, b->d_fsweep[p][0], n, b->d_serial);
+      else k_line_elim_b<1, 8><<<(n + 3) / 4, fl::kThreads, fl::elim_bytes(8), s>>>(F, b->d_S, b->d_fsweep[p][0], n, b->d_serial);
+    }
     else k_film1d_warp_b<<<(n + 3) / 4, 128, 0, s>>>(F, b->d_S, b->d_fsweep[p][0], n);
   }
   if constexpr (p) {
     if (const int n = b->n_fsweep[p][1])
-      k_line_elim_b<4><<<n, fl::kThreads, fl::elim_bytes(fl::kMaxK), s>>>(F, b->d_S, b->d_fsweep[p][1], n, b->d_serial);
+      k_line_elim_b<4, 8><<<n, fl::kThreads, fl::elim_bytes(8), s>>>(F, b->d_S, b->d_fsweep[p][1], n, b->d_serial);
     k = 2;
   }
   for (; k < 5; ++k) {

@@ -432,9 +432,13 @@ k_line_elim(FilmDev<double> F, FieldRef fr, int* __restrict__ serial) {
                        reinterpret_cast<double*>(smraw) + sub * 4 * K * T, &ex);
 }
 // (film << 1) | chain of a batch's films of W warps a line, K by film: one launch
-// for all lengths, so that short lines and long ones run beside each other
-template <int W>
-__global__ void __launch_bounds__(fl::kThreads)
+// for all lengths, so that short lines and long ones run beside each other.  Where
+// none has more than KMAX = 4 rows a lane, five blocks an SM in place of two: 2048
+// films of 40 to 60 rows 31.0 -> 28.0 us a step of both chains (118 registers, and
+// 96 with 96 bytes of spill; no such gain for eight rows: 2048 films of 180 to 250
+// rows 61.9 with 188 registers, 62.3 with 128).
+template <int W, int KMAX>
+__global__ void __launch_bounds__(fl::kThreads, KMAX <= 4 ? 5 : 1)
 k_line_elim_b(const FilmDev<double>* __restrict__ Fs, const ScfDev* __restrict__ Ss, const int* __restrict__ items, int nitems,
               int* __restrict__ serial) {
   extern __shared__ __align__(16) unsigned char smraw[];
@@ -448,14 +452,14 @@ k_line_elim_b(const FilmDev<double>* __restrict__ Fs, const ScfDev* __restrict__
   const double* field = S.hx + (size_t)((*S.iter) % S.slots) * ((size_t)S.ntypes * S.npts);
   if (film_line_serial<double>(F, field, 0, dir, (threadIdx.x & (T - 1)) == 0, serial + f)) return;
   double* chain = dir == 0 ? F.q : F.qd;
-  double* sm = reinterpret_cast<double*>(smraw) + sub * 4 * fl::kMaxK * T;
+  double* sm = reinterpret_cast<double*>(smraw) + sub * 4 * KMAX * T;
   switch (fl::rows_per_lane(F.gz + 1)) {
     case 2: if constexpr (W == 1) fl::chain_elim<2, W>(F, dir, chain, field, sm, &ex); break;
     case 3: fl::chain_elim<3, W>(F, dir, chain, field, sm, &ex); break;
     case 4: fl::chain_elim<4, W>(F, dir, chain, field, sm, &ex); break;
-    case 5: fl::chain_elim<5, W>(F, dir, chain, field, sm, &ex); break;
-    case 6: fl::chain_elim<6, W>(F, dir, chain, field, sm, &ex); break;
-    case 7: fl::chain_elim<7, W>(F, dir, chain, field, sm, &ex); break;
-    default: fl::chain_elim<8, W>(F, dir, chain, field, sm, &ex); break;
+    case 5: if constexpr (KMAX > 4) fl::chain_elim<5, W>(F, dir, chain, field, sm, &ex); break;
+    case 6: if constexpr (KMAX > 4) fl::chain_elim<6, W>(F, dir, chain, field, sm, &ex); break;
+    case 7: if constexpr (KMAX > 4) fl::chain_elim<7, W>(F, dir, chain, field, sm, &ex); break;
+    default: if constexpr (KMAX > 4) fl::chain_elim<8, W>(F, dir, chain, field, sm, &ex); break;
   }
 }
