@@ -185,8 +185,9 @@ void adi_step(const AdiLaunch& A, const FilmDev<T>& D, const FieldRef& fr, int s
 // ADSCF_AUTOTUNE=0 keeps the default shapes.
 struct AdiTuneKey {
   int dev, gx, gy, gz;
+  bool any;                     // the film may run the sweeps on lines of any length
   bool operator<(const AdiTuneKey& o) const {
-    return std::tie(dev, gx, gy, gz) < std::tie(o.dev, o.gx, o.gy, o.gz);
+    return std::tie(dev, gx, gy, gz, any) < std::tie(o.dev, o.gx, o.gy, o.gz, o.any);
   }
 };
 struct AdiTuneVal {
@@ -206,7 +207,7 @@ void adi_defaults(FilmState* F, const FilmDev<float>& D) {
 }
 
 int adi_tune(adscf_ctx* ctx, FilmState* F, const FilmDev<float>& D, const FieldRef& fr) {
-  const AdiTuneKey key{ctx->dev, D.gx, D.gy, D.gz};
+  const AdiTuneKey key{ctx->dev, D.gx, D.gy, D.gz, F->any_ok};
   {
     std::lock_guard<std::mutex> lk(g_adi_mu);
     auto it = g_adi_tune.find(key);

@@ -6,7 +6,7 @@ not."""
 import numpy as np
 import pytest
 
-from adscf_gb300 import FILM_1D, FILM_3D, FP64, Batch, Context, MIX_SIMPLE
+from adscf_gb300 import FILM_1D, FILM_3D, FP64, SPLIT, Batch, Context, MIX_SIMPLE
 from oracle import film as of
 
 pytestmark = pytest.mark.gpu
@@ -55,3 +55,21 @@ def test_planes(rng):
         dens, res = c.propagate_diblock(w)
     assert abs(res.Qsum / ref["Qsum"] - 1.0) < 1e-11
     assert np.max(np.abs(dens - ref["density"])) < 1e-10 * np.max(np.abs(ref["density"]))
+
+
+def test_planes_split_after_a_film_without(rng):
+    """The tuner's choice for the shape was made by a film that may run the sweeps on
+    lines of any length; this one may not.  FP32 rounding of the increments, 6e-8 a
+    step, times the matrices' O(ds / h^2) ~ 1."""
+    gz = 20
+    w = 0.1 * rng.standard_normal((2, gz + 1, 10, 12))
+    w[:, 0] = w[:, -1] = 0.0
+    for back in (False, True, False):
+        kw = dict(film(gz, (12, 10)), precision=SPLIT)
+        if not back:
+            kw["dss"] = np.abs(kw["dss"])
+        ref = oracle(kw, w, lambda p, f, ds: of.adi_step_3d(p, f, kw["dz"], 6.0 / 12, 6.0 / 10, ds))  # noqa: B023
+        with Context(FILM_3D, **kw) as c:
+            dens, res = c.propagate_diblock(w)
+        assert abs(res.Qsum / ref["Qsum"] - 1.0) < 2e-6
+        assert np.max(np.abs(dens - ref["density"])) < 1e-5 * np.max(np.abs(ref["density"]))
