@@ -10,7 +10,7 @@
 // Against the persistent sweep of the line passes (batch.cu), a double step
 // reads and writes the spectrum twice for four times and needs no waits
 // between items.  An SCF iteration of 64 grids of 24^3 to 64^3, 100 to 200
-// steps: split 42.1 -> 23.9 ms, FP64 348 -> 222; of one 64^3 grid 19.1 -> 3.3
+// steps: split 42.1 -> 23.9 ms, FP64 348 -> 213; of one 64^3 grid 19.1 -> 3.3
 // and 153 -> 9.3.
 #include <map>
 #include <new>
@@ -63,7 +63,7 @@ bool plan_class(Class& C, int optin, int gx, int gy, int gz) {
   mxk::Dev<T>& D = M->dev<T>();
   D.gx = gx; D.gy = gy; D.gz = gz;
   // 64-byte column runs: 64 grids of 24^3 to 64^3 split 23.9 ms an iteration, 26.7
-  // with 32 bytes, 27.3 with 128; in FP64 222 and 223 ms
+  // with 32 bytes, 27.3 with 128; the same in FP64
   Geom G;
   if (!default_geometry<T>(M, G)) return false;
   if (!geometry<T>(M, G.cut, 2 * G.cols, G.cap_a, G.cap_b)) geometry<T>(M, G.cut, G.cols, G.cap_a, G.cap_b);
